@@ -119,7 +119,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
   __shared__ float sm_r[2];
   __shared__ int sm_wide[2][2];                 // a loader warp saw a_i - r > 80 (overflow guard)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
   uint8_t* smK = sm;
@@ -167,7 +167,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
   const uint32_t tmem = tmem_base_s;
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       mbar_expect_tx(&kv_full, 2 * TILE_BYTES);
       tma_load_4d(smK, &tm_k, &kv_full, 0, kvhead, tok_chunk + row0, batch);
@@ -192,7 +192,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = mbar_wait(&kv_full, 0, &abort_flag);
       const uint32_t idesc_s = umma_idesc(128, TW, Pack2<T>::is_bf16, false, false);
       const uint32_t idesc_o = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);

@@ -96,7 +96,7 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
   __shared__ float sm_r[2];
   __shared__ int sm_wide[2][2];                 // a loader warp saw r - a_j > 80 (overflow guard)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
   uint8_t* smQ = sm;
@@ -139,7 +139,7 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
   const uint32_t tmem = tmem_base_s;
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&q_full, 2 * TILE_BYTES);
       tma_load_4d(smQ, &tm_q, &q_full, 0, qhead, tok_chunk + row0, batch);
       tma_load_4d(smDY, &tm_dy, &q_full, 0, qhead, tok_chunk + row0, batch);
@@ -163,7 +163,7 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
     // Issuing thread A: S and dP.  One thread issues a product only every ~108 clocks whatever its
     // shape (measured), so the three products of a step are shared between two threads: this one runs
     // ahead with S(J+1) and dP(J+1), thread B follows with dQ(J).
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = mbar_wait(&q_full, 0, &abort_flag);
       const uint32_t idesc_s = umma_idesc(128, TW, Pack2<T>::is_bf16, false, false);
       const uint32_t q_addr = smem_u32(smQ), dy_addr = smem_u32(smDY);
@@ -205,7 +205,7 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
     }
   } else if (warp == 6) {
     // Issuing thread B: dQ += dS(J) K_J, releases the key/value stage
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       const uint32_t idesc_q = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
       for (int J = 0; J < nJ && ok; ++J) {

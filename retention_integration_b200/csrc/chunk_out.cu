@@ -116,7 +116,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   __shared__ float sm_r[2];
   __shared__ int sm_wide[2][2];                 // a loader warp saw r - a_j > 80 (overflow guard)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
   uint8_t* smQ = sm;
@@ -167,7 +167,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
 
   if (warp == 4) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       mbar_expect_tx(&q_full, TILE_BYTES);
       tma_load_4d(smQ, &tm_q, &q_full, 0, qhead, chunk * p.cq + row0, batch);
@@ -196,7 +196,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
     }
   } else if (warp == 5) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = mbar_wait(&q_full, 0, &abort_flag);
       const uint32_t idesc_s = umma_idesc(128, TW, Pack2<T>::is_bf16, false, false);
       const uint32_t idesc_v = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);

@@ -65,7 +65,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
   uint8_t* smX = sm;                          // NS x XT_BYTES (rows = features, 64 tokens)
@@ -113,7 +113,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
 
   if (warp == 4 * NG) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       for (int it = 0; it < total; ++it) {
         const int s = it % NS, ph = (it / NS) & 1;
         const int g = it / kblocks, kb = it % kblocks;
@@ -143,7 +143,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
     // issues and as many per commit or barrier wait, which made one thread serving both groups
     // the slowest stage of the pipeline.
     const int g = warp - (4 * NG + 1);
-    if (lane == 0 && (!gram_cta || g == 0)) {
+    if ((!gram_cta || g == 0) && elect_one()) {
       bool ok = true;
       if (gram_cta) {
         const uint32_t idesc = umma_idesc(128, HD, Pack2<T>::is_bf16, false, false);

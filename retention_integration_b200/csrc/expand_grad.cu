@@ -89,7 +89,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int tile_i = blockIdx.x % p.tiles_per_chunk;
   const int chunk = blockIdx.x / p.tiles_per_chunk;
   const int head = blockIdx.y, batch = blockIdx.z;
@@ -150,7 +150,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
   const int ch = (batch * p.n_chunks + chunk) * p.h + gh;
 
   if (warp == W_TMA) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&w_full, 2 * NRT * TILE_BYTES);
       for (int rt = 0; rt < NRT; ++rt) {
         tma_load_4d(smW + rt * TILE_BYTES, &tm_w, &w_full, 0, head, chunk * p.c + row0 + rt * 128, batch);
@@ -173,7 +173,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
     // needs ~108 clocks per tcgen05.mma it issues and more per commit, whatever the shape (measured), and
     // traced timelines showed one thread per row tile setting the kernel's pace at ~1300 clocks per tile
     // against ~900 for the drain.
-    if (lane == 0) {
+    if (elect_one()) {
       const int rt = (warp - (W_TMA + 1)) >> 1, par = (warp - (W_TMA + 1)) & 1;
       bool ok = mbar_wait(&w_full, 0, &abort_flag);
       const uint32_t w_addr = smem_u32(smW) + rt * TILE_BYTES;
