@@ -20,10 +20,10 @@
  *   - `dtype` is PR_BF16 or PR_FP16 for Q/K/V-like tensors; gates, row sums and
  *     Gram matrices are fp32;
  *   - tensors are dense and row-major in the stated shape;
- *   - head dim d = 64 in this build; deg = 2.
+ *   - head dim d = 64 in this build unless an entry says otherwise; deg = 2.
  *
  * Shapes use b batch, t tokens, h kv heads, hq query heads (multiple of h), d head
- * dim, c chunk length, n = t / c chunks, cp = c rounded up to 64, and
+ * dim, c chunk length, n = t / c chunks rounded up (the last chunk may be shorter; nothing is padded), cp = c rounded up to 64, and
  * D2 = 128*(d/16)*(d/16+1) rows (2560 at d = 64) of the expansion layout the kernels and chunk states
  * use: the reference's own block layout, retention/_update_state/reference.py:5-29 (see layout.cuh).
  * Inference states cross this ABI in the exact layout, d*(d+1)/2 = 2080 rows.
@@ -254,13 +254,14 @@ int pr_decode_step_strided(int dtype, int b, int tk, int h, int hq, int d, const
  * power_retention's chunked branch (retention/power_retention_maker.py:143-193) and its backward
  * (what autograd runs: retention/_query_state/triton.py:544-621, _attention/triton.py:742-810,
  * _discumsum/triton.py:334-355, _update_state/triton.py:329-355 and the gradients of the glue),
- * sequenced in native code over the entry points above.  t must be a multiple of c (the caller
- * pads, as the reference's wrapper does, :71-90); deg = 2. */
+ * sequenced in native code over the entry points above.  t need not be a multiple of c: the last chunk
+ * is then shorter, with the results that the reference's zero padding has (:71-90).  d = 16, 32 or 64 (states
+ * and carries of the chunk-state layout have 128*(d/16)*(d/16+1) rows of d); deg = 2. */
 typedef struct pr_problem {
   int dtype;   /* PR_BF16 / PR_FP16 */
   int b, t;    /* batch, tokens */
   int h, hq;   /* kv heads, query heads (multiple of h) */
-  int d;       /* head dim (64) */
+  int d;       /* head dim */
   int c;       /* chunk length */
   float scale; /* score scale (the reference's default is 1/sqrt(d)) */
 } pr_problem;
@@ -284,7 +285,7 @@ int pr_retention_fwd(const pr_problem* problem, const void* Q, const void* K, co
  * The chunk size blocks the computation of retention/power_retention_maker.py:143-193 without changing its
  * result; on this hardware 1024 is fastest (5.3 ms per step at chunk 128 against 2.6 at 1024 for b1 t65536 h8).
  * pr_retention_fwd / _bwd run whatever pr_problem.c says; a host that wants the fast blocking passes
- * c = pr_fast_chunk(t, its_chunk) and pads t to a multiple of it with zero tokens behind gates of 1. */
+ * c = pr_fast_chunk(t, its_chunk). */
 int pr_fast_chunk(long long t, int requested_chunk);
 
 /* Backward.  dO [b,t,hq,d] -> dQ, dK, dV (shapes of Q, K, V) and dlog_G [b,t,h] fp32 (NULL when
@@ -296,6 +297,17 @@ int pr_fast_chunk(long long t, int requested_chunk);
  * the whole pass on `stream`. */
 int pr_retention_bwd(const pr_problem* problem, const void* Q, const void* K, const void* V, const float* log_G,
                      const void* O, const void* dO, int had_carry, void* saved, void* scratch, void* dQ, void* dK,
+                     void* dV, float* dlog_G, int device, void* stream);
+
+/* The state-free branch (retention/power_retention_maker.py:128-132): causal power attention over the whole
+ * sequence, which is one chunk; deg = 2 or 4, d = 16, 32 or 64 (pr_problem.c is not read).
+ * Workspaces: PR_WS_SAVED (written by the forward, read by the backward) and PR_WS_BWD_SCRATCH, sizes from
+ * pr_attention_workspace_bytes.  The backward forks a second stream like pr_retention_bwd. */
+int pr_attention_workspace_bytes(const pr_problem* problem, int what, size_t* out);
+int pr_attention_fwd(const pr_problem* problem, int deg, const void* Q, const void* K, const void* V,
+                     const float* log_G, void* O, void* saved, int device, void* stream);
+int pr_attention_bwd(const pr_problem* problem, int deg, const void* Q, const void* K, const void* V,
+                     const float* log_G, const void* O, const void* dO, void* saved, void* scratch, void* dQ, void* dK,
                      void* dV, float* dlog_G, int device, void* stream);
 
 /* Between the caller's projection GEMM and the operator (deploy/nanoGPT/model.py:66-84,

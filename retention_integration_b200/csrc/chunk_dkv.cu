@@ -28,14 +28,14 @@ constexpr int TW = 64;                  // queries per step
 constexpr int QD_BYTES = TW * 128;      // one query or dO tile
 constexpr int Z_BYTES = 64 * 128;
 constexpr int R_BYTES = 2 * QD_BYTES;   // one ring stage
-constexpr int DR = ref_dim(HD);
-constexpr int NBLK = DR / 64;           // 40 stages of 64 expanded rows
 constexpr uint32_t TMEM_COLS = 256;     // two CTAs per SM
 constexpr uint32_t COL_S = 0, COL_P = 0, COL_DP = 64, COL_DS = 64, COL_DV = 128, COL_DK = 192, COL_A = 0;
 }  // namespace dkv
 
 struct ChunkDkvParams {
   int hq, h, n_chunks, c, tiles_per_chunk;
+  int t, d;               // tokens (the last chunk may be shorter), features (a multiple of 16)
+  int nblk;               // stages of 64 expanded rows of a state
   int state_chunk_hi;     // chunks <= this have a state-path dV term
   float scale;
   const float* a;         // [b, t, h] or null
@@ -135,7 +135,9 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
   const int ratio = p.hq / p.h;
   const int row0 = tile_j * 128;
   const int tok_chunk = chunk * p.c;
-  const int q_tiles = (p.c + TW - 1) / TW;      // query tiles of TW rows in the chunk
+  const int c = min(p.c, p.t - tok_chunk);      // tokens of this chunk
+  if (row0 >= c) return;
+  const int q_tiles = (c + TW - 1) / TW;        // query tiles of TW rows in the chunk
   const int qt0 = row0 / TW;                    // first query tile that can see this key tile
   const int nI = q_tiles - qt0;
   const int n_steps = nI * ratio;
@@ -173,7 +175,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       tma_load_4d(smK, &tm_k, &kv_full, 0, kvhead, tok_chunk + row0, batch);
       tma_load_4d(smV, &tm_v, &kv_full, 0, kvhead, tok_chunk + row0, batch);
       const int ch = (batch * p.n_chunks + chunk) * p.h + kvhead;
-      const int n_ring = n_steps + (has_state ? NBLK / 2 : 0);
+      const int n_ring = n_steps + (has_state ? p.nblk / 2 : 0);
       for (int g = 0; g < n_ring && ok; ++g) {
         const int s = g % NR, ph = (g / NR) & 1;
         ok = mbar_wait(&r_empty[s], ph ^ 1, &abort_flag);
@@ -186,8 +188,8 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
           tma_load_4d(dst + QD_BYTES, &tm_dy, &r_full[s], 0, qh, tok_chunk + I * TW, batch);
         } else {
           const int blk = 2 * (g - n_steps);
-          tma_load_2d(dst, &tm_ds, &r_full[s], 0, ch * DR + blk * 64);
-          tma_load_2d(dst + Z_BYTES, &tm_ds, &r_full[s], 0, ch * DR + (blk + 1) * 64);
+          tma_load_2d(dst, &tm_ds, &r_full[s], 0, (ch * p.nblk + blk) * 64);
+          tma_load_2d(dst + Z_BYTES, &tm_ds, &r_full[s], 0, (ch * p.nblk + blk + 1) * 64);
         }
       }
     }
@@ -229,7 +231,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       if (ok && has_state) {
         // 128 expanded entries against two state blocks (one ring stage) per item: eight products
         // per pair of waits and commits keep this thread off the critical path
-        for (int k = 0; k < NBLK / 2 && ok; ++k) {
+        for (int k = 0; k < p.nblk / 2 && ok; ++k) {
           const int s = k % NS, ph = (k / NS) & 1;
           const int g = n_steps + k, rs = g % NR;
           ok = mbar_wait(&a_full[s], ph, &abort_flag) && mbar_wait(&r_full[rs], (g / NR) & 1, &abort_flag);
@@ -249,10 +251,10 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
     }
   } else {
     const int row = row0 + tid;  // key index inside the chunk
-    const bool row_valid = row < p.c;
+    const bool row_valid = row < c;
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const bool gated = p.a != nullptr;
-    const size_t tok_base = (size_t)batch * p.n_chunks * p.c + tok_chunk;
+    const size_t tok_base = (size_t)batch * p.t + tok_chunk;
     const float* a_chunk = gated ? p.a + tok_base * p.h + kvhead : nullptr;
     const float a_j = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
     const float s2 = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
@@ -264,7 +266,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       if (tid < TW) {
         const int qp0 = (qt0 + st / ratio) * TW, qh = kvhead * ratio + st % ratio;
         const int qp = qp0 + tid;
-        const bool v = qp < p.c;
+        const bool v = qp < c;
         av_n = (gated && v) ? a_chunk[(size_t)qp * p.h] : 0.f;
         r_n = gated ? a_chunk[(size_t)qp0 * p.h] : 0.f;
         dl_n = v ? p.dl[(tok_base + qp) * p.hq + qh] : 0.f;
@@ -277,7 +279,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       const int qp0 = I * TW;
       const int sb = st & 1;
       if (tid < TW) {
-        const bool v = qp0 + tid < p.c;
+        const bool v = qp0 + tid < c;
         const float il = v ? safe_recip(l_n) : 0.f;
         sm_aq[sb][tid] = av_n;
         sm_dl[sb][tid] = dl_n;
@@ -299,7 +301,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       // come after this warp's keys need no mask; a warp whose keys all come after the step's
       // queries writes zeros without reading the scores.
       const int wrow0 = row0 + (warp << 5);
-      if (qp0 + TW - 1 < wrow0 || wrow0 >= p.c) {
+      if (qp0 + TW - 1 < wrow0 || wrow0 >= c) {
         uint32_t z[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) z[j] = 0u;
@@ -309,12 +311,12 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         tmem_st16(tmem + lane_addr + COL_DS + 16, z);
       } else {
         const float r = sm_r[sb];
-        const bool mask = (wrow0 + 31 > qp0) || (wrow0 + 31 >= p.c);
-        const bool sep = (qp0 + TW - 1 < p.c) && !(sm_wide[sb][0] | sm_wide[sb][1]) &&
+        const bool mask = (wrow0 + 31 > qp0) || (wrow0 + 31 >= c);
+        const bool sep = (qp0 + TW - 1 < c) && !(sm_wide[sb][0] | sm_wide[sb][1]) &&
                          !__any_sync(0xffffffffu, (r - a_j) > 80.f);
         const float c_j = sep ? (float)DEG * s2 * __expf(r - a_j) : (float)DEG * s2;
         const int lo = row_valid ? row - qp0 : TW;  // first query column this key keeps
-        const int hi = p.c - 1 - qp0;               // last column inside the chunk
+        const int hi = c - 1 - qp0;                 // last column inside the chunk
 #pragma unroll 1
         for (int q4 = 0; q4 < TW / 32; ++q4) {
           uint32_t sv[32], pv[32], pk[16], dk[16];
@@ -371,6 +373,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       int k = 0;
       static_for<0, HD / 16>([&](auto yc) {
         constexpr int Y = decltype(yc)::value;
+        if (16 * Y >= p.d) return;
 #pragma unroll 1
         for (int a0 = 0; a0 < 16 * (Y + 1); a0 += 8, ++k) {
           uint32_t r0[32], r1[32];
@@ -405,9 +408,10 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       tmem_ld32(tmem + lane_addr + COL_DV + 32, acc + 32);
       tmem_wait_ld();
       if (row_valid) {
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dV) + (tok * p.h + kvhead) * HD);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dV) + (tok * p.h + kvhead) * p.d);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
+          if (8 * j >= p.d) break;
           uint4 v;
           v.x = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 0]), __uint_as_float(acc[8 * j + 1]));
           v.y = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3]));
@@ -421,11 +425,12 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       tmem_ld32(tmem + lane_addr + COL_DK + 32, acc + 32);
       tmem_wait_ld();
       if (row_valid) {
-        const float4* st = p.dk_state ? reinterpret_cast<const float4*>(p.dk_state + (tok * p.h + kvhead) * HD)
+        const float4* st = p.dk_state ? reinterpret_cast<const float4*>(p.dk_state + (tok * p.h + kvhead) * p.d)
                                       : nullptr;
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dK) + (tok * p.h + kvhead) * HD);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dK) + (tok * p.h + kvhead) * p.d);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
+          if (8 * j >= p.d) break;
           float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
           if (st) {
             s0 = st[2 * j];
@@ -458,8 +463,8 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   using namespace pr::dkv;
   PR_REQUIRE(deg == 2 || (deg == 4 && wdS == nullptr && dk_state == nullptr), PR_ERR_BAD_ARG,
              "deg=%d: states exist for deg 2; deg 4 runs state-free (attention only)", deg);
-  PR_REQUIRE(d == HD, PR_ERR_BAD_ARG, "head dim %d: this build handles d = 64", d);
-  PR_REQUIRE(b > 0 && t > 0 && hq > 0 && h > 0 && hq % h == 0 && c > 0 && t % c == 0, PR_ERR_BAD_ARG,
+  PR_REQUIRE(head_dim_ok(d), PR_ERR_BAD_ARG, "head dim %d: a multiple of 16 up to 64", d);
+  PR_REQUIRE(b > 0 && t > 0 && hq > 0 && h > 0 && hq % h == 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d hq=%d h=%d c=%d", b, t, hq, h, c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(Q && dO && K && V && dl && l && dK && dV && da_k, PR_ERR_BAD_ARG, "null pointer");
@@ -473,7 +478,10 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   ChunkDkvParams p;
   p.hq = hq;
   p.h = h;
-  p.n_chunks = t / c;
+  p.n_chunks = chunks_of(t, c);
+  p.t = t;
+  p.d = d;
+  p.nblk = ref_dim(d) / 64;
   p.c = c;
   p.tiles_per_chunk = (c + 127) / 128;
   p.state_chunk_hi = wdS ? state_chunk_hi : -1;
@@ -500,8 +508,8 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   if ((rc = make_tmap(&tm_k, K, 2, 4, dk, sk, box, true))) return rc;
   if ((rc = make_tmap(&tm_v, V, 2, 4, dk, sk, box, true))) return rc;
   if (wdS) {
-    uint64_t dz[2] = {64, (uint64_t)b * p.n_chunks * h * ref_dim(d)};
-    uint64_t st[2] = {0, 128};
+    uint64_t dz[2] = {(uint64_t)d, (uint64_t)b * p.n_chunks * h * ref_dim(d)};
+    uint64_t st[2] = {0, (uint64_t)d * 2};
     uint32_t bz[2] = {64, 64};
     if ((rc = make_tmap(&tm_ds, wdS, 2, 2, dz, st, bz, true))) return rc;
   } else {

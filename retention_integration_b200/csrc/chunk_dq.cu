@@ -31,6 +31,7 @@ constexpr uint32_t COL_S = 0, COL_DP = 128, COL_ACC = 192;  // S double-buffered
 
 struct ChunkDqParams {
   int hq, h, n_chunks, c, tiles_per_chunk;
+  int t, d;               // tokens (the last chunk may be shorter), features (a multiple of 16)
   float scale;
   const float* a;         // [b, t, h] or null
   const float* dl;        // [b, t, hq]
@@ -109,7 +110,9 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
   const int qhead = blockIdx.y, batch = blockIdx.z;
   const int kvhead = qhead / (p.hq / p.h);
   const int row0 = tile_i * 128;
-  const int nJ = min(p.c - 1, row0 + 127) / TW + 1;
+  const int c = min(p.c, p.t - chunk * p.c);  // tokens of this chunk
+  if (row0 >= c) return;
+  const int nJ = min(c - 1, row0 + 127) / TW + 1;
   const int tok_chunk = chunk * p.c;
   const bool has_st = p.dq_state != nullptr;
 
@@ -224,11 +227,11 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
     }
   } else {
     const int row = row0 + tid;
-    const bool row_valid = row < p.c;
+    const bool row_valid = row < c;
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const bool gated = p.a != nullptr;
-    const size_t tok = (size_t)batch * p.n_chunks * p.c + tok_chunk + row;
-    const float* a_chunk = gated ? p.a + ((size_t)batch * p.n_chunks * p.c + tok_chunk) * p.h + kvhead : nullptr;
+    const size_t tok = (size_t)batch * p.t + tok_chunk + row;
+    const float* a_chunk = gated ? p.a + ((size_t)batch * p.t + tok_chunk) * p.h + kvhead : nullptr;
     const float a_i = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
     const float dl_i = row_valid ? p.dl[tok * p.hq + qhead] : 0.f;
     const float inv_l = row_valid ? safe_recip(p.l[tok * p.hq + qhead]) : 0.f;
@@ -241,8 +244,8 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
     auto load_gates = [&](int J) {
       if (tid < TW && gated) {
         const int kp = J * TW + tid;
-        av_n = kp < p.c ? a_chunk[(size_t)kp * p.h] : 0.f;
-        r_n = a_chunk[(size_t)min(J * TW + TW - 1, p.c - 1) * p.h];
+        av_n = kp < c ? a_chunk[(size_t)kp * p.h] : 0.f;
+        r_n = a_chunk[(size_t)min(J * TW + TW - 1, c - 1) * p.h];
       }
     };
     load_gates(0);
@@ -267,8 +270,8 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
       // diagonal for gates <= 0; if one exceeds 80 (growing gates) the warp takes the per-pair
       // form.  Steps wholly below the diagonal need no mask; a warp whose rows all precede the
       // step's keys writes zeros without reading the scores.
-      const int lim = min(row, p.c - 1) - kp0;  // last column this row keeps
-      if (kp0 > min(wrow0 + 31, p.c - 1)) {
+      const int lim = min(row, c - 1) - kp0;  // last column this row keeps
+      if (kp0 > min(wrow0 + 31, c - 1)) {
         uint32_t z[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) z[j] = 0u;
@@ -276,7 +279,7 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
         tmem_st16(tmem + lane_addr + col_s + 16, z);
       } else {
         const float r = sm_r[sb];
-        const bool mask = (kp0 + TW - 1 > wrow0) || (kp0 + TW - 1 >= p.c);
+        const bool mask = (kp0 + TW - 1 > wrow0) || (kp0 + TW - 1 >= c);
         const bool sep = !(sm_wide[sb][0] | sm_wide[sb][1]) && !__any_sync(0xffffffffu, (a_i - r) > 80.f);
         const float c_i = sep ? s2x2 * __expf(a_i - r) : s2x2;
 #pragma unroll 1
@@ -309,9 +312,10 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
       tmem_ld32(tmem + lane_addr + COL_ACC + 32, acc + 32);
       tmem_wait_ld();
       if (row_valid) {
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dQ) + (tok * p.hq + qhead) * HD);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dQ) + (tok * p.hq + qhead) * p.d);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
+          if (8 * j >= p.d) break;
           float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
           if (has_st) {
             // columns 8j..8j+7: 16-byte chunks 2j, 2j+1 of the row in its 32-column half
@@ -346,8 +350,8 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   using namespace pr::dq;
   PR_REQUIRE(deg == 2 || (deg == 4 && dq_state == nullptr), PR_ERR_BAD_ARG,
              "deg=%d: states exist for deg 2; deg 4 runs state-free (attention only)", deg);
-  PR_REQUIRE(d == HD, PR_ERR_BAD_ARG, "head dim %d: this build handles d = 64", d);
-  PR_REQUIRE(b > 0 && t > 0 && hq > 0 && h > 0 && hq % h == 0 && c > 0 && t % c == 0, PR_ERR_BAD_ARG,
+  PR_REQUIRE(head_dim_ok(d), PR_ERR_BAD_ARG, "head dim %d: a multiple of 16 up to 64", d);
+  PR_REQUIRE(b > 0 && t > 0 && hq > 0 && h > 0 && hq % h == 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d hq=%d h=%d c=%d", b, t, hq, h, c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(Q && dO && K && V && dl && l && dQ && da_q, PR_ERR_BAD_ARG, "null pointer");
@@ -358,7 +362,9 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   ChunkDqParams p;
   p.hq = hq;
   p.h = h;
-  p.n_chunks = t / c;
+  p.n_chunks = chunks_of(t, c);
+  p.t = t;
+  p.d = d;
   p.c = c;
   p.tiles_per_chunk = (c + 127) / 128;
   p.scale = scale;

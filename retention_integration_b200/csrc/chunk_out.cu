@@ -35,8 +35,6 @@ constexpr int TW = 64;                 // keys per attention step
 constexpr int KV_BYTES = TW * 128;     // one key or value tile
 constexpr int Z_BYTES = 64 * 128;      // 64 expanded rows x 64 features
 constexpr int R_BYTES = 2 * KV_BYTES;  // one ring stage
-constexpr int DR = ref_dim(HD);        // 2560 expanded rows
-constexpr int NBLK = DR / 64;          // 40 stages of 64 expanded rows (4 first factors x 16)
 constexpr uint32_t TMEM_COLS = 256;
 constexpr uint32_t COL_ACC = 0, COL_U = 64, COL_S = 128, COL_A = 128;  // S: 2 buffers x 64 columns, P aliased
 }  // namespace co
@@ -45,6 +43,9 @@ struct ChunkOutParams {
   int hq, h;            // query heads, kv heads
   int n_chunks;         // chunks per batch element
   int cq, ck;           // queries / keys per chunk (query i sits at key position i + ck - cq)
+  int tq, tk;           // queries / keys per batch element: the last chunk may be shorter than the others
+  int d;                // features (a multiple of 16; TMA fills the tiles' columns up to 64 with zeros)
+  int nblk;             // stages of 64 expanded rows of a state: ref_dim(d) / 64
   int tiles_per_chunk;  // ceil(cq / 128)
   int state_from_chunk; // chunks >= this read the state (n_chunks: never)
   int q_gate_last;      // 1: gate the state read-out with the gate at the last key (inference)
@@ -130,9 +131,11 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   const int chunk = blockIdx.x / p.tiles_per_chunk;
   const int qhead = blockIdx.y, batch = blockIdx.z;
   const int kvhead = qhead / (p.hq / p.h);
-  const int q_off = p.ck - p.cq;
+  const int cq = min(p.cq, p.tq - chunk * p.cq), ck = min(p.ck, p.tk - chunk * p.ck);  // of this chunk
+  const int q_off = ck - cq;
   const int row0 = tile_i * 128;
-  const int last_key = min(p.ck - 1, row0 + 127 + q_off);
+  if (row0 >= cq) return;  // a tile past the end of a shorter last chunk
+  const int last_key = min(ck - 1, row0 + 127 + q_off);
   const int nJ = p.has_attn ? last_key / TW + 1 : 0;
   const bool has_state = chunk >= p.state_from_chunk;
 
@@ -174,10 +177,10 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       const int ch = (batch * p.n_chunks + chunk) * p.h + kvhead;
       if (has_state) {
         mbar_expect_tx(&g_full, 2 * Z_BYTES);
-        tma_load_2d(smG, &tm_ghi, &g_full, 0, ch * HD);
-        tma_load_2d(smG + Z_BYTES, &tm_glo, &g_full, 0, ch * HD);
+        tma_load_3d(smG, &tm_ghi, &g_full, 0, 0, ch);
+        tma_load_3d(smG + Z_BYTES, &tm_glo, &g_full, 0, 0, ch);
       }
-      const int n_ring = nJ + (has_state ? NBLK / 2 : 0);
+      const int n_ring = nJ + (has_state ? p.nblk / 2 : 0);
       for (int g = 0; g < n_ring && ok; ++g) {
         const int s = g % NR, ph = (g / NR) & 1;
         ok = mbar_wait(&r_empty[s], ph ^ 1, &abort_flag);
@@ -189,8 +192,8 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
           tma_load_4d(dst + KV_BYTES, &tm_v, &r_full[s], 0, kvhead, chunk * p.ck + g * TW, batch);
         } else {
           const int blk = 2 * (g - nJ);
-          tma_load_2d(dst, &tm_z, &r_full[s], 0, ch * DR + blk * 64);
-          tma_load_2d(dst + Z_BYTES, &tm_z, &r_full[s], 0, ch * DR + (blk + 1) * 64);
+          tma_load_2d(dst, &tm_z, &r_full[s], 0, (ch * p.nblk + blk) * 64);
+          tma_load_2d(dst + Z_BYTES, &tm_z, &r_full[s], 0, (ch * p.nblk + blk + 1) * 64);
         }
       }
     }
@@ -247,9 +250,9 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
                       (half > 0 || ks > 0) ? 1u : 0u);
           umma_commit(&a_empty[0]);
         }
-        // ring items 1 .. NBLK/2: 128 expanded entries against two state blocks (one ring stage);
+        // ring items 1 .. nblk/2: 128 expanded entries against two state blocks (one ring stage);
         // eight products per pair of waits and commits keep this thread off the critical path
-        for (int k = 1; k <= NBLK / 2 && ok; ++k) {
+        for (int k = 1; k <= p.nblk / 2 && ok; ++k) {
           const int s = k % NS, ph = (k / NS) & 1;
           const int g = nJ + k - 1, rs = g % NR;
           ok = mbar_wait(&a_full[s], ph, &abort_flag) && mbar_wait(&r_full[rs], (g / NR) & 1, &abort_flag);
@@ -271,11 +274,11 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   } else {
     // --------------------------------------------------------- row-owning warps
     const int row = row0 + tid;                 // query index inside the chunk
-    const bool row_valid = row < p.cq;
+    const bool row_valid = row < cq;
     const int qpos = row + q_off;               // key position of this query
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const bool gated = p.a != nullptr;
-    const float* a_chunk = gated ? p.a + ((size_t)batch * p.n_chunks * p.ck + (size_t)chunk * p.ck) * p.h + kvhead
+    const float* a_chunk = gated ? p.a + ((size_t)batch * p.tk + (size_t)chunk * p.ck) * p.h + kvhead
                                  : nullptr;
     const float a_i = (gated && row_valid) ? a_chunk[(size_t)qpos * p.h] : 0.f;
     const float s2 = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
@@ -286,8 +289,8 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
     auto load_gates = [&](int J) {
       if (tid < TW && gated) {
         const int kp = J * TW + tid;
-        av_n = kp < p.ck ? a_chunk[(size_t)kp * p.h] : 0.f;
-        r_n = a_chunk[(size_t)min(J * TW + TW - 1, p.ck - 1) * p.h];
+        av_n = kp < ck ? a_chunk[(size_t)kp * p.h] : 0.f;
+        r_n = a_chunk[(size_t)min(J * TW + TW - 1, ck - 1) * p.h];
       }
     };
     if (nJ > 0) load_gates(0);
@@ -314,7 +317,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       // diagonal need no mask; a warp whose rows all precede the step's keys writes zeros
       // without reading the scores.
       const int wq0 = row0 + (warp << 5) + q_off;  // key position of this warp's first query
-      if (kp0 > min(wq0 + 31, p.ck - 1)) {
+      if (kp0 > min(wq0 + 31, ck - 1)) {
         uint32_t z[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) z[j] = 0u;
@@ -322,10 +325,10 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         tmem_st16(tmem + lane_addr + col_s + 16, z);
       } else {
         const float r = sm_r[sb];
-        const bool mask = (kp0 + TW - 1 > wq0) || (kp0 + TW - 1 >= p.ck);
+        const bool mask = (kp0 + TW - 1 > wq0) || (kp0 + TW - 1 >= ck);
         const bool sep = !(sm_wide[sb][0] | sm_wide[sb][1]) && !__any_sync(0xffffffffu, (a_i - r) > 80.f);
         const float c_i = sep ? s2 * __expf(a_i - r) : s2;
-        const int lim = min(qpos, p.ck - 1) - kp0;  // last column this row keeps
+        const int lim = min(qpos, ck - 1) - kp0;  // last column this row keeps
 #pragma unroll 1
         for (int q4 = 0; q4 < TW / 32; ++q4) {
           uint32_t sv[32], pk[16];
@@ -353,7 +356,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       ok = mbar_wait(&q_full, 0, &abort_flag);
       float f = p.scale;
       if (gated) {
-        const float a_g = p.q_gate_last ? a_chunk[(size_t)(p.ck - 1) * p.h] : a_i;
+        const float a_g = p.q_gate_last ? a_chunk[(size_t)(ck - 1) * p.h] : a_i;
         f *= __expf(0.5f * a_g);
       }
 #pragma unroll
@@ -377,7 +380,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         __syncwarp();
         if (lane == 0) mbar_arrive(&a_full[0]);
       }
-      // ring items 1..NBLK/2: 128 expanded entries (64 packed products) each.  The gated row goes
+      // ring items 1..nblk/2: 128 expanded entries (64 packed products) each.  The gated row goes
       // back to its own slot of the query tile so that the first factor can be fetched by a runtime
       // index; the loop over first factors then has a body of 64 multiplies per stage.
       if (ok) {
@@ -388,6 +391,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       int k = 1;
       static_for<0, HD / 16>([&](auto yc) {
         constexpr int Y = decltype(yc)::value;
+        if (16 * Y >= p.d) return;
 #pragma unroll 1
         for (int a0 = 0; a0 < 16 * (Y + 1); a0 += 8, ++k) {
           uint32_t r0[32], r1[32];
@@ -438,11 +442,12 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       tmem_ld32(tmem + lane_addr + COL_ACC + 32, acc + 32);
       tmem_wait_ld();
       if (row_valid) {
-        const size_t tok = (size_t)batch * p.n_chunks * p.cq + (size_t)chunk * p.cq + row;
+        const size_t tok = (size_t)batch * p.tq + (size_t)chunk * p.cq + row;
         const float inv = p.normalize ? safe_recip(l) : 1.f;
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.O) + (tok * p.hq + qhead) * HD);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.O) + (tok * p.hq + qhead) * p.d);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
+          if (8 * j >= p.d) break;
           uint4 v;
           v.x = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 0]), inv * __uint_as_float(acc[8 * j + 1]));
           v.y = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 2]), inv * __uint_as_float(acc[8 * j + 3]));
@@ -462,15 +467,16 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
 
 }  // namespace pr
 
-extern "C" int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int hq, int h, int d, const void* Q,
-                            const void* K, const void* V, const float* a, const void* Z, const void* zg_hi,
-                            const void* zg_lo, int state_from_chunk, int q_gate_last, int normalize, float scale,
-                            int deg, void* O, float* l_out, int device, void* stream) {
-  using namespace pr;
+int pr::chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int h, int d, const void* Q, const void* K,
+                  const void* V, const float* a, const void* Z, const void* zg_hi, const void* zg_lo,
+                  int state_from_chunk, int q_gate_last, int normalize, float scale, int deg, void* O, float* l_out,
+                  int device, void* stream) {
   using namespace pr::co;
-  PR_REQUIRE(d == HD, PR_ERR_BAD_ARG, "head dim %d: this build handles d = 64", d);
-  PR_REQUIRE(b > 0 && n_chunks > 0 && cq > 0 && ck >= cq && hq > 0 && h > 0 && hq % h == 0, PR_ERR_BAD_ARG,
-             "bad sizes b=%d n=%d cq=%d ck=%d hq=%d h=%d", b, n_chunks, cq, ck, hq, h);
+  PR_REQUIRE(head_dim_ok(d), PR_ERR_BAD_ARG, "head dim %d: a multiple of 16 up to 64", d);
+  const int n_chunks = cq > 0 ? (tq + cq - 1) / cq : 0;
+  PR_REQUIRE(b > 0 && n_chunks > 0 && cq > 0 && ck >= cq && hq > 0 && h > 0 && hq % h == 0 &&
+                 (n_chunks == 1 || (cq == ck && tq == tk)) && tk >= tq,
+             PR_ERR_BAD_ARG, "bad sizes b=%d n=%d cq=%d ck=%d hq=%d h=%d", b, n_chunks, cq, ck, hq, h);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(deg == 2 || (deg == 4 && Z == nullptr), PR_ERR_BAD_ARG,
              "deg=%d: states exist for deg 2; deg 4 runs state-free (attention only)", deg);
@@ -489,6 +495,10 @@ extern "C" int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int 
   p.n_chunks = n_chunks;
   p.cq = cq;
   p.ck = ck;
+  p.tq = tq;
+  p.tk = tk;
+  p.d = d;
+  p.nblk = ref_dim(d) / 64;
   p.tiles_per_chunk = (cq + 127) / 128;
   p.state_from_chunk = with_state ? state_from_chunk : n_chunks;
   p.q_gate_last = q_gate_last;
@@ -502,11 +512,10 @@ extern "C" int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int 
   if (rc) return rc;
   CUtensorMap tm_q, tm_k, tm_v, tm_z, tm_ghi, tm_glo;
   {
-    const uint64_t tq = (uint64_t)n_chunks * cq, tk = (uint64_t)n_chunks * ck;
-    uint64_t dq[4] = {(uint64_t)d, (uint64_t)hq, tq, (uint64_t)b};
-    uint64_t sq[4] = {0, (uint64_t)d * 2, (uint64_t)hq * d * 2, tq * hq * d * 2};
-    uint64_t dk[4] = {(uint64_t)d, (uint64_t)h, tk, (uint64_t)b};
-    uint64_t sk[4] = {0, (uint64_t)d * 2, (uint64_t)h * d * 2, tk * h * d * 2};
+    uint64_t dq[4] = {(uint64_t)d, (uint64_t)hq, (uint64_t)tq, (uint64_t)b};
+    uint64_t sq[4] = {0, (uint64_t)d * 2, (uint64_t)hq * d * 2, (uint64_t)tq * hq * d * 2};
+    uint64_t dk[4] = {(uint64_t)d, (uint64_t)h, (uint64_t)tk, (uint64_t)b};
+    uint64_t sk[4] = {0, (uint64_t)d * 2, (uint64_t)h * d * 2, (uint64_t)tk * h * d * 2};
     uint32_t box[4] = {64, 1, 128, 1};
     uint32_t box_kv[4] = {64, 1, (uint32_t)TW, 1};
     if ((rc = make_tmap(&tm_q, Q, 2, 4, dq, sq, box, true))) return rc;
@@ -519,13 +528,12 @@ extern "C" int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int 
     }
   }
   if (with_state) {
-    uint64_t dz[2] = {64, (uint64_t)b * n_chunks * h * ref_dim(d)};
-    uint64_t dg[2] = {64, (uint64_t)b * n_chunks * h * d};
-    uint64_t st[2] = {0, 128};
+    uint64_t dz[2] = {(uint64_t)d, (uint64_t)b * n_chunks * h * ref_dim(d)};
+    uint64_t st[2] = {0, (uint64_t)d * 2};
     uint32_t box[2] = {64, 64};
     if ((rc = make_tmap(&tm_z, Z, 2, 2, dz, st, box, true))) return rc;
-    if ((rc = make_tmap(&tm_ghi, zg_hi, 2, 2, dg, st, box, true))) return rc;
-    if ((rc = make_tmap(&tm_glo, zg_lo, 2, 2, dg, st, box, true))) return rc;
+    if ((rc = gram_tmap(&tm_ghi, zg_hi, d, (uint64_t)b * n_chunks * h))) return rc;
+    if ((rc = gram_tmap(&tm_glo, zg_lo, d, (uint64_t)b * n_chunks * h))) return rc;
   } else {
     tm_z = tm_q;
     tm_ghi = tm_q;
@@ -547,4 +555,12 @@ extern "C" int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int 
 #undef PR_LAUNCH_OUT
   PR_CUDA(cudaGetLastError());
   return PR_OK;
+}
+
+extern "C" int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int hq, int h, int d, const void* Q,
+                            const void* K, const void* V, const float* a, const void* Z, const void* zg_hi,
+                            const void* zg_lo, int state_from_chunk, int q_gate_last, int normalize, float scale,
+                            int deg, void* O, float* l_out, int device, void* stream) {
+  return pr::chunk_out(dtype, b, n_chunks * cq, n_chunks * ck, cq, ck, hq, h, d, Q, K, V, a, Z, zg_hi, zg_lo,
+                       state_from_chunk, q_gate_last, normalize, scale, deg, O, l_out, device, stream);
 }

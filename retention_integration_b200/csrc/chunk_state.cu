@@ -45,6 +45,7 @@ struct ChunkStateParams {
   int group;        // operand heads summed into one output head (GQA ratio in backward)
   int c, cp;        // chunk length, padded to 64
   int n_chunks;     // chunks per batch element
+  int t, d;         // tokens (the last chunk may be shorter), features (a multiple of 16)
   int key_weights;  // 1: weight 2 on pairs from different 16-blocks; 0: all weights 1
   void* out;        // [b, n, nh, D2, 64]
   float* gram;      // [b, n, nh, 64, 64] or null
@@ -82,7 +83,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
   const int head = ch % p.nh;
   const int chunk = (ch / p.nh) % p.n_chunks;
   const int batch = ch / (p.nh * p.n_chunks);
-  const int kblocks = p.cp / TOK;
+  const int kblocks = (min(p.c, p.t - chunk * p.c) + TOK - 1) / TOK;
   const int total = kblocks * p.group;
 
   if (tid == 0) {
@@ -118,17 +119,17 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
         const int s = it % NS, ph = (it / NS) & 1;
         const int g = it / kblocks, kb = it % kblocks;
         const int xhead = head * p.group + g;
-        const int xrow = ((batch * p.n_chunks + chunk) * (p.nh * p.group) + xhead) * HD;
+        const int xrow = ((batch * p.n_chunks + chunk) * (p.nh * p.group) + xhead) * p.d;
         if (!gram_cta && !mbar_wait(&x_empty[s], ph ^ 1, &abort_flag)) break;
         if (gram_cta) {
           // two stages only: the padded A operand is twice the size of a value stage
           const int gs = it & 1, gph = (it >> 1) & 1;
           if (!mbar_wait(&w_empty[gs], gph ^ 1, &abort_flag)) break;
-          mbar_expect_tx(&w_full[gs], 2 * XT_BYTES);
+          mbar_expect_tx(&w_full[gs], 2 * p.d * (TOK * 2));
           tma_load_2d(smX + gs * XT_BYTES, &tm_xt, &w_full[gs], kb * TOK, xrow);
           tma_load_2d(smG + gs * GA_BYTES, &tm_xs, &w_full[gs], kb * TOK, xrow);
         } else {
-          mbar_expect_tx(&x_full[s], XT_BYTES);
+          mbar_expect_tx(&x_full[s], p.d * (TOK * 2));
           tma_load_2d(smX + s * XT_BYTES, &tm_xt, &x_full[s], kb * TOK, xrow);
           if (it >= NS && !(mbar_wait(&done[0][s], ph ^ 1, &abort_flag) && mbar_wait(&done[1][s], ph ^ 1, &abort_flag)))
             break;
@@ -182,7 +183,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
     const int grp = warp >> 2;
     const int row_in_tile = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    const int D2 = ref_dim(HD);
+    const int D2 = p.n_tiles * 128;
     // expansion: this thread's row of both tiles (first factors a0 and a0 + 8, common second factor b),
     // tokens [32 grp, 32 grp + 32) of every stage; epilogue: its row of tile `grp`
     const int drow0 = slot * NG * 128 + row_in_tile;
@@ -255,19 +256,20 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
       tmem_ld32(tmem + lane_addr + COL_ACC + grp * 64 + 32, acc + 32);
       tmem_wait_ld();
       if (gram_cta) {
-        if (grp == 0 && row_in_tile < HD && p.gram != nullptr) {
-          float4* dst = reinterpret_cast<float4*>(p.gram + ((size_t)ch * HD + row_in_tile) * HD);
+        if (grp == 0 && row_in_tile < p.d && p.gram != nullptr) {
+          float4* dst = reinterpret_cast<float4*>(p.gram + ((size_t)ch * p.d + row_in_tile) * p.d);
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            dst[j] = make_float4(__uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]),
+            if (4 * j < p.d) dst[j] = make_float4(__uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]),
                                  __uint_as_float(acc[4 * j + 2]), __uint_as_float(acc[4 * j + 3]));
         }
       } else if (valid) {
         const float wgt = p.key_weights ? ref_key_weight(a, b) : 1.f;
-        T* dst = static_cast<T*>(p.out) + ((size_t)ch * D2 + drow) * HD;
+        T* dst = static_cast<T*>(p.out) + ((size_t)ch * D2 + drow) * p.d;
         // four 32-byte stores: a full sector per thread and instruction
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
+          if (16 * j >= p.d) break;
           uint32_t v[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k)
@@ -305,11 +307,10 @@ static int launch_chunk_state(const ChunkStateParams& p, int b, const CUtensorMa
 
 }  // namespace pr
 
-extern "C" int pr_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
-                              const void* v, void* out, float* gram, int key_weights, int device, void* stream) {
-  using namespace pr;
-  PR_REQUIRE(d == cs::HD, PR_ERR_BAD_ARG, "head dim %d: this build handles d = 64", d);
-  PR_REQUIRE(b > 0 && t > 0 && nh > 0 && group > 0 && c > 0 && t % c == 0, PR_ERR_BAD_ARG,
+int pr::chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
+                    const void* v, void* out, float* gram, int key_weights, int device, void* stream) {
+  PR_REQUIRE(head_dim_ok(d), PR_ERR_BAD_ARG, "head dim %d: a multiple of 16 up to 64", d);
+  PR_REQUIRE(b > 0 && t > 0 && nh > 0 && group > 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d heads=%d group=%d c=%d", b, t, nh, group, c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(xt && v && out && aligned16(xt) && aligned16(v) && aligned16(out), PR_ERR_BAD_ARG,
@@ -323,7 +324,9 @@ extern "C" int pr_chunk_state(int dtype, int b, int t, int nh, int group, int d,
   p.group = group;
   p.c = c;
   p.cp = (c + 63) / 64 * 64;
-  p.n_chunks = t / c;
+  p.n_chunks = chunks_of(t, c);
+  p.t = t;
+  p.d = d;
   p.key_weights = key_weights;
   p.out = out;
   p.gram = gram;
@@ -350,4 +353,10 @@ extern "C" int pr_chunk_state(int dtype, int b, int t, int nh, int group, int d,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return dtype == PR_BF16 ? launch_chunk_state<__nv_bfloat16>(p, b, tm_xt, tm_xs, tm_w, s)
                           : launch_chunk_state<__half>(p, b, tm_xt, tm_xs, tm_w, s);
+}
+
+extern "C" int pr_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
+                              const void* v, void* out, float* gram, int key_weights, int device, void* stream) {
+  PR_REQUIRE(d == pr::cs::HD, PR_ERR_BAD_ARG, "head dim %d: this entry point handles d = 64", d);
+  return pr::chunk_state(dtype, b, t, nh, group, d, c, xt, xts, v, out, gram, key_weights, device, stream);
 }

@@ -27,8 +27,6 @@ namespace pr {
 
 namespace eg {
 constexpr int HD = 64;
-constexpr int D2 = ref_dim(HD);          // 2560 expanded rows (block layout, see layout.cuh)
-constexpr int NT = D2 / 128;             // 20 tiles of 128 rows = 8 first factors x 16
 constexpr int TILE_BYTES = 128 * 128;
 constexpr int G_BYTES = 64 * 128;
 // NRT row tiles of 128 tokens per CTA.  Warps: 4 NRT drain warps (one group of four per row tile), one
@@ -62,6 +60,8 @@ constexpr uint32_t OFF_XA = 0, OFF_U = 64;
 struct ExpandGradParams {
   int h, hx;             // gate/state heads, operand heads (hx = h * ratio)
   int n_chunks, c;
+  int t, d;              // tokens (the last chunk may be shorter), features (a multiple of 16)
+  int nt;                // tiles of 128 expanded rows (8 first factors x 16) of a state
   int tiles_per_chunk;
   int chunk_lo, chunk_hi;  // chunks in [lo, hi] have a state term; the others get zeros
   int query_side;
@@ -95,16 +95,17 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
   const int head = blockIdx.y, batch = blockIdx.z;
   const int gh = head / (p.hx / p.h);
   const int row0 = tile_i * ROWS;
-  const size_t tok0 = (size_t)batch * p.n_chunks * p.c + (size_t)chunk * p.c;
+  const size_t tok0 = (size_t)batch * p.t + (size_t)chunk * p.c;
+  const int c = min(p.c, p.t - chunk * p.c);  // tokens of this chunk
+  if (row0 >= c) return;
 
   if (chunk < p.chunk_lo || chunk > p.chunk_hi) {
     // no state term for this chunk: zero gradient
     if (tid < ROWS) {
       const int row = row0 + tid;
-      if (row < p.c) {
-        float4* dst = reinterpret_cast<float4*>(p.dX + ((tok0 + row) * p.hx + head) * HD);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) dst[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row < c) {
+        float4* dst = reinterpret_cast<float4*>(p.dX + ((tok0 + row) * p.hx + head) * p.d);
+        for (int j = 0; j < p.d / 4; ++j) dst[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         p.gdot[(tok0 + row) * p.hx + head] = 0.f;
       }
     }
@@ -157,15 +158,15 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
         tma_load_4d(smX + rt * TILE_BYTES, &tm_x, &w_full, 0, head, chunk * p.c + row0 + rt * 128, batch);
       }
       mbar_expect_tx(&g_full, 2 * G_BYTES);
-      tma_load_2d(smG, &tm_ghi, &g_full, 0, ch * HD);
-      tma_load_2d(smG + G_BYTES, &tm_glo, &g_full, 0, ch * HD);
-      for (int nt = 0; nt < NT; ++nt) {
+      tma_load_3d(smG, &tm_ghi, &g_full, 0, 0, ch);
+      tma_load_3d(smG + G_BYTES, &tm_glo, &g_full, 0, 0, ch);
+      for (int nt = 0; nt < p.nt; ++nt) {
         const int s = nt % NSS, ph = (nt / NSS) & 1;
         if (!mbar_wait(&s_empty[s], ph ^ 1, &abort_flag)) break;
         // the slot lent to the Gram operand is free once the Gram products have completed
         if (Cfg<NRT>::G_IN_RING && nt == NSS - 1 && !mbar_wait(&u_full[0], 0, &abort_flag)) break;
         mbar_expect_tx(&s_full[s], TILE_BYTES);
-        tma_load_2d(smS + s * TILE_BYTES, &tm_s, &s_full[s], 0, ch * D2 + nt * 128);
+        tma_load_2d(smS + s * TILE_BYTES, &tm_s, &s_full[s], 0, (ch * p.nt + nt) * 128);
       }
     }
   } else if (warp > W_TMA) {
@@ -178,7 +179,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
       bool ok = mbar_wait(&w_full, 0, &abort_flag);
       const uint32_t w_addr = smem_u32(smW) + rt * TILE_BYTES;
       const uint32_t idesc = umma_idesc(128, 128, Pack2<T>::is_bf16, false, false);
-      for (int nt = par; nt < NT && ok; nt += 2) {
+      for (int nt = par; nt < p.nt && ok; nt += 2) {
         const int s = nt % NSS, ph = (nt / NSS) & 1;
         const int b = par;
         // buffer 0 has been drained nt/2 times before tile nt; buffer 1 once more (the Gram part)
@@ -217,7 +218,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
     const int rt = warp >> 2;                  // row tile owned by this warp group
     const int r = (warp & 3) * 32 + lane;      // token row inside the tile = TMEM lane
     const int row = row0 + rt * 128 + r;
-    const bool row_valid = row < p.c;
+    const bool row_valid = row < c;
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
 
     float f = p.query_side ? p.scale : 1.f;
@@ -283,6 +284,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
     int nt = 0;
     static_for<0, HD / 16>([&](auto yc) {
       constexpr int Y = decltype(yc)::value;
+      if (16 * Y >= p.d) return;
       // second factors x~[16Y .. 16Y+15] of this block and their gradient accumulators, as pairs:
       // the drain runs on packed fp32 FMAs (two entries per instruction)
       float2 x[8], dx[8];
@@ -361,9 +363,10 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
 
     if (ok && row_valid) {
       float dot = 0.f;
-      float4* dst = reinterpret_cast<float4*>(p.dX + ((tok0 + row) * p.hx + head) * HD);
+      float4* dst = reinterpret_cast<float4*>(p.dX + ((tok0 + row) * p.hx + head) * p.d);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
+        if (8 * j >= p.d) break;
         const uint4 v4 = *reinterpret_cast<const uint4*>(xrow + swz128(r, j));
         const uint32_t w[4] = {v4.x, v4.y, v4.z, v4.w};
         float d8[8];
@@ -398,8 +401,8 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
                               int chunk_hi, float* dX, float* gdot, int device, void* stream) {
   using namespace pr;
   using namespace pr::eg;
-  PR_REQUIRE(d == HD, PR_ERR_BAD_ARG, "head dim %d: this build handles d = 64", d);
-  PR_REQUIRE(b > 0 && t > 0 && h > 0 && hx > 0 && hx % h == 0 && c > 0 && t % c == 0, PR_ERR_BAD_ARG,
+  PR_REQUIRE(head_dim_ok(d), PR_ERR_BAD_ARG, "head dim %d: a multiple of 16 up to 64", d);
+  PR_REQUIRE(b > 0 && t > 0 && h > 0 && hx > 0 && hx % h == 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d h=%d hx=%d c=%d", b, t, h, hx, c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(W && X && State && g_hi && g_lo && dX && gdot, PR_ERR_BAD_ARG, "null pointer");
@@ -408,12 +411,15 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
   PR_REQUIRE((a == nullptr) == (A == nullptr), PR_ERR_BAD_ARG, "a and A must be given together");
   PR_REQUIRE(hx <= 65535 && b <= 65535, PR_ERR_BAD_ARG, "hx and b must be <= 65535");
   PR_CUDA(cudaSetDevice(device));
-  const int n = t / c;
+  const int n = chunks_of(t, c);
   ExpandGradParams p;
   p.h = h;
   p.hx = hx;
   p.n_chunks = n;
   p.c = c;
+  p.t = t;
+  p.d = d;
+  p.nt = ref_dim(d) / 128;
   using C = Cfg<PR_EG_NRT>;
   p.tiles_per_chunk = (c + C::ROWS - 1) / C::ROWS;
   p.chunk_lo = chunk_lo;
@@ -437,13 +443,12 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
     if ((rc = make_tmap(&tm_x, X, 2, 4, dims, str, box, true))) return rc;
   }
   {
-    uint64_t ds[2] = {64, (uint64_t)b * n * h * D2};
-    uint64_t dg[2] = {64, (uint64_t)b * n * h * d};
-    uint64_t st[2] = {0, 128};
-    uint32_t box_s[2] = {64, 128}, box_g[2] = {64, 64};
+    uint64_t ds[2] = {(uint64_t)d, (uint64_t)b * n * h * ref_dim(d)};
+    uint64_t st[2] = {0, (uint64_t)d * 2};
+    uint32_t box_s[2] = {64, 128};
     if ((rc = make_tmap(&tm_s, State, 2, 2, ds, st, box_s, true))) return rc;
-    if ((rc = make_tmap(&tm_ghi, g_hi, 2, 2, dg, st, box_g, true))) return rc;
-    if ((rc = make_tmap(&tm_glo, g_lo, 2, 2, dg, st, box_g, true))) return rc;
+    if ((rc = gram_tmap(&tm_ghi, g_hi, d, (uint64_t)b * n * h))) return rc;
+    if ((rc = gram_tmap(&tm_glo, g_lo, d, (uint64_t)b * n * h))) return rc;
   }
   const size_t smem = C::SMEM;
   dim3 grid(p.tiles_per_chunk * n, hx, b);

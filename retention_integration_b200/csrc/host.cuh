@@ -48,6 +48,31 @@ int status_word(int device, int** dev_ptr, volatile int** host_ptr);
 int make_tmap(CUtensorMap* out, const void* base, int elem_bytes, int rank, const uint64_t* dims,
               const uint64_t* strides_bytes, const uint32_t* box, bool swizzle128);
 
+// A stack of `count` dense d x d 16-bit matrices as boxes of 64 x 64 (rows and columns past d read as zeros).
+inline int gram_tmap(CUtensorMap* out, const void* base, int d, uint64_t count) {
+  const uint64_t dims[3] = {(uint64_t)d, (uint64_t)d, count}, strides[3] = {0, (uint64_t)d * 2, (uint64_t)d * d * 2};
+  const uint32_t box[3] = {64, 64, 1};
+  return make_tmap(out, base, 2, 3, dims, strides, box, true);
+}
+
+// The kernels work on 64 features; narrower heads are widened with zeros by the TMA loads (boxes wider than the
+// tensor) and only their own features are written back.
+inline bool head_dim_ok(int d) { return d >= 16 && d <= 64 && d % 16 == 0; }
+
+// Chunks of a sequence of t tokens; the last one may be shorter.
+inline int chunks_of(int t, int c) { return (t + c - 1) / c; }
+
+// pr_chunk_out for sequences whose last chunk is shorter: tq queries and tk keys per batch element.
+int chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int h, int d, const void* Q, const void* K,
+              const void* V, const float* a, const void* Z, const void* zg_hi, const void* zg_lo, int state_from_chunk,
+              int q_gate_last, int normalize, float scale, int deg, void* O, float* l_out, int device, void* stream);
+// pr_dout_prep with dy optional.
+int dout_prep(int dtype, long long rows, int d, const void* O, const void* dO, const float* l, void* dy, float* dl,
+              int device, void* stream);
+// pr_chunk_state for every head dim of head_dim_ok.
+int chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts, const void* v,
+                void* out, float* gram, int key_weights, int device, void* stream);
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Dynamic shared memory of a kernel: the attribute is raised once per kernel and device (and again only when a

@@ -32,12 +32,13 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
   __shared__ float carry_s;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int n = t / c;
+  const int n = (t + c - 1) / c;
   const int head = blockIdx.x % hx;
   const int chunk = (blockIdx.x / hx) % n;
   const int batch = blockIdx.x / (hx * n);
   const int gh = head / (hx / h);  // gate / kv head of this head
   const size_t tok0 = (size_t)batch * t + (size_t)chunk * c;
+  c = min(c, t - chunk * c);  // the last chunk may be shorter
 
   // ---- the chunk's cumulative log gates: read if a pass before this one has made them, else a
   // block-wide inclusive scan of the log gates
@@ -92,7 +93,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
   T* out2_base = xts ? xts + ((size_t)(batch * n + chunk) * hx + head) * (size_t)d * cp : nullptr;
   // the chunk's 64-token tiles are split over gridDim.y blocks (each recomputes the cheap scan)
   const int tiles = cp / 64, tiles_per = (tiles + gridDim.y - 1) / gridDim.y;
-  const int tb_end = min(cp, (int)(blockIdx.y + 1) * tiles_per * 64);
+  const int tb_end = min((c + 63) & ~63, (int)(blockIdx.y + 1) * tiles_per * 64);
   // The loads of tile k+1 are issued before tile k is transposed and written out, so a CTA always has
   // a tile's worth of reads in flight (64 tokens x d features: up to four 16-byte vectors per thread).
   constexpr int kMaxVec = NV;  // 4 covers d <= 64, 8 covers d <= 128
@@ -217,7 +218,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
 template <typename T>
 __global__ void dout_prep_kernel(const T* __restrict__ O, const T* __restrict__ dO, const float* __restrict__ l,
                                  T* __restrict__ dy, float* __restrict__ dl, size_t rows, int d) {
-  const int lanes_per_row = d / 8;  // 4, 8 or 16 threads share a row
+  const int lanes_per_row = d / 8;  // 2, 4, 8 or 16 threads share a row
   const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t row = gid / lanes_per_row;
   const int sub = (int)(gid % lanes_per_row);
@@ -236,7 +237,8 @@ __global__ void dout_prep_kernel(const T* __restrict__ O, const T* __restrict__ 
     }
   }
   for (int off = lanes_per_row >> 1; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-  if (active) {
+  if (active && sub == 0) dl[row] = -part * inv;
+  if (active && dy != nullptr) {  // the state-free branch has no use for dy
     uint32_t gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -244,7 +246,6 @@ __global__ void dout_prep_kernel(const T* __restrict__ O, const T* __restrict__ 
       gw[k] = Pack2<T>::from_f32(b.x * inv, b.y * inv);
     }
     *reinterpret_cast<uint4*>(dy + row * d + sub * 8) = make_uint4(gw[0], gw[1], gw[2], gw[3]);
-    if (sub == 0) dl[row] = -part * inv;
   }
 }
 
@@ -262,11 +263,12 @@ gate_grad_kernel(const float* __restrict__ da_q, const float* __restrict__ gq, c
   __shared__ float warp_tot[kPrepThreads / 32];
   __shared__ float carry_s, wk_sum_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int n = t / c, ratio = hq / h;
+  const int n = (t + c - 1) / c, ratio = hq / h;
   const int head = blockIdx.x % h;
   const int chunk = (blockIdx.x / h) % n;
   const int batch = blockIdx.x / (h * n);
   const size_t tok0 = (size_t)batch * t + (size_t)chunk * c;
+  c = min(c, t - chunk * c);  // the last chunk may be shorter
 
   // chunk-gate gradient: key discount terms of the chunk + the reverse scans' partial sums
   // ([b, h, scan_blocks, n] and [b, h, gram_blocks, n]), all reduced by the whole block
@@ -327,11 +329,10 @@ gate_grad_kernel(const float* __restrict__ da_q, const float* __restrict__ gq, c
 
 }  // namespace pr
 
-extern "C" int pr_dout_prep(int dtype, long long rows, int d, const void* O, const void* dO, const float* l, void* dy,
-                            float* dl, int device, void* stream) {
-  using namespace pr;
-  PR_REQUIRE(rows > 0 && (d == 32 || d == 64 || d == 128), PR_ERR_BAD_ARG, "rows=%lld d=%d", rows, d);
-  PR_REQUIRE(O && dO && l && dy && dl && aligned16(O) && aligned16(dO) && aligned16(dy), PR_ERR_BAD_ARG,
+int pr::dout_prep(int dtype, long long rows, int d, const void* O, const void* dO, const float* l, void* dy, float* dl,
+                  int device, void* stream) {
+  PR_REQUIRE(rows > 0 && (d == 16 || d == 32 || d == 64 || d == 128), PR_ERR_BAD_ARG, "rows=%lld d=%d", rows, d);
+  PR_REQUIRE(O && dO && l && dl && aligned16(O) && aligned16(dO) && aligned16(dy), PR_ERR_BAD_ARG,
              "null or misaligned pointer");
   PR_CUDA(cudaSetDevice(device));
   const size_t threads = (size_t)rows * (d / 8);
@@ -350,13 +351,19 @@ extern "C" int pr_dout_prep(int dtype, long long rows, int d, const void* O, con
   return PR_OK;
 }
 
+extern "C" int pr_dout_prep(int dtype, long long rows, int d, const void* O, const void* dO, const float* l, void* dy,
+                            float* dl, int device, void* stream) {
+  PR_REQUIRE(dy != nullptr, PR_ERR_BAD_ARG, "null pointer");
+  return pr::dout_prep(dtype, rows, d, O, dO, l, dy, dl, device, stream);
+}
+
 extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c, const float* log_g, const void* x,
                             float* a_out, float* A_out, void* xt, const float* row_scale, void* xts, int query_side,
                             float mult, int write_a, int device, void* stream) {
   using namespace pr;
   PR_REQUIRE(b > 0 && t > 0 && h > 0 && hx > 0 && hx % h == 0, PR_ERR_BAD_ARG, "bad sizes b=%d t=%d h=%d hx=%d", b, t,
              h, hx);
-  PR_REQUIRE(c > 0 && t % c == 0, PR_ERR_BAD_ARG, "t=%d is not a multiple of the chunk size %d", t, c);
+  PR_REQUIRE(c > 0, PR_ERR_BAD_ARG, "chunk size %d", c);
   PR_REQUIRE(d % 8 == 0 && d >= 16 && d <= 128, PR_ERR_BAD_ARG, "head dim %d unsupported", d);
   PR_REQUIRE(c <= 16384, PR_ERR_BAD_ARG, "chunk size %d exceeds 16384", c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
@@ -376,11 +383,11 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
   {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const long long base = (long long)b * (t / c) * hx;
+    const long long base = (long long)b * chunks_of(t, c) * hx;
     const long long want = ((long long)sms * 8 + base - 1) / base;  // eight 128-thread CTAs per SM are resident
     ysplit = (int)std::min<long long>(tiles, std::max<long long>(ysplit, want));
   }
-  const dim3 grid(b * (t / c) * hx, xt ? ysplit : 1);
+  const dim3 grid(b * chunks_of(t, c) * hx, xt ? ysplit : 1);
   // The cumulative gates are scanned once per (batch, chunk, gate head), not once per CTA of the transposing
   // pass: either they are handed in (write_a = 0 with a_out given: the backward reuses the forward's), or a
   // first small launch makes them and the transposing launch reads them.
@@ -405,14 +412,14 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
   } while (0)
   if (dtype == PR_BF16) {
     if (two_pass) {
-      PR_LAUNCH_PREP(__nv_bfloat16, dim3(b * (t / c) * h, 1), log_g, nullptr, nullptr, nullptr, 1);
+      PR_LAUNCH_PREP(__nv_bfloat16, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, nullptr, 1);
       PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_out, xt, xts, 0);
     } else {
       PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_in, xt, xts, write_a);
     }
   } else {
     if (two_pass) {
-      PR_LAUNCH_PREP(__half, dim3(b * (t / c) * h, 1), log_g, nullptr, nullptr, nullptr, 1);
+      PR_LAUNCH_PREP(__half, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, nullptr, 1);
       PR_LAUNCH_PREP(__half, grid, log_g, a_out, xt, xts, 0);
     } else {
       PR_LAUNCH_PREP(__half, grid, log_g, a_in, xt, xts, write_a);
@@ -427,11 +434,11 @@ extern "C" int pr_gate_grad(int b, int t, int h, int hq, int c, const float* da_
                             const float* wk, const float* dA_scan, int scan_blocks, const float* dA_gram,
                             int gram_blocks, float* dlog_g, int device, void* stream) {
   using namespace pr;
-  PR_REQUIRE(b > 0 && t > 0 && h > 0 && hq > 0 && hq % h == 0 && c > 0 && t % c == 0, PR_ERR_BAD_ARG,
+  PR_REQUIRE(b > 0 && t > 0 && h > 0 && hq > 0 && hq % h == 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d h=%d hq=%d c=%d", b, t, h, hq, c);
   PR_REQUIRE(da_q && da_k && dlog_g, PR_ERR_BAD_ARG, "null pointer");
   PR_CUDA(cudaSetDevice(device));
-  gate_grad_kernel<<<b * (t / c) * h, kPrepThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  gate_grad_kernel<<<b * chunks_of(t, c) * h, kPrepThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       da_q, gq, da_k, wk, dA_scan, scan_blocks, dA_gram, gram_blocks, dlog_g, t, h, hq, c);
   PR_CUDA(cudaGetLastError());
   return PR_OK;

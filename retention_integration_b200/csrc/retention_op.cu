@@ -29,12 +29,12 @@ struct Sizes {
 
 int sizes_of(const pr_problem* p, Sizes* s) {
   PR_REQUIRE(p != nullptr, PR_ERR_BAD_ARG, "problem is null");
-  PR_REQUIRE(p->d == 64, PR_ERR_BAD_ARG, "head dim %d: this build handles d = 64", p->d);
+  PR_REQUIRE(p->d == 16 || p->d == 32 || p->d == 64, PR_ERR_BAD_ARG, "head dim %d: this build handles 16, 32 and 64", p->d);
   PR_REQUIRE(p->dtype == PR_BF16 || p->dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", p->dtype);
-  PR_REQUIRE(p->b > 0 && p->t > 0 && p->h > 0 && p->hq > 0 && p->hq % p->h == 0 && p->c > 0 && p->t % p->c == 0,
+  PR_REQUIRE(p->b > 0 && p->t > 0 && p->h > 0 && p->hq > 0 && p->hq % p->h == 0 && p->c > 0,
              PR_ERR_BAD_ARG, "bad sizes b=%d t=%d h=%d hq=%d c=%d", p->b, p->t, p->h, p->hq, p->c);
   const size_t b = p->b, t = p->t, h = p->h, hq = p->hq, d = p->d;
-  s->n = p->t / p->c;
+  s->n = chunks_of(p->t, p->c);
   s->cp = (p->c + 63) / 64 * 64;
   s->DR = ref_dim(p->d);
   s->esz = 2;
@@ -126,6 +126,40 @@ int side_stream_ready(SideStream* s) {
   return PR_OK;
 }
 
+// The fork of one backward pass: begin(), launches on side(), side_done(), launches on the caller's stream, join().
+class Fork {
+ public:
+  int begin(int device, void* stream) {
+    PR_REQUIRE(device >= 0 && device < kMaxDevices, PR_ERR_BAD_ARG, "device ordinal %d out of range", device);
+    main_ = static_cast<cudaStream_t>(stream);
+    if (!overlap_enabled()) return PR_OK;
+    lock_ = std::unique_lock<std::mutex>(g_side[device].mu);
+    PR_CUDA(cudaSetDevice(device));
+    int rc = side_stream_ready(&g_side[device]);
+    if (rc) return rc;
+    PR_CUDA(cudaEventRecord(g_side[device].fork, main_));
+    PR_CUDA(cudaStreamWaitEvent(g_side[device].stream, g_side[device].fork, 0));
+    s_ = &g_side[device];
+    return PR_OK;
+  }
+  void* side() const { return s_ ? s_->stream : main_; }
+  // recorded even after an error, so that a capture of the caller's stream is left in a closable state
+  void side_done() {
+    if (s_) cudaEventRecord(s_->join, s_->stream);
+  }
+  int join(int rc) {
+    if (!s_) return rc;
+    cudaError_t e = cudaStreamWaitEvent(main_, s_->join, 0);
+    lock_.unlock();
+    return (!rc && e != cudaSuccess) ? fail(PR_ERR_CUDA, "joining the second stream failed: %s", cudaGetErrorString(e)) : rc;
+  }
+
+ private:
+  SideStream* s_ = nullptr;
+  cudaStream_t main_ = nullptr;
+  std::unique_lock<std::mutex> lock_;
+};
+
 }  // namespace
 }  // namespace pr
 
@@ -206,12 +240,12 @@ extern "C" int pr_retention_fwd(const pr_problem* prob, const void* Q, const voi
                          nullptr, 0, 1.f, 1, device, stream)))
     return rc;
   // chunk states and Gram matrices, then their scans (in place: Z[m] = state entering chunk m)
-  if ((rc = pr_chunk_state(p.dtype, p.b, p.t, p.h, 1, p.d, p.c, KT, KT, V, sv.Z, gram, 1, device, stream))) return rc;
+  if ((rc = chunk_state(p.dtype, p.b, p.t, p.h, 1, p.d, p.c, KT, KT, V, sv.Z, gram, 1, device, stream))) return rc;
   if ((rc = pr_state_scan_fwd(p.dtype, p.b, s.n, p.h, p.d, E, sv.Z, sv.A, carry_state, final_state, gram, sv.zhi,
                               sv.zlo, sv.zfull, carry_gram, final_gram, device, stream)))
     return rc;
   // attention + state read-out + normalisation
-  return pr_chunk_out(p.dtype, p.b, s.n, p.c, p.c, p.hq, p.h, p.d, Q, K, V, gated ? sv.a : nullptr, sv.Z, sv.zhi,
+  return chunk_out(p.dtype, p.b, p.t, p.t, p.c, p.c, p.hq, p.h, p.d, Q, K, V, gated ? sv.a : nullptr, sv.Z, sv.zhi,
                       sv.zlo, carry_state ? 0 : 1, 0, 1, p.scale, 2, O, sv.l, device, stream);
 }
 
@@ -254,27 +288,15 @@ extern "C" int pr_retention_bwd(const pr_problem* prob, const void* Q, const voi
 
   // ---- query side, on the second stream when there is one: gradient through the read-out's expansion
   // (saved states), then the attention backward merged with it
-  PR_REQUIRE(device >= 0 && device < kMaxDevices, PR_ERR_BAD_ARG, "device ordinal %d out of range", device);
-  SideStream* side = overlap_enabled() ? &g_side[device] : nullptr;
-  std::unique_lock<std::mutex> lock;
-  void* qstream = stream;
-  if (side != nullptr) {
-    lock = std::unique_lock<std::mutex>(side->mu);
-    PR_CUDA(cudaSetDevice(device));
-    if ((rc = side_stream_ready(side))) return rc;
-    PR_CUDA(cudaEventRecord(side->fork, static_cast<cudaStream_t>(stream)));
-    PR_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
-    qstream = side->stream;
-  }
+  Fork fork;
+  if ((rc = fork.begin(device, stream))) return rc;
+  void* qstream = fork.side();
   rc = pr_expand_grad(p.dtype, p.b, p.t, p.h, p.hq, p.d, p.c, dy, Q, sv.Z, sv.zhi, sv.zlo, a, A, dl, 1, p.scale, 2.f,
                       had_carry ? 0 : 1, s.n - 1, dqs, gq, device, qstream);
   if (!rc)
     rc = pr_chunk_dq(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.c, Q, dO, K, V, a, dl, sv.l, dqs, p.scale, 2, dQ, daq, device,
                      qstream);
-  if (side != nullptr) {
-    // joined even after an error, so that a capture of the caller's stream is left in a closable state
-    cudaEventRecord(side->join, side->stream);
-  }
+  fork.side_done();
 
   // ---- key side: gradient of the state read-out (dZ_m, dZg_m from the gated queries; the forward's
   // cumulative gates are read, not rescanned), reverse scans (in place: dZ becomes w (.) dS_m), gradient
@@ -282,7 +304,7 @@ extern "C" int pr_retention_bwd(const pr_problem* prob, const void* Q, const voi
   if (!rc)
     rc = pr_gate_prep(p.dtype, p.b, p.t, p.h, p.hq, p.d, p.c, log_G, Q, gated ? sv.a : nullptr, nullptr, QT, dl, QTs, 1,
                       p.scale, 0, device, stream);
-  if (!rc) rc = pr_chunk_state(p.dtype, p.b, p.t, p.h, group, p.d, p.c, QT, QTs, dy, dZ, dZg, 0, device, stream);
+  if (!rc) rc = chunk_state(p.dtype, p.b, p.t, p.h, group, p.d, p.c, QT, QTs, dy, dZ, dZg, 0, device, stream);
   if (!rc)
     rc = pr_state_scan_bwd(p.dtype, p.b, s.n, p.h, p.d, E, dZ, sv.Z, sv.A, nullptr, nullptr, partS, dZg, sv.zfull, ghi,
                            glo, nullptr, nullptr, partG, device, stream);
@@ -292,14 +314,95 @@ extern "C" int pr_retention_bwd(const pr_problem* prob, const void* Q, const voi
   if (!rc)
     rc = pr_chunk_dkv(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.c, Q, dO, K, V, dZ, a, A, dl, sv.l, dks, s.n - 2, p.scale, 2,
                       dK, dV, dak, device, stream);
-  if (side != nullptr) {
-    cudaError_t e = cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), side->join, 0);
-    if (!rc && e != cudaSuccess) rc = fail(PR_ERR_CUDA, "joining the second stream failed: %s", cudaGetErrorString(e));
-    lock.unlock();
-  }
+  rc = fork.join(rc);
   if (rc) return rc;
   if (gated)
     return pr_gate_grad(p.b, p.t, p.h, p.hq, p.c, daq, gq, dak, wk, partS, s.blocksS, partG, s.blocksG, dlog_G, device,
                         stream);
   return PR_OK;
+}
+
+// ---- The state-free branch: one chunk holds the whole sequence, so there is no state to form, scan or read.
+namespace pr {
+namespace {
+
+// Saved from forward to backward: gate sums, row sums.  Backward scratch: dl, da_q, da_k.
+int attention_check(const pr_problem* p, int deg) {
+  PR_REQUIRE(p != nullptr, PR_ERR_BAD_ARG, "problem is null");
+  PR_REQUIRE(p->d == 16 || p->d == 32 || p->d == 64, PR_ERR_BAD_ARG, "head dim %d: this build handles 16, 32 and 64", p->d);
+  PR_REQUIRE(p->dtype == PR_BF16 || p->dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", p->dtype);
+  PR_REQUIRE(p->b > 0 && p->t > 0 && p->h > 0 && p->hq > 0 && p->hq % p->h == 0, PR_ERR_BAD_ARG,
+             "bad sizes b=%d t=%d h=%d hq=%d", p->b, p->t, p->h, p->hq);
+  PR_REQUIRE(deg == 2 || deg == 4, PR_ERR_BAD_ARG, "deg=%d: 2 or 4", deg);
+  return PR_OK;
+}
+
+}  // namespace
+}  // namespace pr
+
+extern "C" int pr_attention_workspace_bytes(const pr_problem* prob, int what, size_t* out) {
+  using namespace pr;
+  PR_REQUIRE(out != nullptr, PR_ERR_BAD_ARG, "out is null");
+  int rc = attention_check(prob, 2);
+  if (rc) return rc;
+  const size_t a = up((size_t)prob->b * prob->t * prob->h * 4), l = up((size_t)prob->b * prob->t * prob->hq * 4);
+  PR_REQUIRE(what == PR_WS_SAVED || what == PR_WS_BWD_SCRATCH, PR_ERR_BAD_ARG, "workspace kind %d", what);
+  *out = what == PR_WS_SAVED ? a + l : a + 2 * l;
+  return PR_OK;
+}
+
+extern "C" int pr_attention_fwd(const pr_problem* prob, int deg, const void* Q, const void* K, const void* V,
+                                const float* log_G, void* O, void* saved, int device, void* stream) {
+  using namespace pr;
+  int rc = attention_check(prob, deg);
+  if (rc) return rc;
+  PR_REQUIRE(Q && K && V && O && saved, PR_ERR_BAD_ARG, "null pointer");
+  const pr_problem& p = *prob;
+  Carver c{static_cast<uint8_t*>(saved)};
+  float* a = c.take<float>(up((size_t)p.b * p.t * p.h * 4));
+  float* l = c.take<float>(0);
+  // one chunk longer than the chunk-local scan holds in shared memory takes the plain cumulative sum
+  if (log_G != nullptr) {
+    if (p.t > 16384)
+      rc = pr_gate_cumsum(p.b, p.t, p.h, log_G, (long long)p.t * p.h, a, device, stream);
+    else
+      rc = pr_gate_prep(p.dtype, p.b, p.t, p.h, p.h, p.d, p.t, log_G, K, a, nullptr, nullptr, nullptr, nullptr, 0, 1.f,
+                        1, device, stream);
+    if (rc) return rc;
+  }
+  return chunk_out(p.dtype, p.b, p.t, p.t, p.t, p.t, p.hq, p.h, p.d, Q, K, V, log_G ? a : nullptr, nullptr, nullptr,
+                   nullptr, 1, 0, 1, p.scale, deg, O, l, device, stream);
+}
+
+extern "C" int pr_attention_bwd(const pr_problem* prob, int deg, const void* Q, const void* K, const void* V,
+                                const float* log_G, const void* O, const void* dO, void* saved, void* scratch, void* dQ,
+                                void* dK, void* dV, float* dlog_G, int device, void* stream) {
+  using namespace pr;
+  int rc = attention_check(prob, deg);
+  if (rc) return rc;
+  PR_REQUIRE(Q && K && V && O && dO && saved && scratch && dQ && dK && dV, PR_ERR_BAD_ARG, "null pointer");
+  PR_REQUIRE(log_G == nullptr || dlog_G != nullptr, PR_ERR_BAD_ARG, "gated problem without a dlog_G output");
+  const pr_problem& p = *prob;
+  const size_t asz = up((size_t)p.b * p.t * p.h * 4), lsz = up((size_t)p.b * p.t * p.hq * 4);
+  Carver c{static_cast<uint8_t*>(saved)};
+  const float* a = c.take<float>(asz);
+  const float* l = c.take<float>(lsz);
+  if (log_G == nullptr) a = nullptr;
+  Carver w{static_cast<uint8_t*>(scratch)};
+  float* dak = w.take<float>(asz);
+  float* dl = w.take<float>(lsz);
+  float* daq = w.take<float>(lsz);
+  if ((rc = dout_prep(p.dtype, (long long)p.b * p.t * p.hq, p.d, O, dO, l, nullptr, dl, device, stream))) return rc;
+  Fork fork;
+  if ((rc = fork.begin(device, stream))) return rc;
+  rc = pr_chunk_dq(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.t, Q, dO, K, V, a, dl, l, nullptr, p.scale, deg, dQ, daq, device,
+                   fork.side());
+  fork.side_done();
+  if (!rc)
+    rc = pr_chunk_dkv(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.t, Q, dO, K, V, nullptr, a, nullptr, dl, l, nullptr, -1,
+                      p.scale, deg, dK, dV, dak, device, stream);
+  rc = fork.join(rc);
+  if (rc || log_G == nullptr) return rc;
+  return pr_gate_grad(p.b, p.t, p.h, p.hq, p.t, daq, nullptr, dak, nullptr, nullptr, 0, nullptr, 0, dlog_G, device,
+                      stream);
 }
