@@ -16,6 +16,7 @@ PR_BF16, PR_FP16 = 0, 1
 PR_OK = 0
 
 _lib = None
+_host = None
 
 
 class PRError(RuntimeError):
@@ -34,6 +35,21 @@ def lib() -> ctypes.CDLL:
         _lib.pr_last_error.restype = ctypes.c_char_p
         _lib.pr_abi_version.restype = ctypes.c_int
     return _lib
+
+
+def host():
+    """The native host path (csrc/binding.cpp).  Like the library it sits on, it has no fallback."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise PRError(f"the host module is missing or does not load ({e}): build it with "
+                          "`python -m retention_integration_b200.build` (there is no fallback path)") from e
+        module.set_error_type(PRError)
+        _host = module
+    return _host
 
 
 def check(rc: int, what: str) -> None:

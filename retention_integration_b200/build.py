@@ -1,4 +1,5 @@
-"""Builds libpr_b200.so (the C-ABI library of sm_100a kernels) in-tree with nvcc.
+"""Builds libpr_b200.so (the C-ABI library of sm_100a kernels) with nvcc, and _host.so (the Python module of the
+host path, csrc/binding.cpp) on top of it with the C++ compiler, both in-tree.
 
     python -m retention_integration_b200.build [--force] [--verbose]
 
@@ -17,6 +18,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libpr_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 
 NVCC_FLAGS = [
@@ -57,6 +59,30 @@ def _compile(src: str, obj: str, verbose: bool) -> None:
         raise RuntimeError(f"nvcc failed on {src}")
 
 
+def _build_host(force: bool, verbose: bool) -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    src = os.path.join(CSRC, "binding.cpp")
+    deps = [src, os.path.join(INCLUDE, "pr_b200.h")]
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(map(os.path.getmtime, deps)):
+        return
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    incs = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in incs), src,
+           "-o", HOST_PATH, f"-L{PKG_DIR}", "-lpr_b200", f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        raise RuntimeError(f"compiling {src} failed")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ_DIR, exist_ok=True)
     newest_header = max(os.path.getmtime(h) for h in _headers())
@@ -76,6 +102,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link of libpr_b200.so failed")
+    _build_host(force, verbose)
     return LIB_PATH
 
 

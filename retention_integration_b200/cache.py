@@ -23,7 +23,7 @@ import math
 
 import torch
 
-from . import layout, ops
+from . import _lib, layout
 from ._lib import PRError
 from .retention import power_retention_inference
 
@@ -111,7 +111,7 @@ class RetentionCache:
             new_state, new_sok = self.state, self.sum_of_keys  # every row is read and written by one thread
         else:
             new_state, new_sok = torch.empty_like(self.state), torch.empty_like(self.sum_of_keys)
-        y = ops.decode_recurrent(q, k, v, log_g, self.state, self.sum_of_keys, new_state, new_sok, scale)
+        y = _lib.host().decode_recurrent(q, k, v, log_g, self.state, self.sum_of_keys, new_state, new_sok, scale)
         self.state, self.sum_of_keys = new_state, new_sok
         return y
 

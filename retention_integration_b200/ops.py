@@ -20,12 +20,17 @@ class LaunchLog:
     events on the launching stream (used by bench.py for the per-kernel breakdown)."""
 
     def __init__(self):
-        self.count = 0
         self.timing = False
         self.events = []  # (name, start, end)
+        self._python = self._native0 = 0
+
+    @property
+    def count(self) -> int:
+        """Kernels launched since the last reset: from this module, and by the native host path."""
+        return self._python + _lib.host().launches() - self._native0
 
     def reset(self, timing: bool = False):
-        self.count = 0
+        self._python, self._native0 = 0, _lib.host().launches()
         self.timing = timing
         self.events = []
 
@@ -40,10 +45,6 @@ class LaunchLog:
 
 launch_log = LaunchLog()
 
-# kernels launched per entry point (for the launch count reported by bench.py)
-_KERNELS_PER_CALL = {}
-
-
 def _call(name: str, *args):
     fn = getattr(lib(), name)
     if launch_log.timing:
@@ -55,7 +56,7 @@ def _call(name: str, *args):
     else:
         rc = fn(*args)
     check(rc, name)
-    launch_log.count += 1
+    launch_log._python += 1
 
 
 def state_rows(d: int) -> int:
@@ -346,56 +347,6 @@ def state_merge(state, sum_of_keys, S, gram, a_last):
     return new_state, new_sok
 
 
-class _Problem(ctypes.Structure):
-    _fields_ = [("dtype", c_int), ("b", c_int), ("t", c_int), ("h", c_int), ("hq", c_int), ("d", c_int), ("c", c_int),
-                ("scale", c_float)]
-
-
-def _problem(Q, h: int, c: int, scale: float) -> _Problem:
-    b, t, hq, d = Q.shape
-    return _Problem(dtype_code(Q.dtype), b, t, h, hq, d, c, scale)
-
-
-def _workspace(prob: _Problem, what: int, dev) -> torch.Tensor:
-    n = ctypes.c_size_t(0)
-    check(lib().pr_workspace_bytes(ctypes.byref(prob), c_int(what), ctypes.byref(n)), "pr_workspace_bytes")
-    return torch.empty(max(n.value, 16), device=dev, dtype=torch.uint8)
-
-
-def retention_fwd(Q, K, V, log_G, c: int, scale: float, carry=None, want_final: bool = False):
-    """The chunked forward in one library call.  Returns (O, saved workspace, final (state, gram) fp32 carries or
-    (None, None))."""
-    b, t, hq, d = Q.shape
-    h = K.shape[2]
-    prob = _problem(Q, h, c, scale)
-    saved = _workspace(prob, 0, Q.device)
-    scratch = _workspace(prob, 1, Q.device)
-    O = torch.empty_like(Q)
-    Cs, Cg = carry if carry is not None else (None, None)
-    Fs = Fg = None
-    if want_final:
-        Fs = torch.empty(b, h, state_rows(d) * d, device=Q.device, dtype=torch.float32)
-        Fg = torch.empty(b, h, d * d, device=Q.device, dtype=torch.float32)
-    _call("pr_retention_fwd", ctypes.byref(prob), ptr(Q), ptr(K), ptr(V), ptr(log_G), ptr(Cs), ptr(Cg), ptr(O),
-          ptr(saved), ptr(scratch), ptr(Fs), ptr(Fg), c_int(_dev(Q)), stream_ptr(Q.device))
-    launch_log.count += 4  # five kernels behind one call
-    return O, saved, Fs, Fg
-
-
-def retention_bwd(Q, K, V, log_G, O, dO, saved, c: int, scale: float, had_carry: bool):
-    """The chunked backward in one library call.  Returns (dQ, dK, dV, dlog_G or None)."""
-    h = K.shape[2]
-    prob = _problem(Q, h, c, scale)
-    scratch = _workspace(prob, 2, Q.device)
-    dQ, dK, dV = torch.empty_like(Q), torch.empty_like(K), torch.empty_like(V)
-    dG = torch.empty_like(log_G) if log_G is not None else None
-    _call("pr_retention_bwd", ctypes.byref(prob), ptr(Q), ptr(K), ptr(V), ptr(log_G), ptr(O), ptr(dO),
-          c_int(1 if had_carry else 0), ptr(saved), ptr(scratch), ptr(dQ), ptr(dK), ptr(dV), ptr(dG), c_int(_dev(Q)),
-          stream_ptr(Q.device))
-    launch_log.count += 10 if log_G is not None else 9  # eleven (ten ungated) kernels behind one call
-    return dQ, dK, dV, dG
-
-
 def state_to_chunk_layout(state, sum_of_keys, want16: bool = False, want32: bool = False, want_gram: bool = False,
                           want_gram_halves: bool = False):
     """Exact-layout (state [b,h,D,d], sum_of_keys [b,h,D]) -> dict with the requested forms in the kernels'
@@ -413,92 +364,6 @@ def state_to_chunk_layout(state, sum_of_keys, want16: bool = False, want32: bool
           ptr(sum_of_keys), ptr(out["z16"]), ptr(out["z32"]), ptr(out["gram"]), ptr(out["ghi"]), ptr(out["glo"]),
           c_int(_dev(state)), stream_ptr(dev))
     return out
-
-
-_decode_ws = {}
-
-
-def _decode_partials(dev, b: int, h: int, hq: int, d: int):
-    """Partial-sum workspace of a split decode step, or (None, None) when the step runs unsplit.  One
-    workspace per (device, stream, shape): calls that may overlap on the GPU (other streams) get their own;
-    calls on one stream are ordered and share it."""
-    if lib().pr_decode_split(c_int(b), c_int(h), c_int(hq)) <= 1:
-        return None, None
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream, b, hq, d)
-    ws = _decode_ws.get(key)
-    if ws is None:
-        ns = lib().pr_decode_nsplit()
-        ws = (torch.empty(b, hq, ns, d, device=dev, dtype=torch.float32),
-              torch.empty(b, hq, ns, device=dev, dtype=torch.float32))
-        _decode_ws[key] = ws
-    return ws
-
-
-def _batch_strided(t: torch.Tensor):
-    """(tensor, batch stride in elements) with everything inside a batch entry dense.  A slice [:, :tk] of a
-    longer preallocated cache qualifies as it is; anything else is copied."""
-    if t is None:
-        return None, 0
-    if t.dim() >= 2:
-        inner = 1
-        dense = True
-        for size, stride in zip(reversed(t.shape[1:]), reversed(t.stride()[1:])):
-            if size != 1 and stride != inner:
-                dense = False
-                break
-            inner *= size
-        if dense and (t.shape[0] == 1 or t.stride(0) >= inner):
-            return t, (t.stride(0) if t.shape[0] > 1 else inner)
-    t = t.contiguous()
-    return t, (t.stride(0) if t.dim() >= 1 else 0)
-
-
-def decode_step(Q, K, V, log_g, state, sum_of_keys, scale: float, h: int):
-    """One decode step (tq = 1) in a single library call and a single kernel.  Returns O [b,1,hq,d].  Q, K, V
-    and log_g may be slices along the token axis of longer tensors (a preallocated cache): they are read in place.
-    The partial-sum workspace a small problem needs is kept per (device, stream, shape), see _decode_partials."""
-    b, _, hq, d = Q.shape
-    tk = K.shape[1] if K is not None else 0
-    Q, q_bs = _batch_strided(Q)
-    if q_bs % 8 != 0 or Q.data_ptr() % 16:
-        Q = Q.contiguous()
-        q_bs = hq * d
-    K, k_bs = _batch_strided(K)
-    V, v_bs = _batch_strided(V)
-    if K is not None and (k_bs != v_bs or k_bs % 8 != 0 or K.data_ptr() % 16 or V.data_ptr() % 16):
-        K, V = K.contiguous(), V.contiguous()
-        k_bs = v_bs = tk * h * d
-    log_g, g_bs = _batch_strided(log_g)
-    O = torch.empty(b, 1, hq, d, device=Q.device, dtype=Q.dtype)
-    part_y, part_l = _decode_partials(Q.device, b, h, hq, d)
-    _call("pr_decode_step_strided", c_int(dtype_code(Q.dtype)), c_int(b), c_int(tk), c_int(h), c_int(hq), c_int(d),
-          ptr(Q), c_longlong(q_bs), ptr(K), ptr(V), c_longlong(k_bs), ptr(log_g), c_longlong(g_bs), ptr(state),
-          ptr(sum_of_keys), c_float(scale), ptr(None), ptr(part_y), ptr(part_l), ptr(O), c_int(_dev(Q)),
-          stream_ptr(Q.device))
-    return O
-
-
-def decode_recurrent(q, k, v, log_g, state, sum_of_keys, new_state, new_sum_of_keys, scale: float):
-    """Pure-recurrent step: advances (state, sum_of_keys) by the token (k, v, log_g) into (new_state,
-    new_sum_of_keys) - which may be the same tensors when hq / h <= 4 - and reads it with q.  Returns O [b,1,hq,d]."""
-    b, _, hq, d = q.shape
-    h = k.shape[2]
-    q, q_bs = _batch_strided(q)
-    k, k_bs = _batch_strided(k)
-    v, v_bs = _batch_strided(v)
-    if k_bs != v_bs:
-        k, v = k.contiguous(), v.contiguous()
-        k_bs = v_bs = h * d
-    if q_bs % 8 != 0 or q.data_ptr() % 16:
-        q, q_bs = q.contiguous(), hq * d
-    log_g, g_bs = _batch_strided(log_g)
-    O = torch.empty(b, 1, hq, d, device=q.device, dtype=q.dtype)
-    part_y, part_l = _decode_partials(q.device, b, h, hq, d)
-    _call("pr_decode_recurrent", c_int(dtype_code(q.dtype)), c_int(b), c_int(h), c_int(hq), c_int(d), ptr(q),
-          c_longlong(q_bs), ptr(k), ptr(v), c_longlong(k_bs), ptr(log_g), c_longlong(g_bs), ptr(state),
-          ptr(sum_of_keys), ptr(new_state), ptr(new_sum_of_keys), c_float(scale), ptr(part_y), ptr(part_l), ptr(O),
-          c_int(_dev(q)), stream_ptr(q.device))
-    return O
 
 
 def caller_prep_fwd(qkvg, cos, sin, h: int, hq: int, d: int, gated: bool, gate_bias: float, half_split: bool):

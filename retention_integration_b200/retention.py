@@ -2,7 +2,8 @@
 (retention/power_retention_maker.py:72-73 and :287-288), running on libpr_b200.so.
 
 The host side only validates arguments, pads, allocates and sequences kernel launches;
-every arithmetic step of the path is a kernel of the C-ABI library.  There is no
+every arithmetic step of the path is a kernel of the C-ABI library.  That host side is native
+(csrc/binding.cpp); what is left here drives the same kernels one by one from Python.  There is no
 PyTorch or CPU fallback: inputs must be CUDA tensors of dtype bfloat16 or float16.
 """
 from __future__ import annotations
@@ -11,14 +12,13 @@ import math
 
 import torch
 
-from . import layout, ops
+from . import _lib, layout, ops
 from ._lib import PRError
 
 _SUPPORTED_D = (64,)
 
-# True: forward and backward of the chunked branch are one library call each (the launch sequence runs in native
-# code); False: the same kernels are launched one by one from Python (per-kernel timing, the sequence-parallel
-# variant, debugging).  Both orders of launches are identical.
+# True: forward and backward are one native call each; False: the same kernels are launched one by one from
+# Python, on padded sequences (per-kernel timing, debugging).  The results are identical.
 NATIVE_SEQUENCER = True
 
 
@@ -41,7 +41,7 @@ def _check_inputs(Q, K, V, log_G, deg, state_free=False):
 
 
 class _ChunkedRetention(torch.autograd.Function):
-    """Chunked forward/backward.  Sequence length is a multiple of the chunk size here.
+    """Chunked forward/backward, launched from Python.  Sequence length is a multiple of the chunk size here.
 
     `carry` is None or (Cs [b,h,DR*d], Cg [b,h,d*d]) fp32: the state and Gram matrix entering the first
     chunk, in the kernels' chunk-state layout (initial_state).  With `want_final` the state and Gram matrix
@@ -55,13 +55,6 @@ class _ChunkedRetention(torch.autograd.Function):
         Cs, Cg = carry if carry is not None else (None, None)
         first = carry is None
         ctx.c, ctx.scale, ctx.first = c, scale, first
-        ctx.native = NATIVE_SEQUENCER
-        if ctx.native:
-            O, saved, Fs, Fg = ops.retention_fwd(Q, K, V, log_G, c, scale, carry, want_final)
-            ctx.save_for_backward(Q, K, V, log_G, O, saved)
-            if want_final:
-                ctx.mark_non_differentiable(Fs, Fg)
-            return O, Fs, Fg
         a, A, KT = ops.gate_prep(K, log_G, c, query_side=False)
         S, gram = ops.chunk_state(KT, None, V, c, h, key_weights=True, want_gram=True)
         del KT
@@ -75,10 +68,6 @@ class _ChunkedRetention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dO, _dFs=None, _dFg=None):
         c, scale = ctx.c, ctx.scale
-        if ctx.native:
-            Q, K, V, log_G, O, saved = ctx.saved_tensors
-            dQ, dK, dV, dlog_G = ops.retention_bwd(Q, K, V, log_G, O, dO.contiguous(), saved, c, scale, not ctx.first)
-            return dQ, dK, dV, dlog_G, None, None, None, None
         Q, K, V, log_G, a, A, O, l, Z, zhi, zlo, zfull = ctx.saved_tensors
         b, t, hq, d = Q.shape
         h = K.shape[2]
@@ -194,10 +183,18 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     continues from it, and with return_final_state the call returns (out, (state, sum_of_keys)) after the
     last token.  Gradients flow to Q, K, V and log_G; the states are treated as constants.
 
-    Head dims 16, 32 and 48 run on the d = 64 kernels with zero-padded features (exact: the padded
-    features contribute nothing to any dot product); they take no states.
+    Head dims 16, 32 and 48 run on the d = 64 kernels as zero-padded features (exact: the padded
+    features contribute nothing to any dot product; 16 and 32 are widened on the way into shared memory);
+    they take no states.
     """
     assert deg % 2 == 0, f"deg must be even: {deg=}"
+    if NATIVE_SEQUENCER and not ops.launch_log.timing:
+        state, sok = initial_state if initial_state is not None else (None, None)
+        out = _lib.host().power_retention(Q, K, V, log_G, state, sok, return_final_state, deg, scale or 0.0,
+                                          chunk_size or 0, -1 if switch_over_seq_len is None else switch_over_seq_len,
+                                          AUTO_CHUNK)
+        if out is not None:
+            return out
     d_orig = Q.shape[-1]
     if d_orig in (16, 32, 48):
         if initial_state is not None or return_final_state:
@@ -272,69 +269,4 @@ def power_retention_inference(Q, K, V, log_G=None, initial_state=None, sum_of_ke
     States use the exact expansion layout, D = d*(d+1)/2 (2080 at d = 64); the reference's
     padded layout (2560) converts with layout.to_reference_layout / from_reference_layout.
     """
-    has_cache = K is not None and V is not None
-    assert has_cache or initial_state is not None, "initial_state or cache must be provided for inference"
-    assert (initial_state is None) == (sum_of_keys is None), "initial_state and sum_of_keys come together"
-    if deg != 2:
-        raise PRError(f"deg={deg}: the state kernels implement deg=2")
-    if not Q.is_cuda:
-        raise PRError("tensors must be CUDA tensors: this package has no CPU path")
-    b, tq, hq, d = Q.shape
-    if d not in _SUPPORTED_D:
-        raise PRError(f"head dim {d} unsupported by this build (supported: {_SUPPORTED_D})")
-    if has_cache:
-        assert Q.dtype == K.dtype == V.dtype, "dtypes of inputs must match"
-        assert K.shape[1] == V.shape[1], "key and value must have the same seq_len"
-        tk, h = K.shape[1], K.shape[2]
-    else:
-        tk, h = 0, initial_state.shape[1]
-    assert hq % h == 0
-    if initial_state is not None:
-        D = layout.exact_dim(d)
-        assert initial_state.shape == (b, h, D, d), f"state must be [b,h,{D},{d}] (exact layout)"
-        assert sum_of_keys.shape == (b, h, D) and sum_of_keys.dtype == torch.float32
-    scale = 1.0 / math.sqrt(d) if scale is None else scale
-    gated = has_cache and log_G is not None
-    if gated:
-        assert log_G.shape == K.shape[:3]
-        log_G = log_G.to(torch.float32)
-    switch = switch_over_seq_len is not None and tk >= switch_over_seq_len
-    decode = tq == 1 and initial_state is not None
-    if not decode or switch:
-        # every path but the plain decode step wants dense tensors; the decode step reads a query and a cache
-        # that are slices of longer preallocated tensors in place
-        Q = Q.contiguous()
-        if has_cache:
-            K, V = K.contiguous(), V.contiguous()
-        if gated:
-            log_G = log_G.contiguous()
-
-    # ---- read-out
-    a = None
-    if decode:
-        # the decode step proper: one library call (gate cumsum, state read, cache attention)
-        Y = ops.decode_step(Q, K if tk > 0 else None, V if tk > 0 else None, log_G if gated else None,
-                            initial_state.contiguous(), sum_of_keys.contiguous(), scale, h)
-    else:
-        if gated:
-            a, _, _ = ops.gate_prep(K, log_G, tk, query_side=False, want_xt=False)
-        if initial_state is None:
-            Y, _ = ops.chunk_out(Q, K, V, a, None, None, None, 1, tq, tk, 1, scale, want_l=False)
-        else:
-            # several query tokens against a state: the tensor-core path, state converted to its layout
-            conv = ops.state_to_chunk_layout(initial_state.contiguous(), sum_of_keys.contiguous(), want16=True,
-                                             want_gram_halves=True)
-            Z, zhi, zlo = conv["z16"].unsqueeze(1), conv["ghi"].unsqueeze(1), conv["glo"].unsqueeze(1)
-            if tk > 0:
-                Y, _ = ops.chunk_out(Q, K, V, a, Z, zhi, zlo, 1, tq, tk, 0, scale, q_gate_last=True, want_l=False)
-            else:
-                Y, _ = ops.chunk_out(Q, None, None, None, Z, zhi, zlo, 1, tq, tq, 0, scale, want_l=False)
-
-    # ---- optionally compress the cache into the state
-    if switch:
-        a2, _, KT = ops.gate_prep(K, log_G if gated else None, tk, query_side=False)
-        a_last = a2[:, -1, :].contiguous() if a2 is not None else None
-        S, gram = ops.chunk_state(KT, None, V, tk, h, key_weights=True, want_gram=True)
-        new_state, new_sok = ops.state_merge(initial_state, sum_of_keys, S, gram, a_last)
-        return Y, new_state, new_sok
-    return Y, initial_state, sum_of_keys
+    return _lib.host().inference(Q, K, V, log_G, initial_state, sum_of_keys, deg, scale, switch_over_seq_len)
