@@ -12,8 +12,13 @@
 // Because both terms share one fp32 accumulator in tensor memory, the reference's
 // rowmax / sqrt(D) range management is not needed.
 //
-// Warp roles: warps 0-3 own one query row per thread (scores -> weights P, expansion
-// phi(q~), epilogue), warp 4 issues TMA loads, warp 5 issues tcgen05.mma.
+// Warp roles: two groups of four warps own the 128 query rows, one row per thread in each group, and take the steps
+// in turn (scores -> weights P, expansion phi(q~)); there is no running maximum, so a row's two partial sums are
+// simply added at the end, and each group writes half of the output columns.  Warp 8 issues TMA loads, warp 9
+// tcgen05.mma.  What bounds the kernel is the latency of a step's chain - barrier, tensor-memory load, arithmetic,
+// store, barrier: 1950 clocks traced for a 64-key step whose products take 320 and whose arithmetic takes 330 of a
+// scheduler's issue slots.  With one group per CTA the two CTAs of an SM had two chains to overlap, now they have
+// four (and three score buffers, so that a group finds its next scores ready): 637 -> NEW us at b16 t2048 h32.
 //   S = Q K_J^T        : A, B K-major in shared memory (TMA, 128-byte swizzle)
 //   acc += P V_J       : A = P written to tensor memory by the row threads, B = V_J MN-major
 //   acc += phi(q~) Z   : A = expansion written to tensor memory 64 rows at a time,
@@ -29,14 +34,19 @@ namespace co {
 constexpr int HD = 64;
 constexpr int NS = 2;                 // expanded-operand ring in tensor memory: 2 stages of 128 entries (64 columns)
 constexpr int NR = 4;                 // shared-memory ring: stages of 16 KB (a key and a value tile, or two state blocks)
-constexpr int THREADS = 192;
+constexpr int NG = 2;                  // row groups
+constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
+constexpr int THREADS = 32 * (W_MMA + 1);
+constexpr int NB = 3;                  // score buffers in tensor memory
 constexpr int TILE_BYTES = 128 * 128;  // 128 rows x 64 16-bit features
 constexpr int TW = 64;                 // keys per attention step
 constexpr int KV_BYTES = TW * 128;     // one key or value tile
 constexpr int Z_BYTES = 64 * 128;      // 64 expanded rows x 64 features
 constexpr int R_BYTES = 2 * KV_BYTES;  // one ring stage
 constexpr uint32_t TMEM_COLS = 256;
-constexpr uint32_t COL_ACC = 0, COL_U = 64, COL_S = 128, COL_A = 128;  // S: 2 buffers x 64 columns, P aliased
+// the weights P overwrite their scores; the state read-out reuses the score buffers (u in the third)
+constexpr uint32_t COL_ACC = 0, COL_U = 64, COL_A = 128;
+__device__ __forceinline__ constexpr uint32_t col_s(int b) { return b == 2 ? 64u : 128u + 64u * b; }
 }  // namespace co
 
 struct ChunkOutParams {
@@ -108,14 +118,14 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
                  const __grid_constant__ CUtensorMap tm_glo) {
   using namespace co;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t q_full, r_full[NR], r_empty[NR], s_full[2], p_full[2], attn_done, g_full, acc_done;
+  __shared__ uint64_t q_full, r_full[NR], r_empty[NR], s_full[NB], p_full[NB], attn_done, g_full, acc_done;
   __shared__ uint64_t a_full[NS], a_empty[NS];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  __shared__ __align__(16) float sm_ak[2][TW];
-  __shared__ __align__(16) float sm_fk[2][TW];  // e^{r - a_j}, r = gate sum at the step's last key
-  __shared__ float sm_r[2];
-  __shared__ int sm_wide[2][2];                 // a loader warp saw r - a_j > 80 (overflow guard)
+  // Per warp and step parity: gate sums a_j of the step's keys and e^{r - a_j}, r = gate sum at the step's last key.
+  // Every warp makes its own copy, two keys per lane, so that no barrier ties the warps of a step together.
+  __shared__ __align__(16) float sm_ak[4 * NG][2][TW], sm_fk[4 * NG][2][TW];
+  __shared__ float sm_l[NG][128];               // row sums of the two groups
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -142,7 +152,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&q_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < NB; ++s) {
       mbar_init(&s_full[s], 1);
       mbar_init(&p_full[s], 4);
     }
@@ -168,7 +178,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
 
-  if (warp == 4) {
+  if (warp == W_TMA) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one()) {
       bool ok = true;
@@ -197,7 +207,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         }
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == W_MMA) {
     // -------------------------------------------------------------- MMA issuer
     if (elect_one()) {
       bool ok = mbar_wait(&q_full, 0, &abort_flag);
@@ -205,32 +215,32 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       const uint32_t idesc_v = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
       const uint32_t idesc_g = umma_idesc(128, HD, Pack2<T>::is_bf16, false, false);
       const uint32_t q_addr = smem_u32(smQ);
-      // scores of tile J+1 are issued before the P V product of tile J, so the row threads
-      // always have the next tile waiting (two score buffers, two key/value stages)
+      // scores run two steps ahead of the P V products, so that each row group finds its next tile waiting
       auto issue_scores = [&](int J) -> bool {
-        const int s = J & 1;
+        const int s = J % NB;
         if (!mbar_wait(&r_full[J % NR], (J / NR) & 1, &abort_flag)) return false;
         tc_fence_after();
         const uint32_t k_addr = smem_u32(smR + (J % NR) * R_BYTES);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + COL_S + s * TW, umma_desc_sw128(q_addr + ks * 32, 16, 1024),
+          umma_ss(tmem + col_s(s), umma_desc_sw128(q_addr + ks * 32, 16, 1024),
                   umma_desc_sw128(k_addr + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
         umma_commit(&s_full[s]);
         return true;
       };
       if (ok && nJ > 0) ok = issue_scores(0);
+      if (ok && nJ > 1) ok = issue_scores(1);
       for (int J = 0; J < nJ && ok; ++J) {
-        const int s = J & 1;
-        if (J + 1 < nJ) ok = issue_scores(J + 1);
+        const int s = J % NB;
+        if (J + 2 < nJ) ok = issue_scores(J + 2);  // into the buffer whose P V product was issued last
         if (!ok) break;
-        ok = mbar_wait(&p_full[s], (J >> 1) & 1, &abort_flag);
+        ok = mbar_wait(&p_full[s], (J / NB) & 1, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint32_t v_addr = smem_u32(smR + (J % NR) * R_BYTES + KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < TW / 16; ++ks)
-          umma_ts(tmem + COL_ACC, tmem + COL_S + s * TW + ks * 8, umma_desc_sw128(v_addr + ks * 2048, 8192, 1024),
+          umma_ts(tmem + COL_ACC, tmem + col_s(s) + ks * 8, umma_desc_sw128(v_addr + ks * 2048, 8192, 1024),
                   idesc_v, (J > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&r_empty[J % NR]);
         if (J == nJ - 1) umma_commit(&attn_done);
@@ -273,10 +283,12 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
     }
   } else {
     // --------------------------------------------------------- row-owning warps
-    const int row = row0 + tid;                 // query index inside the chunk
+    const int grp = warp >> 2, r = tid & 127;   // row group, row inside the tile
+    const int row = row0 + r;                   // query index inside the chunk
     const bool row_valid = row < cq;
     const int qpos = row + q_off;               // key position of this query
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    const int wrow = (warp & 3) * 32;
+    const uint32_t lane_addr = (uint32_t)wrow << 16;
     const bool gated = p.a != nullptr;
     const float* a_chunk = gated ? p.a + ((size_t)batch * p.tk + (size_t)chunk * p.ck) * p.h + kvhead
                                  : nullptr;
@@ -284,64 +296,64 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
     const float s2 = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
     float l_acc = 0.f;
     bool ok = true;
-    // gate sums of the next step's keys, loaded one step ahead by the first TW threads
-    float av_n = 0.f, r_n = 0.f;
+    // gate sums of this warp's next step, loaded one step ahead
+    float av0 = 0.f, av1 = 0.f, r_n = 0.f;
     auto load_gates = [&](int J) {
-      if (tid < TW && gated) {
-        const int kp = J * TW + tid;
-        av_n = kp < ck ? a_chunk[(size_t)kp * p.h] : 0.f;
+      if (gated) {
+        const int kp = J * TW + lane;
         r_n = a_chunk[(size_t)min(J * TW + TW - 1, ck - 1) * p.h];
+        av0 = kp < ck ? a_chunk[(size_t)kp * p.h] : 0.f;
+        av1 = kp + 32 < ck ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
       }
     };
-    if (nJ > 0) load_gates(0);
+    if (grp < nJ) load_gates(grp);
 
-    for (int J = 0; J < nJ; ++J) {
+    for (int J = grp; J < nJ; J += NG) {
       const int kp0 = J * TW;
-      const int sb = J & 1;
-      if (tid < TW) {
-        sm_ak[sb][tid] = av_n;
-        sm_fk[sb][tid] = __expf(r_n - av_n);
-        const bool wide = __any_sync(0xffffffffu, (r_n - av_n) > 80.f);
-        if (lane == 0) sm_wide[sb][warp] = wide;
-        if (tid == 0) sm_r[sb] = r_n;
-      }
-      named_bar_sync(1, 128);
-      if (J + 1 < nJ) load_gates(J + 1);  // in flight while this step is computed
-      ok = mbar_wait(&s_full[sb], (J >> 1) & 1, &abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t col_s = COL_S + sb * TW;
+      const int sb = J % NB, sp = (J / NG) & 1;
+      float* ak = sm_ak[warp][sp];
+      float* fk = sm_fk[warp][sp];
+      const float rs = r_n;
+      ak[lane] = av0;
+      ak[lane + 32] = av1;
+      fk[lane] = __expf(rs - av0);
+      fk[lane + 32] = __expf(rs - av1);
       // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
       // row and per key instead of one per pair (both exponents <= 0 below the diagonal for gates
       // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps wholly below the
       // diagonal need no mask; a warp whose rows all precede the step's keys writes zeros
       // without reading the scores.
-      const int wq0 = row0 + (warp << 5) + q_off;  // key position of this warp's first query
+      const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - fminf(av0, av1), a_i - rs) > 80.f);
+      __syncwarp();  // ak, fk
+      const float c_i = sep ? s2 * __expf(a_i - rs) : s2;
+      if (J + NG < nJ) load_gates(J + NG);  // in flight while this step is computed
+      ok = mbar_wait(&s_full[sb], (J / NB) & 1, &abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t cs = tmem + lane_addr + col_s(sb);
+      const int wq0 = row0 + wrow + q_off;  // key position of this warp's first query
       if (kp0 > min(wq0 + 31, ck - 1)) {
         uint32_t z[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) z[j] = 0u;
-        tmem_st16(tmem + lane_addr + col_s, z);
-        tmem_st16(tmem + lane_addr + col_s + 16, z);
+        tmem_st16(cs, z);
+        tmem_st16(cs + 16, z);
       } else {
-        const float r = sm_r[sb];
         const bool mask = (kp0 + TW - 1 > wq0) || (kp0 + TW - 1 >= ck);
-        const bool sep = !(sm_wide[sb][0] | sm_wide[sb][1]) && !__any_sync(0xffffffffu, (a_i - r) > 80.f);
-        const float c_i = sep ? s2 * __expf(a_i - r) : s2;
         const int lim = min(qpos, ck - 1) - kp0;  // last column this row keeps
 #pragma unroll 1
         for (int q4 = 0; q4 < TW / 32; ++q4) {
           uint32_t sv[32], pk[16];
-          tmem_ld32(tmem + lane_addr + col_s + q4 * 32, sv);
+          tmem_ld32(cs + q4 * 32, sv);
           tmem_wait_ld();
           const int lm = lim - q4 * 32;
           if (sep) {
-            if (mask) out_half<T, DEG, true, true>(sv, sm_fk[sb] + q4 * 32, c_i, a_i, lm, pk, l_acc);
-            else out_half<T, DEG, true, false>(sv, sm_fk[sb] + q4 * 32, c_i, a_i, lm, pk, l_acc);
+            if (mask) out_half<T, DEG, true, true>(sv, fk + q4 * 32, c_i, a_i, lm, pk, l_acc);
+            else out_half<T, DEG, true, false>(sv, fk + q4 * 32, c_i, a_i, lm, pk, l_acc);
           } else {
-            out_half<T, DEG, false, true>(sv, sm_ak[sb] + q4 * 32, c_i, a_i, lm, pk, l_acc);
+            out_half<T, DEG, false, true>(sv, ak + q4 * 32, c_i, a_i, lm, pk, l_acc);
           }
-          tmem_st16(tmem + lane_addr + col_s + q4 * 16, pk);
+          tmem_st16(cs + q4 * 16, pk);
         }
       }
       tmem_wait_st();
@@ -351,9 +363,9 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
     }
 
     // gated, scaled query row as 32 packed pairs
-    uint32_t q2[32];
-    if (ok && has_state) {
-      ok = mbar_wait(&q_full, 0, &abort_flag);
+    if (has_state) {  // whether a wait has run out or not: the barriers below want every thread
+      uint32_t q2[32];
+      if (ok) ok = mbar_wait(&q_full, 0, &abort_flag);
       float f = p.scale;
       if (gated) {
         const float a_g = p.q_gate_last ? a_chunk[(size_t)(ck - 1) * p.h] : a_i;
@@ -361,7 +373,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(tid, j));
+        const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(r, j));
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -372,7 +384,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       // the P columns alias the expansion ring: wait until the last P V product has read them
       if (ok && nJ > 0) ok = mbar_wait(&attn_done, 0, &abort_flag);
       tc_fence_after();
-      if (ok) {
+      if (ok && grp == 0) {
         // item 0: q~ itself (A operand of u = q~ Zg)
         tmem_st32(tmem + lane_addr + COL_A, q2);
         tmem_wait_st();
@@ -380,24 +392,27 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         __syncwarp();
         if (lane == 0) mbar_arrive(&a_full[0]);
       }
-      // ring items 1..nblk/2: 128 expanded entries (64 packed products) each.  The gated row goes
-      // back to its own slot of the query tile so that the first factor can be fetched by a runtime
-      // index; the loop over first factors then has a body of 64 multiplies per stage.
-      if (ok) {
+      // The gated row goes back to its own slot of the query tile (both groups have read the raw one, and the score
+      // products that read it have completed) so that the first factor can be fetched by a runtime index; the loop
+      // over first factors then has a body of 64 multiplies per stage.
+      named_bar_sync(1, 128 * NG);
+      if (grp == 0) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-          *reinterpret_cast<uint4*>(smQ + swz128(tid, j)) = make_uint4(q2[4 * j], q2[4 * j + 1], q2[4 * j + 2], q2[4 * j + 3]);
+          *reinterpret_cast<uint4*>(smQ + swz128(r, j)) = make_uint4(q2[4 * j], q2[4 * j + 1], q2[4 * j + 2], q2[4 * j + 3]);
       }
-      int k = 1;
+      named_bar_sync(1, 128 * NG);
+      // ring items 1..nblk/2: 128 expanded entries (64 packed products) each.  A block of second factors has an even
+      // number of items, so group 1 takes the odd items (first factors 0-7, 16-23 ...) and group 0 the even ones.
+      const int s = grp;
+      int k = 2 - grp;
       static_for<0, HD / 16>([&](auto yc) {
         constexpr int Y = decltype(yc)::value;
         if (16 * Y >= p.d) return;
 #pragma unroll 1
-        for (int a0 = 0; a0 < 16 * (Y + 1); a0 += 8, ++k) {
-          uint32_t r0[32], r1[32];
-          expand_stage<T, Y>(smQ, tid, a0, q2, r0);
-          expand_stage<T, Y>(smQ, tid, a0 + 4, q2, r1);
-          const int s = k % NS;
+        for (int a0 = 8 * (1 - grp); a0 < 16 * (Y + 1); a0 += 16, k += NG) {
+          uint32_t x[32];
+          expand_stage<T, Y>(smQ, r, a0, q2, x);
           // the slot was last used by item k - 2: the Gram item (its own barrier) or a ring item, whose
           // completion the issuing thread reports on the ring stage's barrier
           if (ok && k == 2) ok = mbar_wait(&a_empty[0], 0, &abort_flag);
@@ -405,10 +420,11 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
             const int g2 = nJ + k - 3;
             ok = mbar_wait(&r_empty[g2 % NR], (g2 / NR) & 1, &abort_flag);
           }
+          tc_fence_after();
+          if (ok) tmem_st32(tmem + lane_addr + COL_A + s * 64, x);
+          expand_stage<T, Y>(smQ, r, a0 + 4, q2, x);
           if (ok) {
-            tc_fence_after();
-            tmem_st32(tmem + lane_addr + COL_A + s * 64, r0);
-            tmem_st32(tmem + lane_addr + COL_A + s * 64 + 32, r1);
+            tmem_st32(tmem + lane_addr + COL_A + s * 64 + 32, x);
             tmem_wait_st();
             tc_fence_before();
           }
@@ -420,34 +436,40 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
 
     if (ok) ok = mbar_wait(&acc_done, 0, &abort_flag);
     tc_fence_after();
-    if (ok) {
-      float l = l_acc;
-      if (has_state) {
-        // the state part of the row sum first, so that u and the accumulators are not live together
-        uint32_t u[64];
-        tmem_ld32(tmem + lane_addr + COL_U, u);
-        tmem_ld32(tmem + lane_addr + COL_U + 32, u + 32);
-        tmem_wait_ld();
-        float ls0 = 0.f, ls1 = 0.f;
+    // Each group finishes 32 of the row's 64 columns: half of <u, q~> for the row sum, half of the output.
+    const uint32_t half = 32 * grp;
+    if (ok && has_state) {
+      uint32_t u[32];
+      tmem_ld32(tmem + lane_addr + COL_U + half, u);
+      tmem_wait_ld();
+      float ls0 = 0.f, ls1 = 0.f;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float2 qv = Pack2<T>::to_f32(q2[j]);
-          ls0 = fmaf(__uint_as_float(u[2 * j]), qv.x, ls0);
-          ls1 = fmaf(__uint_as_float(u[2 * j + 1]), qv.y, ls1);
+      for (int j = 0; j < 4; ++j) {
+        const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(r, 4 * grp + j));  // the gated row
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 qv = Pack2<T>::to_f32(w[k]);
+          ls0 = fmaf(__uint_as_float(u[8 * j + 2 * k]), qv.x, ls0);
+          ls1 = fmaf(__uint_as_float(u[8 * j + 2 * k + 1]), qv.y, ls1);
         }
-        l += ls0 + ls1;
       }
-      uint32_t acc[64];
-      tmem_ld32(tmem + lane_addr + COL_ACC, acc);
-      tmem_ld32(tmem + lane_addr + COL_ACC + 32, acc + 32);
+      l_acc += ls0 + ls1;
+    }
+    sm_l[grp][r] = l_acc;
+    named_bar_sync(1, 128 * NG);
+    if (ok) {
+      const float l = sm_l[0][r] + sm_l[1][r];
+      uint32_t acc[32];
+      tmem_ld32(tmem + lane_addr + COL_ACC + half, acc);
       tmem_wait_ld();
       if (row_valid) {
         const size_t tok = (size_t)batch * p.tq + (size_t)chunk * p.cq + row;
         const float inv = p.normalize ? safe_recip(l) : 1.f;
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.O) + (tok * p.hq + qhead) * p.d);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.O) + (tok * p.hq + qhead) * p.d + half);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (8 * j >= p.d) break;
+        for (int j = 0; j < 4; ++j) {
+          if ((int)half + 8 * j >= p.d) break;
           uint4 v;
           v.x = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 0]), inv * __uint_as_float(acc[8 * j + 1]));
           v.y = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 2]), inv * __uint_as_float(acc[8 * j + 3]));
@@ -455,7 +477,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
           v.w = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 6]), inv * __uint_as_float(acc[8 * j + 7]));
           dst[j] = v;
         }
-        if (p.l_out != nullptr) p.l_out[tok * p.hq + qhead] = l;
+        if (p.l_out != nullptr && grp == 0) p.l_out[tok * p.hq + qhead] = l;
       }
     }
   }
