@@ -377,8 +377,10 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
 #pragma unroll 1
         for (int a0 = 0; a0 < 16 * (Y + 1); a0 += 8, ++k) {
           uint32_t r0[32], r1[32];
-          expand_stage<T, Y>(smK, tid, a0, k2, r0);
-          expand_stage<T, Y>(smK, tid, a0 + 4, k2, r1);
+          uint32_t x2[8];
+          expand_second(smK, tid, Y, x2);
+          expand_stage<T>(smK, tid, a0, x2, r0);
+          expand_stage<T>(smK, tid, a0 + 4, x2, r1);
           const int s = k % NS;
           if (ok && k >= NS) {
             // the slot was last used by item k - NS, whose completion is reported on its ring stage's barrier

@@ -12,13 +12,20 @@
 // Because both terms share one fp32 accumulator in tensor memory, the reference's
 // rowmax / sqrt(D) range management is not needed.
 //
-// Warp roles: two groups of four warps own the 128 query rows, one row per thread in each group, and take the steps
-// in turn (scores -> weights P, expansion phi(q~)); there is no running maximum, so a row's two partial sums are
-// simply added at the end, and each group writes half of the output columns.  Warp 8 issues TMA loads, warp 9
-// tcgen05.mma.  What bounds the kernel is the latency of a step's chain - barrier, tensor-memory load, arithmetic,
-// store, barrier: 1950 clocks traced for a 64-key step whose products take 320 and whose arithmetic takes 330 of a
-// scheduler's issue slots.  With one group per CTA the two CTAs of an SM had two chains to overlap, now they have
-// four (and three score buffers, so that a group finds its next scores ready): 637 -> NEW us at b16 t2048 h32.
+// Warp roles: two groups of four warps own the query rows, one row per thread in each group, and take the steps in
+// turn (scores -> weights P, expansion phi(q~)); there is no running maximum, so a row's partial sums are simply
+// added at the end.  One more warp issues TMA loads and one tcgen05.mma.
+//
+// What bounded the earlier form (one row group per CTA, 637 us at b16 t2048 h32 without states, 317 us at
+// b1 t65536 h8 with chunks of 1024 and states): the latency of a step's chain, about 2000 clocks traced for a 64-key
+// step whose products take 320 - two groups and three buffers overlap four such chains per SM (494, 287 us) -
+// and then, for a third of the time, 10 thousand clocks per CTA of set-up, first loads, cold instructions and
+// write-out.  So the kernel is persistent: two CTAs per SM take over tile after tile (ClcRing), the loads and the
+// first scores of a tile overlap the write-out of the one before, and ring stages, buffers and groups go on
+// rotating across tiles; and the issuing thread keeps running positions and prepared descriptors, since every
+// instruction it executes between two batches leaves the tensor pipe idle (with divisions and a second commit per
+// operand: 459, 301 us).  Now 451 and 265 us.  Slower: three groups per CTA (520 us); 256 rows per CTA at one CTA per SM
+// (439 us, but 360 with states, where every gap of the one or two issuing threads is exposed).
 //   S = Q K_J^T        : A, B K-major in shared memory (TMA, 128-byte swizzle)
 //   acc += P V_J       : A = P written to tensor memory by the row threads, B = V_J MN-major
 //   acc += phi(q~) Z   : A = expansion written to tensor memory 64 rows at a time,
@@ -32,21 +39,22 @@ namespace pr {
 
 namespace co {
 constexpr int HD = 64;
-constexpr int NS = 2;                 // expanded-operand ring in tensor memory: 2 stages of 128 entries (64 columns)
-constexpr int NR = 4;                 // shared-memory ring: stages of 16 KB (a key and a value tile, or two state blocks)
 constexpr int NG = 2;                  // row groups
+constexpr int NB = 3;                  // buffers of 64 columns in tensor memory
+constexpr int NR = 4;                  // ring stages of 16 KB (key and value tile, Gram operand, two state blocks)
 constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
 constexpr int THREADS = 32 * (W_MMA + 1);
-constexpr int NB = 3;                  // score buffers in tensor memory
+constexpr uint32_t TMEM_COLS = 256;    // two CTAs per SM
+constexpr size_t SMEM = 1024 + 2 * 128 * 128 + NR * 16384;
 constexpr int TILE_BYTES = 128 * 128;  // 128 rows x 64 16-bit features
 constexpr int TW = 64;                 // keys per attention step
 constexpr int KV_BYTES = TW * 128;     // one key or value tile
 constexpr int Z_BYTES = 64 * 128;      // 64 expanded rows x 64 features
 constexpr int R_BYTES = 2 * KV_BYTES;  // one ring stage
-constexpr uint32_t TMEM_COLS = 256;
-// the weights P overwrite their scores; the state read-out reuses the score buffers (u in the third)
-constexpr uint32_t COL_ACC = 0, COL_U = 64, COL_A = 128;
-__device__ __forceinline__ constexpr uint32_t col_s(int b) { return b == 2 ? 64u : 128u + 64u * b; }
+// Tensor memory: the accumulator, then the buffers.  A buffer holds scores, overwritten by their weights P; in the
+// state read-out 128 expanded entries, and for a while u = q~ Zg.  Operand number u of a CTA goes to buffer u % NB and
+// is written by group u % NG.
+__device__ __forceinline__ constexpr uint32_t col_b(int b) { return 64u * (uint32_t)(1 + b); }
 }  // namespace co
 
 struct ChunkOutParams {
@@ -64,6 +72,7 @@ struct ChunkOutParams {
   float scale;          // s
   const float* a;       // [b, n*ck, h] cumulative log gates inside each chunk, or null
   void* O;              // [b, n*cq, hq, 64]
+  int o_aligned32;      // O starts on a 32-byte boundary
   float* l_out;         // [b, n*cq, hq] or null
   int* status;
 };
@@ -71,19 +80,46 @@ struct ChunkOutParams {
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 
-// One 32-column half of an attention step for one query row: p = s^2 S^2 g into `pk`, row sum into
+// What a CTA index stands for: a tile of 128 query rows of one (batch, chunk, query head).
+struct OutTile {
+  int chunk, qhead, kvhead, batch, row0;
+  int cq, ck, q_off;   // queries and keys of the chunk; key position of query 0
+  int nJ;              // attention steps: rows see keys up to their position
+  int nI;              // operands of the state read-out: q~ itself, then 128 expanded entries each
+  bool empty;          // past the end of a shorter last chunk
+  __device__ __forceinline__ OutTile(const ChunkOutParams& p, const dim3& cta) {
+    const int x = (int)cta.x;
+    // the longest tiles of a head first
+    const int tile_i = p.tiles_per_chunk - 1 - x % p.tiles_per_chunk;
+    chunk = x / p.tiles_per_chunk;
+    qhead = (int)cta.y;
+    batch = (int)cta.z;
+    kvhead = qhead / (p.hq / p.h);
+    cq = min(p.cq, p.tq - chunk * p.cq);
+    ck = min(p.ck, p.tk - chunk * p.ck);
+    q_off = ck - cq;
+    row0 = tile_i * 128;
+    empty = row0 >= cq;
+    nJ = (p.has_attn && !empty) ? min(ck - 1, row0 + 127 + q_off) / co::TW + 1 : 0;
+    nI = (chunk >= p.state_from_chunk && !empty) ? 1 + p.nblk / 2 : 0;
+  }
+};
+
+// One 16-column piece of an attention step for one query row: p = s^2 S^2 g into `pk`, row sum into
 // l_acc.  SEP: the gate factor is c_i * fk[col] (c_i carries s^2); otherwise s^2 e^{a_i - ak[col]} per
 // pair.  MASK: columns beyond `lim` (the row's own key position, relative to the step) are dropped.
 template <typename T, int DEG, bool SEP, bool MASK>
-__device__ __forceinline__ void out_half(const uint32_t (&sv)[32], const float* __restrict__ fk, float c_i, float a_i,
-                                         int lim, uint32_t (&pk)[16], float& l_acc) {
+__device__ __forceinline__ void out_piece(const uint32_t (&sv)[16], const float* __restrict__ fk, float c_i, float a_i,
+                                          int lim, uint32_t (&pk)[8], float2& acc) {
   // two columns per instruction: packed fp32 multiplies and adds
   const float4* f4 = reinterpret_cast<const float4*>(fk);
   const float2 c2 = make_float2(c_i, c_i);
-  float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int j = 0; j < 32; j += 4) {
+  for (int j = 0; j < 16; j += 4) {
     const float4 f = f4[j >> 2];
     const float2 fv[2] = {make_float2(f.x, f.y), make_float2(f.z, f.w)};
 #pragma unroll
@@ -107,6 +143,22 @@ __device__ __forceinline__ void out_half(const uint32_t (&sv)[32], const float* 
       pk[col >> 1] = Pack2<T>::from_f32(pv.x, pv.y);
     }
   }
+}
+
+// A whole step: the load of the next piece is in flight while one is computed.
+template <typename T, int DEG, bool SEP, bool MASK>
+__device__ __forceinline__ void out_step(uint32_t cs, const float* __restrict__ fk, float c_i, float a_i, int lim,
+                                         float& l_acc) {
+  uint32_t sv[2][16], pk[8];
+  float2 acc = make_float2(0.f, 0.f);
+  tmem_ld16(cs, sv[0]);
+#pragma unroll
+  for (int q = 0; q < co::TW / 16; ++q) {
+    tmem_wait_ld();
+    if (q + 1 < co::TW / 16) tmem_ld16(cs + (q + 1) * 16, sv[(q + 1) & 1]);
+    out_piece<T, DEG, SEP, MASK>(sv[q & 1], fk + q * 16, c_i, a_i, lim - q * 16, pk, acc);
+    tmem_st8(cs + q * 8, pk);
+  }
   l_acc += acc.x + acc.y;
 }
 
@@ -118,373 +170,430 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
                  const __grid_constant__ CUtensorMap tm_glo) {
   using namespace co;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t q_full, r_full[NR], r_empty[NR], s_full[NB], p_full[NB], attn_done, g_full, acc_done;
-  __shared__ uint64_t a_full[NS], a_empty[NS];
+  // q_*: the query tiles, two in flight.  r_*: the ring of operand tiles; operand number u takes stage u % NR, and
+  // r_empty says that the products that read both have completed.  s_full: scores in a buffer; op_full: a group has
+  // written an A operand (weights, q~, expansion) into it.  u_full: the Gram product; acc_full / acc_free:
+  // accumulator complete / read out; rows: the row warps meet.
+  __shared__ uint64_t q_full[2], q_free[2], r_full[NR], r_empty[NR], s_full[NB], op_full[NB];
+  __shared__ uint64_t u_full, acc_full, acc_free, rows;
+  __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  // Per warp and step parity: gate sums a_j of the step's keys and e^{r - a_j}, r = gate sum at the step's last key.
-  // Every warp makes its own copy, two keys per lane, so that no barrier ties the warps of a step together.
-  __shared__ __align__(16) float sm_ak[4 * NG][2][TW], sm_fk[4 * NG][2][TW];
-  __shared__ float sm_l[NG][128];               // row sums of the two groups
+  // Per warp and step parity: e^{r - a_j} of the step's keys, r = gate sum at its last key (or a_j itself where the
+  // exponentials do not separate).  Every warp makes its own copy, two keys per lane, so that no barrier ties the
+  // warps of a step together.
+  __shared__ __align__(16) float sm_fk[4 * NG][2][TW];
+  __shared__ float sm_l[2][NG][128];            // row sums of the groups
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
-  uint8_t* smQ = sm;
-  // One ring serves both phases: attention step J takes stage J % NR (key tile, then value tile);
-  // the state read-out goes on with the same stage counter, two 64-row state blocks per stage,
-  // so state blocks stream in while the last attention steps are still being computed.
-  uint8_t* smR = smQ + TILE_BYTES;        // NR x R_BYTES
-  uint8_t* smG = smR + NR * R_BYTES;      // hi, lo: 2 x Z_BYTES
+  uint8_t* smQ0 = sm;                         // 2 x TILE_BYTES
+  // One ring serves both phases: an attention step takes a stage (key tile, then value tile); the state read-out goes
+  // on with the same stage counter, two 64-row state blocks per stage, and so does the next tile, so the operands of
+  // what comes next stream in while the last steps are still being computed.
+  uint8_t* smR = smQ0 + 2 * TILE_BYTES;       // NR x R_BYTES
 
-  const int tile_i = blockIdx.x % p.tiles_per_chunk;
-  const int chunk = blockIdx.x / p.tiles_per_chunk;
-  const int qhead = blockIdx.y, batch = blockIdx.z;
-  const int kvhead = qhead / (p.hq / p.h);
-  const int cq = min(p.cq, p.tq - chunk * p.cq), ck = min(p.ck, p.tk - chunk * p.ck);  // of this chunk
-  const int q_off = ck - cq;
-  const int row0 = tile_i * 128;
-  if (row0 >= cq) return;  // a tile past the end of a shorter last chunk
-  const int last_key = min(ck - 1, row0 + 127 + q_off);
-  const int nJ = p.has_attn ? last_key / TW + 1 : 0;
-  const bool has_state = chunk >= p.state_from_chunk;
-
-  if (tid == 0) {
-    abort_flag = 0;
-    mbar_init(&q_full, 1);
-    for (int s = 0; s < NB; ++s) {
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 4);
+  if (warp == W_TMA) {
+    if (elect_one()) {
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+      abort_flag = 0;
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(&q_full[s], 1);
+        mbar_init(&q_free[s], 4 * NG);
+      }
+      for (int s = 0; s < NR; ++s) {
+        mbar_init(&r_full[s], 1);
+        mbar_init(&r_empty[s], 1);
+      }
+      for (int s = 0; s < NB; ++s) {
+        mbar_init(&s_full[s], 1);
+        mbar_init(&op_full[s], 4);
+      }
+      mbar_init(&u_full, 1);
+      mbar_init(&acc_full, 1);
+      mbar_init(&acc_free, 4 * NG);
+      mbar_init(&rows, 4 * NG);
+      clc_init(&clc, 4 * NG + 2);
+      fence_mbar_init();
     }
-    for (int s = 0; s < NR; ++s) {
-      mbar_init(&r_full[s], 1);
-      mbar_init(&r_empty[s], 1);
+    __syncwarp();
+    named_bar_arrive(1, THREADS);  // the first loads need not wait for the tensor memory
+  } else {
+    if (warp == 0) {
+      tmem_alloc(&tmem_base_s, TMEM_COLS);
+      tmem_relinquish();
     }
-    mbar_init(&attn_done, 1);
-    mbar_init(&g_full, 1);
-    mbar_init(&acc_done, 1);
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(&a_full[s], 4);
-      mbar_init(&a_empty[s], 1);
-    }
-    fence_mbar_init();
+    tc_fence_before();
+    named_bar_sync(1, THREADS);
+    tc_fence_after();
   }
-  if (warp == 0) {
-    tmem_alloc(&tmem_base_s, TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
 
   if (warp == W_TMA) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one()) {
       bool ok = true;
-      mbar_expect_tx(&q_full, TILE_BYTES);
-      tma_load_4d(smQ, &tm_q, &q_full, 0, qhead, chunk * p.cq + row0, batch);
-      const int ch = (batch * p.n_chunks + chunk) * p.h + kvhead;
-      if (has_state) {
-        mbar_expect_tx(&g_full, 2 * Z_BYTES);
-        tma_load_3d(smG, &tm_ghi, &g_full, 0, 0, ch);
-        tma_load_3d(smG + Z_BYTES, &tm_glo, &g_full, 0, 0, ch);
-      }
-      const int n_ring = nJ + (has_state ? p.nblk / 2 : 0);
-      for (int g = 0; g < n_ring && ok; ++g) {
-        const int s = g % NR, ph = (g / NR) & 1;
-        ok = mbar_wait(&r_empty[s], ph ^ 1, &abort_flag);
+      dim3 cta = blockIdx;
+      int g = 0;  // ring stages so far
+      for (int it = 0; ok; ++it) {
+        const OutTile w(p, cta);
+        if (ok && it >= 2) ok = mbar_wait(&q_free[it & 1], ((it >> 1) - 1) & 1, &abort_flag);
         if (!ok) break;
-        mbar_expect_tx(&r_full[s], R_BYTES);
-        uint8_t* dst = smR + s * R_BYTES;
-        if (g < nJ) {
-          tma_load_4d(dst, &tm_k, &r_full[s], 0, kvhead, chunk * p.ck + g * TW, batch);
-          tma_load_4d(dst + KV_BYTES, &tm_v, &r_full[s], 0, kvhead, chunk * p.ck + g * TW, batch);
+        if (!w.empty) {
+          mbar_expect_tx(&q_full[it & 1], TILE_BYTES);
+          tma_load_4d(smQ0 + (it & 1) * TILE_BYTES, &tm_q, &q_full[it & 1], 0, w.qhead, w.chunk * p.cq + w.row0, w.batch);
+          const int ch = (w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead;
+          for (int i = 0; i < w.nJ + w.nI && ok; ++i, ++g) {
+            if (i == 1) ok = clc_ask(&clc, it, &abort_flag);  // after the loads that the tile starts with
+            const int s = g % NR;
+            ok = ok && mbar_wait(&r_empty[s], ((g / NR) & 1) ^ 1, &abort_flag);
+            if (!ok) break;
+            mbar_expect_tx(&r_full[s], R_BYTES);
+            uint8_t* dst = smR + s * R_BYTES;
+            const int k = i - w.nJ;
+            if (k < 0) {
+              tma_load_4d(dst, &tm_k, &r_full[s], 0, w.kvhead, w.chunk * p.ck + i * TW, w.batch);
+              tma_load_4d(dst + KV_BYTES, &tm_v, &r_full[s], 0, w.kvhead, w.chunk * p.ck + i * TW, w.batch);
+            } else if (k == 0) {
+              tma_load_3d(dst, &tm_ghi, &r_full[s], 0, 0, ch);
+              tma_load_3d(dst + Z_BYTES, &tm_glo, &r_full[s], 0, 0, ch);
+            } else {
+              tma_load_2d(dst, &tm_z, &r_full[s], 0, (ch * p.nblk + 2 * (k - 1)) * 64);
+              tma_load_2d(dst + Z_BYTES, &tm_z, &r_full[s], 0, (ch * p.nblk + 2 * (k - 1) + 1) * 64);
+            }
+          }
+          if (ok && w.nJ + w.nI == 1) ok = clc_ask(&clc, it, &abort_flag);
         } else {
-          const int blk = 2 * (g - nJ);
-          tma_load_2d(dst, &tm_z, &r_full[s], 0, (ch * p.nblk + blk) * 64);
-          tma_load_2d(dst + Z_BYTES, &tm_z, &r_full[s], 0, (ch * p.nblk + blk + 1) * 64);
+          mbar_arrive(&q_full[it & 1]);  // nothing to load: the phase passes all the same
+          ok = clc_ask(&clc, it, &abort_flag);
         }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
     }
   } else if (warp == W_MMA) {
+    const uint32_t tmem = tmem_base_s;
     // -------------------------------------------------------------- MMA issuer
     if (elect_one()) {
-      bool ok = mbar_wait(&q_full, 0, &abort_flag);
       const uint32_t idesc_s = umma_idesc(128, TW, Pack2<T>::is_bf16, false, false);
       const uint32_t idesc_v = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
       const uint32_t idesc_g = umma_idesc(128, HD, Pack2<T>::is_bf16, false, false);
-      const uint32_t q_addr = smem_u32(smQ);
-      // scores run two steps ahead of the P V products, so that each row group finds its next tile waiting
-      auto issue_scores = [&](int J) -> bool {
-        const int s = J % NB;
-        if (!mbar_wait(&r_full[J % NR], (J / NR) & 1, &abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(smR + (J % NR) * R_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + col_s(s), umma_desc_sw128(q_addr + ks * 32, 16, 1024),
-                  umma_desc_sw128(k_addr + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(&s_full[s]);
-        return true;
-      };
-      if (ok && nJ > 0) ok = issue_scores(0);
-      if (ok && nJ > 1) ok = issue_scores(1);
-      for (int J = 0; J < nJ && ok; ++J) {
-        const int s = J % NB;
-        if (J + 2 < nJ) ok = issue_scores(J + 2);  // into the buffer whose P V product was issued last
-        if (!ok) break;
-        ok = mbar_wait(&p_full[s], (J / NB) & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t v_addr = smem_u32(smR + (J % NR) * R_BYTES + KV_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < TW / 16; ++ks)
-          umma_ts(tmem + COL_ACC, tmem + col_s(s) + ks * 8, umma_desc_sw128(v_addr + ks * 2048, 8192, 1024),
-                  idesc_v, (J > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&r_empty[J % NR]);
-        if (J == nJ - 1) umma_commit(&attn_done);
-      }
-      if (ok && has_state) {
-        // item 0: u = q~ Zg (hi then lo)
-        ok = mbar_wait(&a_full[0], 0, &abort_flag) && mbar_wait(&g_full, 0, &abort_flag);
-        if (ok) {
-          tc_fence_after();
-          const uint32_t g_addr = smem_u32(smG);
-#pragma unroll
-          for (int half = 0; half < 2; ++half)
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              umma_ts(tmem + COL_U, tmem + COL_A + ks * 8,
-                      umma_desc_sw128(g_addr + half * Z_BYTES + ks * 32, 16, 1024), idesc_g,
-                      (half > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&a_empty[0]);
+      bool ok = true;
+      dim3 cta = blockIdx;
+      // Positions in the rotation of buffers and ring stages, with the phases of op_full and r_full there: of the next
+      // operand (b, s), and of the next scores, which run up to NB operands ahead.
+      struct Pos {
+        int b = 0, s = 0;
+        uint32_t b_ph = 0, s_ph = 0;
+        __device__ __forceinline__ void step() {
+          if (++b == NB) b = 0, b_ph ^= 1;
+          if (++s == NR) s = 0, s_ph ^= 1;
         }
-        // ring items 1 .. nblk/2: 128 expanded entries against two state blocks (one ring stage);
-        // eight products per pair of waits and commits keep this thread off the critical path
-        for (int k = 1; k <= p.nblk / 2 && ok; ++k) {
-          const int s = k % NS, ph = (k / NS) & 1;
-          const int g = nJ + k - 1, rs = g % NR;
-          ok = mbar_wait(&a_full[s], ph, &abort_flag) && mbar_wait(&r_full[rs], (g / NR) & 1, &abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t z_addr = smem_u32(smR + rs * R_BYTES);
+      } at, sc;
+      int tiles = 0;
+      const uint32_t ring = smem_u32(smR);
+      // descriptors of stage 0; a stage on is R_BYTES >> 4 on in the address field
+      const uint64_t d_k = umma_desc_sw128(ring, 16, 1024), d_v = umma_desc_sw128(ring + KV_BYTES, 8192, 1024),
+                     d_z = umma_desc_sw128(ring, 8192, 1024);
+      for (int it = 0; ok; ++it) {
+        const OutTile w(p, cta);
+        if (!w.empty) {
+          const uint64_t d_q = umma_desc_sw128(smem_u32(smQ0 + (it & 1) * TILE_BYTES), 16, 1024);
+          ok = mbar_wait(&q_full[it & 1], (it >> 1) & 1, &abort_flag);
+          auto issue_scores = [&]() -> bool {
+            if (!mbar_wait(&r_full[sc.s], sc.s_ph, &abort_flag)) return false;
+            tc_fence_after();
+            const uint64_t d = d_k + (uint32_t)sc.s * (R_BYTES >> 4);
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            umma_ts(tmem + COL_ACC, tmem + COL_A + s * 64 + ks * 8,
-                    umma_desc_sw128(z_addr + (ks >> 2) * Z_BYTES + (ks & 3) * 2048, 8192, 1024), idesc_v,
-                    (nJ > 0 || k > 1 || ks > 0) ? 1u : 0u);
-          // one commit per item: it frees the ring stage for the TMA thread and, two items on, the
-          // tensor-memory slot for the expansion warps (a commit costs this thread ~150 clocks, a sixth of an item)
-          umma_commit(&r_empty[rs]);
+            for (int ks = 0; ks < 4; ++ks) umma_ss(tmem + col_b(sc.b), d_q + 2 * ks, d + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+            umma_commit(&s_full[sc.b]);
+            sc.step();
+            return true;
+          };
+          sc = at;
+          for (int J = 0; J < min(w.nJ, NB) && ok; ++J) ok = issue_scores();
+          // the accumulator of the tile before has been read out
+          if (ok && tiles > 0) ok = mbar_wait(&acc_free, (tiles - 1) & 1, &abort_flag);
+          for (int J = 0; J < w.nJ && ok; ++J) {
+            ok = mbar_wait(&op_full[at.b], at.b_ph, &abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t d = d_v + (uint32_t)at.s * (R_BYTES >> 4);
+#pragma unroll
+            for (int ks = 0; ks < TW / 16; ++ks)
+              umma_ts(tmem, tmem + col_b(at.b) + ks * 8, d + ks * (2048 >> 4), idesc_v, (J > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(&r_empty[at.s]);
+            at.step();
+            // the next scores, into the buffer that the product just issued reads (products execute in order)
+            if (J + NB < w.nJ) ok = issue_scores();
+          }
+          for (int k = 0; k < w.nI && ok; ++k) {
+            ok = mbar_wait(&op_full[at.b], at.b_ph, &abort_flag) && mbar_wait(&r_full[at.s], at.s_ph, &abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            if (k == 0) {
+              // u = q~ Zg (hi then lo), into the buffer of the operand after next
+              const uint64_t d = d_k + (uint32_t)at.s * (R_BYTES >> 4);
+              const int bu = at.b == 0 ? 2 : at.b - 1;
+#pragma unroll
+              for (int hl = 0; hl < 2; ++hl)
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                  umma_ts(tmem + col_b(bu), tmem + col_b(at.b) + ks * 8, d + hl * (Z_BYTES >> 4) + 2 * ks, idesc_g,
+                          (hl > 0 || ks > 0) ? 1u : 0u);
+              umma_commit(&u_full);
+            } else {
+              // 128 expanded entries against two state blocks
+              const uint64_t d = d_z + (uint32_t)at.s * (R_BYTES >> 4);
+#pragma unroll
+              for (int ks = 0; ks < 8; ++ks)
+                umma_ts(tmem, tmem + col_b(at.b) + ks * 8, d + (ks >> 2) * (Z_BYTES >> 4) + (ks & 3) * (2048 >> 4), idesc_v,
+                        (w.nJ > 0 || k > 1 || ks > 0) ? 1u : 0u);
+            }
+            umma_commit(&r_empty[at.s]);
+            at.step();
+          }
+          if (ok) umma_commit(&acc_full);
+          ++tiles;
         }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
-      if (ok) umma_commit(&acc_done);
     }
   } else {
     // --------------------------------------------------------- row-owning warps
-    const int grp = warp >> 2, r = tid & 127;   // row group, row inside the tile
-    const int row = row0 + r;                   // query index inside the chunk
-    const bool row_valid = row < cq;
-    const int qpos = row + q_off;               // key position of this query
+    const uint32_t tmem = tmem_base_s;
+    const int grp = warp >> 2, r = tid & 127;   // row group, row inside a tile
     const int wrow = (warp & 3) * 32;
     const uint32_t lane_addr = (uint32_t)wrow << 16;
-    const bool gated = p.a != nullptr;
-    const float* a_chunk = gated ? p.a + ((size_t)batch * p.tk + (size_t)chunk * p.ck) * p.h + kvhead
-                                 : nullptr;
-    const float a_i = (gated && row_valid) ? a_chunk[(size_t)qpos * p.h] : 0.f;
     const float s2 = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
-    float l_acc = 0.f;
+    const bool gated = p.a != nullptr;
     bool ok = true;
-    // gate sums of this warp's next step, loaded one step ahead
-    float av0 = 0.f, av1 = 0.f, r_n = 0.f;
-    auto load_gates = [&](int J) {
-      if (gated) {
-        const int kp = J * TW + lane;
-        r_n = a_chunk[(size_t)min(J * TW + TW - 1, ck - 1) * p.h];
-        av0 = kp < ck ? a_chunk[(size_t)kp * p.h] : 0.f;
-        av1 = kp + 32 < ck ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
-      }
+    dim3 cta = blockIdx;
+    int u0 = 0, tiles = 0, grams = 0;  // operands before this tile, tiles with rows, Gram products so far
+    uint32_t s_base = 0, row_ph = 0;   // phase of each buffer's s_full at the tile's start (one bit each), and of rows
+    // the row warps meet; bounded like every wait
+    auto meet = [&]() {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&rows);
+      if (ok) ok = mbar_wait(&rows, row_ph, &abort_flag);
+      row_ph ^= 1;
     };
-    if (grp < nJ) load_gates(grp);
-
-    for (int J = grp; J < nJ; J += NG) {
-      const int kp0 = J * TW;
-      const int sb = J % NB, sp = (J / NG) & 1;
-      float* ak = sm_ak[warp][sp];
-      float* fk = sm_fk[warp][sp];
-      const float rs = r_n;
-      ak[lane] = av0;
-      ak[lane + 32] = av1;
-      fk[lane] = __expf(rs - av0);
-      fk[lane + 32] = __expf(rs - av1);
-      // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
-      // row and per key instead of one per pair (both exponents <= 0 below the diagonal for gates
-      // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps wholly below the
-      // diagonal need no mask; a warp whose rows all precede the step's keys writes zeros
-      // without reading the scores.
-      const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - fminf(av0, av1), a_i - rs) > 80.f);
-      __syncwarp();  // ak, fk
-      const float c_i = sep ? s2 * __expf(a_i - rs) : s2;
-      if (J + NG < nJ) load_gates(J + NG);  // in flight while this step is computed
-      ok = mbar_wait(&s_full[sb], (J / NB) & 1, &abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t cs = tmem + lane_addr + col_s(sb);
-      const int wq0 = row0 + wrow + q_off;  // key position of this warp's first query
-      if (kp0 > min(wq0 + 31, ck - 1)) {
-        uint32_t z[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) z[j] = 0u;
-        tmem_st16(cs, z);
-        tmem_st16(cs + 16, z);
-      } else {
-        const bool mask = (kp0 + TW - 1 > wq0) || (kp0 + TW - 1 >= ck);
-        const int lim = min(qpos, ck - 1) - kp0;  // last column this row keeps
-#pragma unroll 1
-        for (int q4 = 0; q4 < TW / 32; ++q4) {
-          uint32_t sv[32], pk[16];
-          tmem_ld32(cs + q4 * 32, sv);
-          tmem_wait_ld();
-          const int lm = lim - q4 * 32;
-          if (sep) {
-            if (mask) out_half<T, DEG, true, true>(sv, fk + q4 * 32, c_i, a_i, lm, pk, l_acc);
-            else out_half<T, DEG, true, false>(sv, fk + q4 * 32, c_i, a_i, lm, pk, l_acc);
-          } else {
-            out_half<T, DEG, false, true>(sv, ak + q4 * 32, c_i, a_i, lm, pk, l_acc);
-          }
-          tmem_st16(cs + q4 * 16, pk);
-        }
-      }
+    auto operand_written = [&](int u) {
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[sb]);
-    }
-
-    // gated, scaled query row as 32 packed pairs
-    if (has_state) {  // whether a wait has run out or not: the barriers below want every thread
-      uint32_t q2[32];
-      if (ok) ok = mbar_wait(&q_full, 0, &abort_flag);
-      float f = p.scale;
-      if (gated) {
-        const float a_g = p.q_gate_last ? a_chunk[(size_t)(ck - 1) * p.h] : a_i;
-        f *= __expf(0.5f * a_g);
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(r, j));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 x = Pack2<T>::to_f32(w[k]);
-          q2[4 * j + k] = Pack2<T>::from_f32(x.x * f, x.y * f);
-        }
-      }
-      // the P columns alias the expansion ring: wait until the last P V product has read them
-      if (ok && nJ > 0) ok = mbar_wait(&attn_done, 0, &abort_flag);
+      if (lane == 0) mbar_arrive(&op_full[u % NB]);
+    };
+    // buffer u % NB is free once the products that read its operand before u have completed
+    auto buffer_free = [&](int u) {
+      if (ok && u >= NB) ok = mbar_wait(&r_empty[(u - NB) % NR], ((u - NB) / NR) & 1, &abort_flag);
       tc_fence_after();
-      if (ok && grp == 0) {
-        // item 0: q~ itself (A operand of u = q~ Zg)
-        tmem_st32(tmem + lane_addr + COL_A, q2);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&a_full[0]);
-      }
-      // The gated row goes back to its own slot of the query tile (both groups have read the raw one, and the score
-      // products that read it have completed) so that the first factor can be fetched by a runtime index; the loop
-      // over first factors then has a body of 64 multiplies per stage.
-      named_bar_sync(1, 128 * NG);
-      if (grp == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          *reinterpret_cast<uint4*>(smQ + swz128(r, j)) = make_uint4(q2[4 * j], q2[4 * j + 1], q2[4 * j + 2], q2[4 * j + 3]);
-      }
-      named_bar_sync(1, 128 * NG);
-      // ring items 1..nblk/2: 128 expanded entries (64 packed products) each.  A block of second factors has an even
-      // number of items, so group 1 takes the odd items (first factors 0-7, 16-23 ...) and group 0 the even ones.
-      const int s = grp;
-      int k = 2 - grp;
-      static_for<0, HD / 16>([&](auto yc) {
-        constexpr int Y = decltype(yc)::value;
-        if (16 * Y >= p.d) return;
-#pragma unroll 1
-        for (int a0 = 8 * (1 - grp); a0 < 16 * (Y + 1); a0 += 16, k += NG) {
-          uint32_t x[32];
-          expand_stage<T, Y>(smQ, r, a0, q2, x);
-          // the slot was last used by item k - 2: the Gram item (its own barrier) or a ring item, whose
-          // completion the issuing thread reports on the ring stage's barrier
-          if (ok && k == 2) ok = mbar_wait(&a_empty[0], 0, &abort_flag);
-          if (ok && k >= 3) {
-            const int g2 = nJ + k - 3;
-            ok = mbar_wait(&r_empty[g2 % NR], (g2 / NR) & 1, &abort_flag);
+    };
+    for (int it = 0; ok; ++it) {
+      const OutTile w(p, cta);
+      if (!w.empty) {
+        uint8_t* smQ = smQ0 + (it & 1) * TILE_BYTES;
+        const float* a_chunk =
+            gated ? p.a + ((size_t)w.batch * p.tk + (size_t)w.chunk * p.ck) * p.h + w.kvhead : nullptr;
+        const int row = w.row0 + r;             // query index inside the chunk
+        const int qpos = row + w.q_off;         // its key position
+        const float a_i = (gated && row < w.cq) ? a_chunk[(size_t)qpos * p.h] : 0.f;
+        float l_acc = 0.f;
+        // gate sums of this warp's next step, loaded one step ahead
+        float av0 = 0.f, av1 = 0.f, r_n = 0.f;
+        auto load_gates = [&](int J) {
+          if (gated) {
+            const int kp = J * TW + lane;
+            r_n = a_chunk[(size_t)min(J * TW + TW - 1, w.ck - 1) * p.h];
+            av0 = kp < w.ck ? a_chunk[(size_t)kp * p.h] : 0.f;
+            av1 = kp + 32 < w.ck ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
           }
-          tc_fence_after();
-          if (ok) tmem_st32(tmem + lane_addr + COL_A + s * 64, x);
-          expand_stage<T, Y>(smQ, r, a0 + 4, q2, x);
-          if (ok) {
-            tmem_st32(tmem + lane_addr + COL_A + s * 64 + 32, x);
-            tmem_wait_st();
-            tc_fence_before();
-          }
-          __syncwarp();
-          if (ok && lane == 0) mbar_arrive(&a_full[s]);
-        }
-      });
-    }
+        };
+        const int first = (u0 + grp) & 1;       // this group's first operand in the tile
+        static_assert(NG == 2, "the group of operand u is u & 1");
+        if (first < w.nJ) load_gates(first);
 
-    if (ok) ok = mbar_wait(&acc_done, 0, &abort_flag);
-    tc_fence_after();
-    // Each group finishes 32 of the row's 64 columns: half of <u, q~> for the row sum, half of the output.
-    const uint32_t half = 32 * grp;
-    if (ok && has_state) {
-      uint32_t u[32];
-      tmem_ld32(tmem + lane_addr + COL_U + half, u);
-      tmem_wait_ld();
-      float ls0 = 0.f, ls1 = 0.f;
+        for (int J = first; J < w.nJ && ok; J += NG) {
+          const int u = u0 + J, b = u % NB;
+          const int kp0 = J * TW;
+          float* fk = sm_fk[warp][(J >> 1) & 1];
+          const float rs = r_n;
+          // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
+          // row and per key instead of one per pair (both exponents <= 0 below the diagonal for gates
+          // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps wholly below the
+          // diagonal need no mask; a warp whose rows all precede the step's keys writes zeros
+          // without reading the scores.
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - fminf(av0, av1), a_i - rs) > 80.f);
+          const float c_i = sep ? s2 * __expf(a_i - rs) : s2;
+          fk[lane] = sep ? __expf(rs - av0) : av0;
+          fk[lane + 32] = sep ? __expf(rs - av1) : av1;
+          __syncwarp();
+          if (J + NG < w.nJ) load_gates(J + NG);  // in flight while this step is computed
+          ok = mbar_wait(&s_full[b], ((s_base >> b) + J / NB) & 1, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t cs = tmem + lane_addr + col_b(b);
+          const int wq0 = w.row0 + wrow + w.q_off;  // key position of this warp's first query
+          if (kp0 > min(wq0 + 31, w.ck - 1)) {
+            uint32_t z[16];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(r, 4 * grp + j));  // the gated row
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 qv = Pack2<T>::to_f32(w[k]);
-          ls0 = fmaf(__uint_as_float(u[8 * j + 2 * k]), qv.x, ls0);
-          ls1 = fmaf(__uint_as_float(u[8 * j + 2 * k + 1]), qv.y, ls1);
+            for (int j = 0; j < 16; ++j) z[j] = 0u;
+            tmem_st16(cs, z);
+            tmem_st16(cs + 16, z);
+          } else {
+            const bool mask = (kp0 + TW - 1 > wq0) || (kp0 + TW - 1 >= w.ck);
+            const int lim = min(qpos, w.ck - 1) - kp0;  // last column this row keeps
+            if (!sep) out_step<T, DEG, false, true>(cs, fk, c_i, a_i, lim, l_acc);
+            else if (mask) out_step<T, DEG, true, true>(cs, fk, c_i, a_i, lim, l_acc);
+            else out_step<T, DEG, true, false>(cs, fk, c_i, a_i, lim, l_acc);
+          }
+          operand_written(u);
         }
-      }
-      l_acc += ls0 + ls1;
-    }
-    sm_l[grp][r] = l_acc;
-    named_bar_sync(1, 128 * NG);
-    if (ok) {
-      const float l = sm_l[0][r] + sm_l[1][r];
-      uint32_t acc[32];
-      tmem_ld32(tmem + lane_addr + COL_ACC + half, acc);
-      tmem_wait_ld();
-      if (row_valid) {
-        const size_t tok = (size_t)batch * p.tq + (size_t)chunk * p.cq + row;
-        const float inv = p.normalize ? safe_recip(l) : 1.f;
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.O) + (tok * p.hq + qhead) * p.d + half);
+
+        if (w.nI > 0) {
+          meet();  // every score product of the tile has completed: the query tile may be rewritten
+          // The gated, scaled row q~ takes the row's place in the query tile, where the expansion fetches its factors
+          // by a runtime index; each group does every other 16-byte piece.
+          if (ok) ok = mbar_wait(&q_full[it & 1], (it >> 1) & 1, &abort_flag);
+          const float f =
+              p.scale * (gated ? __expf(0.5f * (p.q_gate_last ? a_chunk[(size_t)(w.ck - 1) * p.h] : a_i)) : 1.f);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if ((int)half + 8 * j >= p.d) break;
-          uint4 v;
-          v.x = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 0]), inv * __uint_as_float(acc[8 * j + 1]));
-          v.y = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 2]), inv * __uint_as_float(acc[8 * j + 3]));
-          v.z = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 4]), inv * __uint_as_float(acc[8 * j + 5]));
-          v.w = Pack2<T>::from_f32(inv * __uint_as_float(acc[8 * j + 6]), inv * __uint_as_float(acc[8 * j + 7]));
-          dst[j] = v;
+          for (int jj = 0; jj < 4; ++jj) {
+            uint4* slot = reinterpret_cast<uint4*>(smQ + swz128(r, 2 * jj + grp));
+            const uint4 v = *slot;
+            uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float2 f2 = Pack2<T>::to_f32(x[k]);
+              x[k] = Pack2<T>::from_f32(f2.x * f, f2.y * f);
+            }
+            *slot = make_uint4(x[0], x[1], x[2], x[3]);
+          }
+          meet();  // q~ is in place
+          const int ui = u0 + w.nJ;
+          if ((ui & 1) == grp) {
+            // operand 0: q~ itself (for u = q~ Zg); then u comes out of the buffer of operand 2, which is this group's
+            // too: its dot product with q~ is the state's part of the row sum
+            buffer_free(ui);
+            {
+              uint32_t q2[32];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(r, j));
+                q2[4 * j] = v.x;
+                q2[4 * j + 1] = v.y;
+                q2[4 * j + 2] = v.z;
+                q2[4 * j + 3] = v.w;
+              }
+              if (ok) {
+                tmem_st32(tmem + lane_addr + col_b(ui % NB), q2);
+                operand_written(ui);
+              }
+            }
+            if (ok) ok = mbar_wait(&u_full, grams & 1, &abort_flag);
+            tc_fence_after();
+            if (ok) {
+              float ls0 = 0.f, ls1 = 0.f;
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) {
+                uint32_t u[32];
+                tmem_ld32(tmem + lane_addr + col_b((ui + 2) % NB) + 32 * hf, u);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const uint4 v = *reinterpret_cast<const uint4*>(smQ + swz128(r, 4 * hf + j));
+                  const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) {
+                    const float2 qv = Pack2<T>::to_f32(x[k]);
+                    ls0 = fmaf(__uint_as_float(u[8 * j + 2 * k]), qv.x, ls0);
+                    ls1 = fmaf(__uint_as_float(u[8 * j + 2 * k + 1]), qv.y, ls1);
+                  }
+                }
+              }
+              l_acc += ls0 + ls1;
+              tc_fence_before();
+            }
+          }
+          ++grams;
+          // operands 1 .. nblk/2: 128 expanded entries (64 packed products) each
+          for (int k = (ui & 1) == grp ? 2 : 1; k < w.nI; k += NG) {
+            // operands 1-2, 3-6, 7-12, 13-20 have their second factors in block Y = 0, 1, 2, 3
+            const int Y = (k > 2) + (k > 6) + (k > 12);
+            const int a0 = 8 * (k - 1 - Y * (Y + 1));
+            const uint32_t ca = tmem + lane_addr + col_b((ui + k) % NB);
+            uint32_t x2[8], x[32];
+            expand_second(smQ, r, Y, x2);
+            expand_stage<T>(smQ, r, a0, x2, x);
+            buffer_free(ui + k);
+            if (ok) tmem_st32(ca, x);
+            expand_stage<T>(smQ, r, a0 + 4, x2, x);
+            if (ok) {
+              tmem_st32(ca + 32, x);
+              operand_written(ui + k);
+            }
+          }
         }
-        if (p.l_out != nullptr && grp == 0) p.l_out[tok * p.hq + qhead] = l;
+        // the query tile may be refilled (its last reads come before the async proxy's writes)
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&q_free[it & 1]);
+
+        sm_l[tiles & 1][grp][r] = l_acc;
+        meet();
+        if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
+        tc_fence_after();
+        // each group writes two pieces of 16 of the row's 64 columns, one 32-byte store each
+        if (ok) {
+          const float l = sm_l[tiles & 1][0][r] + sm_l[tiles & 1][1][r];
+          const float inv = p.normalize ? safe_recip(l) : 1.f;
+          const size_t tok = (size_t)w.batch * p.tq + (size_t)w.chunk * p.cq + row;
+          uint32_t acc[2][16];
+          tmem_ld16(tmem + lane_addr + 32 * grp, acc[0]);
+          tmem_ld16(tmem + lane_addr + 32 * grp + 16, acc[1]);
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_free);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int c0 = 32 * grp + 16 * q;
+            if (row < w.cq && c0 < p.d) {
+              uint32_t v[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                v[j] = Pack2<T>::from_f32(inv * __uint_as_float(acc[q][2 * j]), inv * __uint_as_float(acc[q][2 * j + 1]));
+              T* dst = static_cast<T*>(p.O) + (tok * p.hq + w.qhead) * p.d + c0;
+              if (p.o_aligned32) {
+                st_global_v8(dst, v);
+              } else {
+                reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+                reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+              }
+            }
+          }
+          if (p.l_out != nullptr && grp == 0 && row < w.cq) p.l_out[tok * p.hq + w.qhead] = l;
+        }
+        // the score products of the tile: buffer b had one for every step J with (u0 + J) % NB == b
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const int j0 = (b - u0 % NB + NB) % NB;
+          if (j0 < w.nJ) s_base ^= (((w.nJ - 1 - j0) / NB + 1) & 1) << b;
+        }
+        u0 += w.nJ + w.nI;
+        ++tiles;
+      } else {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&q_free[it & 1]);
       }
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
     }
   }
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && abort_flag) *p.status = ST_TIMEOUT;
-  if (warp == 0) tmem_dealloc(tmem, co::TMEM_COLS);
+  if (warp == 0) tmem_dealloc(tmem_base_s, TMEM_COLS);
 }
 
 }  // namespace pr
@@ -529,6 +638,7 @@ int pr::chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int 
   p.scale = scale;
   p.a = a;
   p.O = O;
+  p.o_aligned32 = (reinterpret_cast<uintptr_t>(O) & 31u) == 0;
   p.l_out = l_out;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;
@@ -561,13 +671,12 @@ int pr::chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int 
     tm_ghi = tm_q;
     tm_glo = tm_q;
   }
-  const size_t smem = 1024 + TILE_BYTES + NR * R_BYTES + 2 * Z_BYTES;
   dim3 grid(p.tiles_per_chunk * n_chunks, hq, b);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define PR_LAUNCH_OUT(TT, DG)                                                                                      \
   do {                                                                                                             \
-    PR_SMEM_ATTR((chunk_out_kernel<TT, DG>), smem, device, true);                                                   \
-    chunk_out_kernel<TT, DG><<<grid, THREADS, smem, s>>>(p, tm_q, tm_k, tm_v, tm_z, tm_ghi, tm_glo);                 \
+    PR_SMEM_ATTR((chunk_out_kernel<TT, DG>), SMEM, device, true);                                                   \
+    chunk_out_kernel<TT, DG><<<grid, THREADS, SMEM, s>>>(p, tm_q, tm_k, tm_v, tm_z, tm_ghi, tm_glo);                 \
   } while (0)
   if (dtype == PR_BF16) {
     if (deg == 4) PR_LAUNCH_OUT(__nv_bfloat16, 4); else PR_LAUNCH_OUT(__nv_bfloat16, 2);

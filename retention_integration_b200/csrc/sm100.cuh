@@ -139,6 +139,55 @@ __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (i
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// ------------------------------------------------------- taking over CTAs
+// A persistent kernel keeps its grid: when a CTA has planned its tile, one thread asks for the index of a CTA of the
+// same grid that has not been launched yet and the CTA does that one's work next (cluster launch control), so set-up,
+// cold instruction fetches and the write-out of one tile overlap the next tile, and long and short tiles balance.
+// Two responses in flight: `full` completes when a response has arrived (16 bytes), `empty` when every reading
+// warp has taken it.
+struct ClcRing {
+  uint4 resp[2];
+  uint64_t full[2], empty[2];
+};
+__device__ __forceinline__ void clc_init(ClcRing* c, uint32_t readers) {
+  for (int i = 0; i < 2; ++i) {
+    mbar_init(&c->full[i], 1);
+    mbar_init(&c->empty[i], readers);
+  }
+}
+// one thread asks for the tile after tile number `it`
+__device__ __forceinline__ bool clc_ask(ClcRing* c, int it, volatile int* abort_flag) {
+  const int s = it & 1;
+  if (it >= 2 && !mbar_wait(&c->empty[s], ((it >> 1) - 1) & 1, abort_flag)) return false;
+  mbar_expect_tx(&c->full[s], 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(&c->resp[s])),
+               "r"(smem_u32(&c->full[s]))
+               : "memory");
+  return true;
+}
+// Every reading warp (or its one issuing thread): the tile after tile number `it` into `x, y, z`; false when there is
+// none.  `arrive`: this thread reports the warp's reading.
+__device__ __forceinline__ bool clc_next(ClcRing* c, int it, dim3* next, bool arrive, bool warp_wide,
+                                         volatile int* abort_flag) {
+  const int s = it & 1;
+  if (!mbar_wait(&c->full[s], (it >> 1) & 1, abort_flag)) return false;
+  uint32_t got, x, y, z;
+  asm volatile(
+      "{\n .reg .b128 h;\n .reg .pred p;\n ld.shared.b128 h, [%4];\n"
+      " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n selp.u32 %0, 1, 0, p;\n"
+      " mov.u32 %1, 0;\n mov.u32 %2, 0;\n mov.u32 %3, 0;\n"
+      " @p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, h;\n}"
+      : "=r"(got), "=r"(x), "=r"(y), "=r"(z)
+      : "r"(smem_u32(&c->resp[s]))
+      : "memory");
+  fence_async_smem();  // the read comes before the next response's write
+  if (warp_wide) __syncwarp();
+  if (arrive) mbar_arrive(&c->empty[s]);
+  *next = dim3(x, y, z);
+  return got != 0;
+}
+
 // --------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -191,6 +240,13 @@ __device__ __forceinline__ void bulk_wait_group_read() {
 template <int N>
 __device__ __forceinline__ void bulk_wait_group() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// one full 32-byte sector per thread; `dst` 32-byte aligned
+__device__ __forceinline__ void st_global_v8(void* dst, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
 }
 
 // -------------------------------------------------------------------- TMEM
@@ -358,11 +414,11 @@ struct Pack2<__half> {
   static constexpr bool is_bf16 = false;
 };
 // Expansion of one stage of the block layout (see layout.cuh): the 64 entries of four
-// consecutive first factors a0..a0+3 (a0 a multiple of 4) against the 16 second factors of
-// block Y, as 32 packed products.  `row` is the thread's own gated row in shared memory
-// (128 bytes, 128-byte swizzle, row index `r`), `x2` the same row as 32 packed registers.
-template <typename T, int Y>
-__device__ __forceinline__ void expand_stage(const uint8_t* tile, int r, int a0, const uint32_t (&x2)[32],
+// consecutive first factors a0..a0+3 (a0 a multiple of 4) against the 16 second factors x2 of
+// one block, as 32 packed products.  `r` is the thread's own gated row in the tile in shared memory
+// (128 bytes, 128-byte swizzle); expand_second() fetches the block's second factors from it.
+template <typename T>
+__device__ __forceinline__ void expand_stage(const uint8_t* tile, int r, int a0, const uint32_t (&x2)[8],
                                              uint32_t (&out)[32]) {
   const uint2 h = *reinterpret_cast<const uint2*>(tile + swz128(r, a0 >> 3) + ((a0 & 7) << 1));
   const uint32_t xa[4] = {__byte_perm(h.x, h.x, 0x1010), __byte_perm(h.x, h.x, 0x3232),
@@ -370,7 +426,13 @@ __device__ __forceinline__ void expand_stage(const uint8_t* tile, int r, int a0,
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) out[8 * k + j] = Pack2<T>::mul(xa[k], x2[8 * Y + j]);
+    for (int j = 0; j < 8; ++j) out[8 * k + j] = Pack2<T>::mul(xa[k], x2[j]);
+}
+__device__ __forceinline__ void expand_second(const uint8_t* tile, int r, int Y, uint32_t (&x2)[8]) {
+  const uint4 lo = *reinterpret_cast<const uint4*>(tile + swz128(r, 2 * Y));
+  const uint4 hi = *reinterpret_cast<const uint4*>(tile + swz128(r, 2 * Y + 1));
+  x2[0] = lo.x; x2[1] = lo.y; x2[2] = lo.z; x2[3] = lo.w;
+  x2[4] = hi.x; x2[5] = hi.y; x2[6] = hi.z; x2[7] = hi.w;
 }
 
 // duplicate the low / high 16-bit half of a packed pair into both halves
