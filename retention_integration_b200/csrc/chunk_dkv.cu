@@ -2,16 +2,24 @@
 // state-path gradients (the reference's attn_bwd_dkdv, retention/_attention/triton.py:390-493,
 // and the dV part of retention/_update_state/reference.py:55-60).
 //
-// One CTA owns 128 key rows (tile J) of one (batch, chunk, kv head); thread = key row.  For
-// every tile of 64 queries at or after the key tile, of every query head of the group (tiles
-// double-buffered in shared memory; 256 tensor memory columns, two CTAs per SM):
+// A tile is 128 key rows of one (batch, chunk, kv head).  For every tile of 64 queries at or after the key
+// tile, of every query head of the group:
 //     S^T = K_J Q_I^T,  dP^T = V_J dO_I^T                (tensor cores)
-//     p = (s S)^2 e^{a_i-a_j},  dp = dP / l_i + dl_i,  dS = 2 s^2 S e^{a_i-a_j} dp
+//     p / l = (s S)^2 e^{a_i-a_j} / l_i,  dS = 2 s^2 S e^{a_i-a_j} (dP + delta_i) / l_i,  delta_i = -<O_i, dO_i>
 //     dV += (P / l)^T dO_I,   dK += dS^T Q_I             (A operands from tensor memory)
 //     da_j -= sum_i p dp                                 (gate gradient, key side)
 // then the state path of the values, dV += phi(k~_j)^T (w (.) dS_m) with k~ the discounted
 // key (same expansion pipeline as the forward read-out).  The epilogue adds the state-path
 // key gradient (fp32, from the expansion-gradient kernel) and writes dK, dV.
+//
+// Three groups of four warps own the key rows, one row per thread in each group, and take the steps in turn, each in
+// its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma.  One persistent CTA per SM takes over
+// tile after tile (ClcRing).  A step is a serial chain - S and dP products, barrier, tensor-memory loads, arithmetic,
+// stores, barrier, dV and dK products - of about 4000 clocks in the earlier form, whose one buffer per CTA
+// made every part of it wait for the others; with three buffers the products of the next steps run while the rows work.
+// Per column of a step a thread reads two factors from shared memory, 1/l times the gate's and delta, where four were
+// read (a broadcast read costs the shared-memory pipe as much as a full one).
+// 490 -> NEW us at b1 t65536 h8 with chunks of 1024 and states.
 #include "host.cuh"
 #include "layout.cuh"
 #include "sm100.cuh"
@@ -20,16 +28,21 @@ namespace pr {
 
 namespace dkv {
 constexpr int HD = 64;
-constexpr int NS = 2;                    // expanded-operand ring in tensor memory: 2 stages of 128 entries (64 columns)
-constexpr int NR = 4;                    // shared-memory ring: stages of 16 KB (a query and a dO tile, or two state blocks)
-constexpr int THREADS = 192;
+constexpr int NG = 3;                    // row groups, each with its own buffer in tensor memory
+constexpr int NR = 7;                    // shared-memory ring: stages of 16 KB (a query and a dO tile, or two state blocks)
+constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
+constexpr int THREADS = 32 * (W_MMA + 1);
 constexpr int TILE_BYTES = 128 * 128;   // 128 key rows x 64 features
 constexpr int TW = 64;                  // queries per step
 constexpr int QD_BYTES = TW * 128;      // one query or dO tile
 constexpr int Z_BYTES = 64 * 128;
 constexpr int R_BYTES = 2 * QD_BYTES;   // one ring stage
-constexpr uint32_t TMEM_COLS = 256;     // two CTAs per SM
-constexpr uint32_t COL_S = 0, COL_P = 0, COL_DP = 64, COL_DS = 64, COL_DV = 128, COL_DK = 192, COL_A = 0;
+constexpr size_t SMEM = 1024 + 4 * TILE_BYTES + NR * R_BYTES;
+constexpr uint32_t TMEM_COLS = 512;
+// A buffer is 128 columns: S and dP, overwritten by P / l and dS (the first half of each); in the state phase 256
+// expanded entries.
+constexpr uint32_t COL_DV = 0, COL_DK = 64;
+__device__ __forceinline__ constexpr uint32_t col_b(int grp) { return 128u + 128u * (uint32_t)grp; }
 }  // namespace dkv
 
 struct ChunkDkvParams {
@@ -42,417 +55,505 @@ struct ChunkDkvParams {
   const float* A;         // [b, n, h] or null
   const float* dl;        // [b, t, hq]
   const float* l;         // [b, t, hq] row sums saved by the forward
-  const float* dk_state;  // [b, t, h, 64] fp32 or null
+  const float* dk_state;  // [b, t, h, d] fp32 or null
   void* dK;
   void* dV;
+  int aligned32;          // dK and dV start on 32-byte boundaries
   float* da_k;            // [b, t, h]
   int* status;
 };
 
-// One 32-column half of a step for one key row: P / l into `pk`, dS into `dk`, twice the row sum of
-// p * dp into da2.  SEP: the gate factor is c_j * fq[col] (c_j carries 2 s^2); otherwise
-// 2 s^2 e^{aq[col] - a_j} per pair, with columns beyond `hi` (past the chunk) dropped as well.
-// MASK: columns before `lo` (queries that precede this key) are dropped.
+struct DkvTile {
+  int chunk, kvhead, batch, row0, tok_chunk;
+  int c;        // tokens of the chunk
+  int qt0;      // first query tile that can see this key tile
+  int n_steps;  // (query tiles from qt0 on) x (query heads of the group)
+  int nI;       // state items of 256 expanded entries
+  bool empty;   // past the end of a shorter last chunk
+  __device__ __forceinline__ DkvTile(const ChunkDkvParams& p, const dim3& cta) {
+    const int x = (int)cta.x;
+    const int tile_j = x % p.tiles_per_chunk;  // the longest tiles of a head first
+    chunk = x / p.tiles_per_chunk;
+    kvhead = (int)cta.y;
+    batch = (int)cta.z;
+    row0 = tile_j * 128;
+    tok_chunk = chunk * p.c;
+    c = min(p.c, p.t - tok_chunk);
+    empty = row0 >= c;
+    qt0 = row0 / dkv::TW;
+    n_steps = empty ? 0 : ((c + dkv::TW - 1) / dkv::TW - qt0) * (p.hq / p.h);
+    nI = (!empty && chunk <= p.state_chunk_hi) ? p.nblk / 4 : 0;
+  }
+};
+
+// One 16-column piece of a step for one key row: P / l into `pk`, dS into `dk`, deg times the row sum of p * dp into
+// acc.  SEP: the gate factor is c_j * fq[col] (c_j carries s^deg, fq 1 / l); otherwise s^deg e^{aq[col] - a_j} fq[col].
+// de: deg * delta.  MASK: columns before `lo` (queries that precede this key) are dropped.
 template <typename T, int DEG, bool SEP, bool MASK>
-__device__ __forceinline__ void dkv_half(const uint32_t (&sv)[32], const uint32_t (&pv)[32], const float* __restrict__ fq,
-                                         const float* __restrict__ il, const float* __restrict__ hl,
-                                         const float* __restrict__ dl, float c_j, float a_j, int lo, int hi,
-                                         uint32_t (&pk)[16], uint32_t (&dk)[16], float& da2) {
+__device__ __forceinline__ void dkv_piece(const uint32_t (&sv)[16], const uint32_t (&pv)[16], const float* __restrict__ fq,
+                                          const float* __restrict__ de, const float* __restrict__ aq, float c_j, float a_j,
+                                          int lo, uint32_t (&pk)[8], uint32_t (&dk)[8], float2& acc) {
   // two columns per instruction: packed fp32 multiplies and FMAs
   const float4* f4 = reinterpret_cast<const float4*>(fq);
-  const float4* i4 = reinterpret_cast<const float4*>(il);
-  const float4* h4 = reinterpret_cast<const float4*>(hl);
-  const float4* d4 = reinterpret_cast<const float4*>(dl);
-  const float2 c2 = make_float2(c_j, c_j);
-  float2 acc = make_float2(0.f, 0.f);
+  const float4* d4 = reinterpret_cast<const float4*>(de);
+  const float4* a4 = reinterpret_cast<const float4*>(aq);
+  const float2 c2 = make_float2(c_j, c_j), deg2 = make_float2((float)DEG, (float)DEG);
 #pragma unroll
-  for (int j = 0; j < 32; j += 4) {
-    const float4 f = f4[j >> 2], iq = i4[j >> 2], hq = h4[j >> 2], dq = d4[j >> 2];
+  for (int j = 0; j < 16; j += 4) {
+    const float4 f = f4[j >> 2], dq = d4[j >> 2];
     const float2 fv[2] = {make_float2(f.x, f.y), make_float2(f.z, f.w)};
-    const float2 iv[2] = {make_float2(iq.x, iq.y), make_float2(iq.z, iq.w)};
-    const float2 hv[2] = {make_float2(hq.x, hq.y), make_float2(hq.z, hq.w)};
     const float2 dv[2] = {make_float2(dq.x, dq.y), make_float2(dq.z, dq.w)};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int col = j + 2 * u;
       const float2 s = make_float2(__uint_as_float(sv[col]), __uint_as_float(sv[col + 1]));
       const float2 p = make_float2(__uint_as_float(pv[col]), __uint_as_float(pv[col + 1]));
-      float2 g;
-      if (SEP) {
-        g = __fmul2_rn(c2, fv[u]);
-      } else {
-        g = make_float2(c_j * __expf(fv[u].x - a_j), c_j * __expf(fv[u].y - a_j));
-        g.x = (col <= hi) ? g.x : 0.f;
-        g.y = (col + 1 <= hi) ? g.y : 0.f;
+      float2 g = __fmul2_rn(c2, fv[u]);
+      if (!SEP) {
+        const float4 a = a4[j >> 2];
+        g.x *= __expf((u ? a.z : a.x) - a_j);
+        g.y *= __expf((u ? a.w : a.y) - a_j);
       }
       if (MASK) {
         g.x = (col >= lo) ? g.x : 0.f;
         g.y = (col + 1 >= lo) ? g.y : 0.f;
       }
       const float2 sp = DEG == 4 ? __fmul2_rn(s, __fmul2_rn(s, s)) : s;  // S^(deg-1)
-      const float2 sg2 = __fmul2_rn(sp, g);  // deg s^deg S^(deg-1) e^{a_i-a_j}
-      const float2 dp = __ffma2_rn(p, iv[u], dv[u]);
-      const float2 ds = __fmul2_rn(sg2, dp);
+      const float2 sg = __fmul2_rn(sp, g);             // s^deg S^(deg-1) e^{a_i-a_j} / l_i
+      const float2 dp = __ffma2_rn(p, deg2, dv[u]);    // deg (dP + delta)
+      const float2 ds = __fmul2_rn(sg, dp);
       acc = __ffma2_rn(ds, s, acc);
-      const float2 pw = __fmul2_rn(__fmul2_rn(sg2, s), hv[u]);
+      const float2 pw = __fmul2_rn(sg, s);
       pk[col >> 1] = Pack2<T>::from_f32(pw.x, pw.y);
       dk[col >> 1] = Pack2<T>::from_f32(ds.x, ds.y);
     }
   }
-  da2 += acc.x + acc.y;
+}
+
+// A whole step: the loads of the next piece are in flight while one is computed.
+template <typename T, int DEG, bool SEP, bool MASK>
+__device__ __forceinline__ void dkv_step(uint32_t cb, const float* __restrict__ fq, const float* __restrict__ de,
+                                         const float* __restrict__ aq, float c_j, float a_j, int lo, float& da) {
+  uint32_t sv[2][16], pv[2][16], pk[8], dk[8];
+  float2 acc = make_float2(0.f, 0.f);
+  tmem_ld16(cb, sv[0]);
+  tmem_ld16(cb + 64, pv[0]);
+#pragma unroll
+  for (int q = 0; q < dkv::TW / 16; ++q) {
+    tmem_wait_ld();
+    if (q + 1 < dkv::TW / 16) {
+      tmem_ld16(cb + (q + 1) * 16, sv[(q + 1) & 1]);
+      tmem_ld16(cb + 64 + (q + 1) * 16, pv[(q + 1) & 1]);
+    }
+    dkv_piece<T, DEG, SEP, MASK>(sv[q & 1], pv[q & 1], fq + q * 16, de + q * 16, aq + q * 16, c_j, a_j, lo - q * 16, pk, dk,
+                                 acc);
+    tmem_st8(cb + q * 8, pk);
+    tmem_st8(cb + 64 + q * 8, dk);
+  }
+  da += acc.x + acc.y;
 }
 
 template <typename T, int DEG>
-__global__ void __launch_bounds__(dkv::THREADS, 2)
+__global__ void __launch_bounds__(dkv::THREADS, 1)
 chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_ds) {
   using namespace dkv;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t kv_full, r_full[NR], r_empty[NR], sp_full, pd_full, attn_done, acc_done;
-  __shared__ uint64_t a_full[NS];
+  // kv_*: the key and value tiles, two pairs in flight.  r_*: the ring of operand tiles.  s_full: S and dP in a
+  // group's buffer; op_full: the group has written its A operands.  acc_full / acc_free: accumulators complete / read
+  // out; rows: the row warps meet.
+  __shared__ uint64_t kv_full[2], kv_free[2], r_full[NR], r_empty[NR], s_full[NG], op_full[NG], acc_full, acc_free, rows;
+  __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  __shared__ __align__(16) float sm_aq[2][TW], sm_dl[2][TW], sm_il[2][TW];
-  __shared__ __align__(16) float sm_fq[2][TW];  // e^{a_i - r}, r = gate sum at the step's first query
-  __shared__ __align__(16) float sm_hl[2][TW];  // 1 / (2 l_i)
-  __shared__ float sm_r[2];
-  __shared__ int sm_wide[2][2];                 // a loader warp saw a_i - r > 80 (overflow guard)
+  // Per warp and step parity, each warp its own copy: e^{a_i - r} / l_i (r = gate sum at the step's first query),
+  // deg * delta_i, and a_i where the exponentials do not separate (the first is 1 / l_i then).
+  __shared__ __align__(16) float sm_fq[4 * NG][2][TW], sm_de[4 * NG][2][TW], sm_aq[4 * NG][TW];
+  __shared__ float sm_da[2][NG][128];
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
-  uint8_t* smK = sm;
-  uint8_t* smV = smK + TILE_BYTES;
-  // One ring serves both phases: attention step st takes stage st % NR (query tile, then dO tile);
-  // the state phase goes on with the same stage counter, two 64-row state blocks per stage, so
-  // state blocks stream in while the last attention steps are still being computed.
-  uint8_t* smR = smV + TILE_BYTES;       // NR x R_BYTES
+  uint8_t* smKV = sm;                    // 2 x (key tile, value tile)
+  // One ring serves both phases and all tiles: an attention step takes a stage (query tile, then dO tile), a state
+  // item two (two 64-row state blocks each), so operands stream in while the steps before are still being computed.
+  uint8_t* smR = smKV + 4 * TILE_BYTES;  // NR x R_BYTES
 
-  const int tile_j = blockIdx.x % p.tiles_per_chunk;
-  const int chunk = blockIdx.x / p.tiles_per_chunk;
-  const int kvhead = blockIdx.y, batch = blockIdx.z;
+  if (warp == W_TMA) {
+    if (elect_one()) {
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_dy);
+      abort_flag = 0;
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(&kv_full[s], 1);
+        mbar_init(&kv_free[s], 4 * NG);
+      }
+      for (int s = 0; s < NR; ++s) {
+        mbar_init(&r_full[s], 1);
+        mbar_init(&r_empty[s], 1);
+      }
+      for (int s = 0; s < NG; ++s) {
+        mbar_init(&s_full[s], 1);
+        mbar_init(&op_full[s], 4);
+      }
+      mbar_init(&acc_full, 1);
+      mbar_init(&acc_free, 4 * NG);
+      mbar_init(&rows, 4 * NG);
+      clc_init(&clc, 4 * NG + 2);
+      fence_mbar_init();
+    }
+    __syncwarp();
+    named_bar_arrive(1, THREADS);  // the first loads need not wait for the tensor memory
+  } else {
+    if (warp == 0) {
+      tmem_alloc(&tmem_base_s, TMEM_COLS);
+      tmem_relinquish();
+    }
+    tc_fence_before();
+    named_bar_sync(1, THREADS);
+    tc_fence_after();
+  }
   const int ratio = p.hq / p.h;
-  const int row0 = tile_j * 128;
-  const int tok_chunk = chunk * p.c;
-  const int c = min(p.c, p.t - tok_chunk);      // tokens of this chunk
-  if (row0 >= c) return;
-  const int q_tiles = (c + TW - 1) / TW;        // query tiles of TW rows in the chunk
-  const int qt0 = row0 / TW;                    // first query tile that can see this key tile
-  const int nI = q_tiles - qt0;
-  const int n_steps = nI * ratio;
-  const bool has_state = chunk <= p.state_chunk_hi;
 
-  if (tid == 0) {
-    abort_flag = 0;
-    mbar_init(&kv_full, 1);
-    for (int s = 0; s < NR; ++s) {
-      mbar_init(&r_full[s], 1);
-      mbar_init(&r_empty[s], 1);
-    }
-    mbar_init(&sp_full, 1);
-    mbar_init(&pd_full, 4);
-    mbar_init(&attn_done, 1);
-    mbar_init(&acc_done, 1);
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(&a_full[s], 4);
-    }
-    fence_mbar_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(&tmem_base_s, TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
-
-  if (warp == 4) {
+  if (warp == W_TMA) {
     if (elect_one()) {
       bool ok = true;
-      mbar_expect_tx(&kv_full, 2 * TILE_BYTES);
-      tma_load_4d(smK, &tm_k, &kv_full, 0, kvhead, tok_chunk + row0, batch);
-      tma_load_4d(smV, &tm_v, &kv_full, 0, kvhead, tok_chunk + row0, batch);
-      const int ch = (batch * p.n_chunks + chunk) * p.h + kvhead;
-      const int n_ring = n_steps + (has_state ? p.nblk / 2 : 0);
-      for (int g = 0; g < n_ring && ok; ++g) {
-        const int s = g % NR, ph = (g / NR) & 1;
-        ok = mbar_wait(&r_empty[s], ph ^ 1, &abort_flag);
+      dim3 cta = blockIdx;
+      int s = 0;           // ring stage and its phase
+      uint32_t s_ph = 0;
+      auto next_stage = [&]() -> uint8_t* {
+        ok = ok && mbar_wait(&r_empty[s], s_ph ^ 1, &abort_flag);
+        if (ok) mbar_expect_tx(&r_full[s], R_BYTES);
+        return smR + s * R_BYTES;
+      };
+      auto advance = [&]() {
+        if (++s == NR) s = 0, s_ph ^= 1;
+      };
+      for (int it = 0; ok; ++it) {
+        const DkvTile w(p, cta);
+        if (it >= 2) ok = mbar_wait(&kv_free[it & 1], ((it >> 1) - 1) & 1, &abort_flag);
         if (!ok) break;
-        mbar_expect_tx(&r_full[s], R_BYTES);
-        uint8_t* dst = smR + s * R_BYTES;
-        if (g < n_steps) {
-          const int I = qt0 + g / ratio, qh = kvhead * ratio + g % ratio;
-          tma_load_4d(dst, &tm_q, &r_full[s], 0, qh, tok_chunk + I * TW, batch);
-          tma_load_4d(dst + QD_BYTES, &tm_dy, &r_full[s], 0, qh, tok_chunk + I * TW, batch);
+        if (!w.empty) {
+          uint8_t* kv = smKV + (it & 1) * 2 * TILE_BYTES;
+          mbar_expect_tx(&kv_full[it & 1], 2 * TILE_BYTES);
+          tma_load_4d(kv, &tm_k, &kv_full[it & 1], 0, w.kvhead, w.tok_chunk + w.row0, w.batch);
+          tma_load_4d(kv + TILE_BYTES, &tm_v, &kv_full[it & 1], 0, w.kvhead, w.tok_chunk + w.row0, w.batch);
+          for (int st = 0; st < w.n_steps && ok; ++st) {
+            const int I = w.qt0 + st / ratio, qh = w.kvhead * ratio + st % ratio;
+            uint8_t* dst = next_stage();
+            if (!ok) break;
+            tma_load_4d(dst, &tm_q, &r_full[s], 0, qh, w.tok_chunk + I * TW, w.batch);
+            tma_load_4d(dst + QD_BYTES, &tm_dy, &r_full[s], 0, qh, w.tok_chunk + I * TW, w.batch);
+            advance();
+            if (st == 0) ok = clc_ask(&clc, it, &abort_flag);
+          }
+          const int blk0 = ((w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead) * p.nblk;
+          for (int k = 0; k < 2 * w.nI && ok; ++k) {
+            uint8_t* dst = next_stage();
+            if (!ok) break;
+            tma_load_2d(dst, &tm_ds, &r_full[s], 0, (blk0 + 2 * k) * 64);
+            tma_load_2d(dst + Z_BYTES, &tm_ds, &r_full[s], 0, (blk0 + 2 * k + 1) * 64);
+            advance();
+          }
         } else {
-          const int blk = 2 * (g - n_steps);
-          tma_load_2d(dst, &tm_ds, &r_full[s], 0, (ch * p.nblk + blk) * 64);
-          tma_load_2d(dst + Z_BYTES, &tm_ds, &r_full[s], 0, (ch * p.nblk + blk + 1) * 64);
+          mbar_arrive(&kv_full[it & 1]);  // nothing to load: the phase passes all the same
+          ok = clc_ask(&clc, it, &abort_flag);
         }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == W_MMA) {
+    const uint32_t tmem = tmem_base_s;
     if (elect_one()) {
-      bool ok = mbar_wait(&kv_full, 0, &abort_flag);
       const uint32_t idesc_s = umma_idesc(128, TW, Pack2<T>::is_bf16, false, false);
       const uint32_t idesc_o = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
-      const uint32_t k_addr = smem_u32(smK), v_addr = smem_u32(smV);
-      for (int st = 0; st < n_steps && ok; ++st) {
-        const int sg = st % NR;
-        ok = mbar_wait(&r_full[sg], (st / NR) & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t q_addr = smem_u32(smR + sg * R_BYTES), dy_addr = q_addr + QD_BYTES;
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + COL_S, umma_desc_sw128(k_addr + ks * 32, 16, 1024),
-                  umma_desc_sw128(q_addr + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + COL_DP, umma_desc_sw128(v_addr + ks * 32, 16, 1024),
-                  umma_desc_sw128(dy_addr + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(&sp_full);
-        ok = mbar_wait(&pd_full, st & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < TW / 16; ++ks)
-          umma_ts(tmem + COL_DV, tmem + COL_P + ks * 8, umma_desc_sw128(dy_addr + ks * 2048, 8192, 1024), idesc_o,
-                  (st > 0 || ks > 0) ? 1u : 0u);
-#pragma unroll
-        for (int ks = 0; ks < TW / 16; ++ks)
-          umma_ts(tmem + COL_DK, tmem + COL_DS + ks * 8, umma_desc_sw128(q_addr + ks * 2048, 8192, 1024), idesc_o,
-                  (st > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&r_empty[sg]);
-        if (st == n_steps - 1) umma_commit(&attn_done);
-      }
-      if (ok && has_state) {
-        // 128 expanded entries against two state blocks (one ring stage) per item: eight products
-        // per pair of waits and commits keep this thread off the critical path
-        for (int k = 0; k < p.nblk / 2 && ok; ++k) {
-          const int s = k % NS, ph = (k / NS) & 1;
-          const int g = n_steps + k, rs = g % NR;
-          ok = mbar_wait(&a_full[s], ph, &abort_flag) && mbar_wait(&r_full[rs], (g / NR) & 1, &abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t z_addr = smem_u32(smR + rs * R_BYTES);
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            umma_ts(tmem + COL_DV, tmem + COL_A + s * 64 + ks * 8,
-                    umma_desc_sw128(z_addr + (ks >> 2) * Z_BYTES + (ks & 3) * 2048, 8192, 1024), idesc_o, 1u);
-          // one commit per item: it frees the ring stage for the TMA thread and, two items on, the
-          // tensor-memory slot for the expansion warps
-          umma_commit(&r_empty[rs]);
+      // positions in the rotation: group and ring stage with the phases of op_full and r_full there, of the next
+      // operand and of the next scores, which run NG operands ahead
+      struct Pos {
+        int g = 0, s = 0;
+        uint32_t g_ph = 0, s_ph = 0;
+        __device__ __forceinline__ void stage() {
+          if (++s == NR) s = 0, s_ph ^= 1;
         }
+        __device__ __forceinline__ void group() {
+          if (++g == NG) g = 0, g_ph ^= 1;
+        }
+      } at, sc;
+      // descriptors of stage 0; a stage on is R_BYTES >> 4 on in the address field
+      const uint32_t ring = smem_u32(smR);
+      const uint64_t d_qk = umma_desc_sw128(ring, 16, 1024), d_dk = umma_desc_sw128(ring + QD_BYTES, 16, 1024),
+                     d_qm = umma_desc_sw128(ring, 8192, 1024), d_dm = umma_desc_sw128(ring + QD_BYTES, 8192, 1024);
+      bool ok = true;
+      dim3 cta = blockIdx;
+      int tiles = 0;
+      for (int it = 0; ok; ++it) {
+        const DkvTile w(p, cta);
+        if (!w.empty) {
+          const uint32_t kv = smem_u32(smKV + (it & 1) * 2 * TILE_BYTES);
+          const uint64_t d_k = umma_desc_sw128(kv, 16, 1024), d_v = umma_desc_sw128(kv + TILE_BYTES, 16, 1024);
+          ok = mbar_wait(&kv_full[it & 1], (it >> 1) & 1, &abort_flag);
+          auto issue_scores = [&]() -> bool {
+            if (!mbar_wait(&r_full[sc.s], sc.s_ph, &abort_flag)) return false;
+            tc_fence_after();
+            const uint32_t off = (uint32_t)sc.s * (R_BYTES >> 4), cb = tmem + col_b(sc.g);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) umma_ss(cb, d_k + 2 * ks, d_qk + off + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) umma_ss(cb + 64, d_v + 2 * ks, d_dk + off + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+            umma_commit(&s_full[sc.g]);
+            sc.stage();
+            sc.group();
+            return true;
+          };
+          sc = at;
+          for (int st = 0; st < min(w.n_steps, NG) && ok; ++st) ok = issue_scores();
+          // the accumulators of the tile before have been read out
+          if (ok && tiles > 0) ok = mbar_wait(&acc_free, (tiles - 1) & 1, &abort_flag);
+          for (int st = 0; st < w.n_steps && ok; ++st) {
+            ok = mbar_wait(&op_full[at.g], at.g_ph, &abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t off = (uint32_t)at.s * (R_BYTES >> 4), cb = tmem + col_b(at.g);
+#pragma unroll
+            for (int ks = 0; ks < TW / 16; ++ks)
+              umma_ts(tmem + COL_DV, cb + ks * 8, d_dm + off + ks * (2048 >> 4), idesc_o, (st > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+            for (int ks = 0; ks < TW / 16; ++ks)
+              umma_ts(tmem + COL_DK, cb + 64 + ks * 8, d_qm + off + ks * (2048 >> 4), idesc_o, (st > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(&r_empty[at.s]);
+            at.stage();
+            at.group();
+            // the group's next scores, into the buffer that the products just issued read (products execute in order)
+            if (st + NG < w.n_steps) ok = issue_scores();
+          }
+          for (int k = 0; k < w.nI && ok; ++k) {
+            // 256 expanded entries against four state blocks (two ring stages)
+            ok = mbar_wait(&op_full[at.g], at.g_ph, &abort_flag);
+            for (int hf = 0; hf < 2 && ok; ++hf) {
+              ok = mbar_wait(&r_full[at.s], at.s_ph, &abort_flag);
+              if (!ok) break;
+              tc_fence_after();
+              const uint32_t off = (uint32_t)at.s * (R_BYTES >> 4), cb = tmem + col_b(at.g) + 64 * hf;
+#pragma unroll
+              for (int ks = 0; ks < 8; ++ks)
+                umma_ts(tmem + COL_DV, cb + ks * 8, d_qm + off + (ks >> 2) * (Z_BYTES >> 4) + (ks & 3) * (2048 >> 4), idesc_o, 1u);
+              umma_commit(&r_empty[at.s]);
+              at.stage();
+            }
+            at.group();
+          }
+          if (ok) umma_commit(&acc_full);
+          ++tiles;
+        }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
-      if (ok) umma_commit(&acc_done);
     }
   } else {
-    const int row = row0 + tid;  // key index inside the chunk
-    const bool row_valid = row < c;
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    const uint32_t tmem = tmem_base_s;
+    const int grp = warp >> 2, r = tid & 127;  // row group, key row inside the tile
+    const int wrow = (warp & 3) * 32;
+    const uint32_t lane_addr = (uint32_t)wrow << 16;
+    const uint32_t cb = tmem + lane_addr + col_b(grp);
     const bool gated = p.a != nullptr;
-    const size_t tok_base = (size_t)batch * p.t + tok_chunk;
-    const float* a_chunk = gated ? p.a + tok_base * p.h + kvhead : nullptr;
-    const float a_j = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
-    const float s2 = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
-    float da2 = 0.f;  // twice the row sum of p * dp
+    const float sdeg = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
     bool ok = true;
-    // per-query values of the next step, loaded one step ahead by the first TW threads
-    float av_n = 0.f, r_n = 0.f, dl_n = 0.f, l_n = 1.f;
-    auto load_cols = [&](int st) {
-      if (tid < TW) {
-        const int qp0 = (qt0 + st / ratio) * TW, qh = kvhead * ratio + st % ratio;
-        const int qp = qp0 + tid;
-        const bool v = qp < c;
-        av_n = (gated && v) ? a_chunk[(size_t)qp * p.h] : 0.f;
-        r_n = gated ? a_chunk[(size_t)qp0 * p.h] : 0.f;
-        dl_n = v ? p.dl[(tok_base + qp) * p.hq + qh] : 0.f;
-        l_n = v ? p.l[(tok_base + qp) * p.hq + qh] : 1.f;
-      }
+    dim3 cta = blockIdx;
+    int tiles = 0, own = 0;    // tiles with rows, operands of this group so far
+    int grp0 = 0, g0 = 0;      // group of the tile's first operand, ring stages before the tile
+    int last_g = -1;           // last ring stage that this group's latest operand was multiplied with
+    uint32_t s_ph = 0, row_ph = 0;
+    // the row warps meet; bounded like every wait
+    auto meet = [&]() {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&rows);
+      if (ok) ok = mbar_wait(&rows, row_ph, &abort_flag);
+      row_ph ^= 1;
     };
-    if (n_steps > 0) load_cols(0);
-    for (int st = 0; st < n_steps; ++st) {
-      const int I = qt0 + st / ratio;
-      const int qp0 = I * TW;
-      const int sb = st & 1;
-      if (tid < TW) {
-        const bool v = qp0 + tid < c;
-        const float il = v ? safe_recip(l_n) : 0.f;
-        sm_aq[sb][tid] = av_n;
-        sm_dl[sb][tid] = dl_n;
-        sm_il[sb][tid] = il;
-        sm_hl[sb][tid] = (1.f / DEG) * il;
-        sm_fq[sb][tid] = v ? __expf(av_n - r_n) : 0.f;
-        const bool wide = __any_sync(0xffffffffu, (av_n - r_n) > 80.f);
-        if (lane == 0) sm_wide[sb][warp] = wide;
-        if (tid == 0) sm_r[sb] = r_n;
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (st + 1 < n_steps) load_cols(st + 1);  // in flight while this step is computed
-      ok = mbar_wait(&sp_full, st & 1, &abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
-      // key and per query instead of one per pair (both exponents <= 0 off the diagonal for gates
-      // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps whose queries all
-      // come after this warp's keys need no mask; a warp whose keys all come after the step's
-      // queries writes zeros without reading the scores.
-      const int wrow0 = row0 + (warp << 5);
-      if (qp0 + TW - 1 < wrow0 || wrow0 >= c) {
-        uint32_t z[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) z[j] = 0u;
-        tmem_st16(tmem + lane_addr + COL_P, z);
-        tmem_st16(tmem + lane_addr + COL_P + 16, z);
-        tmem_st16(tmem + lane_addr + COL_DS, z);
-        tmem_st16(tmem + lane_addr + COL_DS + 16, z);
-      } else {
-        const float r = sm_r[sb];
-        const bool mask = (wrow0 + 31 > qp0) || (wrow0 + 31 >= c);
-        const bool sep = (qp0 + TW - 1 < c) && !(sm_wide[sb][0] | sm_wide[sb][1]) &&
-                         !__any_sync(0xffffffffu, (r - a_j) > 80.f);
-        const float c_j = sep ? (float)DEG * s2 * __expf(r - a_j) : (float)DEG * s2;
-        const int lo = row_valid ? row - qp0 : TW;  // first query column this key keeps
-        const int hi = c - 1 - qp0;                 // last column inside the chunk
-#pragma unroll 1
-        for (int q4 = 0; q4 < TW / 32; ++q4) {
-          uint32_t sv[32], pv[32], pk[16], dk[16];
-          tmem_ld32(tmem + lane_addr + COL_S + q4 * 32, sv);
-          tmem_ld32(tmem + lane_addr + COL_DP + q4 * 32, pv);
-          tmem_wait_ld();
-          const float* il = sm_il[sb] + q4 * 32;
-          const float* hl = sm_hl[sb] + q4 * 32;
-          const float* dl = sm_dl[sb] + q4 * 32;
-          const int lo4 = lo - q4 * 32, hi4 = hi - q4 * 32;
-          if (sep) {
-            if (mask) dkv_half<T, DEG, true, true>(sv, pv, sm_fq[sb] + q4 * 32, il, hl, dl, c_j, a_j, lo4, hi4, pk, dk, da2);
-            else dkv_half<T, DEG, true, false>(sv, pv, sm_fq[sb] + q4 * 32, il, hl, dl, c_j, a_j, lo4, hi4, pk, dk, da2);
-          } else {
-            dkv_half<T, DEG, false, true>(sv, pv, sm_aq[sb] + q4 * 32, il, hl, dl, c_j, a_j, lo4, hi4, pk, dk, da2);
-          }
-          tmem_st16(tmem + lane_addr + COL_P + q4 * 16, pk);
-          tmem_st16(tmem + lane_addr + COL_DS + q4 * 16, dk);
-        }
-      }
+    auto operand_written = [&](int g) {
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&pd_full);
-    }
-
-    if (ok && has_state) {
-      ok = mbar_wait(&kv_full, 0, &abort_flag);
-      float f = 1.f;
-      if (gated) {
-        const float A = p.A[(batch * p.n_chunks + chunk) * p.h + kvhead];
-        f = __expf(0.5f * (A - a_j));
-      }
-      uint32_t k2[32];
+      if (lane == 0) mbar_arrive(&op_full[grp]);
+      last_g = g;
+      ++own;
+    };
+    for (int it = 0; ok; ++it) {
+      const DkvTile w(p, cta);
+      if (!w.empty) {
+        uint8_t* smK = smKV + (it & 1) * 2 * TILE_BYTES;
+        const int row = w.row0 + r;  // key index inside the chunk
+        const bool row_valid = row < w.c;
+        const size_t tok_base = (size_t)w.batch * p.t + w.tok_chunk;
+        const float* a_chunk = gated ? p.a + tok_base * p.h + w.kvhead : nullptr;
+        const float a_j = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
+        float da = 0.f;  // deg times the row sum of p * dp
+        // per-query values of this warp's next step, two per lane, loaded one step ahead
+        float av[2], dlv[2], lv[2], r_n = 0.f;
+        auto load_cols = [&](int st) {
+          const int qp0 = (w.qt0 + st / ratio) * TW, qh = w.kvhead * ratio + st % ratio;
+          r_n = gated ? a_chunk[(size_t)qp0 * p.h] : 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(smK + swz128(tid, j));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 x = Pack2<T>::to_f32(w[k]);
-          k2[4 * j + k] = Pack2<T>::from_f32(x.x * f, x.y * f);
-        }
-      }
-      if (ok && n_steps > 0) ok = mbar_wait(&attn_done, 0, &abort_flag);
-      tc_fence_after();
-      // the discounted row goes back to its own slot of the key tile (first factors are fetched
-      // by a runtime index); the attention products that read the tile have completed
-      if (ok) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          *reinterpret_cast<uint4*>(smK + swz128(tid, j)) = make_uint4(k2[4 * j], k2[4 * j + 1], k2[4 * j + 2], k2[4 * j + 3]);
-      }
-      int k = 0;
-      static_for<0, HD / 16>([&](auto yc) {
-        constexpr int Y = decltype(yc)::value;
-        if (16 * Y >= p.d) return;
-#pragma unroll 1
-        for (int a0 = 0; a0 < 16 * (Y + 1); a0 += 8, ++k) {
-          uint32_t r0[32], r1[32];
-          uint32_t x2[8];
-          expand_second(smK, tid, Y, x2);
-          expand_stage<T>(smK, tid, a0, x2, r0);
-          expand_stage<T>(smK, tid, a0 + 4, x2, r1);
-          const int s = k % NS;
-          if (ok && k >= NS) {
-            // the slot was last used by item k - NS, whose completion is reported on its ring stage's barrier
-            const int g2 = n_steps + k - NS;
-            ok = mbar_wait(&r_empty[g2 % NR], (g2 / NR) & 1, &abort_flag);
+          for (int k = 0; k < 2; ++k) {
+            const int qp = qp0 + lane + 32 * k;
+            const bool v = qp < w.c;
+            av[k] = !v ? -1e30f : gated ? a_chunk[(size_t)qp * p.h] : 0.f;
+            dlv[k] = v ? p.dl[(tok_base + qp) * p.hq + qh] : 0.f;
+            lv[k] = v ? p.l[(tok_base + qp) * p.hq + qh] : 0.f;  // 0: no such query
           }
-          if (ok) {
-            tc_fence_after();
-            tmem_st32(tmem + lane_addr + COL_A + s * 64, r0);
-            tmem_st32(tmem + lane_addr + COL_A + s * 64 + 32, r1);
-            tmem_wait_st();
-            tc_fence_before();
+        };
+        const int first = (grp - grp0 + NG) % NG;  // this group's first operand in the tile
+        if (first < w.n_steps) load_cols(first);
+        for (int st = first; st < w.n_steps && ok; st += NG) {
+          const int qp0 = (w.qt0 + st / ratio) * TW;
+          float* fq = sm_fq[warp][own & 1];
+          float* de = sm_de[warp][own & 1];
+          const float rs = r_n;
+          // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
+          // key and per query instead of one per pair (both exponents <= 0 off the diagonal for gates
+          // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps whose queries all
+          // come after this warp's keys need no mask; a warp whose keys all come after the step's
+          // queries writes zeros without reading the scores.
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(fmaxf(av[0], av[1]) - rs, rs - a_j) > 80.f);
+          const float c_j = sep ? sdeg * __expf(rs - a_j) : sdeg;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const bool v = qp0 + lane + 32 * k < w.c;
+            const float il = v ? safe_recip(lv[k]) : 0.f;
+            fq[lane + 32 * k] = (sep && v) ? il * __expf(av[k] - rs) : il;
+            de[lane + 32 * k] = (float)DEG * dlv[k] * lv[k];
+            if (!sep) sm_aq[warp][lane + 32 * k] = av[k];
           }
           __syncwarp();
-          if (ok && lane == 0) mbar_arrive(&a_full[s]);
-        }
-      });
-    }
-
-    if (ok) ok = mbar_wait(&acc_done, 0, &abort_flag);
-    tc_fence_after();
-    if (ok) {
-      uint32_t acc[64];
-      const size_t tok = tok_base + row;
-      // dV
-      tmem_ld32(tmem + lane_addr + COL_DV, acc);
-      tmem_ld32(tmem + lane_addr + COL_DV + 32, acc + 32);
-      tmem_wait_ld();
-      if (row_valid) {
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dV) + (tok * p.h + kvhead) * p.d);
+          if (st + NG < w.n_steps) load_cols(st + NG);  // in flight while this step is computed
+          ok = mbar_wait(&s_full[grp], s_ph, &abort_flag);
+          s_ph ^= 1;
+          if (!ok) break;
+          tc_fence_after();
+          const int wrow0 = w.row0 + wrow;
+          if (qp0 + TW - 1 < wrow0 || wrow0 >= w.c) {
+            uint32_t z[16];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (8 * j >= p.d) break;
-          uint4 v;
-          v.x = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 0]), __uint_as_float(acc[8 * j + 1]));
-          v.y = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3]));
-          v.z = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 4]), __uint_as_float(acc[8 * j + 5]));
-          v.w = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7]));
-          dst[j] = v;
-        }
-      }
-      // dK
-      tmem_ld32(tmem + lane_addr + COL_DK, acc);
-      tmem_ld32(tmem + lane_addr + COL_DK + 32, acc + 32);
-      tmem_wait_ld();
-      if (row_valid) {
-        const float4* st = p.dk_state ? reinterpret_cast<const float4*>(p.dk_state + (tok * p.h + kvhead) * p.d)
-                                      : nullptr;
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dK) + (tok * p.h + kvhead) * p.d);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (8 * j >= p.d) break;
-          float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-          if (st) {
-            s0 = st[2 * j];
-            s1 = st[2 * j + 1];
+            for (int j = 0; j < 16; ++j) z[j] = 0u;
+            tmem_st16(cb, z);
+            tmem_st16(cb + 16, z);
+            tmem_st16(cb + 64, z);
+            tmem_st16(cb + 80, z);
+          } else {
+            const bool mask = (wrow0 + 31 > qp0) || (wrow0 + 31 >= w.c);
+            const int lo = row_valid ? row - qp0 : TW;  // first query column this key keeps
+            if (!sep) dkv_step<T, DEG, false, true>(cb, fq, de, sm_aq[warp], c_j, a_j, lo, da);
+            else if (mask) dkv_step<T, DEG, true, true>(cb, fq, de, fq, c_j, a_j, lo, da);
+            else dkv_step<T, DEG, true, false>(cb, fq, de, fq, c_j, a_j, lo, da);
           }
-          uint4 v;
-          v.x = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 0]) + s0.x, __uint_as_float(acc[8 * j + 1]) + s0.y);
-          v.y = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 2]) + s0.z, __uint_as_float(acc[8 * j + 3]) + s0.w);
-          v.z = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 4]) + s1.x, __uint_as_float(acc[8 * j + 5]) + s1.y);
-          v.w = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 6]) + s1.z, __uint_as_float(acc[8 * j + 7]) + s1.w);
-          dst[j] = v;
+          operand_written(g0 + st);
         }
-        p.da_k[tok * p.h + kvhead] = (-1.f / DEG) * da2;
+
+        if (w.nI > 0) {
+          meet();  // every score product of the tile has completed: the key tile may be rewritten
+          // The discounted key takes the row's place in the key tile, where the expansion fetches its factors by a
+          // runtime index; each group does every third 16-byte piece.
+          if (ok) ok = mbar_wait(&kv_full[it & 1], (it >> 1) & 1, &abort_flag);
+          float f = 1.f;
+          if (gated) f = __expf(0.5f * (p.A[(w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead] - a_j));
+          for (int j = grp; j < 8; j += NG) {
+            uint4* slot = reinterpret_cast<uint4*>(smK + swz128(r, j));
+            const uint4 v = *slot;
+            uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float2 f2 = Pack2<T>::to_f32(x[k]);
+              x[k] = Pack2<T>::from_f32(f2.x * f, f2.y * f);
+            }
+            *slot = make_uint4(x[0], x[1], x[2], x[3]);
+          }
+          meet();
+          // items of 16 first factors x 16 second factors: block Y of second factors has Y + 1 of them
+          int k = (grp - (grp0 + w.n_steps) % NG + NG) % NG;
+          for (; k < w.nI; k += NG) {
+            const int Y = (k > 0) + (k > 2) + (k > 5);
+            const int a0 = 16 * (k - Y * (Y + 1) / 2);
+            uint32_t x2[8], x[32];
+            expand_second(smK, r, Y, x2);
+            expand_stage<T>(smK, r, a0, x2, x);
+            // the buffer is free once the products that read its last operand have completed
+            if (ok && last_g >= 0) ok = mbar_wait(&r_empty[last_g % NR], (last_g / NR) & 1, &abort_flag);
+            tc_fence_after();
+            if (ok) tmem_st32(cb, x);
+#pragma unroll
+            for (int q = 1; q < 4; ++q) {
+              expand_stage<T>(smK, r, a0 + 4 * q, x2, x);
+              if (ok) tmem_st32(cb + 32 * q, x);
+            }
+            if (ok) operand_written(g0 + w.n_steps + 2 * k + 1);
+          }
+        }
+        // the key and value tiles may be refilled (their last reads come before the async proxy's writes; the products
+        // that read them have completed with the scores)
+        fence_async_smem();
+        sm_da[tiles & 1][grp][r] = da;
+        meet();
+        if (lane == 0) mbar_arrive(&kv_free[it & 1]);
+
+        const size_t tok = tok_base + row;
+        const float* st = p.dk_state ? p.dk_state + (tok * p.h + w.kvhead) * p.d : nullptr;
+        if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
+        tc_fence_after();
+        // the groups share the write-out: 16 of the 64 columns of dV (units 0-3) or dK (units 4-7) at a time
+        for (int unit = grp; ok && unit < 8; unit += NG) {
+          const int c0 = 16 * (unit & 3);
+          uint32_t acc[16];
+          tmem_ld16(tmem + lane_addr + 16 * unit, acc);
+          const bool mine = row_valid && c0 < p.d;
+          float4 add[4];
+          if (unit >= 4 && st != nullptr && mine) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) add[j] = reinterpret_cast<const float4*>(st + c0)[j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) add[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+          tmem_wait_ld();
+          if (mine) {
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + add[j].x, __uint_as_float(acc[4 * j + 1]) + add[j].y);
+              v[2 * j + 1] =
+                  Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + add[j].z, __uint_as_float(acc[4 * j + 3]) + add[j].w);
+            }
+            T* dst = static_cast<T*>(unit < 4 ? p.dV : p.dK) + (tok * p.h + w.kvhead) * p.d + c0;
+            if (p.aligned32) {
+              st_global_v8(dst, v);
+            } else {
+              reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+              reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_free);
+        if (grp == 0 && row_valid) {
+          const float sum = (sm_da[tiles & 1][0][r] + sm_da[tiles & 1][1][r]) + sm_da[tiles & 1][2][r];
+          p.da_k[tok * p.h + w.kvhead] = (-1.f / DEG) * sum;
+        }
+        grp0 = (grp0 + w.n_steps + w.nI) % NG;
+        g0 += w.n_steps + 2 * w.nI;
+        ++tiles;
+      } else {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&kv_free[it & 1]);
       }
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
     }
   }
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && abort_flag) *p.status = ST_TIMEOUT;
-  if (warp == 0) tmem_dealloc(tmem, dkv::TMEM_COLS);
+  if (warp == 0) tmem_dealloc(tmem_base_s, TMEM_COLS);
 }
 
 }  // namespace pr
@@ -495,6 +596,7 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   p.dk_state = dk_state;
   p.dK = dK;
   p.dV = dV;
+  p.aligned32 = ((reinterpret_cast<uintptr_t>(dK) | reinterpret_cast<uintptr_t>(dV)) & 31u) == 0;
   p.da_k = da_k;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;
@@ -517,13 +619,12 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   } else {
     tm_ds = tm_q;
   }
-  const size_t smem = 1024 + 2 * TILE_BYTES + NR * R_BYTES;
   dim3 grid(p.tiles_per_chunk * p.n_chunks, h, b);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define PR_LAUNCH_DKV(TT, DG)                                                                                      \
   do {                                                                                                             \
-    PR_SMEM_ATTR((chunk_dkv_kernel<TT, DG>), smem, device, true);                                                   \
-    chunk_dkv_kernel<TT, DG><<<grid, THREADS, smem, s>>>(p, tm_k, tm_v, tm_q, tm_dy, tm_ds);                         \
+    PR_SMEM_ATTR((chunk_dkv_kernel<TT, DG>), SMEM, device, true);                                                   \
+    chunk_dkv_kernel<TT, DG><<<grid, THREADS, SMEM, s>>>(p, tm_k, tm_v, tm_q, tm_dy, tm_ds);                         \
   } while (0)
   if (dtype == PR_BF16) {
     if (deg == 4) PR_LAUNCH_DKV(__nv_bfloat16, 4); else PR_LAUNCH_DKV(__nv_bfloat16, 2);

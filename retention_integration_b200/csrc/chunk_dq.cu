@@ -2,9 +2,7 @@
 // state-path query gradient (the reference's attn_bwd_dq, retention/_attention/triton.py:496-603,
 // for deg = 2 without the division by the score).
 //
-// One CTA owns 128 query rows of one (batch, chunk, query head); thread = row.  For every
-// tile of 64 keys up to the diagonal (tiles double-buffered in shared memory; 256 tensor
-// memory columns, so two CTAs share an SM and hide each other's waits):
+// A tile is 128 query rows of one (batch, chunk, query head).  For every tile of 64 keys up to the diagonal:
 //     S  = Q K_J^T,  dP = dO V_J^T                      (tensor cores, fp32 in tensor memory)
 //     p  = (s S)^2 e^{a_i-a_j},  dp = dP / l_i + dl_i,  e = p dp,  dS = 2 s^2 S e^{a_i-a_j} dp
 //     dQ += dS K_J                                      (A = dS from tensor memory)
@@ -13,6 +11,12 @@
 // 1/l_i is applied in fp32, so the cancellation between dP / l and dl (exact for a row with a
 // single key) is not spoiled by a 16-bit rounding of dO / l.  The epilogue adds the
 // state-path gradient (fp32, from the expansion-gradient kernel) and writes dQ.
+//
+// Three groups of four warps own the query rows, one row per thread in each group, and take the steps in turn, each in
+// its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma.  One persistent CTA per SM takes over
+// tile after tile (ClcRing).  Bound by the latency of a step's chain (products, barrier, tensor-memory loads,
+// arithmetic, stores, barrier, product); two CTAs per SM with one row group each overlapped two of them and spent
+// a third of the time on set-up and write-out: 232 -> NEW us at b1 t65536 h8 with chunks of 1024.
 #include "host.cuh"
 #include "sm100.cuh"
 
@@ -20,13 +24,18 @@ namespace pr {
 
 namespace dq {
 constexpr int HD = 64;
-constexpr int THREADS = 224;             // warps 0-3 rows, 4 TMA, 5 and 6 issue tcgen05.mma
+constexpr int NG = 3;                    // row groups, each with its own buffer in tensor memory
+constexpr int NR = 6;                    // shared-memory ring: stages of a key and a value tile
+constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
+constexpr int THREADS = 32 * (W_MMA + 1);
 constexpr int TILE_BYTES = 128 * 128;   // 128 query rows x 64 features
 constexpr int TW = 64;                  // keys per step
 constexpr int KV_BYTES = TW * 128;      // one key or value tile
-constexpr int NKV = 4;                  // key/value tiles in flight
-constexpr uint32_t TMEM_COLS = 256;     // two CTAs per SM
-constexpr uint32_t COL_S = 0, COL_DP = 128, COL_ACC = 192;  // S double-buffered (2 x 64); dS overwrites its S
+constexpr int R_BYTES = 2 * KV_BYTES;
+constexpr size_t SMEM = 1024 + 4 * TILE_BYTES + NR * R_BYTES;
+constexpr uint32_t TMEM_COLS = 512;
+// the accumulator, then a buffer of 128 columns per group: S, overwritten by dS (its first half), and dP
+__device__ __forceinline__ constexpr uint32_t col_b(int grp) { return 128u + 128u * (uint32_t)grp; }
 }  // namespace dq
 
 struct ChunkDqParams {
@@ -36,25 +45,46 @@ struct ChunkDqParams {
   const float* a;         // [b, t, h] or null
   const float* dl;        // [b, t, hq]
   const float* l;         // [b, t, hq] row sums saved by the forward
-  const float* dq_state;  // [b, t, hq, 64] fp32 or null
-  void* dQ;               // [b, t, hq, 64]
+  const float* dq_state;  // [b, t, hq, d] fp32 or null
+  void* dQ;               // [b, t, hq, d]
+  int aligned32;          // dQ starts on a 32-byte boundary
   float* da_q;            // [b, t, hq]
   int* status;
 };
 
-// One 32-column half of a step for one row: dS = 2 s^2 S g dp into `pk`, row sum of dS * S into da2.
-// SEP: the gate factor is c_i * fk[col] (c_i carries 2 s^2); otherwise 2 s^2 e^{a_i - ak[col]} per pair.
+struct DqTile {
+  int chunk, qhead, kvhead, batch, row0, tok_chunk;
+  int c;        // tokens of the chunk
+  int nJ;       // steps: key tiles up to the diagonal
+  bool empty;   // past the end of a shorter last chunk
+  __device__ __forceinline__ DqTile(const ChunkDqParams& p, const dim3& cta) {
+    const int x = (int)cta.x;
+    // the longest tiles of a head first
+    const int tile_i = p.tiles_per_chunk - 1 - x % p.tiles_per_chunk;
+    chunk = x / p.tiles_per_chunk;
+    qhead = (int)cta.y;
+    batch = (int)cta.z;
+    kvhead = qhead / (p.hq / p.h);
+    row0 = tile_i * 128;
+    tok_chunk = chunk * p.c;
+    c = min(p.c, p.t - tok_chunk);
+    empty = row0 >= c;
+    nJ = empty ? 0 : min(c - 1, row0 + 127) / dq::TW + 1;
+  }
+};
+
+// One 16-column piece of a step for one row: dS = deg s^deg S^(deg-1) g dp into `pk`, row sum of dS * S into acc.
+// SEP: the gate factor is c_i * fk[col] (c_i carries deg s^deg); otherwise c_i e^{a_i - ak[col]} per pair.
 // MASK: columns beyond `lim` (the row's own position, relative to the step) are dropped.
 template <typename T, int DEG, bool SEP, bool MASK>
-__device__ __forceinline__ void dq_half(const uint32_t (&sv)[32], const uint32_t (&pv)[32], const float* __restrict__ fk,
-                                        float c_i, float a_i, float inv_l, float dl_i, int lim, uint32_t (&pk)[16],
-                                        float& da2) {
+__device__ __forceinline__ void dq_piece(const uint32_t (&sv)[16], const uint32_t (&pv)[16], const float* __restrict__ fk,
+                                         float c_i, float a_i, float inv_l, float dl_i, int lim, uint32_t (&pk)[8],
+                                         float2& acc) {
   // two columns per instruction: packed fp32 multiplies and FMAs
   const float4* f4 = reinterpret_cast<const float4*>(fk);
   const float2 c2 = make_float2(c_i, c_i), il2 = make_float2(inv_l, inv_l), dl2 = make_float2(dl_i, dl_i);
-  float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int j = 0; j < 32; j += 4) {
+  for (int j = 0; j < 16; j += 4) {
     const float4 f = f4[j >> 2];
     const float2 fv[2] = {make_float2(f.x, f.y), make_float2(f.z, f.w)};
 #pragma unroll
@@ -79,265 +109,318 @@ __device__ __forceinline__ void dq_half(const uint32_t (&sv)[32], const uint32_t
       pk[col >> 1] = Pack2<T>::from_f32(ds.x, ds.y);
     }
   }
-  da2 += acc.x + acc.y;
+}
+
+// A whole step: the loads of the next piece are in flight while one is computed.
+template <typename T, int DEG, bool SEP, bool MASK>
+__device__ __forceinline__ void dq_step(uint32_t cb, const float* __restrict__ fk, float c_i, float a_i, float inv_l,
+                                        float dl_i, int lim, float& da) {
+  uint32_t sv[2][16], pv[2][16], pk[8];
+  float2 acc = make_float2(0.f, 0.f);
+  tmem_ld16(cb, sv[0]);
+  tmem_ld16(cb + 64, pv[0]);
+#pragma unroll
+  for (int q = 0; q < dq::TW / 16; ++q) {
+    tmem_wait_ld();
+    if (q + 1 < dq::TW / 16) {
+      tmem_ld16(cb + (q + 1) * 16, sv[(q + 1) & 1]);
+      tmem_ld16(cb + 64 + (q + 1) * 16, pv[(q + 1) & 1]);
+    }
+    dq_piece<T, DEG, SEP, MASK>(sv[q & 1], pv[q & 1], fk + q * 16, c_i, a_i, inv_l, dl_i, lim - q * 16, pk, acc);
+    tmem_st8(cb + q * 8, pk);
+  }
+  da += acc.x + acc.y;
 }
 
 template <typename T, int DEG>
-__global__ void __launch_bounds__(dq::THREADS, 2)
+__global__ void __launch_bounds__(dq::THREADS, 1)
 chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
                 const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_st) {
+                const __grid_constant__ CUtensorMap tm_v) {
   using namespace dq;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t q_full, kv_full[NKV], kv_empty[NKV], sp_full, ds_full, acc_done, qdy_free, st_full, dq_done[2];
+  // q_*: the query and dO tiles, two pairs in flight.  r_*: the ring of key and value tiles.  s_full: S and dP in a
+  // group's buffer; op_full: the group has written dS.  acc_full / acc_free: accumulator complete / read out; rows: the
+  // row warps meet.
+  __shared__ uint64_t q_full[2], q_free[2], r_full[NR], r_empty[NR], s_full[NG], op_full[NG], acc_full, acc_free, rows;
+  __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  __shared__ __align__(16) float sm_ak[2][TW];  // gate sums a_j of the step's keys
-  __shared__ __align__(16) float sm_fk[2][TW];  // e^{r - a_j}, r = gate sum at the step's last key
-  __shared__ float sm_r[2];
-  __shared__ int sm_wide[2][2];                 // a loader warp saw r - a_j > 80 (overflow guard)
+  // Per warp and step parity, each warp its own copy: e^{r - a_j} of the step's keys, r = gate sum at its last key (or
+  // a_j itself where the exponentials do not separate).
+  __shared__ __align__(16) float sm_fk[4 * NG][2][TW];
+  __shared__ float sm_da[2][NG][128];
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
-  uint8_t* smQ = sm;
-  uint8_t* smDY = smQ + TILE_BYTES;
-  uint8_t* smK = smDY + TILE_BYTES;      // NKV stages x KV_BYTES
-  uint8_t* smV = smK + NKV * KV_BYTES;   // NKV stages x KV_BYTES
+  uint8_t* smQD = sm;                    // 2 x (query tile, dO tile)
+  uint8_t* smR = smQD + 4 * TILE_BYTES;  // NR x R_BYTES
 
-  const int tile_i = blockIdx.x % p.tiles_per_chunk;
-  const int chunk = blockIdx.x / p.tiles_per_chunk;
-  const int qhead = blockIdx.y, batch = blockIdx.z;
-  const int kvhead = qhead / (p.hq / p.h);
-  const int row0 = tile_i * 128;
-  const int c = min(p.c, p.t - chunk * p.c);  // tokens of this chunk
-  if (row0 >= c) return;
-  const int nJ = min(c - 1, row0 + 127) / TW + 1;
-  const int tok_chunk = chunk * p.c;
-  const bool has_st = p.dq_state != nullptr;
-
-  if (tid == 0) {
-    abort_flag = 0;
-    mbar_init(&q_full, 1);
-    for (int s = 0; s < NKV; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
-    }
-    mbar_init(&sp_full, 1);
-    mbar_init(&ds_full, 4);
-    mbar_init(&acc_done, 1);
-    mbar_init(&qdy_free, 1);
-    mbar_init(&st_full, 1);
-    mbar_init(&dq_done[0], 1);
-    mbar_init(&dq_done[1], 1);
-    fence_mbar_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(&tmem_base_s, TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
-
-  if (warp == 4) {
+  if (warp == W_TMA) {
     if (elect_one()) {
-      mbar_expect_tx(&q_full, 2 * TILE_BYTES);
-      tma_load_4d(smQ, &tm_q, &q_full, 0, qhead, tok_chunk + row0, batch);
-      tma_load_4d(smDY, &tm_dy, &q_full, 0, qhead, tok_chunk + row0, batch);
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_dy);
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+      abort_flag = 0;
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(&q_full[s], 1);
+        mbar_init(&q_free[s], 1);
+      }
+      for (int s = 0; s < NR; ++s) {
+        mbar_init(&r_full[s], 1);
+        mbar_init(&r_empty[s], 1);
+      }
+      for (int s = 0; s < NG; ++s) {
+        mbar_init(&s_full[s], 1);
+        mbar_init(&op_full[s], 4);
+      }
+      mbar_init(&acc_full, 1);
+      mbar_init(&acc_free, 4 * NG);
+      mbar_init(&rows, 4 * NG);
+      clc_init(&clc, 4 * NG + 2);
+      fence_mbar_init();
+    }
+    __syncwarp();
+    named_bar_arrive(1, THREADS);  // the first loads need not wait for the tensor memory
+  } else {
+    if (warp == 0) {
+      tmem_alloc(&tmem_base_s, TMEM_COLS);
+      tmem_relinquish();
+    }
+    tc_fence_before();
+    named_bar_sync(1, THREADS);
+    tc_fence_after();
+  }
+
+  if (warp == W_TMA) {
+    if (elect_one()) {
       bool ok = true;
-      for (int J = 0; J < nJ; ++J) {
-        const int s = J % NKV, ph = (J / NKV) & 1;
-        if (!(ok = mbar_wait(&kv_empty[s], ph ^ 1, &abort_flag))) break;
-        mbar_expect_tx(&kv_full[s], 2 * KV_BYTES);
-        tma_load_4d(smK + s * KV_BYTES, &tm_k, &kv_full[s], 0, kvhead, tok_chunk + J * TW, batch);
-        tma_load_4d(smV + s * KV_BYTES, &tm_v, &kv_full[s], 0, kvhead, tok_chunk + J * TW, batch);
-      }
-      // The query and dO tiles are dead once the last S and dP are computed: the fp32
-      // state-path gradient of these rows (two 32-column halves) takes their place.
-      if (ok && has_st && mbar_wait(&qdy_free, 0, &abort_flag)) {
-        mbar_expect_tx(&st_full, 2 * TILE_BYTES);
-        tma_load_4d(smQ, &tm_st, &st_full, 0, qhead, tok_chunk + row0, batch);
-        tma_load_4d(smDY, &tm_st, &st_full, 32, qhead, tok_chunk + row0, batch);
+      dim3 cta = blockIdx;
+      int s = 0;           // ring stage and its phase
+      uint32_t s_ph = 0;
+      for (int it = 0; ok; ++it) {
+        const DqTile w(p, cta);
+        if (it >= 2) ok = mbar_wait(&q_free[it & 1], ((it >> 1) - 1) & 1, &abort_flag);
+        if (!ok) break;
+        if (!w.empty) {
+          uint8_t* qd = smQD + (it & 1) * 2 * TILE_BYTES;
+          mbar_expect_tx(&q_full[it & 1], 2 * TILE_BYTES);
+          tma_load_4d(qd, &tm_q, &q_full[it & 1], 0, w.qhead, w.tok_chunk + w.row0, w.batch);
+          tma_load_4d(qd + TILE_BYTES, &tm_dy, &q_full[it & 1], 0, w.qhead, w.tok_chunk + w.row0, w.batch);
+          for (int J = 0; J < w.nJ; ++J) {
+            if (!(ok = mbar_wait(&r_empty[s], s_ph ^ 1, &abort_flag))) break;
+            mbar_expect_tx(&r_full[s], R_BYTES);
+            tma_load_4d(smR + s * R_BYTES, &tm_k, &r_full[s], 0, w.kvhead, w.tok_chunk + J * TW, w.batch);
+            tma_load_4d(smR + s * R_BYTES + KV_BYTES, &tm_v, &r_full[s], 0, w.kvhead, w.tok_chunk + J * TW, w.batch);
+            if (++s == NR) s = 0, s_ph ^= 1;
+            if (J == 0 && !(ok = clc_ask(&clc, it, &abort_flag))) break;
+          }
+        } else {
+          mbar_arrive(&q_full[it & 1]);  // nothing to load: the phase passes all the same
+          ok = clc_ask(&clc, it, &abort_flag);
+        }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
     }
-  } else if (warp == 5) {
-    // Issuing thread A: S and dP.  One thread issues a product only every ~108 clocks whatever its
-    // shape (measured), so the three products of a step are shared between two threads: this one runs
-    // ahead with S(J+1) and dP(J+1), thread B follows with dQ(J).
+  } else if (warp == W_MMA) {
+    const uint32_t tmem = tmem_base_s;
     if (elect_one()) {
-      bool ok = mbar_wait(&q_full, 0, &abort_flag);
       const uint32_t idesc_s = umma_idesc(128, TW, Pack2<T>::is_bf16, false, false);
-      const uint32_t q_addr = smem_u32(smQ), dy_addr = smem_u32(smDY);
-      auto issue_s = [&](int J) {
-        const uint32_t k_addr = smem_u32(smK + (J % NKV) * KV_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + COL_S + (J & 1) * TW, umma_desc_sw128(q_addr + ks * 32, 16, 1024),
-                  umma_desc_sw128(k_addr + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-      };
-      auto issue_dp = [&](int J) {
-        const uint32_t v_addr = smem_u32(smV + (J % NKV) * KV_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + COL_DP, umma_desc_sw128(dy_addr + ks * 32, 16, 1024),
-                  umma_desc_sw128(v_addr + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(&sp_full);
-        if (J == nJ - 1) umma_commit(&qdy_free);
-      };
-      if (ok) ok = mbar_wait(&kv_full[0], 0, &abort_flag);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0);
-        issue_dp(0);
-      }
-      for (int J = 0; J + 1 < nJ && ok; ++J) {
-        ok = mbar_wait(&kv_full[(J + 1) % NKV], ((J + 1) / NKV) & 1, &abort_flag);
-        // S(J+1) overwrites the buffer whose dS fed dQ(J-1): that product must have completed
-        if (ok && J >= 1) ok = mbar_wait(&dq_done[(J + 1) & 1], ((J - 1) >> 1) & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        issue_s(J + 1);
-        // dP(J+1) overwrites dP(J), which the rows have read once dS(J) is in tensor memory
-        ok = mbar_wait(&ds_full, J & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        issue_dp(J + 1);
-      }
-    }
-  } else if (warp == 6) {
-    // Issuing thread B: dQ += dS(J) K_J, releases the key/value stage
-    if (elect_one()) {
-      bool ok = true;
       const uint32_t idesc_q = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
-      for (int J = 0; J < nJ && ok; ++J) {
-        ok = mbar_wait(&ds_full, J & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(smK + (J % NKV) * KV_BYTES);
+      // positions in the rotation: group and ring stage with the phases of op_full and r_full there, of the next
+      // operand and of the next scores, which run NG operands ahead
+      struct Pos {
+        int g = 0, s = 0;
+        uint32_t g_ph = 0, s_ph = 0;
+        __device__ __forceinline__ void step() {
+          if (++g == NG) g = 0, g_ph ^= 1;
+          if (++s == NR) s = 0, s_ph ^= 1;
+        }
+      } at, sc;
+      // descriptors of stage 0; a stage on is R_BYTES >> 4 on in the address field
+      const uint32_t ring = smem_u32(smR);
+      const uint64_t d_k = umma_desc_sw128(ring, 16, 1024), d_v = umma_desc_sw128(ring + KV_BYTES, 16, 1024),
+                     d_km = umma_desc_sw128(ring, 8192, 1024);
+      bool ok = true;
+      dim3 cta = blockIdx;
+      int tiles = 0;
+      for (int it = 0; ok; ++it) {
+        const DqTile w(p, cta);
+        ok = mbar_wait(&q_full[it & 1], (it >> 1) & 1, &abort_flag);
+        if (!w.empty) {
+          const uint32_t qd = smem_u32(smQD + (it & 1) * 2 * TILE_BYTES);
+          const uint64_t d_q = umma_desc_sw128(qd, 16, 1024), d_dy = umma_desc_sw128(qd + TILE_BYTES, 16, 1024);
+          auto issue_scores = [&](bool last) -> bool {
+            if (!mbar_wait(&r_full[sc.s], sc.s_ph, &abort_flag)) return false;
+            tc_fence_after();
+            const uint32_t off = (uint32_t)sc.s * (R_BYTES >> 4), cb = tmem + col_b(sc.g);
 #pragma unroll
-        for (int ks = 0; ks < TW / 16; ++ks)
-          umma_ts(tmem + COL_ACC, tmem + COL_S + (J & 1) * TW + ks * 8,
-                  umma_desc_sw128(k_addr + ks * 2048, 8192, 1024), idesc_q, (J > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&kv_empty[J % NKV]);
-        umma_commit(&dq_done[J & 1]);
+            for (int ks = 0; ks < 4; ++ks) umma_ss(cb, d_q + 2 * ks, d_k + off + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) umma_ss(cb + 64, d_dy + 2 * ks, d_v + off + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+            umma_commit(&s_full[sc.g]);
+            if (last) umma_commit(&q_free[it & 1]);  // the query and dO tiles have been read
+            sc.step();
+            return true;
+          };
+          sc = at;
+          for (int J = 0; J < min(w.nJ, NG) && ok; ++J) ok = issue_scores(J == w.nJ - 1);
+          // the accumulator of the tile before has been read out
+          if (ok && tiles > 0) ok = mbar_wait(&acc_free, (tiles - 1) & 1, &abort_flag);
+          for (int J = 0; J < w.nJ && ok; ++J) {
+            ok = mbar_wait(&op_full[at.g], at.g_ph, &abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t off = (uint32_t)at.s * (R_BYTES >> 4), cb = tmem + col_b(at.g);
+#pragma unroll
+            for (int ks = 0; ks < TW / 16; ++ks)
+              umma_ts(tmem, cb + ks * 8, d_km + off + ks * (2048 >> 4), idesc_q, (J > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(&r_empty[at.s]);
+            at.step();
+            // the group's next scores, into the buffer that the product just issued reads (products execute in order)
+            if (J + NG < w.nJ) ok = issue_scores(J + NG == w.nJ - 1);
+          }
+          if (ok) umma_commit(&acc_full);
+          ++tiles;
+        } else {
+          mbar_arrive(&q_free[it & 1]);
+        }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
-      if (ok) umma_commit(&acc_done);
     }
   } else {
-    const int row = row0 + tid;
-    const bool row_valid = row < c;
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    const uint32_t tmem = tmem_base_s;
+    const int grp = warp >> 2, r = tid & 127;  // row group, query row inside the tile
+    const int wrow = (warp & 3) * 32;
+    const uint32_t lane_addr = (uint32_t)wrow << 16;
+    const uint32_t cb = tmem + lane_addr + col_b(grp);
     const bool gated = p.a != nullptr;
-    const size_t tok = (size_t)batch * p.t + tok_chunk + row;
-    const float* a_chunk = gated ? p.a + ((size_t)batch * p.t + tok_chunk) * p.h + kvhead : nullptr;
-    const float a_i = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
-    const float dl_i = row_valid ? p.dl[tok * p.hq + qhead] : 0.f;
-    const float inv_l = row_valid ? safe_recip(p.l[tok * p.hq + qhead]) : 0.f;
-    const float s2x2 = DEG == 4 ? 4.f * (p.scale * p.scale) * (p.scale * p.scale) : 2.f * p.scale * p.scale;  // deg s^deg
-    const int wrow0 = row0 + (warp << 5);  // first row of this warp
-    float da2 = 0.f;                       // twice the row sum of p * dp
+    const float sdeg = DEG == 4 ? 4.f * (p.scale * p.scale) * (p.scale * p.scale) : 2.f * p.scale * p.scale;  // deg s^deg
     bool ok = true;
-    // gate sums of the next step's keys, loaded one step ahead by the first TW threads
-    float av_n = 0.f, r_n = 0.f;
-    auto load_gates = [&](int J) {
-      if (tid < TW && gated) {
-        const int kp = J * TW + tid;
-        av_n = kp < c ? a_chunk[(size_t)kp * p.h] : 0.f;
-        r_n = a_chunk[(size_t)min(J * TW + TW - 1, c - 1) * p.h];
-      }
-    };
-    load_gates(0);
-    for (int J = 0; J < nJ; ++J) {
-      const int kp0 = J * TW;
-      const int sb = J & 1;
-      const uint32_t col_s = COL_S + sb * TW;
-      if (tid < TW) {
-        sm_ak[sb][tid] = av_n;
-        sm_fk[sb][tid] = __expf(r_n - av_n);
-        const bool wide = __any_sync(0xffffffffu, (r_n - av_n) > 80.f);
-        if (lane == 0) sm_wide[sb][warp] = wide;
-        if (tid == 0) sm_r[sb] = r_n;
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (J + 1 < nJ) load_gates(J + 1);  // in flight while this step is computed
-      ok = mbar_wait(&sp_full, J & 1, &abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential
-      // per row and per key instead of one per pair.  Both exponents are <= 0 below the
-      // diagonal for gates <= 0; if one exceeds 80 (growing gates) the warp takes the per-pair
-      // form.  Steps wholly below the diagonal need no mask; a warp whose rows all precede the
-      // step's keys writes zeros without reading the scores.
-      const int lim = min(row, c - 1) - kp0;  // last column this row keeps
-      if (kp0 > min(wrow0 + 31, c - 1)) {
-        uint32_t z[16];
+    dim3 cta = blockIdx;
+    int tiles = 0, own = 0, grp0 = 0;  // tiles with rows, steps of this group so far; group of the tile's first step
+    uint32_t row_ph = 0;
+    for (int it = 0; ok; ++it) {
+      const DqTile w(p, cta);
+      if (!w.empty) {
+        const int row = w.row0 + r;
+        const bool row_valid = row < w.c;
+        const size_t tok0 = (size_t)w.batch * p.t + w.tok_chunk;
+        const size_t ix = (tok0 + row) * p.hq + w.qhead;
+        const float* a_chunk = gated ? p.a + tok0 * p.h + w.kvhead : nullptr;
+        const float a_i = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
+        const float dl_i = row_valid ? p.dl[ix] : 0.f;
+        const float inv_l = row_valid ? safe_recip(p.l[ix]) : 0.f;
+        const int wrow0 = w.row0 + wrow;  // first row of this warp
+        float da = 0.f;                   // deg times the row sum of p * dp
+        // gate sums of this warp's next step, two keys per lane, loaded one step ahead
+        float av0 = 0.f, av1 = 0.f, r_n = 0.f;
+        auto load_gates = [&](int J) {
+          if (gated) {
+            const int kp = J * TW + lane;
+            r_n = a_chunk[(size_t)min(J * TW + TW - 1, w.c - 1) * p.h];
+            av0 = kp < w.c ? a_chunk[(size_t)kp * p.h] : 0.f;
+            av1 = kp + 32 < w.c ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
+          }
+        };
+        const int first = (grp - grp0 + NG) % NG;  // this group's first step in the tile
+        if (first < w.nJ) load_gates(first);
+        for (int J = first; J < w.nJ && ok; J += NG, ++own) {
+          const int kp0 = J * TW;
+          float* fk = sm_fk[warp][own & 1];
+          const float rs = r_n;
+          // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential
+          // per row and per key instead of one per pair.  Both exponents are <= 0 below the
+          // diagonal for gates <= 0; if one exceeds 80 (growing gates) the warp takes the per-pair
+          // form.  Steps wholly below the diagonal need no mask; a warp whose rows all precede the
+          // step's keys writes zeros without reading the scores.
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - fminf(av0, av1), a_i - rs) > 80.f);
+          const float c_i = sep ? sdeg * __expf(a_i - rs) : sdeg;
+          fk[lane] = sep ? __expf(rs - av0) : av0;
+          fk[lane + 32] = sep ? __expf(rs - av1) : av1;
+          __syncwarp();
+          if (J + NG < w.nJ) load_gates(J + NG);  // in flight while this step is computed
+          ok = mbar_wait(&s_full[grp], own & 1, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (kp0 > min(wrow0 + 31, w.c - 1)) {
+            uint32_t z[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) z[j] = 0u;
-        tmem_st16(tmem + lane_addr + col_s, z);
-        tmem_st16(tmem + lane_addr + col_s + 16, z);
-      } else {
-        const float r = sm_r[sb];
-        const bool mask = (kp0 + TW - 1 > wrow0) || (kp0 + TW - 1 >= c);
-        const bool sep = !(sm_wide[sb][0] | sm_wide[sb][1]) && !__any_sync(0xffffffffu, (a_i - r) > 80.f);
-        const float c_i = sep ? s2x2 * __expf(a_i - r) : s2x2;
-#pragma unroll 1
-        for (int q4 = 0; q4 < TW / 32; ++q4) {
-          uint32_t sv[32], pv[32], pk[16];
-          tmem_ld32(tmem + lane_addr + col_s + q4 * 32, sv);
-          tmem_ld32(tmem + lane_addr + COL_DP + q4 * 32, pv);
-          tmem_wait_ld();
-          const int lm = lim - q4 * 32;
-          if (sep) {
-            if (mask) dq_half<T, DEG, true, true>(sv, pv, sm_fk[sb] + q4 * 32, c_i, a_i, inv_l, dl_i, lm, pk, da2);
-            else dq_half<T, DEG, true, false>(sv, pv, sm_fk[sb] + q4 * 32, c_i, a_i, inv_l, dl_i, lm, pk, da2);
+            for (int j = 0; j < 16; ++j) z[j] = 0u;
+            tmem_st16(cb, z);
+            tmem_st16(cb + 16, z);
           } else {
-            dq_half<T, DEG, false, true>(sv, pv, sm_ak[sb] + q4 * 32, c_i, a_i, inv_l, dl_i, lm, pk, da2);
+            const bool mask = (kp0 + TW - 1 > wrow0) || (kp0 + TW - 1 >= w.c);
+            const int lim = min(row, w.c - 1) - kp0;  // last column this row keeps
+            if (!sep) dq_step<T, DEG, false, true>(cb, fk, c_i, a_i, inv_l, dl_i, lim, da);
+            else if (mask) dq_step<T, DEG, true, true>(cb, fk, c_i, a_i, inv_l, dl_i, lim, da);
+            else dq_step<T, DEG, true, false>(cb, fk, c_i, a_i, inv_l, dl_i, lim, da);
           }
-          tmem_st16(tmem + lane_addr + col_s + q4 * 16, pk);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&op_full[grp]);
         }
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_full);
-    }
-    if (ok) ok = mbar_wait(&acc_done, 0, &abort_flag);
-    if (ok && has_st) ok = mbar_wait(&st_full, 0, &abort_flag);
-    tc_fence_after();
-    if (ok) {
-      uint32_t acc[64];
-      tmem_ld32(tmem + lane_addr + COL_ACC, acc);
-      tmem_ld32(tmem + lane_addr + COL_ACC + 32, acc + 32);
-      tmem_wait_ld();
-      if (row_valid) {
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(p.dQ) + (tok * p.hq + qhead) * p.d);
+        sm_da[tiles & 1][grp][r] = da;
+        // the row warps meet; bounded like every wait
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&rows);
+        // the groups share the write-out, 16 of the 64 columns at a time; the state-path gradient comes in meanwhile
+        const float* st = p.dq_state ? p.dq_state + ix * p.d : nullptr;
+        float4 add[2][4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (8 * j >= p.d) break;
-          float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-          if (has_st) {
-            // columns 8j..8j+7: 16-byte chunks 2j, 2j+1 of the row in its 32-column half
-            const uint8_t* half = (j < 4) ? smQ : smDY;
-            s0 = *reinterpret_cast<const float4*>(half + swz128(tid, (2 * j) & 7));
-            s1 = *reinterpret_cast<const float4*>(half + swz128(tid, (2 * j + 1) & 7));
-          }
-          uint4 v;
-          v.x = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 0]) + s0.x, __uint_as_float(acc[8 * j + 1]) + s0.y);
-          v.y = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 2]) + s0.z, __uint_as_float(acc[8 * j + 3]) + s0.w);
-          v.z = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 4]) + s1.x, __uint_as_float(acc[8 * j + 5]) + s1.y);
-          v.w = Pack2<T>::from_f32(__uint_as_float(acc[8 * j + 6]) + s1.z, __uint_as_float(acc[8 * j + 7]) + s1.w);
-          dst[j] = v;
+        for (int q = 0; q < 2; ++q) {
+          const int c0 = 16 * (grp + NG * q);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            add[q][j] = (st != nullptr && row_valid && c0 < p.d && c0 < HD) ? reinterpret_cast<const float4*>(st + c0)[j]
+                                                                           : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        p.da_q[tok * p.hq + qhead] = (1.f / DEG) * da2;
+        if (ok) ok = mbar_wait(&rows, row_ph, &abort_flag);
+        row_ph ^= 1;
+        if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
+        tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int c0 = 16 * (grp + NG * q);
+          if (!ok || c0 >= HD) continue;
+          uint32_t acc[16];
+          tmem_ld16(tmem + lane_addr + c0, acc);
+          tmem_wait_ld();
+          if (row_valid && c0 < p.d) {
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + add[q][j].x, __uint_as_float(acc[4 * j + 1]) + add[q][j].y);
+              v[2 * j + 1] =
+                  Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + add[q][j].z, __uint_as_float(acc[4 * j + 3]) + add[q][j].w);
+            }
+            T* dst = static_cast<T*>(p.dQ) + ix * p.d + c0;
+            if (p.aligned32) {
+              st_global_v8(dst, v);
+            } else {
+              reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+              reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_free);
+        if (grp == NG - 1 && row_valid)
+          p.da_q[ix] = (1.f / DEG) * ((sm_da[tiles & 1][0][r] + sm_da[tiles & 1][1][r]) + sm_da[tiles & 1][2][r]);
+        grp0 = (grp0 + w.nJ) % NG;
+        ++tiles;
       }
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
     }
   }
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && abort_flag) *p.status = ST_TIMEOUT;
-  if (warp == 0) tmem_dealloc(tmem, dq::TMEM_COLS);
+  if (warp == 0) tmem_dealloc(tmem_base_s, TMEM_COLS);
 }
 
 }  // namespace pr
@@ -373,10 +456,11 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   p.l = l;
   p.dq_state = dq_state;
   p.dQ = dQ;
+  p.aligned32 = (reinterpret_cast<uintptr_t>(dQ) & 31u) == 0;
   p.da_q = da_q;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;
-  CUtensorMap tm_q, tm_dy, tm_k, tm_v, tm_st;
+  CUtensorMap tm_q, tm_dy, tm_k, tm_v;
   uint64_t dq_[4] = {(uint64_t)d, (uint64_t)hq, (uint64_t)t, (uint64_t)b};
   uint64_t sq[4] = {0, (uint64_t)d * 2, (uint64_t)hq * d * 2, (uint64_t)t * hq * d * 2};
   uint64_t dk[4] = {(uint64_t)d, (uint64_t)h, (uint64_t)t, (uint64_t)b};
@@ -387,19 +471,12 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   uint32_t box_kv[4] = {64, 1, (uint32_t)TW, 1};
   if ((rc = make_tmap(&tm_k, K, 2, 4, dk, sk, box_kv, true))) return rc;
   if ((rc = make_tmap(&tm_v, V, 2, 4, dk, sk, box_kv, true))) return rc;
-  tm_st = tm_q;  // unused without a state-path gradient
-  if (dq_state) {
-    uint64_t ss[4] = {0, (uint64_t)d * 4, (uint64_t)hq * d * 4, (uint64_t)t * hq * d * 4};
-    uint32_t box_st[4] = {32, 1, 128, 1};
-    if ((rc = make_tmap(&tm_st, dq_state, 4, 4, dq_, ss, box_st, true))) return rc;
-  }
-  const size_t smem = 1024 + 2 * TILE_BYTES + 2 * NKV * KV_BYTES;
   dim3 grid(p.tiles_per_chunk * p.n_chunks, hq, b);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define PR_LAUNCH_DQ(TT, DG)                                                                                      \
   do {                                                                                                           \
-    PR_SMEM_ATTR((chunk_dq_kernel<TT, DG>), smem, device, true);                                                   \
-    chunk_dq_kernel<TT, DG><<<grid, THREADS, smem, s>>>(p, tm_q, tm_dy, tm_k, tm_v, tm_st);                         \
+    PR_SMEM_ATTR((chunk_dq_kernel<TT, DG>), SMEM, device, true);                                                   \
+    chunk_dq_kernel<TT, DG><<<grid, THREADS, SMEM, s>>>(p, tm_q, tm_dy, tm_k, tm_v);                         \
   } while (0)
   if (dtype == PR_BF16) {
     if (deg == 4) PR_LAUNCH_DQ(__nv_bfloat16, 4); else PR_LAUNCH_DQ(__nv_bfloat16, 2);

@@ -77,13 +77,6 @@ struct ChunkOutParams {
   int* status;
 };
 
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
 // What a CTA index stands for: a tile of 128 query rows of one (batch, chunk, query head).
 struct OutTile {
   int chunk, qhead, kvhead, batch, row0;

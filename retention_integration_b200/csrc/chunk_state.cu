@@ -162,17 +162,18 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
         }
       } else {
         const uint32_t idesc = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
+        const uint64_t d_w0 = umma_desc_sw128(smem_u32(smW), 8192, 1024);
         for (int it = 0; it < total && ok; ++it) {
           const int s = it % NS, ph = (it / NS) & 1;
           const int sa = it % NSA, pha = (it / NSA) & 1;
           ok = mbar_wait(&w_full[s], ph, &abort_flag) && mbar_wait(&a_full[g][sa], pha, &abort_flag);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t b_addr = smem_u32(smW + s * W_BYTES);
+          const uint64_t d_w = d_w0 + (uint32_t)s * (W_BYTES >> 4);
 #pragma unroll
           for (int ks = 0; ks < TOK / 16; ++ks)
             umma_ts(tmem + COL_ACC + g * 64, tmem + COL_A + (g * NSA + sa) * 32 + ks * 8,
-                    umma_desc_sw128(b_addr + ks * 2048, 8192, 1024), idesc, (it > 0 || ks > 0) ? 1u : 0u);
+                    d_w + ks * (2048 >> 4), idesc, (it > 0 || ks > 0) ? 1u : 0u);
           umma_commit(&done[g][s]);
         }
       }

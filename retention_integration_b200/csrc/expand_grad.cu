@@ -177,7 +177,9 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
     if (elect_one()) {
       const int rt = (warp - (W_TMA + 1)) >> 1, par = (warp - (W_TMA + 1)) & 1;
       bool ok = mbar_wait(&w_full, 0, &abort_flag);
-      const uint32_t w_addr = smem_u32(smW) + rt * TILE_BYTES;
+      // prepared descriptors: a state tile on is TILE_BYTES >> 4 on in the address field
+      const uint64_t d_w = umma_desc_sw128(smem_u32(smW) + rt * TILE_BYTES, 16, 1024),
+                     d_s0 = umma_desc_sw128(smem_u32(smS), 16, 1024);
       const uint32_t idesc = umma_idesc(128, 128, Pack2<T>::is_bf16, false, false);
       for (int nt = par; nt < p.nt && ok; nt += 2) {
         const int s = nt % NSS, ph = (nt / NSS) & 1;
@@ -187,11 +189,10 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
              mbar_wait(&s_full[s], ph, &abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t s_addr = smem_u32(smS + s * TILE_BYTES);
+        const uint64_t d_s = d_s0 + (uint32_t)s * (TILE_BYTES >> 4);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + col_d(rt, b), umma_desc_sw128(w_addr + ks * 32, 16, 1024),
-                  umma_desc_sw128(s_addr + ks * 32, 16, 1024), idesc, ks > 0 ? 1u : 0u);
+          umma_ss(tmem + col_d(rt, b), d_w + 2 * ks, d_s + 2 * ks, idesc, ks > 0 ? 1u : 0u);
         umma_commit(&d_full[rt][b]);
         umma_commit(&s_empty[s]);
         if (nt == 0) {

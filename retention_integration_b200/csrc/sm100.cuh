@@ -139,6 +139,13 @@ __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (i
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+
 // ------------------------------------------------------- taking over CTAs
 // A persistent kernel keeps its grid: when a CTA has planned its tile, one thread asks for the index of a CTA of the
 // same grid that has not been launched yet and the CTA does that one's work next (cluster launch control), so set-up,
