@@ -234,8 +234,10 @@ py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G,
   V = aligned(V);
   if (scale == 0) scale = 1.0 / std::sqrt((double)d);
   if (quadratic) c = with_state ? t : 0;  // a short sequence that carries a state is one chunk of the chunked form
-  const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || K.requires_grad() || V.requires_grad() ||
-                                                   (G.defined() && G.requires_grad()));
+  // the autograd node also where an input carries a tangent: forward mode is not implemented, and the node says so
+  auto any_of = [&](auto f) { return f(Q) || f(K) || f(V) || (G.defined() && f(G)); };
+  const bool grad = (at::GradMode::is_enabled() && any_of([](const Tensor& t) { return t.requires_grad(); })) ||
+                    any_of([](const Tensor& t) { return t._fw_grad(0).defined(); });
   Tensor Cs, Cg;
   if (state.has_value()) {
     pr_require(sok.has_value(), "initial_state is the pair (state, sum_of_keys)");
