@@ -16,7 +16,6 @@
 // Arithmetic as deploy/nanoGPT/model.py:159-164: x * cos and rotate(x) * sin are rounded fp32
 // products, their sum is rounded once more, then cast to the input's dtype (no fused multiply-add,
 // so that the 16-bit results are the reference's bit for bit).
-#include <algorithm>
 
 #include "host.cuh"
 #include "sm100.cuh"
@@ -25,6 +24,7 @@ namespace pr {
 namespace {
 
 constexpr int kCpThreads = 256;
+constexpr int kCpVectors = 4;  // 16-byte vectors per thread
 
 // numerically safe log(sigmoid(x)) = min(x, 0) - log1p(exp(-|x|))
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(__expf(-fabsf(x))); }
@@ -62,84 +62,101 @@ struct CallerPrepParams {
   size_t tokens;          // b * t
 };
 
-// One work item = one 16-byte vector of q or k (a pair of vectors when the rotary pairs are
-// half-split) or of v; consecutive threads take consecutive items, so a warp reads 512 contiguous
-// bytes of a token's row and writes 512 contiguous bytes of Q, K or V.  The item number is split
-// into (token, vector) with 32-bit arithmetic whenever the problem allows (IDX = unsigned): the
-// 64-bit divisions of the general case cost as many issue slots as the rest of the item.
+// A head row is cut into units: one 16-byte vector, or (half-split pairs) the two vectors that rotate into each other;
+// the same cut for q, k and v heads.  A thread takes kCpVectors vectors of one token that sit at the same place of
+// their heads, W units apart: one pair of table loads and one split of the index serve all of them, and all of a
+// thread's loads are in flight together, which HBM needs (one vector per turn of a grid-stride loop, as this kernel had
+// it, reached 70-76 % of the copy bandwidth and read the tables once per vector).  Consecutive threads take
+// consecutive units, so a warp reads and writes 512 contiguous bytes per vector.  The index is split with 32-bit
+// arithmetic whenever the problem allows (IDX = unsigned).
 // GRAD: inputs are dQ, dK, dV, dlog_g and the saved projection output (for the gate's derivative);
 // the output is the gradient with respect to the projection output.
 template <typename T, bool GRAD, bool HALF, typename IDX>
-__global__ void __launch_bounds__(kCpThreads, HALF ? 4 : 8)
+__global__ void __launch_bounds__(kCpThreads, 4)
 caller_prep_kernel(const CallerPrepParams p, const T* __restrict__ in, const float* __restrict__ cosT,
                    const float* __restrict__ sinT, T* __restrict__ Q, T* __restrict__ K, T* __restrict__ V,
                    float* __restrict__ log_g, T* __restrict__ grad_in) {
-  const int d = p.d, vpr = d / 8;                 // vectors per head row
-  const int units_rot = HALF ? vpr / 2 : vpr;     // work items per rotated head row
-  const int n_rot = (p.hq + p.h) * units_rot;     // q heads, then k heads: one contiguous span of the row
-  const IDX per_tok = (IDX)(n_rot + p.h * vpr);
-  const long long off_v = (long long)(p.hq + p.h) * d, off_g = off_v + (long long)p.h * d;
-  const IDX total = (IDX)p.tokens * per_tok;
-  const IDX step = (IDX)gridDim.x * kCpThreads;
+  constexpr int NV = HALF ? 2 : 1, R = kCpVectors / NV;  // vectors per unit, units per thread
+  const int d = p.d, ur = d / 8 / NV;                    // units per head row
+  const int heads = p.hq + 2 * p.h, n_rot = p.hq + p.h, hstep = (heads + R - 1) / R;
+  const IDX W = (IDX)(hstep * ur);
   const float sign = GRAD ? -1.f : 1.f;
-  for (IDX idx = (IDX)blockIdx.x * kCpThreads + threadIdx.x; idx < total; idx += step) {
-    const IDX tok_i = idx / per_tok;
-    const int u = (int)(idx - tok_i * per_tok);
-    const size_t tok = tok_i;
-    const T* row_in = in + tok * p.in_stride;
-    T* row_g = GRAD ? grad_in + tok * p.in_stride : nullptr;
-    if (u < n_rot) {
-      const int head = u / units_rot, j = u - head * units_rot;
-      const bool is_q = head < p.hq;
-      const long long col = (long long)head * d + j * 8;
-      T* dense = (is_q ? Q + (tok * p.hq + head) * d : K + (tok * p.h + (head - p.hq)) * d) + j * 8;
-      const IDX batch = tok_i / (IDX)p.t;
-      const size_t trow = (size_t)batch * p.cs_bstride + (size_t)(tok_i - batch * (IDX)p.t) * (d / 2) + (HALF ? j * 8 : j * 4);
-      const T* src = GRAD ? dense : row_in + col;
-      T* dst = GRAD ? row_g + col : dense;
-      if (!HALF) {
-        const uint4 v = *reinterpret_cast<const uint4*>(src);
-        const float4 c4 = *reinterpret_cast<const float4*>(cosT + trow), s4 = *reinterpret_cast<const float4*>(sinT + trow);
-        float x[8], y[8];
-        unpack8<T>(v, x);
-        const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+  const IDX idx = (IDX)blockIdx.x * kCpThreads + threadIdx.x;
+  const IDX tok_i = idx / W;
+  if (tok_i >= (IDX)p.tokens) return;
+  const int u = (int)(idx - tok_i * W);
+  const int head0 = u / ur, j = u - head0 * ur;
+  const size_t tok = tok_i;
+  const T* row_in = in + tok * p.in_stride;
+  T* row_g = GRAD ? grad_in + tok * p.in_stride : nullptr;
+  // the token's vector of Q, K or V
+  auto dense = [&](int head) -> T* {
+    T* base = head < p.hq ? Q + (tok * p.hq + head) * d
+                          : (head < n_rot ? K + (tok * p.h + (head - p.hq)) * d : V + (tok * p.h + (head - n_rot)) * d);
+    return base + j * 8;
+  };
+
+  uint4 v[R][NV];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) rotate_pair(x[2 * e], x[2 * e + 1], c[e], s[e], sign, &y[2 * e], &y[2 * e + 1]);
-        *reinterpret_cast<uint4*>(dst) = pack8<T>(y);
+  for (int i = 0; i < R; ++i) {
+    const int head = head0 + i * hstep;
+    if (head < heads) {
+      const T* src = GRAD ? dense(head) : row_in + (long long)head * d + j * 8;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[i][k] = *reinterpret_cast<const uint4*>(src + k * (d / 2));
+    }
+  }
+  // a gate rides with the first unit of its value head
+  float gate[R], up[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int gh = head0 + i * hstep - n_rot;
+    if (p.gated && j == 0 && gh >= 0 && gh < p.h) {
+      gate[i] = float(row_in[(long long)heads * d + gh]) + p.gate_bias;
+      if (GRAD) up[i] = log_g[tok * p.h + gh];
+    }
+  }
+  // cosines and sines of this place: 4 pairs of a vector, or 8 of a unit of two
+  constexpr int NP = 4 * NV;
+  float c[NP], s[NP];
+  if (head0 < n_rot) {
+    const IDX batch = tok_i / (IDX)p.t;
+    const size_t trow = (size_t)batch * p.cs_bstride + (size_t)(tok_i - batch * (IDX)p.t) * (d / 2) + j * NP;
+#pragma unroll
+    for (int k = 0; k < NP; k += 4) {
+      *reinterpret_cast<float4*>(c + k) = *reinterpret_cast<const float4*>(cosT + trow + k);
+      *reinterpret_cast<float4*>(s + k) = *reinterpret_cast<const float4*>(sinT + trow + k);
+    }
+  }
+
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int head = head0 + i * hstep;
+    if (head >= heads) break;
+    if (head < n_rot) {
+      float x[NV][8], y[NV][8];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) unpack8<T>(v[i][k], x[k]);
+      if constexpr (!HALF) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) rotate_pair(x[0][2 * e], x[0][2 * e + 1], c[e], s[e], sign, &y[0][2 * e], &y[0][2 * e + 1]);
       } else {
         // elements 8j..8j+7 pair with 8j + d/2 .. 8j + d/2 + 7
-        const uint4 va = *reinterpret_cast<const uint4*>(src), vb = *reinterpret_cast<const uint4*>(src + d / 2);
-        float c[8], s[8], x0[8], x1[8], y0[8], y1[8];
-        *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cosT + trow);
-        *reinterpret_cast<float4*>(c + 4) = *reinterpret_cast<const float4*>(cosT + trow + 4);
-        *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sinT + trow);
-        *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(sinT + trow + 4);
-        unpack8<T>(va, x0);
-        unpack8<T>(vb, x1);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) rotate_pair(x0[e], x1[e], c[e], s[e], sign, &y0[e], &y1[e]);
-        *reinterpret_cast<uint4*>(dst) = pack8<T>(y0);
-        *reinterpret_cast<uint4*>(dst + d / 2) = pack8<T>(y1);
+        for (int e = 0; e < 8; ++e) rotate_pair(x[0][e], x[NV - 1][e], c[e], s[e], sign, &y[0][e], &y[NV - 1][e]);
       }
-    } else {
-      const int w = u - n_rot;            // vector of the token's value span
-      const int head = w / vpr;
-      T* dense = V + tok * ((size_t)p.h * d) + (size_t)w * 8;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[i][k] = pack8<T>(y[k]);
+    }
+    T* dst = GRAD ? row_g + (long long)head * d + j * 8 : dense(head);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) *reinterpret_cast<uint4*>(dst + k * (d / 2)) = v[i][k];
+    const int gh = head - n_rot;
+    if (p.gated && j == 0 && gh >= 0) {
       if (GRAD)
-        *reinterpret_cast<uint4*>(row_g + off_v + (long long)w * 8) = *reinterpret_cast<const uint4*>(dense);
+        row_g[(long long)heads * d + gh] = T(up[i] * (1.f / (1.f + __expf(gate[i]))));  // d/dx log sigmoid(x) = sigmoid(-x)
       else
-        *reinterpret_cast<uint4*>(dense) = *reinterpret_cast<const uint4*>(row_in + off_v + (long long)w * 8);
-      // the token's gate columns ride with the first vector of each value head: one gate per thread
-      if (p.gated && w - head * vpr == 0) {
-        const float pre = float(row_in[off_g + head]) + p.gate_bias;
-        if (GRAD) {
-          // d/dx log sigmoid(x) = sigmoid(-x)
-          const float sg = 1.f / (1.f + __expf(pre));
-          row_g[off_g + head] = T(log_g[tok * p.h + head] * sg);
-        } else {
-          log_g[tok * p.h + head] = log_sigmoid(pre);
-        }
-      }
+        log_g[tok * p.h + gh] = log_sigmoid(gate[i]);
     }
   }
 }
@@ -147,16 +164,12 @@ caller_prep_kernel(const CallerPrepParams p, const T* __restrict__ in, const flo
 template <typename T>
 int launch_caller_prep(bool grad, const CallerPrepParams& p, const void* in, const float* cosT, const float* sinT, void* Q,
                        void* K, void* V, float* log_g, void* grad_in, cudaStream_t s) {
-  const int vpr = p.d / 8, ur = p.half_split ? vpr / 2 : vpr;
-  const size_t per_tok = (size_t)(p.hq + p.h) * ur + (size_t)p.h * vpr;
-  const size_t total = p.tokens * per_tok;
-  // every thread takes a few items; the grid is a multiple of the SM count (eight CTAs resident per SM)
-  int sms = 148, dev = 0;
-  PR_CUDA(cudaGetDevice(&dev));
-  PR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const size_t want = (total + kCpThreads - 1) / kCpThreads;
-  const unsigned grid = (unsigned)std::min<size_t>(want, (size_t)sms * 32);
-  const bool small = total + (size_t)grid * kCpThreads < ((size_t)1 << 32);  // the item counter may not wrap
+  const int nv = p.half_split ? 2 : 1, r = kCpVectors / nv;
+  const size_t per_tok = (size_t)((p.hq + 2 * p.h + r - 1) / r) * (p.d / 8 / nv);
+  const size_t ctas = (p.tokens * per_tok + kCpThreads - 1) / kCpThreads;
+  PR_REQUIRE(ctas < ((size_t)1 << 31), PR_ERR_BAD_ARG, "%zu CTAs exceed the grid limit", ctas);
+  const unsigned grid = (unsigned)ctas;
+  const bool small = ctas * kCpThreads < ((size_t)1 << 32);  // the index may not wrap
 #define PR_LAUNCH_CP(G, H)                                                                                         \
   do {                                                                                                             \
     if (small)                                                                                                     \
