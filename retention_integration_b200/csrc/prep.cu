@@ -15,7 +15,7 @@ namespace pr {
 constexpr int kPrepThreads = 256;   // gate_grad
 constexpr int kGpThreads = 128;     // gate_prep: small CTAs, eight per SM, four 16-byte loads in flight per thread
 
-template <typename T, int NV, bool PAIRED>
+template <typename T, int NV, bool PAIRED, bool SCALED>
 __global__ void __launch_bounds__(kGpThreads, NV == 4 ? 8 : 4)
 gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in, const T* __restrict__ x,
                  float* __restrict__ a_out, float* __restrict__ A_out, T* __restrict__ xt,
@@ -42,8 +42,14 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
 
   // ---- the chunk's cumulative log gates: read if a pass before this one has made them, else a
   // block-wide inclusive scan of the log gates
+  // (read: of this CTA's own tokens, and the total; a token's gate lies h floats from its neighbour's, so each costs a
+  // sector, and all of the chunk's for every CTA were more sectors than the tokens themselves)
+  const int tiles = cp / 64, tiles_per = (tiles + gridDim.y - 1) / gridDim.y;
+  const int tb_begin = blockIdx.y * tiles_per * 64, tb_end = min((c + 63) & ~63, (int)(blockIdx.y + 1) * tiles_per * 64);
+  float A = 0.f;
   if (a_in != nullptr) {
-    for (int i = tid; i < c; i += kGpThreads) sm_a[i] = a_in[(tok0 + i) * h + gh];
+    A = a_in[(tok0 + c - 1) * h + gh];
+    for (int i = tb_begin + tid; i < min(c, tb_end); i += kGpThreads) sm_a[i] = a_in[(tok0 + i) * h + gh];
     __syncthreads();
   } else if (log_g != nullptr) {
     if (tid == 0) carry_s = 0.f;
@@ -79,7 +85,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
     for (int i = tid; i < c; i += kGpThreads) sm_a[i] = 0.f;
     __syncthreads();
   }
-  const float A = sm_a[c - 1];
+  if (a_in == nullptr) A = sm_a[c - 1];
   if (write_a && blockIdx.y == 0) {
     if (a_out != nullptr)
       for (int i = tid; i < c; i += kGpThreads) a_out[(tok0 + i) * h + gh] = sm_a[i];
@@ -90,10 +96,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
   // ---- gated transpose, 64 tokens at a time
   const int vec_per_row = d / 8;
   T* out_base = xt + ((size_t)(batch * n + chunk) * hx + head) * (size_t)d * cp;
-  T* out2_base = xts ? xts + ((size_t)(batch * n + chunk) * hx + head) * (size_t)d * cp : nullptr;
-  // the chunk's 64-token tiles are split over gridDim.y blocks (each recomputes the cheap scan)
-  const int tiles = cp / 64, tiles_per = (tiles + gridDim.y - 1) / gridDim.y;
-  const int tb_end = min((c + 63) & ~63, (int)(blockIdx.y + 1) * tiles_per * 64);
+  T* out2_base = SCALED ? xts + ((size_t)(batch * n + chunk) * hx + head) * (size_t)d * cp : nullptr;
   // The loads of tile k+1 are issued before tile k is transposed and written out, so a CTA always has
   // a tile's worth of reads in flight (64 tokens x d features: up to four 16-byte vectors per thread).
   constexpr int kMaxVec = NV;  // 4 covers d <= 64, 8 covers d <= 128
@@ -127,12 +130,12 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
         if (i < c) {
           raw[q] = *reinterpret_cast<const uint4*>(x + ((tok0 + i) * hx + head) * (size_t)d + v * 8);
           fac[q] = query_side ? mult * __expf(0.5f * sm_a[i]) : mult * __expf(0.5f * (A - sm_a[i]));
-          if (xts != nullptr) rsc[q] = row_scale[(tok0 + i) * hx + head];
+          if (SCALED) rsc[q] = row_scale[(tok0 + i) * hx + head];
         }
       }
     }
   };
-  const int tb_begin = blockIdx.y * tiles_per * 64;
+  // the chunk's 64-token tiles are split over gridDim.y blocks
   if (tb_begin < tb_end) load_tile(tb_begin);
   for (int tb = tb_begin; tb < tb_end; tb += 64) {
     __syncthreads();
@@ -171,7 +174,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
           dst[(2 * k) * 32] = __byte_perm(wa[k], w[k], 0x5410);
           dst[(2 * k + 1) * 32] = __byte_perm(wa[k], w[k], 0x7632);
         }
-        if (xts != nullptr) {
+        if (SCALED) {
           uint32_t* dst2 = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(tile2) + (v * 8) * 64 + pos);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -189,7 +192,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
         dst[(2 * k) * 64] = (uint16_t)(w[k] & 0xffffu);
         dst[(2 * k + 1) * 64] = (uint16_t)(w[k] >> 16);
       }
-      if (xts != nullptr) {
+      if (SCALED) {
         uint16_t* dst2 = reinterpret_cast<uint16_t*>(tile2) + (v * 8) * 64 + pos;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -206,7 +209,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
       const int chunk8 = ((tv ^ (row >> 3)) & 7) << 3;
       *reinterpret_cast<uint4*>(out_base + (size_t)row * cp + tb + tv * 8) =
           *reinterpret_cast<const uint4*>(tile + row * 64 + chunk8);
-      if (xts != nullptr)
+      if (SCALED)
         *reinterpret_cast<uint4*>(out2_base + (size_t)row * cp + tb + tv * 8) =
             *reinterpret_cast<const uint4*>(tile2 + row * 64 + chunk8);
     }
@@ -401,31 +404,39 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
                                           WRITE);                                                              \
     PR_CUDA(cudaGetLastError());                                                                               \
   } while (0)
-#define PR_LAUNCH_PREP(TT, GRID, LG, AIN, XT, XTS, WRITE)                                                       \
+#define PR_LAUNCH_PREP_S(TT, SC, GRID, LG, AIN, XT, XTS, WRITE)                                                 \
   do {                                                                                                         \
     if (d == 64)                                                                                               \
-      PR_LAUNCH_PREP_K((gate_prep_kernel<TT, 4, true>), TT, GRID, LG, AIN, XT, XTS, WRITE);                    \
+      PR_LAUNCH_PREP_K((gate_prep_kernel<TT, 4, true, SC>), TT, GRID, LG, AIN, XT, XTS, WRITE);                    \
     else if (d < 64)                                                                                           \
-      PR_LAUNCH_PREP_K((gate_prep_kernel<TT, 4, false>), TT, GRID, LG, AIN, XT, XTS, WRITE);                   \
+      PR_LAUNCH_PREP_K((gate_prep_kernel<TT, 4, false, SC>), TT, GRID, LG, AIN, XT, XTS, WRITE);                   \
     else                                                                                                       \
-      PR_LAUNCH_PREP_K((gate_prep_kernel<TT, 8, false>), TT, GRID, LG, AIN, XT, XTS, WRITE);                   \
+      PR_LAUNCH_PREP_K((gate_prep_kernel<TT, 8, false, SC>), TT, GRID, LG, AIN, XT, XTS, WRITE);                   \
+  } while (0)
+#define PR_LAUNCH_PREP(TT, GRID, LG, AIN, XT, XTS, WRITE)                                                       \
+  do {                                                                                                         \
+    if (XTS != nullptr)                                                                                        \
+      PR_LAUNCH_PREP_S(TT, true, GRID, LG, AIN, XT, XTS, WRITE);                                               \
+    else                                                                                                       \
+      PR_LAUNCH_PREP_S(TT, false, GRID, LG, AIN, XT, XTS, WRITE);                                              \
   } while (0)
   if (dtype == PR_BF16) {
     if (two_pass) {
-      PR_LAUNCH_PREP(__nv_bfloat16, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, nullptr, 1);
+      PR_LAUNCH_PREP(__nv_bfloat16, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, (void*)nullptr, 1);
       PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_out, xt, xts, 0);
     } else {
       PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_in, xt, xts, write_a);
     }
   } else {
     if (two_pass) {
-      PR_LAUNCH_PREP(__half, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, nullptr, 1);
+      PR_LAUNCH_PREP(__half, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, (void*)nullptr, 1);
       PR_LAUNCH_PREP(__half, grid, log_g, a_out, xt, xts, 0);
     } else {
       PR_LAUNCH_PREP(__half, grid, log_g, a_in, xt, xts, write_a);
     }
   }
 #undef PR_LAUNCH_PREP
+#undef PR_LAUNCH_PREP_S
 #undef PR_LAUNCH_PREP_K
   return PR_OK;
 }
