@@ -217,7 +217,14 @@ int pr_gate_grad(int b, int t, int h, int hq, int c, const float* da_q, const fl
  * absent) + the partials (may be absent) -> O [b,1,hq,d].
  * pr_state_merge: the switch-over of :366-382: new_state = state*exp(a_last) + S, with
  * S [b,1,h,D2,d] and gram [b,1,h,d,d] from pr_chunk_state over the cached tokens; state and
- * sum_of_keys may be NULL (first compression). */
+ * sum_of_keys may be NULL (first compression).
+ * pr_compress_cache: pr_chunk_state and pr_state_merge in one kernel, without the chunk state in memory: the tk cached
+ * tokens (xt from pr_gate_prep with c = tk, V [b,tk,h,64]) go straight into new_state = state*exp(a_last) + S and its
+ * sum_of_keys.  state, sum_of_keys and a_last may be NULL; the new pair may not overlap the old one; new_state on a
+ * 32-byte boundary. */
+int pr_compress_cache(int dtype, int b, int tk, int h, int d, const void* xt, const void* v, const void* state,
+                      const float* sum_of_keys, const float* a_last, void* new_state, float* new_sum_of_keys,
+                      int device, void* stream);
 int pr_decode_nsplit(void);
 /* Parts the decode step of a given shape is split into, in [1, pr_decode_nsplit()]; 1 means that
  * pr_decode_step / pr_decode_recurrent need no part_y / part_l.  Negative on bad sizes. */

@@ -184,13 +184,12 @@ void check_state(const Tensor& state, const Tensor& sok, int64_t b, int64_t h, i
   pr_require(state.is_cuda() && sok.is_cuda(), "the state must live on a CUDA device: this package has no CPU path");
 }
 
-// new_state = state e^a_last + S, exact layout; S [b,1,h,DR,d] in the chunk-state layout (a_last [b,h] or none)
-std::tuple<Tensor, Tensor> merge_state(const Tensor& state, const Tensor& sok, const Tensor& S, const Tensor& gram,
-                                       const Tensor& a_last, int64_t b, int64_t h, int64_t d, const On& on) {
+// The pair after the last token in the exact layout, from the scans' carries.
+std::tuple<Tensor, Tensor> final_state(const Tensor& S, const Tensor& gram, int64_t b, int64_t h, int64_t d, const On& on) {
   const int64_t D = d * (d + 1) / 2;
   const Tensor ns = at::empty({b, h, D, d}, S.options()), nk = empty_f32({b, h, D}, S);
-  check(pr_state_merge(dtype_code(S), (int)b, (int)h, (int)d, cptr(state), fptr(sok), cptr(S), fptr(gram), fptr(a_last),
-                       mptr(ns), fmptr(nk), on.device, on.stream),
+  check(pr_state_merge(dtype_code(S), (int)b, (int)h, (int)d, nullptr, nullptr, cptr(S), fptr(gram), nullptr, mptr(ns),
+                       fmptr(nk), on.device, on.stream),
         "pr_state_merge", 1);
   return {ns, nk};
 }
@@ -267,7 +266,7 @@ py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G,
   }
   if (!want_final) return py::cast(O);
   const On on(Q);
-  const auto [ns, nk] = merge_state(Tensor(), Tensor(), Fs.detach().to(Q.scalar_type()), Fg.detach(), Tensor(), b, h, d, on);
+  const auto [ns, nk] = final_state(Fs.detach().to(Q.scalar_type()), Fg.detach(), b, h, d, on);
   return py::make_tuple(O, py::make_tuple(ns, nk));
 }
 
@@ -429,11 +428,11 @@ py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, 
   if (!compress) return py::make_tuple(Y, state_, sok_);
 
   // ---- the cache becomes a new state
-  const Tensor S = at::empty({b, 1, h, state_rows(d), d}, Q.options()), gram = empty_f32({b, 1, h, d, d}, Q);
-  check(pr_chunk_state(dt, (int)b, (int)tk, (int)h, 1, (int)d, (int)tk, cptr(xt), cptr(xt), cptr(V), mptr(S), fmptr(gram), 1,
-                       on.device, on.stream),
-        "pr_chunk_state", 1);
-  const auto [ns, nk] = merge_state(state, sok, S, gram, total, b, h, d, on);
+  const int64_t D = d * (d + 1) / 2;
+  const Tensor ns = at::empty({b, h, D, d}, Q.options()), nk = empty_f32({b, h, D}, Q);
+  check(pr_compress_cache(dt, (int)b, (int)tk, (int)h, (int)d, cptr(xt), cptr(V), cptr(state), fptr(sok), fptr(total),
+                          mptr(ns), fmptr(nk), on.device, on.stream),
+        "pr_compress_cache", 1);
   return py::make_tuple(Y, ns, nk);
 }
 

@@ -18,6 +18,11 @@
 // for the tensor core), which is why the second factor is read once for two products; the values come in by TMA as the MN-major B operand; fp32 accumulation in
 // tensor memory.  The last grid slot in x computes the Gram matrix with both operands
 // in shared memory.
+//
+// EXACT (a token cache compressed into an inference state, retention/power_retention_maker.py:374-388): the read-out
+// writes the state in the exact layout, state * e^a_last + the cache's part in fp32, and sum_of_keys from the Gram
+// matrix.  Pairs that the block layout holds twice are written from one of their rows, with weight 2.  A pass of its
+// own that converted and added cost 75 us at b16 t2048 h32, half as much again as the bytes it moved needed.
 #include "host.cuh"
 #include "layout.cuh"
 #include "sm100.cuh"
@@ -49,10 +54,16 @@ struct ChunkStateParams {
   int key_weights;  // 1: weight 2 on pairs from different 16-blocks; 0: all weights 1
   void* out;        // [b, n, nh, D2, 64]
   float* gram;      // [b, n, nh, 64, 64] or null
+  // EXACT: the state to add to (null: none) with its sum_of_keys, the log decay [b, nh] (null: none), and the new
+  // sum_of_keys; `out` is the new state [b, nh, d(d+1)/2, d], `gram` is not written
+  const void* state;
+  const float* sok;
+  const float* a_last;
+  float* new_sok;
   int* status;
 };
 
-template <typename T>
+template <typename T, bool EXACT>
 __global__ void __maxnreg__(80)
 chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap tm_xt,
                    const __grid_constant__ CUtensorMap tm_xs, const __grid_constant__ CUtensorMap tm_w) {
@@ -76,7 +87,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
   // grid.x = slots * (batch, chunk, head) triples, slot fastest: the CTAs of one triple run together and
   // share their operand tiles through L2, and the triple count is not bound by the 65535 limit of grid.y
   const int n_tile_ctas = (p.n_tiles + NG - 1) / NG;
-  const int slots = n_tile_ctas + (p.gram ? 1 : 0);
+  const int slots = n_tile_ctas + (EXACT || p.gram ? 1 : 0);
   const int slot = (int)(blockIdx.x % (unsigned)slots);
   const bool gram_cta = (slot == n_tile_ctas);
   const int ch = (int)(blockIdx.x / (unsigned)slots);  // (batch * n + chunk) * nh + head
@@ -256,13 +267,50 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
       tmem_ld32(tmem + lane_addr + COL_ACC + grp * 64, acc);
       tmem_ld32(tmem + lane_addr + COL_ACC + grp * 64 + 32, acc + 32);
       tmem_wait_ld();
+      const float decay = !EXACT || p.state == nullptr ? 0.f : (p.a_last ? __expf(p.a_last[ch]) : 1.f);
       if (gram_cta) {
-        if (grp == 0 && row_in_tile < p.d && p.gram != nullptr) {
+        if (EXACT) {
+          if (grp == 0 && row_in_tile < HD) {
+            // row a of the Gram matrix holds the pairs (a, b >= a), which lie side by side
+            const size_t at = (size_t)ch * exact_dim(HD) + exact_row(HD, row_in_tile, row_in_tile) - row_in_tile;
+#pragma unroll
+            for (int j = 0; j < HD; ++j)
+              if (j >= row_in_tile)
+                p.new_sok[at + j] = (p.sok != nullptr ? p.sok[at + j] * decay : 0.f) +
+                                    __uint_as_float(acc[j]) * (j == row_in_tile ? 1.f : 2.f);
+          }
+        } else if (grp == 0 && row_in_tile < p.d && p.gram != nullptr) {
           float4* dst = reinterpret_cast<float4*>(p.gram + ((size_t)ch * p.d + row_in_tile) * p.d);
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             if (4 * j < p.d) dst[j] = make_float4(__uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]),
                                  __uint_as_float(acc[4 * j + 2]), __uint_as_float(acc[4 * j + 3]));
+        }
+      } else if (EXACT) {
+        if (valid && a <= b) {
+          const float wgt = a == b ? 1.f : 2.f;
+          const size_t at = ((size_t)ch * exact_dim(HD) + exact_row(HD, a, b)) * HD;
+          T* dst = static_cast<T*>(p.out) + at;
+          const T* old = static_cast<const T*>(p.state) + at;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint4 o[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+            if (p.state != nullptr) {
+              o[0] = *reinterpret_cast<const uint4*>(old + 16 * j);
+              o[1] = *reinterpret_cast<const uint4*>(old + 16 * j + 8);
+            }
+            const uint32_t ow[8] = {o[0].x, o[0].y, o[0].z, o[0].w, o[1].x, o[1].y, o[1].z, o[1].w};
+            uint32_t v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              // the reference rounds state * decay to the state's dtype before adding (:374-382)
+              const float2 raw = Pack2<T>::to_f32(ow[k]);
+              const float2 od = Pack2<T>::to_f32(Pack2<T>::from_f32(raw.x * decay, raw.y * decay));
+              v[k] = Pack2<T>::from_f32(od.x + wgt * __uint_as_float(acc[16 * j + 2 * k]),
+                                        od.y + wgt * __uint_as_float(acc[16 * j + 2 * k + 1]));
+            }
+            st_global_v8(dst + 16 * j, v);
+          }
         }
       } else if (valid) {
         const float wgt = p.key_weights ? ref_key_weight(a, b) : 1.f;
@@ -289,7 +337,7 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
   if (warp == 0) tmem_dealloc(tmem, cs::TMEM_COLS);
 }
 
-template <typename T>
+template <typename T, bool EXACT>
 static int launch_chunk_state(const ChunkStateParams& p, int b, const CUtensorMap& tm_xt, const CUtensorMap& tm_xs,
                               const CUtensorMap& tm_w, cudaStream_t stream) {
   using namespace cs;
@@ -297,13 +345,51 @@ static int launch_chunk_state(const ChunkStateParams& p, int b, const CUtensorMa
   static_assert(2 * GA_BYTES <= NS * W_BYTES, "Gram stages must fit in the value ring");
   int device = 0;
   PR_CUDA(cudaGetDevice(&device));  // the entry point has made the caller's device current
-  PR_SMEM_ATTR(chunk_state_kernel<T>, smem, device, true);
-  const long long ctas = (long long)((p.n_tiles + NG - 1) / NG + (p.gram ? 1 : 0)) * b * p.n_chunks * p.nh;
+  PR_SMEM_ATTR((chunk_state_kernel<T, EXACT>), smem, device, true);
+  const long long ctas = (long long)((p.n_tiles + NG - 1) / NG + (EXACT || p.gram ? 1 : 0)) * b * p.n_chunks * p.nh;
   PR_REQUIRE(ctas < (1ll << 31), PR_ERR_BAD_ARG, "%lld CTAs exceed the grid limit", ctas);
   dim3 grid((unsigned)ctas);
-  chunk_state_kernel<T><<<grid, THREADS, smem, stream>>>(p, tm_xt, tm_xs, tm_w);
+  chunk_state_kernel<T, EXACT><<<grid, THREADS, smem, stream>>>(p, tm_xt, tm_xs, tm_w);
   PR_CUDA(cudaGetLastError());
   return PR_OK;
+}
+
+// Fills the sizes and tensor maps and launches.
+template <bool EXACT>
+static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
+                           const void* v, ChunkStateParams p, int device, void* stream) {
+  PR_CUDA(cudaSetDevice(device));
+  p.n_tiles = (ref_dim(d) + 127) / 128;
+  p.nh = nh;
+  p.group = group;
+  p.c = c;
+  p.cp = (c + 63) / 64 * 64;
+  p.n_chunks = chunks_of(t, c);
+  p.t = t;
+  p.d = d;
+  int rc = status_word(device, &p.status, nullptr);
+  if (rc) return rc;
+  const int hx = nh * group;
+  CUtensorMap tm_xt, tm_xs, tm_w;
+  {
+    uint64_t dims[2] = {(uint64_t)p.cp, (uint64_t)b * p.n_chunks * hx * d};
+    uint64_t strides[2] = {0, (uint64_t)p.cp * 2};
+    uint32_t box[2] = {64, (uint32_t)d};
+    rc = make_tmap(&tm_xt, xt, 2, 2, dims, strides, box, true);
+    if (rc) return rc;
+    rc = make_tmap(&tm_xs, xts, 2, 2, dims, strides, box, true);
+    if (rc) return rc;
+  }
+  {
+    uint64_t dims[4] = {(uint64_t)d, (uint64_t)hx, (uint64_t)t, (uint64_t)b};
+    uint64_t strides[4] = {0, (uint64_t)d * 2, (uint64_t)hx * d * 2, (uint64_t)t * hx * d * 2};
+    uint32_t box[4] = {64, 1, 64, 1};
+    rc = make_tmap(&tm_w, v, 2, 4, dims, strides, box, true);
+    if (rc) return rc;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return dtype == PR_BF16 ? launch_chunk_state<__nv_bfloat16, EXACT>(p, b, tm_xt, tm_xs, tm_w, s)
+                          : launch_chunk_state<__half, EXACT>(p, b, tm_xt, tm_xs, tm_w, s);
 }
 
 }  // namespace pr
@@ -318,46 +404,35 @@ int pr::chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, co
              "null or misaligned pointer");
   PR_REQUIRE(gram == nullptr || (xts != nullptr && aligned16(xts) && aligned16(gram)), PR_ERR_BAD_ARG,
              "gram requested without a scaled operand");
-  PR_CUDA(cudaSetDevice(device));
-  ChunkStateParams p;
-  p.n_tiles = (ref_dim(d) + 127) / 128;
-  p.nh = nh;
-  p.group = group;
-  p.c = c;
-  p.cp = (c + 63) / 64 * 64;
-  p.n_chunks = chunks_of(t, c);
-  p.t = t;
-  p.d = d;
+  ChunkStateParams p{};
   p.key_weights = key_weights;
   p.out = out;
   p.gram = gram;
-  int rc = status_word(device, &p.status, nullptr);
-  if (rc) return rc;
-  const int hx = nh * group;
-  CUtensorMap tm_xt, tm_xs, tm_w;
-  {
-    uint64_t dims[2] = {(uint64_t)p.cp, (uint64_t)b * p.n_chunks * hx * d};
-    uint64_t strides[2] = {0, (uint64_t)p.cp * 2};
-    uint32_t box[2] = {64, (uint32_t)d};
-    rc = make_tmap(&tm_xt, xt, 2, 2, dims, strides, box, true);
-    if (rc) return rc;
-    rc = make_tmap(&tm_xs, gram ? xts : xt, 2, 2, dims, strides, box, true);
-    if (rc) return rc;
-  }
-  {
-    uint64_t dims[4] = {(uint64_t)d, (uint64_t)hx, (uint64_t)t, (uint64_t)b};
-    uint64_t strides[4] = {0, (uint64_t)d * 2, (uint64_t)hx * d * 2, (uint64_t)t * hx * d * 2};
-    uint32_t box[4] = {64, 1, 64, 1};
-    rc = make_tmap(&tm_w, v, 2, 4, dims, strides, box, true);
-    if (rc) return rc;
-  }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return dtype == PR_BF16 ? launch_chunk_state<__nv_bfloat16>(p, b, tm_xt, tm_xs, tm_w, s)
-                          : launch_chunk_state<__half>(p, b, tm_xt, tm_xs, tm_w, s);
+  return run_chunk_state<false>(dtype, b, t, nh, group, d, c, xt, gram ? xts : xt, v, p, device, stream);
 }
 
 extern "C" int pr_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
                               const void* v, void* out, float* gram, int key_weights, int device, void* stream) {
   PR_REQUIRE(d == pr::cs::HD, PR_ERR_BAD_ARG, "head dim %d: this entry point handles d = 64", d);
   return pr::chunk_state(dtype, b, t, nh, group, d, c, xt, xts, v, out, gram, key_weights, device, stream);
+}
+
+extern "C" int pr_compress_cache(int dtype, int b, int tk, int h, int d, const void* xt, const void* v, const void* state,
+                                 const float* sum_of_keys, const float* a_last, void* new_state, float* new_sum_of_keys,
+                                 int device, void* stream) {
+  using namespace pr;
+  PR_REQUIRE(d == cs::HD, PR_ERR_BAD_ARG, "head dim %d: inference states are built for d = 64", d);
+  PR_REQUIRE(b > 0 && tk > 0 && h > 0, PR_ERR_BAD_ARG, "bad sizes b=%d tk=%d h=%d", b, tk, h);
+  PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
+  PR_REQUIRE(xt && v && new_state && new_sum_of_keys, PR_ERR_BAD_ARG, "null pointer");
+  PR_REQUIRE((state == nullptr) == (sum_of_keys == nullptr), PR_ERR_BAD_ARG, "state and sum_of_keys come together");
+  PR_REQUIRE(aligned16(xt) && aligned16(v) && aligned16(state) && (reinterpret_cast<uintptr_t>(new_state) & 31u) == 0,
+             PR_ERR_BAD_ARG, "misaligned pointer (new_state: 32 bytes)");
+  ChunkStateParams p{};
+  p.out = new_state;
+  p.state = state;
+  p.sok = sum_of_keys;
+  p.a_last = a_last;
+  p.new_sok = new_sum_of_keys;
+  return run_chunk_state<true>(dtype, b, tk, h, 1, d, tk, xt, xt, v, p, device, stream);
 }

@@ -30,6 +30,9 @@ __host__ __device__ inline void ref_decode(int idx, int* a, int* b) {
   *a = rem >> 4;
   *b = 16 * y + (rem & 15);
 }
+// exact layout (inference states): the pairs a <= b in order, row (a, b)
+__host__ __device__ constexpr int exact_dim(int d) { return d * (d + 1) / 2; }
+__host__ __device__ constexpr int exact_row(int d, int a, int b) { return a * d - a * (a - 1) / 2 + (b - a); }
 // key-side weight of entry (a, b): 2 when a lies left of b's 16-block
 __host__ __device__ inline float ref_key_weight(int a, int b) { return a < (b & ~15) ? 2.f : 1.f; }
 
