@@ -493,7 +493,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         // the key and value tiles may be refilled (their last reads come before the async proxy's writes; the products
         // that read them have completed with the scores)
         fence_async_smem();
-        sm_da[tiles & 1][grp][r] = da;
+        sm_da[tiles & 1][first][r] = da;  // by step, not by group: a fixed order of the sum whatever the CTA did before
         meet();
         if (lane == 0) mbar_arrive(&kv_free[it & 1]);
 

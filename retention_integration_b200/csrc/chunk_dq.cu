@@ -363,7 +363,7 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
           __syncwarp();
           if (lane == 0) mbar_arrive(&op_full[grp]);
         }
-        sm_da[tiles & 1][grp][r] = da;
+        sm_da[tiles & 1][first][r] = da;  // by step, not by group: a fixed order of the sum whatever the CTA did before
         // the row warps meet; bounded like every wait
         __syncwarp();
         if (lane == 0) mbar_arrive(&rows);

@@ -137,3 +137,16 @@ def test_compressed_cache(cuda_device, tk, h, gated, old, dtype):
     tol = 4 * 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
     assert rel_l2(s1.double().cpu(), want.cpu()) < tol
     assert rel_l2(n1.double().cpu(), want_n.cpu()) < tol
+
+
+def test_same_bits_whatever_else_is_in_the_launch(cuda_device):
+    """Which tiles a persistent CTA has worked on before does not change the order of any sum."""
+    import retention_integration_b200 as prb
+
+    leaves, dO = _inputs(cuda_device, 4, 640, 48, 1, 64, True, torch.bfloat16, seed=9)
+    fn = lambda *x: prb.power_retention(*x, deg=2, chunk_size=320)
+    full = _grads(fn, leaves, dO)
+    for lo in (0, 17, 45):
+        part = _grads(fn, [x[:, :, lo:lo + 3].contiguous() for x in leaves], dO[:, :, lo:lo + 3].contiguous())
+        for name, x, y in zip(("O", "dQ", "dK", "dV", "dlog_G"), part, full):
+            assert torch.equal(x, y[:, :, lo:lo + 3]), (name, lo)
