@@ -50,6 +50,7 @@ struct ChunkStateParams {
   int group;        // operand heads summed into one output head (GQA ratio in backward)
   int c, cp;        // chunk length, padded to 64
   int n_chunks;     // chunks per batch element
+  int chunk0, n_run;  // the chunks that are wanted: n_run from chunk0 on
   int t, d;         // tokens (the last chunk may be shorter), features (a multiple of 16)
   int key_weights;  // 1: weight 2 on pairs from different 16-blocks; 0: all weights 1
   void* out;        // [b, n, nh, D2, 64]
@@ -90,10 +91,11 @@ chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap
   const int slots = n_tile_ctas + (EXACT || p.gram ? 1 : 0);
   const int slot = (int)(blockIdx.x % (unsigned)slots);
   const bool gram_cta = (slot == n_tile_ctas);
-  const int ch = (int)(blockIdx.x / (unsigned)slots);  // (batch * n + chunk) * nh + head
-  const int head = ch % p.nh;
-  const int chunk = (ch / p.nh) % p.n_chunks;
-  const int batch = ch / (p.nh * p.n_chunks);
+  const int which = (int)(blockIdx.x / (unsigned)slots);
+  const int head = which % p.nh;
+  const int chunk = p.chunk0 + (which / p.nh) % p.n_run;
+  const int batch = which / (p.nh * p.n_run);
+  const int ch = (batch * p.n_chunks + chunk) * p.nh + head;
   const int kblocks = (min(p.c, p.t - chunk * p.c) + TOK - 1) / TOK;
   const int total = kblocks * p.group;
 
@@ -346,7 +348,7 @@ static int launch_chunk_state(const ChunkStateParams& p, int b, const CUtensorMa
   int device = 0;
   PR_CUDA(cudaGetDevice(&device));  // the entry point has made the caller's device current
   PR_SMEM_ATTR((chunk_state_kernel<T, EXACT>), smem, device, true);
-  const long long ctas = (long long)((p.n_tiles + NG - 1) / NG + (EXACT || p.gram ? 1 : 0)) * b * p.n_chunks * p.nh;
+  const long long ctas = (long long)((p.n_tiles + NG - 1) / NG + (EXACT || p.gram ? 1 : 0)) * b * p.n_run * p.nh;
   PR_REQUIRE(ctas < (1ll << 31), PR_ERR_BAD_ARG, "%lld CTAs exceed the grid limit", ctas);
   dim3 grid((unsigned)ctas);
   chunk_state_kernel<T, EXACT><<<grid, THREADS, smem, stream>>>(p, tm_xt, tm_xs, tm_w);
@@ -357,8 +359,11 @@ static int launch_chunk_state(const ChunkStateParams& p, int b, const CUtensorMa
 // Fills the sizes and tensor maps and launches.
 template <bool EXACT>
 static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
-                           const void* v, ChunkStateParams p, int device, void* stream) {
+                           const void* v, ChunkStateParams p, int chunk0, int n_run, int device, void* stream) {
+  if (n_run <= 0) return PR_OK;
   PR_CUDA(cudaSetDevice(device));
+  p.chunk0 = chunk0;
+  p.n_run = n_run;
   p.n_tiles = (ref_dim(d) + 127) / 128;
   p.nh = nh;
   p.group = group;
@@ -395,7 +400,8 @@ static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, in
 }  // namespace pr
 
 int pr::chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
-                    const void* v, void* out, float* gram, int key_weights, int device, void* stream) {
+                    const void* v, void* out, float* gram, int key_weights, int chunk0, int n_run, int device,
+                    void* stream) {
   PR_REQUIRE(head_dim_ok(d), PR_ERR_BAD_ARG, "head dim %d: a multiple of 16 up to 64", d);
   PR_REQUIRE(b > 0 && t > 0 && nh > 0 && group > 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d heads=%d group=%d c=%d", b, t, nh, group, c);
@@ -408,13 +414,14 @@ int pr::chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, co
   p.key_weights = key_weights;
   p.out = out;
   p.gram = gram;
-  return run_chunk_state<false>(dtype, b, t, nh, group, d, c, xt, gram ? xts : xt, v, p, device, stream);
+  return run_chunk_state<false>(dtype, b, t, nh, group, d, c, xt, gram ? xts : xt, v, p, chunk0, n_run, device, stream);
 }
 
 extern "C" int pr_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
                               const void* v, void* out, float* gram, int key_weights, int device, void* stream) {
   PR_REQUIRE(d == pr::cs::HD, PR_ERR_BAD_ARG, "head dim %d: this entry point handles d = 64", d);
-  return pr::chunk_state(dtype, b, t, nh, group, d, c, xt, xts, v, out, gram, key_weights, device, stream);
+  return pr::chunk_state(dtype, b, t, nh, group, d, c, xt, xts, v, out, gram, key_weights, 0,
+                         pr::chunks_of(t, c > 0 ? c : 1), device, stream);
 }
 
 extern "C" int pr_compress_cache(int dtype, int b, int tk, int h, int d, const void* xt, const void* v, const void* state,
@@ -434,5 +441,5 @@ extern "C" int pr_compress_cache(int dtype, int b, int tk, int h, int d, const v
   p.sok = sum_of_keys;
   p.a_last = a_last;
   p.new_sok = new_sum_of_keys;
-  return run_chunk_state<true>(dtype, b, tk, h, 1, d, tk, xt, xt, v, p, device, stream);
+  return run_chunk_state<true>(dtype, b, tk, h, 1, d, tk, xt, xt, v, p, 0, 1, device, stream);
 }

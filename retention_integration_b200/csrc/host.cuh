@@ -69,9 +69,13 @@ int chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int h, i
 // pr_dout_prep with dy optional.
 int dout_prep(int dtype, long long rows, int d, const void* O, const void* dO, const float* l, void* dy, float* dl,
               int device, void* stream);
-// pr_chunk_state for every head dim of head_dim_ok.
+// pr_gate_prep / pr_chunk_state for the chunks [chunk0, chunk0 + n_run) only (pr_gate_prep: the copies; the gate sums are
+// made for all); chunk_state for every head dim of head_dim_ok.
+int gate_prep(int dtype, int b, int t, int h, int hx, int d, int c, const float* log_g, const void* x, float* a_out,
+              float* A_out, void* xt, const float* row_scale, void* xts, int query_side, float mult, int write_a,
+              int chunk0, int n_run, int device, void* stream);
 int chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts, const void* v,
-                void* out, float* gram, int key_weights, int device, void* stream);
+                void* out, float* gram, int key_weights, int chunk0, int n_run, int device, void* stream);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

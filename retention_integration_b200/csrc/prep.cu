@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(kGpThreads, NV == 4 ? 8 : 4)
 gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in, const T* __restrict__ x,
                  float* __restrict__ a_out, float* __restrict__ A_out, T* __restrict__ xt,
                  const float* __restrict__ row_scale, T* __restrict__ xts, int t, int h, int hx, int d, int c, int cp,
-                 int query_side, float mult, int write_a) {
+                 int query_side, float mult, int write_a, int chunk0, int chunk1) {
   extern __shared__ float sm_f[];
   float* sm_a = sm_f;                                    // [c] cumulative gates (given, or scanned here)
   // transposed tiles [d features][64 tokens], 128-byte rows; the 16-byte chunk holding tokens 8j..8j+7 of
@@ -91,7 +91,7 @@ gate_prep_kernel(const float* __restrict__ log_g, const float* __restrict__ a_in
       for (int i = tid; i < c; i += kGpThreads) a_out[(tok0 + i) * h + gh] = sm_a[i];
     if (tid == 0 && A_out != nullptr) A_out[((size_t)batch * n + chunk) * h + gh] = A;
   }
-  if (xt == nullptr) return;
+  if (xt == nullptr || chunk < chunk0 || chunk >= chunk1) return;
 
   // ---- gated transpose, 64 tokens at a time
   const int vec_per_row = d / 8;
@@ -360,10 +360,9 @@ extern "C" int pr_dout_prep(int dtype, long long rows, int d, const void* O, con
   return pr::dout_prep(dtype, rows, d, O, dO, l, dy, dl, device, stream);
 }
 
-extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c, const float* log_g, const void* x,
-                            float* a_out, float* A_out, void* xt, const float* row_scale, void* xts, int query_side,
-                            float mult, int write_a, int device, void* stream) {
-  using namespace pr;
+int pr::gate_prep(int dtype, int b, int t, int h, int hx, int d, int c, const float* log_g, const void* x, float* a_out,
+                  float* A_out, void* xt, const float* row_scale, void* xts, int query_side, float mult, int write_a,
+                  int chunk0, int n_run, int device, void* stream) {
   PR_REQUIRE(b > 0 && t > 0 && h > 0 && hx > 0 && hx % h == 0, PR_ERR_BAD_ARG, "bad sizes b=%d t=%d h=%d hx=%d", b, t,
              h, hx);
   PR_REQUIRE(c > 0, PR_ERR_BAD_ARG, "chunk size %d", c);
@@ -374,6 +373,7 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
              "x / xt null or misaligned");
   PR_REQUIRE(xts == nullptr || (xt != nullptr && row_scale != nullptr && aligned16(xts)), PR_ERR_BAD_ARG,
              "scaled copy requested without xt or row_scale");
+  if (n_run <= 0 && !write_a) return PR_OK;
   PR_CUDA(cudaSetDevice(device));
   const int cp = (c + 63) / 64 * 64;
   const size_t smem = (size_t)((c + 3) & ~3) * 4 + (size_t)2 * 64 * d * 2;
@@ -401,7 +401,7 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
     PR_SMEM_ATTR(KERNEL, smem, device, false);                                                                 \
     KERNEL<<<GRID, kGpThreads, smem, s>>>(LG, AIN, static_cast<const TT*>(x), a_out, A_out, static_cast<TT*>(XT), \
                                           row_scale, static_cast<TT*>(XTS), t, h, hx, d, c, cp, query_side, mult, \
-                                          WRITE);                                                              \
+                                          WRITE, chunk0, chunk0 + n_run);                                                              \
     PR_CUDA(cudaGetLastError());                                                                               \
   } while (0)
 #define PR_LAUNCH_PREP_S(TT, SC, GRID, LG, AIN, XT, XTS, WRITE)                                                 \
@@ -423,14 +423,14 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
   if (dtype == PR_BF16) {
     if (two_pass) {
       PR_LAUNCH_PREP(__nv_bfloat16, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, (void*)nullptr, 1);
-      PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_out, xt, xts, 0);
+      if (n_run > 0) PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_out, xt, xts, 0);
     } else {
       PR_LAUNCH_PREP(__nv_bfloat16, grid, log_g, a_in, xt, xts, write_a);
     }
   } else {
     if (two_pass) {
       PR_LAUNCH_PREP(__half, dim3(b * chunks_of(t, c) * h, 1), log_g, nullptr, nullptr, (void*)nullptr, 1);
-      PR_LAUNCH_PREP(__half, grid, log_g, a_out, xt, xts, 0);
+      if (n_run > 0) PR_LAUNCH_PREP(__half, grid, log_g, a_out, xt, xts, 0);
     } else {
       PR_LAUNCH_PREP(__half, grid, log_g, a_in, xt, xts, write_a);
     }
@@ -439,6 +439,13 @@ extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c
 #undef PR_LAUNCH_PREP_S
 #undef PR_LAUNCH_PREP_K
   return PR_OK;
+}
+
+extern "C" int pr_gate_prep(int dtype, int b, int t, int h, int hx, int d, int c, const float* log_g, const void* x,
+                            float* a_out, float* A_out, void* xt, const float* row_scale, void* xts, int query_side,
+                            float mult, int write_a, int device, void* stream) {
+  return pr::gate_prep(dtype, b, t, h, hx, d, c, log_g, x, a_out, A_out, xt, row_scale, xts, query_side, mult, write_a, 0,
+                       1 << 30, device, stream);
 }
 
 extern "C" int pr_gate_grad(int b, int t, int h, int hq, int c, const float* da_q, const float* gq, const float* da_k,

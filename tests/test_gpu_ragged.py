@@ -150,3 +150,19 @@ def test_same_bits_whatever_else_is_in_the_launch(cuda_device):
         part = _grads(fn, [x[:, :, lo:lo + 3].contiguous() for x in leaves], dO[:, :, lo:lo + 3].contiguous())
         for name, x, y in zip(("O", "dQ", "dK", "dV", "dlog_G"), part, full):
             assert torch.equal(x, y[:, :, lo:lo + 3]), (name, lo)
+
+
+@pytest.mark.parametrize("t,chunk", [(200, 128), (640, 128), (100, 128)])
+def test_states_that_nothing_reads_are_not_made(cuda_device, t, chunk):
+    """The last chunk's state (no final state asked for) and the gradient of the first one's stay unwritten in the
+    workspaces: whatever lies there, NaN here, reaches no result."""
+    import retention_integration_b200 as prb
+
+    leaves, dO = _inputs(cuda_device, 2, t, 2, 2, 64, True, torch.bfloat16, seed=t)
+    want = _grads(lambda *x: prb.power_retention(*x, return_final_state=True, chunk_size=chunk)[0], leaves, dO)
+    torch.cuda.empty_cache()
+    for mb in (1, 2, 4, 8, 16, 32, 64):  # what the caching allocator hands out next
+        torch.full((mb << 18,), float("nan"), device=cuda_device)
+    got = _grads(lambda *x: prb.power_retention(*x, chunk_size=chunk, switch_over_seq_len=1), leaves, dO)
+    for name, x, y in zip(("O", "dQ", "dK", "dV", "dlog_G"), got, want):
+        assert torch.equal(x, y), name
