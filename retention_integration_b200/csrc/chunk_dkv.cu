@@ -544,6 +544,9 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         g0 += w.n_steps + 2 * w.nI;
         ++tiles;
       } else {
+        // Not before the producer has come to this tile, and so has seen the last phase of this slot's kv_free: in a
+        // run of empty tiles the row warps could pass it, and two phases on the parity that it waits for looks open.
+        ok = mbar_wait(&kv_full[it & 1], (it >> 1) & 1, &abort_flag);
         __syncwarp();
         if (lane == 0) mbar_arrive(&kv_free[it & 1]);
       }

@@ -577,6 +577,9 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         u0 += w.nJ + w.nI;
         ++tiles;
       } else {
+        // Not before the producer has come to this tile, and so has seen the last phase of this slot's q_free: in a
+        // run of empty tiles the row warps could pass it, and two phases on the parity that it waits for looks open.
+        ok = mbar_wait(&q_full[it & 1], (it >> 1) & 1, &abort_flag);
         __syncwarp();
         if (lane == 0) mbar_arrive(&q_free[it & 1]);
       }
