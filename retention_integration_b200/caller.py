@@ -16,7 +16,7 @@ import math
 
 import torch
 
-from . import _lib
+from . import _lib, ops
 
 __all__ = ["rotary_tables", "prepare_qkvg", "GATE_BIAS"]
 
@@ -33,6 +33,24 @@ def rotary_tables(t: int, d: int, device):
     return torch.sin(ang), torch.cos(ang)
 
 
+class _TracedPrepareQKVG(torch.autograd.Function):
+    """prepare_qkvg as torch.jit.trace can record it: the tracer sees an autograd.Function as one node, and of the
+    native call only the allocations."""
+
+    @staticmethod
+    def forward(ctx, qkvg, sin, cos, h, hq, d, gated, gate_bias, half_split):
+        ctx.save_for_backward(qkvg, sin, cos)
+        ctx.cfg = (h, hq, d, gated, gate_bias, half_split)
+        out = ops.caller_prep_fwd(qkvg, cos, sin, *ctx.cfg)
+        return out if gated else out[:3]
+
+    @staticmethod
+    def backward(ctx, *grads):
+        qkvg, sin, cos = ctx.saved_tensors
+        grads = [x.contiguous() for x in grads] + [None] * (4 - len(grads))
+        return (ops.caller_prep_bwd(qkvg, cos, sin, *ctx.cfg, *grads), *[None] * 8)
+
+
 def prepare_qkvg(qkvg, sin, cos, h: int, hq: int, d: int, gated: bool = True, gate_bias: float = GATE_BIAS,
                  half_split: bool = False):
     """qkvg [b, t, W]: a token's row holds hq*d query, h*d key, h*d value features and (gated) h gate
@@ -42,4 +60,10 @@ def prepare_qkvg(qkvg, sin, cos, h: int, hq: int, d: int, gated: bool = True, ga
 
     W must be a multiple of 8 for 16-byte rows; a narrower projection (W = (hq+2h)d + h with h not a multiple
     of 8) is padded here with one extra copy - size `c_attn`'s out_features to a multiple of 8 to avoid it."""
-    return _lib.host().prepare_qkvg(qkvg, sin, cos, h, hq, d, gated, gate_bias, half_split)
+    out = _lib.host().prepare_qkvg(qkvg, sin, cos, h, hq, d, gated, gate_bias, half_split)
+    if out is not None:
+        return out
+    x = torch.nn.functional.pad(qkvg, (0, -qkvg.shape[-1] % 8)).contiguous()
+    out = _TracedPrepareQKVG.apply(x, sin.float().contiguous(), cos.float().contiguous(), h, hq, d, bool(gated),
+                                   float(gate_bias), bool(half_split))
+    return out if gated else (*out, None)

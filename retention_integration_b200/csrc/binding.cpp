@@ -7,6 +7,7 @@
 // Everything runs on torch's current stream of the tensors' device.  Workspaces come from the caching allocator on
 // every call: they are tied to the stream, so calls from several threads and streams do not share any.
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -194,11 +195,17 @@ std::tuple<Tensor, Tensor> final_state(const Tensor& S, const Tensor& gram, int6
   return {ns, nk};
 }
 
+// torch.jit.trace records torch's own operators.  Of a call made here it would see the allocations of the results and
+// none of the kernels, and the trace would give back memory that nothing has written.  The Python callers have an
+// autograd.Function for this case, which the tracer records as one node: the entry points answer None.
+bool being_traced() { return at::tracer::impl::is_dispatch_enabled(); }
+
 // power_retention with the blocking chosen here.  chunk 0 / switch_over -1: not given.  Returns None for the head
-// dims that the caller has to widen first.
+// dims that the caller has to widen first, and where the caller's own path has to run.
 py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G, const OptTensor& state,
                            const OptTensor& sok, bool want_final, int64_t deg, double scale, int64_t chunk,
                            int64_t switch_over, bool auto_chunk) {
+  if (being_traced()) return py::none();
   require(deg % 2 == 0, "deg must be even");
   require(Q.dim() == 4 && K.dim() == 4 && V.dim() == 4, "Q, K, V must be [batch, seq_len, heads, dim]");
   const int64_t b = Q.size(0), t = Q.size(1), hq = Q.size(2), d = Q.size(3), h = K.size(2);
@@ -521,8 +528,8 @@ class PrepareQKVG : public torch::autograd::Function<PrepareQKVG> {
   }
 };
 
-py::tuple prepare_qkvg(Tensor x, Tensor sin, Tensor cos, int64_t h, int64_t hq, int64_t d, bool gated, double bias,
-                       bool half_split) {
+py::object prepare_qkvg(Tensor x, Tensor sin, Tensor cos, int64_t h, int64_t hq, int64_t d, bool gated, double bias,
+                        bool half_split) {
   pr_require(x.is_cuda() && x.dim() == 3 && (x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf),
              "prepare_qkvg wants a CUDA bf16/fp16 tensor [b, t, W]");
   const int64_t used = (hq + 2 * h) * d + (gated ? h : 0), t = x.size(1);
@@ -539,6 +546,7 @@ py::tuple prepare_qkvg(Tensor x, Tensor sin, Tensor cos, int64_t h, int64_t hq, 
                  (sin.dim() == 2 || (sin.dim() == 3 && sin.size(0) == x.size(0))) && sin.device() == x.device() &&
                  cos.device() == x.device(),
              "sin / cos must be [t, d/2] (or [b, t, d/2]) for the tokens of the projection");
+  if (being_traced()) return py::none();
   const variable_list out = PrepareQKVG::apply(x, sin, cos, h, hq, d, gated, bias, half_split);
   if (gated) return py::make_tuple(out[0], out[1], out[2], out[3]);
   return py::make_tuple(out[0], out[1], out[2], py::none());

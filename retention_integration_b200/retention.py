@@ -18,7 +18,8 @@ from ._lib import PRError
 _SUPPORTED_D = (64,)
 
 # True: forward and backward are one native call each; False: the same kernels are launched one by one from
-# Python, on padded sequences (per-kernel timing, debugging).  The results are identical.
+# Python, on padded sequences (per-kernel timing, debugging; torch.jit.trace also takes this path, because it can record
+# the autograd.Functions here and not the native call).  The results are identical.
 NATIVE_SEQUENCER = True
 
 

@@ -1,0 +1,50 @@
+"""The native host path (csrc/binding.cpp) under the tools that a caller may wrap around it."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(dev, b, t, h, hq, d=64, seed=0):
+    g = torch.Generator(dev).manual_seed(seed)
+    Q, K, V = (torch.randn(b, t, n, d, generator=g, device=dev).to(torch.bfloat16) for n in (hq, h, h))
+    return [Q, K, V, F.logsigmoid(torch.randn(b, t, h, generator=g, device=dev))]
+
+
+def _traced(fn, example, leaves):
+    """(results, gradients) of the trace made from `example` and of `fn` itself, both on `leaves`."""
+    out = []
+    for f in (torch.jit.trace(fn, tuple(example), check_trace=False), fn):
+        y = f(*leaves)
+        y = list(y) if isinstance(y, (tuple, list)) else [y]
+        out.append(y + list(torch.autograd.grad(sum((i + 1) * x.float().sum() for i, x in enumerate(y)), leaves)))
+    return out
+
+
+@pytest.mark.parametrize("t,d,chunk", [(256, 64, None), (256, 64, 64), (200, 64, 64), (96, 32, None)])
+def test_a_trace_computes(cuda_device, t, d, chunk):
+    """torch.jit.trace records the operator, not just the allocation of its result."""
+    import retention_integration_b200 as prb
+
+    leaves = [x.requires_grad_() for x in _inputs(cuda_device, 1, t, 2, 4, d, seed=1)]
+    got, want = _traced(lambda *x: prb.power_retention(*x, chunk_size=chunk), _inputs(cuda_device, 1, t, 2, 4, d), leaves)
+    for x, y in zip(got, want):
+        # the traced path pads the sequence, which regroups no sum but those over whole zero tiles
+        assert float((x.float() - y.float()).norm()) <= 1e-3 * float(y.float().norm())
+
+
+@pytest.mark.parametrize("gated,half_split,extra", [(True, False, 0), (False, True, 0), (True, True, 6)])
+def test_a_trace_of_the_glue_computes(cuda_device, gated, half_split, extra):
+    import retention_integration_b200 as prb
+
+    t, h, hq, d = 40, 2, 4, 64
+    W = (hq + 2 * h) * d + (h if gated else 0) + extra
+    g = torch.Generator(cuda_device).manual_seed(0)
+    a, b = (torch.randn(2, t, W, generator=g, device=cuda_device).to(torch.bfloat16) for _ in range(2))
+    sin, cos = prb.rotary_tables(t, d, cuda_device)
+    fn = lambda x: tuple(y for y in prb.prepare_qkvg(x, sin, cos, h, hq, d, gated=gated, half_split=half_split)
+                         if y is not None)
+    got, want = _traced(fn, [a], [b.requires_grad_()])
+    for x, y in zip(got, want):
+        assert torch.equal(x, y)
