@@ -13,9 +13,11 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <optional>
 #include <string>
 #include <tuple>
@@ -200,23 +202,25 @@ std::tuple<Tensor, Tensor> final_state(const Tensor& S, const Tensor& gram, int6
 // autograd.Function for this case, which the tracer records as one node: the entry points answer None.
 bool being_traced() { return at::tracer::impl::is_dispatch_enabled(); }
 
-// power_retention with the blocking chosen here.  chunk 0 / switch_over -1: not given.  Returns None for the head
-// dims that the caller has to widen first, and where the caller's own path has to run.
+// power_retention with the blocking chosen here.  Returns None for the head dims that the caller has to widen first, and
+// where the caller's own path has to run.  switch_over is a double because callers say "never" with infinity.
 py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G, const OptTensor& state,
-                           const OptTensor& sok, bool want_final, int64_t deg, double scale, int64_t chunk,
-                           int64_t switch_over, bool auto_chunk) {
+                           const OptTensor& sok, bool want_final, int64_t deg, double scale,
+                           std::optional<int64_t> chunk_size, std::optional<double> switch_over, bool auto_chunk) {
   if (being_traced()) return py::none();
   require(deg % 2 == 0, "deg must be even");
+  pr_require(!chunk_size.has_value() || *chunk_size > 0, "chunk_size must be positive");
+  pr_require(state.has_value() == sok.has_value(), "initial_state is the pair (state, sum_of_keys)");
+  const int64_t chunk = chunk_size.value_or(0);  // 0: not given
   require(Q.dim() == 4 && K.dim() == 4 && V.dim() == 4, "Q, K, V must be [batch, seq_len, heads, dim]");
   const int64_t b = Q.size(0), t = Q.size(1), hq = Q.size(2), d = Q.size(3), h = K.size(2);
   const bool with_state = state.has_value() || want_final;
   if ((d == 16 || d == 32) && with_state)
     throw PrError("states are kept for head dim 64 only (got " + std::to_string(d) + ")");
   if (d == 48) return py::none();
-  int64_t c = (auto_chunk && deg == 2) ? pr_fast_chunk(t, (int)chunk) : chunk;
-  if (c != chunk) switch_over = c ? c : -1;
-  else if (c > 0 && switch_over < 0) switch_over = c;
-  const bool quadratic = switch_over < 0 || c == 0 || (t + c - 1) / c * c <= switch_over;
+  int64_t c = (auto_chunk && deg == 2) ? pr_fast_chunk(t, (int)std::min<int64_t>(chunk, std::numeric_limits<int>::max())) : chunk;
+  if (c != chunk || !switch_over.has_value()) switch_over = c ? std::optional<double>((double)c) : std::nullopt;
+  const bool quadratic = !switch_over.has_value() || c == 0 || (double)((t + c - 1) / c * c) <= *switch_over;
   if (deg != 2 && !(deg == 4 && quadratic && !with_state))
     throw PrError("deg=" + std::to_string(deg) +
                   ": the state kernels implement deg=2 (as the reference's state operators do); "
@@ -246,7 +250,6 @@ py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G,
                     any_of([](const Tensor& t) { return t._fw_grad(0).defined(); });
   Tensor Cs, Cg;
   if (state.has_value()) {
-    pr_require(sok.has_value(), "initial_state is the pair (state, sum_of_keys)");
     check_state(*state, *sok, b, h, d);
     const On on(Q);
     const Tensor s = aligned(state->detach().to(Q.scalar_type())), k = aligned(sok->detach());
@@ -347,13 +350,12 @@ void gate_sums(const Tensor& K, const Tensor& G, const Tensor& a, const Tensor& 
 }
 
 py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, const OptTensor& log_G,
-                    const OptTensor& state_, const OptTensor& sok_, int64_t deg, std::optional<double> scale_,
-                    std::optional<int64_t> switch_over) {
+                    const OptTensor& state_, const OptTensor& sok_, std::optional<double> scale_,
+                    std::optional<double> switch_over) {
   const at::NoGradGuard no_grad;
   const bool has_cache = K_.has_value() && V_.has_value(), has_state = state_.has_value();
   require(has_cache || has_state, "initial_state or cache must be provided for inference");
   require(has_state == sok_.has_value(), "initial_state and sum_of_keys come together");
-  if (deg != 2) throw PrError("deg=" + std::to_string(deg) + ": the state kernels implement deg=2");
   require(Q0.dim() == 4, "Q must be [batch, tokens, heads, dim]");
   pr_require(Q0.is_cuda(), "tensors must be CUDA tensors: this package has no CPU path");
   const int64_t b = Q0.size(0), tq = Q0.size(1), hq = Q0.size(2), d = Q0.size(3);
@@ -390,7 +392,7 @@ py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, 
     require(G.device() == Q0.device(), "tensors must live on one device");
     if (G.scalar_type() != at::kFloat) G = G.to(at::kFloat);
   }
-  const bool compress = switch_over.has_value() && tk >= *switch_over;
+  const bool compress = switch_over.has_value() && (double)tk >= *switch_over;
 
   Tensor Y;
   if (tq == 1 && has_state && !compress) {

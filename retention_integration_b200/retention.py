@@ -191,9 +191,8 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     assert deg % 2 == 0, f"deg must be even: {deg=}"
     if NATIVE_SEQUENCER and not ops.launch_log.timing:
         state, sok = initial_state if initial_state is not None else (None, None)
-        out = _lib.host().power_retention(Q, K, V, log_G, state, sok, return_final_state, deg, scale or 0.0,
-                                          chunk_size or 0, -1 if switch_over_seq_len is None else switch_over_seq_len,
-                                          AUTO_CHUNK)
+        out = _lib.host().power_retention(Q, K, V, log_G, state, sok, return_final_state, int(deg), scale or 0.0,
+                                          chunk_size, switch_over_seq_len, AUTO_CHUNK)
         if out is not None:
             return out
     d_orig = Q.shape[-1]
@@ -270,4 +269,6 @@ def power_retention_inference(Q, K, V, log_G=None, initial_state=None, sum_of_ke
     States use the exact expansion layout, D = d*(d+1)/2 (2080 at d = 64); the reference's
     padded layout (2560) converts with layout.to_reference_layout / from_reference_layout.
     """
-    return _lib.host().inference(Q, K, V, log_G, initial_state, sum_of_keys, deg, scale, switch_over_seq_len)
+    if deg != 2:
+        raise PRError(f"deg={deg}: the state kernels implement deg=2")
+    return _lib.host().inference(Q, K, V, log_G, initial_state, sum_of_keys, scale, switch_over_seq_len)

@@ -1,0 +1,45 @@
+"""What the public calls accept and refuse of their plain arguments.  CPU tensors are refused last of all, so a call that
+gets as far as that has had its other arguments accepted; nothing here needs a GPU."""
+import math
+
+import pytest
+import torch
+
+import retention_integration_b200 as prb
+from retention_integration_b200 import retention
+
+Q = torch.zeros(1, 256, 2, 64, dtype=torch.bfloat16)
+
+
+@pytest.mark.parametrize("value", [math.inf, 512.0, 100.5, 0, -1, 2 ** 40, None])
+def test_switch_over_may_be_any_number(value):
+    with pytest.raises(prb.PRError, match="CUDA"):
+        prb.power_retention(Q, Q, Q, chunk_size=128, switch_over_seq_len=value)
+    with pytest.raises(prb.PRError, match="CUDA"):
+        prb.power_retention_inference(Q, Q, Q, switch_over_seq_len=value)
+
+
+def test_deg_may_be_a_whole_float():
+    with pytest.raises(prb.PRError, match="CUDA"):
+        prb.power_retention(Q, Q, Q, deg=2.0)
+    with pytest.raises(prb.PRError, match="CUDA"):
+        prb.power_retention_inference(Q, Q, Q, deg=2.0)
+    with pytest.raises(prb.PRError, match="deg=4"):
+        prb.power_retention_inference(Q, Q, Q, deg=4)
+    with pytest.raises(AssertionError):
+        prb.power_retention(Q, Q, Q, deg=2.5)
+
+
+@pytest.mark.parametrize("auto", [False, True])
+@pytest.mark.parametrize("chunk", [0, -1, -128])
+def test_a_chunk_has_tokens(monkeypatch, auto, chunk):
+    monkeypatch.setattr(retention, "AUTO_CHUNK", auto)
+    with pytest.raises(prb.PRError, match="chunk_size"):
+        prb.power_retention(Q, Q, Q, chunk_size=chunk)
+
+
+def test_half_a_state_is_refused():
+    sok = torch.zeros(1, 2, 2080)
+    for pair in ((None, sok), (torch.zeros(1, 2, 2080, 64, dtype=torch.bfloat16), None)):
+        with pytest.raises(prb.PRError, match="pair"):
+            prb.power_retention(Q, Q, Q, initial_state=pair)
