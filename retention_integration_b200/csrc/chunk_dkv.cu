@@ -413,10 +413,18 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
           const float rs = r_n;
           // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
           // key and per query instead of one per pair (both exponents <= 0 off the diagonal for gates
-          // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps whose queries all
+          // <= 0; a warp falls back to the per-pair form if one exceeds 80).  The query's factor also holds 1 / l_i, so
+          // the key's exponent is tested together with the largest log l_i: near the diagonal, where the gates'
+          // factors make up for each other, e^{a_i - r} / l_i would lose its bits below the smallest normal number
+          // otherwise (15 % off in dK and dV with gates of -1.24 a token and row sums of 1e12).  It cannot grow too large:
+          // l_i >= e^{a_i - r} (s q_i.k_r)^deg, the weight of the key at r.  Steps whose queries all
           // come after this warp's keys need no mask; a warp whose keys all come after the step's
           // queries writes zeros without reading the scores.
-          const bool sep = !__any_sync(0xffffffffu, fmaxf(fmaxf(av[0], av[1]) - rs, rs - a_j) > 80.f);
+          float log_l = 0.f;
+          if (gated)
+            log_l = __logf(__uint_as_float(
+                __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fabsf(lv[0]), fabsf(lv[1])), 1.f)))));
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(fmaxf(av[0], av[1]) - rs, rs - a_j + log_l) > 80.f);
           const float c_j = sep ? sdeg * __expf(rs - a_j) : sdeg;
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
