@@ -8,6 +8,7 @@
 // Memory: the caller allocates everything.  `saved` is what the backward needs from the
 // forward (gate sums, row sums, scanned states and Gram matrices); `scratch` is dead when the
 // call returns its work to the stream and may be reused by the next call on the same stream.
+#include <atomic>
 #include <mutex>
 
 #include "host.cuh"
@@ -97,17 +98,27 @@ Saved carve_saved(void* base, const Sizes& s) {
 // saved states, then chunk_dq) needs nothing from the reverse scan, which heads the key side
 // (gate_prep, chunk_state, scan, expand_grad, chunk_dkv).  The query side is enqueued on a second
 // stream, forked from and joined back into the caller's stream with events, so that its CTAs fill
-// the partial last wave of each key-side launch (and vice versa).  One stream and event pair per
-// device, created on first use (outside any stream capture: a capture of the caller's stream
-// then records the fork and the join like any cross-stream dependency); `mu` is held while a
-// backward is being enqueued, so concurrent callers take turns at using the pair.
+// the partial last wave of each key-side launch (and vice versa).
+//
+// A device has kSideStreams such streams, created together by its first backward outside a capture and kept for the
+// process.  Which one a backward uses depends on its caller's stream, so that callers on different streams seldom wait
+// for one another; `mu` is held while a backward is being enqueued.  While a caller's stream is being captured, the
+// second stream belongs to that capture until it ends (the fork and the join are recorded like any cross-stream
+// dependency): a backward of another stream that comes to it meanwhile is enqueued on its caller's stream alone,
+// because it could neither join that capture nor leave it undisturbed.
 struct SideStream {
   std::mutex mu;
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
 constexpr int kMaxDevices = 64;
-SideStream g_side[kMaxDevices];
+constexpr int kSideStreams = 8;
+struct DeviceSides {
+  std::mutex mu;  // creation
+  std::atomic<bool> ready{false};
+  SideStream side[kSideStreams];
+};
+DeviceSides g_side[kMaxDevices];
 
 bool overlap_enabled() {
   static const bool on = [] {
@@ -117,12 +128,35 @@ bool overlap_enabled() {
   return on;
 }
 
-// with s->mu held
-int side_stream_ready(SideStream* s) {
-  if (s->stream != nullptr) return PR_OK;
-  PR_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-  PR_CUDA(cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming));
-  PR_CUDA(cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming));
+// The capture that a stream takes part in; 0: none, ~0: one that has failed and not ended yet.
+int capture_of(cudaStream_t stream, unsigned long long* id) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  *id = 0;
+  PR_CUDA(cudaStreamGetCaptureInfo(stream, &status, id));
+  if (status != cudaStreamCaptureStatusActive) *id = status == cudaStreamCaptureStatusNone ? 0 : ~0ull;
+  return PR_OK;
+}
+
+// The device's streams, or none yet (*out = null) when the first backward is being captured.
+int side_streams(int device, cudaStream_t caller, DeviceSides** out) {
+  DeviceSides& d = g_side[device];
+  *out = &d;
+  if (d.ready.load(std::memory_order_acquire)) return PR_OK;
+  std::lock_guard<std::mutex> lock(d.mu);
+  if (d.ready.load(std::memory_order_relaxed)) return PR_OK;
+  unsigned long long capture = 0;
+  int rc = capture_of(caller, &capture);
+  if (rc) return rc;
+  if (capture) {
+    *out = nullptr;
+    return PR_OK;
+  }
+  for (SideStream& s : d.side) {
+    if (!s.stream) PR_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+    if (!s.fork) PR_CUDA(cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming));
+    if (!s.join) PR_CUDA(cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming));
+  }
+  d.ready.store(true, std::memory_order_release);
   return PR_OK;
 }
 
@@ -133,13 +167,25 @@ class Fork {
     PR_REQUIRE(device >= 0 && device < kMaxDevices, PR_ERR_BAD_ARG, "device ordinal %d out of range", device);
     main_ = static_cast<cudaStream_t>(stream);
     if (!overlap_enabled()) return PR_OK;
-    lock_ = std::unique_lock<std::mutex>(g_side[device].mu);
     PR_CUDA(cudaSetDevice(device));
-    int rc = side_stream_ready(&g_side[device]);
-    if (rc) return rc;
-    PR_CUDA(cudaEventRecord(g_side[device].fork, main_));
-    PR_CUDA(cudaStreamWaitEvent(g_side[device].stream, g_side[device].fork, 0));
-    s_ = &g_side[device];
+    DeviceSides* d = nullptr;
+    int rc = side_streams(device, main_, &d);
+    if (rc || !d) return rc;
+    // handles are pointers or small numbers: mixed so that both spread over the streams
+    const uint64_t mix = reinterpret_cast<uintptr_t>(stream) * 0x9E3779B97F4A7C15ull;
+    SideStream& s = d->side[mix >> 61];
+    static_assert(kSideStreams == 8, "three bits of the mixed handle");
+    std::unique_lock<std::mutex> lock(s.mu);
+    unsigned long long theirs = 0, ours = 0;
+    if ((rc = capture_of(s.stream, &theirs))) return rc;
+    if (theirs) {
+      if ((rc = capture_of(main_, &ours))) return rc;
+      if (ours != theirs) return PR_OK;  // another caller's capture
+    }
+    PR_CUDA(cudaEventRecord(s.fork, main_));
+    PR_CUDA(cudaStreamWaitEvent(s.stream, s.fork, 0));
+    lock_ = std::move(lock);
+    s_ = &s;
     return PR_OK;
   }
   void* side() const { return s_ ? s_->stream : main_; }

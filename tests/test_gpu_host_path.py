@@ -48,3 +48,72 @@ def test_a_trace_of_the_glue_computes(cuda_device, gated, half_split, extra):
     got, want = _traced(fn, [a], [b.requires_grad_()])
     for x, y in zip(got, want):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("chunk", [None, 64])
+def test_a_capture_leaves_other_streams_alone(cuda_device, chunk):
+    """While one stream is being captured, forward and backward run on others, and the capture holds its own work alone.
+    (More streams than the library keeps for overlapping, so that some share the captured caller's.)"""
+    import retention_integration_b200 as prb
+
+    def step(leaves, dO):
+        return torch.autograd.grad(prb.power_retention(*leaves, chunk_size=chunk), leaves, dO)
+
+    args = []
+    for seed in (0, 1):
+        leaves = [x.requires_grad_() for x in _inputs(cuda_device, 1, 256, 2, 4, seed=seed)]
+        args.append((leaves, torch.randn_like(leaves[0])))
+    want = [step(*a) for a in args]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(24)]
+    for s in streams:  # memory for the calls below: the allocator need not ask the driver during the capture
+        with torch.cuda.stream(s):
+            step(*args[1])
+    torch.cuda.synchronize()
+    graph, others = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        captured = [step(*args[0])]
+        for s in streams:
+            with torch.cuda.stream(s):
+                others.append(step(*args[1]))
+        captured.append(step(*args[0]))
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    for got, ref in [(c, want[0]) for c in captured] + [(o, want[1]) for o in others]:
+        for x, y in zip(got, ref):
+            assert torch.equal(x, y)
+
+
+def test_callers_on_many_streams_and_threads(cuda_device):
+    """Backward passes enqueued from several threads on streams of their own, overlapping on the GPU."""
+    import threading
+
+    import retention_integration_b200 as prb
+
+    cases = []
+    for seed, (t, chunk) in enumerate([(256, None), (640, 128), (300, 128), (128, None)] * 3):
+        leaves = [x.requires_grad_() for x in _inputs(cuda_device, 1, t, 2, 4, seed=seed)]
+        cases.append((leaves, torch.randn_like(leaves[0]), chunk))
+
+    def step(leaves, dO, chunk):
+        return torch.autograd.grad(prb.power_retention(*leaves, chunk_size=chunk), leaves, dO)
+
+    want = [step(*c) for c in cases]
+    torch.cuda.synchronize()
+    got = [None] * len(cases)
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                got[i] = step(*cases[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(cases))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        for x, y in zip(g, w):
+            assert torch.equal(x, y)
