@@ -10,6 +10,7 @@
 #include <ATen/TracerMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -36,7 +37,9 @@ std::atomic<long long> g_launches{0};  // kernels launched through this module
 PyObject* g_error = nullptr;           // the package's PRError
 
 // Messages of the three kinds of failure a caller can see.  c10::Error would reach Python as RuntimeError too, but
-// PRError and AssertionError are what the package promises.
+// PRError and AssertionError are what the package promises.  The module's exception translator turns them into those for
+// a call from Python; a backward pass is called by the autograd engine, which knows torch's own carrier of a Python
+// exception (in_engine).
 struct PrError : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
@@ -53,6 +56,19 @@ void check(int rc, const char* what, int kernels) {
   if (rc != PR_OK)
     throw PrError(std::string(what) + " failed with code " + std::to_string(rc) + ": " + pr_last_error());
   g_launches.fetch_add(kernels, std::memory_order_relaxed);
+}
+
+template <typename F>
+auto in_engine(F&& f) -> decltype(f()) {
+  try {
+    return f();
+  } catch (const PrError& e) {
+    py::gil_scoped_acquire gil;
+    PyErr_SetString(g_error ? g_error : PyExc_RuntimeError, e.what());
+    python_error carried;
+    carried.persist();
+    throw carried;
+  }
 }
 
 int dtype_code(const Tensor& t) {
@@ -145,6 +161,9 @@ class Retention : public torch::autograd::Function<Retention> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return in_engine([&] { return run_backward(ctx, grads); });
+  }
+  static variable_list run_backward(AutogradContext* ctx, const variable_list& grads) {
     const auto s = ctx->get_saved_variables();
     const Tensor &Q = s[0], &K = s[1], &V = s[2], &G = s[3], &O = s[4], &saved = s[5];
     variable_list out(10);
@@ -505,6 +524,9 @@ class PrepareQKVG : public torch::autograd::Function<PrepareQKVG> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return in_engine([&] { return run_backward(ctx, grads); });
+  }
+  static variable_list run_backward(AutogradContext* ctx, const variable_list& grads) {
     const auto s = ctx->get_saved_variables();
     const Tensor &x = s[0], &sin = s[1], &cos = s[2];
     const On on(x);

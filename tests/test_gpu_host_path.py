@@ -117,3 +117,35 @@ def test_callers_on_many_streams_and_threads(cuda_device):
     for g, w in zip(got, want):
         for x, y in zip(g, w):
             assert torch.equal(x, y)
+
+
+def _widened():
+    """Saved 16-bit tensors come back in 32 bits, which the backward pass refuses before it launches anything."""
+    return torch.autograd.graph.saved_tensors_hooks(lambda x: x, lambda x: x.float() if x.dtype == torch.bfloat16 else x)
+
+
+@pytest.mark.parametrize("chunk", [None, 64])
+def test_a_failed_backward_raises_the_packages_error(cuda_device, chunk):
+    import retention_integration_b200 as prb
+
+    leaves = [x.requires_grad_() for x in _inputs(cuda_device, 1, 256, 2, 4)]
+    with _widened():
+        out = prb.power_retention(*leaves, chunk_size=chunk)
+    with pytest.raises(prb.PRError, match="float16"):
+        out.sum().backward()
+    with torch.autograd.detect_anomaly(check_nan=False):
+        with _widened():
+            out = prb.power_retention(*leaves, chunk_size=chunk)
+        with pytest.raises(prb.PRError, match="float16"):
+            out.sum().backward()
+
+
+def test_a_failed_backward_of_the_glue_raises_the_packages_error(cuda_device):
+    import retention_integration_b200 as prb
+
+    x = torch.randn(1, 64, 4 * 64 + 8, device=cuda_device).to(torch.bfloat16).requires_grad_()
+    sin, cos = prb.rotary_tables(64, 64, cuda_device)
+    with _widened():
+        Q, K, V, log_g = prb.prepare_qkvg(x, sin, cos, 1, 2, 64)
+    with pytest.raises(prb.PRError, match="float16"):
+        Q.sum().backward()
