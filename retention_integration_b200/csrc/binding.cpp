@@ -22,6 +22,7 @@
 #include <optional>
 #include <string>
 #include <tuple>
+#include <variant>
 
 #include "../../include/pr_b200.h"
 
@@ -206,8 +207,10 @@ void check_state(const Tensor& state, const Tensor& sok, int64_t b, int64_t h, i
   pr_require(state.is_cuda() && sok.is_cuda(), "the state must live on a CUDA device: this package has no CPU path");
 }
 
+using StatePair = std::tuple<Tensor, Tensor>;
+
 // The pair after the last token in the exact layout, from the scans' carries.
-std::tuple<Tensor, Tensor> final_state(const Tensor& S, const Tensor& gram, int64_t b, int64_t h, int64_t d, const On& on) {
+StatePair final_state(const Tensor& S, const Tensor& gram, int64_t b, int64_t h, int64_t d, const On& on) {
   const int64_t D = d * (d + 1) / 2;
   const Tensor ns = at::empty({b, h, D, d}, S.options()), nk = empty_f32({b, h, D}, S);
   check(pr_state_merge(dtype_code(S), (int)b, (int)h, (int)d, nullptr, nullptr, cptr(S), fptr(gram), nullptr, mptr(ns),
@@ -221,12 +224,15 @@ std::tuple<Tensor, Tensor> final_state(const Tensor& S, const Tensor& gram, int6
 // autograd.Function for this case, which the tracer records as one node: the entry points answer None.
 bool being_traced() { return at::tracer::impl::is_dispatch_enabled(); }
 
+using Retained = std::variant<Tensor, std::tuple<Tensor, StatePair>>;  // with a final state: (output, pair)
+
 // power_retention with the blocking chosen here.  Returns None for the head dims that the caller has to widen first, and
 // where the caller's own path has to run.  switch_over is a double because callers say "never" with infinity.
-py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G, const OptTensor& state,
-                           const OptTensor& sok, bool want_final, int64_t deg, double scale,
-                           std::optional<int64_t> chunk_size, std::optional<double> switch_over, bool auto_chunk) {
-  if (being_traced()) return py::none();
+std::optional<Retained> power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G, const OptTensor& state,
+                                        const OptTensor& sok, bool want_final, int64_t deg, double scale,
+                                        std::optional<int64_t> chunk_size, std::optional<double> switch_over,
+                                        bool auto_chunk) {
+  if (being_traced()) return std::nullopt;
   require(deg % 2 == 0, "deg must be even");
   pr_require(!chunk_size.has_value() || *chunk_size > 0, "chunk_size must be positive");
   pr_require(state.has_value() == sok.has_value(), "initial_state is the pair (state, sum_of_keys)");
@@ -236,7 +242,7 @@ py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G,
   const bool with_state = state.has_value() || want_final;
   if ((d == 16 || d == 32) && with_state)
     throw PrError("states are kept for head dim 64 only (got " + std::to_string(d) + ")");
-  if (d == 48) return py::none();
+  if (d == 48) return std::nullopt;
   int64_t c = (auto_chunk && deg == 2) ? pr_fast_chunk(t, (int)std::min<int64_t>(chunk, std::numeric_limits<int>::max())) : chunk;
   if (c != chunk || !switch_over.has_value()) switch_over = c ? std::optional<double>((double)c) : std::nullopt;
   const bool quadratic = !switch_over.has_value() || c == 0 || (double)((t + c - 1) / c * c) <= *switch_over;
@@ -293,10 +299,9 @@ py::object power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G,
     Fs = r.Fs;
     Fg = r.Fg;
   }
-  if (!want_final) return py::cast(O);
+  if (!want_final) return Retained(O);
   const On on(Q);
-  const auto [ns, nk] = final_state(Fs.detach().to(Q.scalar_type()), Fg.detach(), b, h, d, on);
-  return py::make_tuple(O, py::make_tuple(ns, nk));
+  return Retained(std::make_tuple(O, final_state(Fs.detach().to(Q.scalar_type()), Fg.detach(), b, h, d, on)));
 }
 
 // ------------------------------------------------------------------------------------------------ inference
@@ -318,14 +323,16 @@ Tensor batch_strided(const Tensor& t, int64_t unit, int64_t* stride) {
 }
 
 struct Partials {
-  Tensor y, l;
+  Tensor both;  // one allocation: rows of d, then their sums
+  float *y = nullptr, *l = nullptr;
   int kernels = 1;
   // workspace of a decode step that is split over several CTAs per (batch, head); none when it is not
   Partials(int64_t b, int64_t h, int64_t hq, int64_t d, const Tensor& like) {
     if (pr_decode_split((int)b, (int)h, (int)hq) <= 1) return;
     const int64_t ns = pr_decode_nsplit();
-    y = empty_f32({b, hq, ns, d}, like);
-    l = empty_f32({b, hq, ns}, like);
+    both = empty_f32({b * hq * ns * (d + 1)}, like);
+    y = fmptr(both);
+    l = y + b * hq * ns * d;
     kernels = 2;
   }
 };
@@ -350,7 +357,7 @@ Tensor decode_step(const Tensor& Q0, const Tensor& K0, const Tensor& V0, const T
   const Tensor O = at::empty({b, 1, hq, d}, Q.options());
   const Partials part(b, h, hq, d, Q);
   check(pr_decode_step_strided(dtype_code(Q), (int)b, (int)tk, (int)h, (int)hq, (int)d, cptr(Q), qs, cptr(K), cptr(V), ks,
-                               fptr(G), gs, cptr(state), fptr(sok), (float)scale, nullptr, fmptr(part.y), fmptr(part.l),
+                               fptr(G), gs, cptr(state), fptr(sok), (float)scale, nullptr, part.y, part.l,
                                mptr(O), on.device, on.stream),
         "pr_decode_step_strided", part.kernels);
   return O;
@@ -368,9 +375,10 @@ void gate_sums(const Tensor& K, const Tensor& G, const Tensor& a, const Tensor& 
         "pr_gate_prep", a.defined() && xt.defined() ? 2 : 1);
 }
 
-py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, const OptTensor& log_G,
-                    const OptTensor& state_, const OptTensor& sok_, std::optional<double> scale_,
-                    std::optional<double> switch_over) {
+std::tuple<Tensor, OptTensor, OptTensor> inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_,
+                                                   const OptTensor& log_G, const OptTensor& state_,
+                                                   const OptTensor& sok_, std::optional<double> scale_,
+                                                   std::optional<double> switch_over) {
   const at::NoGradGuard no_grad;
   const bool has_cache = K_.has_value() && V_.has_value(), has_state = state_.has_value();
   require(has_cache || has_state, "initial_state or cache must be provided for inference");
@@ -416,7 +424,7 @@ py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, 
   Tensor Y;
   if (tq == 1 && has_state && !compress) {
     Y = decode_step(Q0, K, V, G, state, sok, scale, h);
-    return py::make_tuple(Y, *state_, *sok_);
+    return {Y, state_, sok_};
   }
   const On on(Q0);
   const Tensor Q = aligned(Q0);
@@ -453,7 +461,7 @@ py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, 
                        has_state && attn, 1, (float)scale, 2, mptr(Y), nullptr, on.device, on.stream),
           "pr_chunk_out", 1);
   }
-  if (!compress) return py::make_tuple(Y, state_, sok_);
+  if (!compress) return {Y, state_, sok_};
 
   // ---- the cache becomes a new state
   const int64_t D = d * (d + 1) / 2;
@@ -461,7 +469,7 @@ py::tuple inference(const Tensor& Q0, const OptTensor& K_, const OptTensor& V_, 
   check(pr_compress_cache(dt, (int)b, (int)tk, (int)h, (int)d, cptr(xt), cptr(V), cptr(state), fptr(sok), fptr(total),
                           mptr(ns), fmptr(nk), on.device, on.stream),
         "pr_compress_cache", 1);
-  return py::make_tuple(Y, ns, nk);
+  return {Y, ns, nk};
 }
 
 Tensor decode_recurrent(const Tensor& q0, const Tensor& k0, const Tensor& v0, const OptTensor& log_g, const Tensor& state,
@@ -492,8 +500,8 @@ Tensor decode_recurrent(const Tensor& q0, const Tensor& k0, const Tensor& v0, co
   const Tensor O = at::empty({b, 1, hq, d}, q.options());
   const Partials part(b, h, hq, d, q);
   check(pr_decode_recurrent(dtype_code(q), (int)b, (int)h, (int)hq, (int)d, cptr(q), qs, cptr(k), cptr(v), ks, fptr(g), gs,
-                            cptr(state), fptr(sok), mptr(new_state), fmptr(new_sok), (float)scale, fmptr(part.y),
-                            fmptr(part.l), mptr(O), on.device, on.stream),
+                            cptr(state), fptr(sok), mptr(new_state), fmptr(new_sok), (float)scale, part.y,
+                            part.l, mptr(O), on.device, on.stream),
         "pr_decode_recurrent", part.kernels);
   return O;
 }
@@ -552,8 +560,10 @@ class PrepareQKVG : public torch::autograd::Function<PrepareQKVG> {
   }
 };
 
-py::object prepare_qkvg(Tensor x, Tensor sin, Tensor cos, int64_t h, int64_t hq, int64_t d, bool gated, double bias,
-                        bool half_split) {
+using Prepared = std::tuple<Tensor, Tensor, Tensor, OptTensor>;
+
+std::optional<Prepared> prepare_qkvg(Tensor x, Tensor sin, Tensor cos, int64_t h, int64_t hq, int64_t d, bool gated,
+                                     double bias, bool half_split) {
   pr_require(x.is_cuda() && x.dim() == 3 && (x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf),
              "prepare_qkvg wants a CUDA bf16/fp16 tensor [b, t, W]");
   const int64_t used = (hq + 2 * h) * d + (gated ? h : 0), t = x.size(1);
@@ -570,10 +580,9 @@ py::object prepare_qkvg(Tensor x, Tensor sin, Tensor cos, int64_t h, int64_t hq,
                  (sin.dim() == 2 || (sin.dim() == 3 && sin.size(0) == x.size(0))) && sin.device() == x.device() &&
                  cos.device() == x.device(),
              "sin / cos must be [t, d/2] (or [b, t, d/2]) for the tokens of the projection");
-  if (being_traced()) return py::none();
+  if (being_traced()) return std::nullopt;
   const variable_list out = PrepareQKVG::apply(x, sin, cos, h, hq, d, gated, bias, half_split);
-  if (gated) return py::make_tuple(out[0], out[1], out[2], out[3]);
-  return py::make_tuple(out[0], out[1], out[2], py::none());
+  return Prepared(out[0], out[1], out[2], gated ? OptTensor(out[3]) : std::nullopt);
 }
 
 }  // namespace
@@ -591,8 +600,10 @@ PYBIND11_MODULE(_host, m) {
   });
   m.def("set_error_type", [](py::object cls) { g_error = cls.release().ptr(); });
   m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
-  m.def("power_retention", &power_retention);
-  m.def("inference", &inference);
-  m.def("decode_recurrent", &decode_recurrent);
-  m.def("prepare_qkvg", &prepare_qkvg);
+  // Without the interpreter lock: a launch into a full queue waits for the GPU, and other Python threads go on meanwhile.
+  using no_gil = py::call_guard<py::gil_scoped_release>;
+  m.def("power_retention", &power_retention, no_gil());
+  m.def("inference", &inference, no_gil());
+  m.def("decode_recurrent", &decode_recurrent, no_gil());
+  m.def("prepare_qkvg", &prepare_qkvg, no_gil());
 }

@@ -149,3 +149,56 @@ def test_a_failed_backward_of_the_glue_raises_the_packages_error(cuda_device):
         Q, K, V, log_g = prb.prepare_qkvg(x, sin, cos, 1, 2, 64)
     with pytest.raises(prb.PRError, match="float16"):
         Q.sum().backward()
+
+
+def _entry(name, dev):
+    import retention_integration_b200 as prb
+
+    Q, K, V, G = _inputs(dev, 1, 64, 1, 1)
+    if name == "power_retention":
+        return lambda: prb.power_retention(Q, K, V, G)
+    if name == "prepare_qkvg":
+        x = torch.zeros(1, 64, 200, device=dev, dtype=torch.bfloat16)
+        sin, cos = prb.rotary_tables(64, 64, dev)
+        return lambda: prb.prepare_qkvg(x, sin, cos, 1, 1, 64)
+    one = [x[:, :1].contiguous() for x in (Q, K, V, G)]
+    cache = prb.RetentionCache(1, 1, 64, recurrent=True)
+    cache.decode(*one)
+    if name == "recurrent":
+        return lambda: cache.decode(*one)
+    return lambda: prb.power_retention_inference(one[0], K, V, G, cache.state, cache.sum_of_keys)
+
+
+@pytest.mark.parametrize("name", ["power_retention", "prepare_qkvg", "recurrent", "inference"])
+def test_other_threads_run_while_a_launch_waits(cuda_device, name):
+    """Behind half a second of GPU work the launch queue fills up, and one of the calls waits for room in it."""
+    import threading
+    import time
+
+    call = _entry(name, cuda_device)
+    with torch.no_grad():
+        call()
+        torch.cuda.synchronize()
+        gaps, stop = [], threading.Event()
+
+        def watch():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(1e-3)
+                last, before = time.perf_counter(), last
+                gaps.append(last - before)
+
+        watcher = threading.Thread(target=watch)
+        watcher.start()
+        torch.cuda._sleep(1_000_000_000)  # clocks
+        longest = 0.0
+        for _ in range(3000):
+            t0 = time.perf_counter()
+            call()
+            longest = max(longest, time.perf_counter() - t0)
+        stop.set()
+        watcher.join()
+        torch.cuda.synchronize()
+    if longest < 0.1:
+        pytest.skip("no launch had to wait")
+    assert max(gaps) < longest / 2
