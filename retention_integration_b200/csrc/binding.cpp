@@ -197,14 +197,15 @@ class Retention : public torch::autograd::Function<Retention> {
   }
 };
 
-// A state pair in the exact layout, checked.
-void check_state(const Tensor& state, const Tensor& sok, int64_t b, int64_t h, int64_t d) {
+// A state pair in the exact layout, on the device of `like`.
+void check_state(const Tensor& state, const Tensor& sok, int64_t b, int64_t h, int64_t d, const Tensor& like) {
   const int64_t D = d * (d + 1) / 2;
   require(state.dim() == 4 && state.size(0) == b && state.size(1) == h && state.size(2) == D && state.size(3) == d,
           "state must be [b,h,d(d+1)/2,d] (exact layout)");
   require(sok.dim() == 3 && sok.size(0) == b && sok.size(1) == h && sok.size(2) == D && sok.scalar_type() == at::kFloat,
           "sum_of_keys must be [b,h,d(d+1)/2] float32");
   pr_require(state.is_cuda() && sok.is_cuda(), "the state must live on a CUDA device: this package has no CPU path");
+  require(state.device() == like.device() && sok.device() == like.device(), "tensors must live on one device");
 }
 
 using StatePair = std::tuple<Tensor, Tensor>;
@@ -275,7 +276,7 @@ std::optional<Retained> power_retention(Tensor Q, Tensor K, Tensor V, const OptT
                     any_of([](const Tensor& t) { return t._fw_grad(0).defined(); });
   Tensor Cs, Cg;
   if (state.has_value()) {
-    check_state(*state, *sok, b, h, d);
+    check_state(*state, *sok, b, h, d, Q);
     const On on(Q);
     const Tensor s = aligned(state->detach().to(Q.scalar_type())), k = aligned(sok->detach());
     Cs = empty_f32({b, h, state_rows(d) * d}, Q);
@@ -406,9 +407,8 @@ std::tuple<Tensor, OptTensor, OptTensor> inference(const Tensor& Q0, const OptTe
   dtype_code(Q0);
   Tensor state, sok;
   if (has_state) {
-    check_state(*state_, *sok_, b, h, d);
+    check_state(*state_, *sok_, b, h, d, Q0);
     pr_require(state_->scalar_type() == Q0.scalar_type(), "the state's dtype must be the query's");
-    require(state_->device() == Q0.device() && sok_->device() == Q0.device(), "tensors must live on one device");
     state = aligned(*state_);
     sok = aligned(*sok_);
   }
@@ -475,14 +475,23 @@ std::tuple<Tensor, OptTensor, OptTensor> inference(const Tensor& Q0, const OptTe
 Tensor decode_recurrent(const Tensor& q0, const Tensor& k0, const Tensor& v0, const OptTensor& log_g, const Tensor& state,
                         const Tensor& sok, const Tensor& new_state, const Tensor& new_sok, double scale) {
   const at::NoGradGuard no_grad;
-  pr_require(q0.is_cuda() && k0.is_cuda() && v0.is_cuda(), "tensors must be CUDA tensors: this package has no CPU path");
-  require(q0.dim() == 4 && k0.dim() == 4 && v0.dim() == 4 && q0.size(1) == 1 && k0.size(1) == 1 && k0.sizes() == v0.sizes(),
+  require(q0.dim() == 4 && k0.dim() == 4 && v0.dim() == 4 && q0.size(1) == 1 && k0.size(1) == 1 && k0.sizes() == v0.sizes() &&
+              k0.size(0) == q0.size(0) && k0.size(3) == q0.size(3),
           "q, k, v must be [batch, 1, heads, dim]");
-  require(q0.scalar_type() == k0.scalar_type() && q0.scalar_type() == v0.scalar_type(), "dtypes of inputs must match");
-  const On on(q0);
   const int64_t b = q0.size(0), hq = q0.size(2), d = q0.size(3), h = k0.size(2);
-  check_state(state, sok, b, h, d);
-  check_state(new_state, new_sok, b, h, d);
+  require(h > 0 && hq % h == 0, "Q heads must be a multiple of KV heads");
+  require(!log_g.has_value() || (log_g->dim() >= 1 && log_g->size(0) == b && log_g->numel() == b * h),
+          "log_g must be [batch, 1, kv_heads]");
+  require(q0.scalar_type() == k0.scalar_type() && q0.scalar_type() == v0.scalar_type(), "dtypes of inputs must match");
+  dtype_code(q0);
+  pr_require(state.scalar_type() == q0.scalar_type() && new_state.scalar_type() == q0.scalar_type(),
+             "the state's dtype must be the query's");
+  pr_require(q0.is_cuda() && k0.is_cuda() && v0.is_cuda(), "tensors must be CUDA tensors: this package has no CPU path");
+  require(k0.device() == q0.device() && v0.device() == q0.device() && (!log_g.has_value() || log_g->device() == q0.device()),
+          "tensors must live on one device");
+  check_state(state, sok, b, h, d, q0);
+  check_state(new_state, new_sok, b, h, d, q0);
+  const On on(q0);
   require(state.is_contiguous() && sok.is_contiguous() && new_state.is_contiguous() && new_sok.is_contiguous(),
           "states must be contiguous");
   int64_t qs = 0, ks = 0, vs = 0, gs = 0;

@@ -43,3 +43,36 @@ def test_half_a_state_is_refused():
     for pair in ((None, sok), (torch.zeros(1, 2, 2080, 64, dtype=torch.bfloat16), None)):
         with pytest.raises(prb.PRError, match="pair"):
             prb.power_retention(Q, Q, Q, initial_state=pair)
+
+
+def _step(b=2, h=2, hq=4, d=64, dtype=torch.bfloat16):
+    return [torch.zeros(b, 1, n, d, dtype=dtype) for n in (hq, h, h)] + [torch.zeros(b, 1, h)]
+
+
+def _decode(q, k, v, g, dtype=torch.bfloat16):
+    return prb.RetentionCache(2, 2, 64, dtype=dtype, device="cpu", recurrent=True).decode(q, k, v, g)
+
+
+def test_a_recurrent_step_is_accepted_up_to_the_device():
+    q, k, v, g = _step()
+    for gates in (g, g[:, 0], None):
+        with pytest.raises(prb.PRError, match="CUDA"):
+            _decode(q, k, v, gates)
+
+
+@pytest.mark.parametrize("change", [
+    lambda q, k, v, g: (q, k[:1], v[:1], g),                       # fewer sequences than the queries have
+    lambda q, k, v, g: (q, k[..., :32], v[..., :32], g),           # narrower keys
+    lambda q, k, v, g: (q, k, v, g[:1]),                           # gates of fewer sequences
+    lambda q, k, v, g: (q, k, v, g[..., :1]),                      # gates of fewer heads
+    lambda q, k, v, g: (q, k, v, g.flatten()),
+    lambda q, k, v, g: (q[:, :, :3], k, v, g),                     # heads that do not divide
+])
+def test_a_recurrent_step_of_other_shapes_is_refused(change):
+    with pytest.raises(AssertionError):
+        _decode(*change(*_step()))
+
+
+def test_a_recurrent_step_of_another_dtype_than_the_state_is_refused():
+    with pytest.raises(prb.PRError, match="state"):
+        _decode(*_step(dtype=torch.float16))
