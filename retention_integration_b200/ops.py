@@ -70,6 +70,14 @@ def _dev(t: torch.Tensor) -> int:
     return t.device.index if t.device.index is not None else torch.cuda.current_device()
 
 
+def _chunks(t: int, c: int) -> int:
+    """Chunks of a sequence.  The C entries take a shorter last chunk; the tensors of these wrappers are sized for whole
+    ones."""
+    if c <= 0 or t % c:
+        raise _lib.PRError(f"t={t} is not a multiple of the chunk size {c}")
+    return t // c
+
+
 def selftest_umma(variant: int, a: torch.Tensor, b: torch.Tensor, n: int, k: int) -> torch.Tensor:
     out = torch.empty(128, n, device=a.device, dtype=torch.float32)
     _call("pr_selftest_umma", c_int(variant), c_int(dtype_code(a.dtype)), c_int(n), c_int(k), ptr(a), ptr(b),
@@ -84,7 +92,7 @@ def gate_prep(x: torch.Tensor, log_g, c: int, query_side: bool, mult: float = 1.
     With row_scale [b,t,hx] fp32 a fourth result is the copy of xT scaled per token."""
     b, t, hx, d = x.shape
     h = log_g.shape[2] if log_g is not None else hx
-    n = t // c
+    n = _chunks(t, c)
     cp = (c + 63) // 64 * 64
     write = want_gates and not query_side
     if not want_xt and c > 16384:
@@ -125,6 +133,7 @@ def chunk_state(xt: torch.Tensor, xts, v: torch.Tensor, c: int, nh: int, key_wei
     """xt [b,n,hx,d,cp] (hx = nh*group), v [b,t,hx,d] -> (S [b,n,nh,DR,d], gram [b,n,nh,d,d] fp32 or None)."""
     b, n, hx, d, cp = xt.shape
     t = v.shape[1]
+    _chunks(t, c)
     group = hx // nh
     out = torch.empty(b, n, nh, state_rows(d), d, device=xt.device, dtype=xt.dtype)
     gram = torch.empty(b, n, nh, d, d, device=xt.device, dtype=torch.float32) if want_gram else None
@@ -264,6 +273,7 @@ def expand_grad(W, X, State, g_hi, g_lo, a, A, row_g, c: int, h: int, query_side
     """Gradient through the expansion.  W, X [b,t,hx,d]; State [b,n,h,DR,d]; g_hi/g_lo [b,n,h,d,d].
     Returns (dX [b,t,hx,d] fp32, gdot [b,t,hx] fp32)."""
     b, t, hx, d = X.shape
+    _chunks(t, c)
     dX = torch.empty(b, t, hx, d, device=X.device, dtype=torch.float32)
     gdot = torch.empty(b, t, hx, device=X.device, dtype=torch.float32)
     _call("pr_expand_grad", c_int(dtype_code(X.dtype)), c_int(b), c_int(t), c_int(h), c_int(hx), c_int(d), c_int(c),
@@ -277,6 +287,7 @@ def chunk_dq(Q, dO, K, V, a, dl, l, dq_state, c: int, scale: float, deg: int = 2
     """Returns (dQ [b,t,hq,d], da_q [b,t,hq] fp32)."""
     b, t, hq, d = Q.shape
     h = K.shape[2]
+    _chunks(t, c)
     dQ = torch.empty_like(Q)
     da_q = torch.empty(b, t, hq, device=Q.device, dtype=torch.float32)
     _call("pr_chunk_dq", c_int(dtype_code(Q.dtype)), c_int(b), c_int(t), c_int(hq), c_int(h), c_int(d), c_int(c),
@@ -289,6 +300,7 @@ def chunk_dkv(Q, dO, K, V, wdS, a, A, dl, l, dk_state, c: int, state_chunk_hi: i
     """Returns (dK, dV [b,t,h,d], da_k [b,t,h] fp32)."""
     b, t, hq, d = Q.shape
     h = K.shape[2]
+    _chunks(t, c)
     dK, dV = torch.empty_like(K), torch.empty_like(V)
     da_k = torch.empty(b, t, h, device=Q.device, dtype=torch.float32)
     _call("pr_chunk_dkv", c_int(dtype_code(Q.dtype)), c_int(b), c_int(t), c_int(hq), c_int(h), c_int(d), c_int(c),
@@ -303,6 +315,7 @@ def gate_grad(da_q, gq, da_k, wk, dA_scan, dA_gram, c: int):
     (dA_scan [b,h,blocks,n], dA_gram [b,h,blocks2,n])."""
     b, t, hq = da_q.shape
     h = da_k.shape[2]
+    _chunks(t, c)
     out = torch.empty(b, t, h, device=da_q.device, dtype=torch.float32)
     blocks = dA_scan.shape[2] if dA_scan is not None else 0
     gblocks = dA_gram.shape[2] if dA_gram is not None else 0

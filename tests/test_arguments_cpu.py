@@ -76,3 +76,20 @@ def test_a_recurrent_step_of_other_shapes_is_refused(change):
 def test_a_recurrent_step_of_another_dtype_than_the_state_is_refused():
     with pytest.raises(prb.PRError, match="state"):
         _decode(*_step(dtype=torch.float16))
+
+
+def test_operator_wrappers_want_whole_chunks():
+    """The tensors that the wrappers allocate hold whole chunks: a ragged sequence would be written past their ends."""
+    from retention_integration_b200 import ops
+
+    x, g, f = torch.zeros(1, 100, 2, 64, dtype=torch.bfloat16), torch.zeros(1, 100, 2), torch.zeros(1, 100, 2)
+    xt = torch.zeros(1, 1, 2, 64, 64, dtype=torch.bfloat16)
+    S, gr = torch.zeros(1, 1, 2, 2560, 64, dtype=torch.bfloat16), torch.zeros(1, 1, 2, 64, 64, dtype=torch.bfloat16)
+    for call in (lambda: ops.gate_prep(x, g, 64, query_side=False),
+                 lambda: ops.chunk_state(xt, None, x, 64, 2, True, True),
+                 lambda: ops.expand_grad(x, x, S, gr, gr, None, None, f, 64, 2, True, 1.0, 2.0, 0, 0),
+                 lambda: ops.chunk_dq(x, x, x, x, None, f, f, None, 64, 1.0),
+                 lambda: ops.chunk_dkv(x, x, x, x, None, None, None, f, f, None, 64, -1, 1.0),
+                 lambda: ops.gate_grad(f, None, f, None, None, None, 64)):
+        with pytest.raises(prb.PRError, match="multiple of the chunk"):
+            call()
