@@ -13,7 +13,8 @@
  *   - returns PR_OK (0) or a negative PR_ERR_* code; pr_last_error() gives a
  *     thread-local message for the last failure on the calling thread;
  *   - never aborts, traps or allocates device memory: the caller passes every
- *     input, output and workspace as a raw device pointer (16-byte aligned);
+ *     input, output and workspace as a raw device pointer (16-byte aligned; the workspaces of
+ *     pr_retention_fwd / _bwd, `out` of pr_chunk_state and `dX` of pr_expand_grad 32-byte);
  *   - work is enqueued on the given stream (a cudaStream_t passed as void*) of
  *     the given device ordinal; the call sets that device current itself, so it
  *     may be called from any thread (autograd's backward thread included);

@@ -607,7 +607,7 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   p.dk_state = dk_state;
   p.dK = dK;
   p.dV = dV;
-  p.aligned32 = ((reinterpret_cast<uintptr_t>(dK) | reinterpret_cast<uintptr_t>(dV)) & 31u) == 0;
+  p.aligned32 = aligned32(dK) && aligned32(dV);
   p.da_k = da_k;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;

@@ -456,7 +456,7 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   p.l = l;
   p.dq_state = dq_state;
   p.dQ = dQ;
-  p.aligned32 = (reinterpret_cast<uintptr_t>(dQ) & 31u) == 0;
+  p.aligned32 = aligned32(dQ);
   p.da_q = da_q;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;

@@ -634,7 +634,7 @@ int pr::chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int 
   p.scale = scale;
   p.a = a;
   p.O = O;
-  p.o_aligned32 = (reinterpret_cast<uintptr_t>(O) & 31u) == 0;
+  p.o_aligned32 = aligned32(O);
   p.l_out = l_out;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;

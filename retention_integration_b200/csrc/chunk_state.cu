@@ -406,8 +406,8 @@ int pr::chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, co
   PR_REQUIRE(b > 0 && t > 0 && nh > 0 && group > 0 && c > 0, PR_ERR_BAD_ARG,
              "bad sizes b=%d t=%d heads=%d group=%d c=%d", b, t, nh, group, c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
-  PR_REQUIRE(xt && v && out && aligned16(xt) && aligned16(v) && aligned16(out), PR_ERR_BAD_ARG,
-             "null or misaligned pointer");
+  PR_REQUIRE(xt && v && out && aligned16(xt) && aligned16(v) && aligned32(out), PR_ERR_BAD_ARG,
+             "null or misaligned pointer (out: 32 bytes)");
   PR_REQUIRE(gram == nullptr || (xts != nullptr && aligned16(xts) && aligned16(gram)), PR_ERR_BAD_ARG,
              "gram requested without a scaled operand");
   ChunkStateParams p{};
@@ -433,7 +433,7 @@ extern "C" int pr_compress_cache(int dtype, int b, int tk, int h, int d, const v
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(xt && v && new_state && new_sum_of_keys, PR_ERR_BAD_ARG, "null pointer");
   PR_REQUIRE((state == nullptr) == (sum_of_keys == nullptr), PR_ERR_BAD_ARG, "state and sum_of_keys come together");
-  PR_REQUIRE(aligned16(xt) && aligned16(v) && aligned16(state) && (reinterpret_cast<uintptr_t>(new_state) & 31u) == 0,
+  PR_REQUIRE(aligned16(xt) && aligned16(v) && aligned16(state) && aligned32(new_state),
              PR_ERR_BAD_ARG, "misaligned pointer (new_state: 32 bytes)");
   ChunkStateParams p{};
   p.out = new_state;

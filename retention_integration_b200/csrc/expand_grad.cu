@@ -407,7 +407,7 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
              "bad sizes b=%d t=%d h=%d hx=%d c=%d", b, t, h, hx, c);
   PR_REQUIRE(dtype == PR_BF16 || dtype == PR_FP16, PR_ERR_BAD_ARG, "dtype %d", dtype);
   PR_REQUIRE(W && X && State && g_hi && g_lo && dX && gdot, PR_ERR_BAD_ARG, "null pointer");
-  PR_REQUIRE(aligned16(W) && aligned16(X) && aligned16(State) && aligned16(g_hi) && aligned16(g_lo) && aligned16(dX),
+  PR_REQUIRE(aligned16(W) && aligned16(X) && aligned16(State) && aligned16(g_hi) && aligned16(g_lo) && aligned32(dX),
              PR_ERR_BAD_ARG, "misaligned pointer");
   PR_REQUIRE((a == nullptr) == (A == nullptr), PR_ERR_BAD_ARG, "a and A must be given together");
   PR_REQUIRE(hx <= 65535 && b <= 65535, PR_ERR_BAD_ARG, "hx and b must be <= 65535");

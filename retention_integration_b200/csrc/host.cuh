@@ -78,6 +78,8 @@ int chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const 
                 void* out, float* gram, int key_weights, int chunk0, int n_run, int device, void* stream);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+// what a thread's 32-byte stores want
+inline bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
 
 // Dynamic shared memory of a kernel: the attribute is raised once per kernel and device (and again only when a
 // later launch needs more), not on every launch.  The record is kept per kernel function, not per call site: a

@@ -271,7 +271,7 @@ extern "C" int pr_retention_fwd(const pr_problem* prob, const void* Q, const voi
   int rc = sizes_of(prob, &s);
   if (rc) return rc;
   PR_REQUIRE(Q && K && V && O && saved && scratch, PR_ERR_BAD_ARG, "null pointer");
-  PR_REQUIRE(aligned16(saved) && aligned16(scratch), PR_ERR_BAD_ARG, "workspaces must be 16-byte aligned");
+  PR_REQUIRE(aligned32(saved) && aligned32(scratch), PR_ERR_BAD_ARG, "workspaces must be 32-byte aligned");
   PR_REQUIRE((carry_state == nullptr) == (carry_gram == nullptr), PR_ERR_BAD_ARG, "the two carries come together");
   PR_REQUIRE((final_state == nullptr) == (final_gram == nullptr), PR_ERR_BAD_ARG, "the two final carries come together");
   const pr_problem& p = *prob;
@@ -308,7 +308,7 @@ extern "C" int pr_retention_bwd(const pr_problem* prob, const void* Q, const voi
   int rc = sizes_of(prob, &s);
   if (rc) return rc;
   PR_REQUIRE(Q && K && V && O && dO && saved && scratch && dQ && dK && dV, PR_ERR_BAD_ARG, "null pointer");
-  PR_REQUIRE(aligned16(saved) && aligned16(scratch), PR_ERR_BAD_ARG, "workspaces must be 16-byte aligned");
+  PR_REQUIRE(aligned32(saved) && aligned32(scratch), PR_ERR_BAD_ARG, "workspaces must be 32-byte aligned");
   const pr_problem& p = *prob;
   const bool gated = log_G != nullptr;
   PR_REQUIRE(!gated || dlog_G != nullptr, PR_ERR_BAD_ARG, "gated problem without a dlog_G output");

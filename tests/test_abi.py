@@ -38,6 +38,28 @@ def test_bad_arguments_return_codes_not_crashes():
     assert rc == -1 and b"variant" in lib.pr_last_error()
 
 
+def test_pointers_that_a_kernel_would_fault_on_are_refused():
+    """Addresses only: every one of these calls returns before it touches the device."""
+    from retention_integration_b200 import _lib
+
+    lib = _lib.lib()
+    P = lambda a: ctypes.c_void_p(a)
+    ok, off = P(1 << 20), P((1 << 20) + 16)  # 16 bytes short of the boundary that 32-byte stores want
+    f = ctypes.c_float(1.0)
+    rc = lib.pr_chunk_state(0, 1, 128, 1, 1, 64, 128, ok, ok, ok, off, None, 1, 0, None)
+    assert rc == -1 and b"misaligned" in lib.pr_last_error()
+    rc = lib.pr_expand_grad(0, 1, 128, 1, 1, 64, 128, ok, ok, ok, ok, ok, None, None, ok, 1, f, f, 0, 0, off, ok, 0, None)
+    assert rc == -1 and b"misaligned" in lib.pr_last_error()
+
+    class Problem(ctypes.Structure):
+        _fields_ = [(n, ctypes.c_int) for n in ("dtype", "b", "t", "h", "hq", "d", "c")] + [("scale", ctypes.c_float)]
+
+    prob = Problem(0, 1, 128, 1, 1, 64, 128, 1.0)
+    for saved, scratch in ((off, ok), (ok, off)):
+        rc = lib.pr_retention_fwd(ctypes.byref(prob), ok, ok, ok, None, None, None, ok, saved, scratch, None, None, 0, None)
+        assert rc == -1 and b"32-byte" in lib.pr_last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from retention_integration_b200 import _lib
 
