@@ -159,7 +159,7 @@ int pr_state_scan_bwd(int dtype, int b, int n, int h, int d, long long E, void* 
  * retention/_attention/cuda.py:34, and compute_query_states, retention/_query_state/cuda.py:42-44).
  * Q [b,n*cq,hq,d]; K,V [b,n*ck,h,d] or NULL (state only); a [b,n*ck,h] or NULL;
  * Z [b,n,h,D2,d], zg_hi/zg_lo [b,n,h,d,d] or NULL.  Query i of a chunk sits at key
- * position i + ck - cq.  Chunks >= state_from_chunk read the state.  O [b,n*cq,hq,d] =
+ * position i + ck - cq.  Chunks >= state_from_chunk read the state (all of them where there are no keys).  O [b,n*cq,hq,d] =
  * y / l (normalize=1) or y; l_out [b,n*cq,hq] or NULL.  deg = 2, or 4 without a state (the
  * reference's attention takes any even degree, its state operators degree 2 only). */
 int pr_chunk_out(int dtype, int b, int n_chunks, int cq, int ck, int hq, int h, int d, const void* Q,

@@ -610,7 +610,8 @@ int pr::chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int 
   const bool has_attn = (K != nullptr && V != nullptr);
   PR_REQUIRE(Q && O && aligned16(Q) && aligned16(O) && aligned16(K) && aligned16(V), PR_ERR_BAD_ARG,
              "null or misaligned pointer");
-  PR_REQUIRE(has_attn || Z != nullptr, PR_ERR_BAD_ARG, "neither keys/values nor a state were given");
+  PR_REQUIRE(has_attn || (Z != nullptr && state_from_chunk <= 0), PR_ERR_BAD_ARG,
+             "a chunk with neither keys / values nor a state");
   const bool with_state = (Z != nullptr) && state_from_chunk < n_chunks;
   PR_REQUIRE(!with_state || (zg_hi && zg_lo && aligned16(Z) && aligned16(zg_hi) && aligned16(zg_lo)), PR_ERR_BAD_ARG,
              "state given without its Gram matrices");

@@ -58,6 +58,9 @@ def test_pointers_that_a_kernel_would_fault_on_are_refused():
     for saved, scratch in ((off, ok), (ok, off)):
         rc = lib.pr_retention_fwd(ctypes.byref(prob), ok, ok, ok, None, None, None, ok, saved, scratch, None, None, 0, None)
         assert rc == -1 and b"32-byte" in lib.pr_last_error()
+    # no keys, and a first chunk that does not read the state either
+    rc = lib.pr_chunk_out(0, 1, 2, 128, 128, 1, 1, 64, ok, None, None, None, ok, ok, ok, 1, 0, 1, f, 2, ok, None, 0, None)
+    assert rc == -1 and b"neither" in lib.pr_last_error()
 
 
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
