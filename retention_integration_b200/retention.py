@@ -123,6 +123,15 @@ class _QuadraticRetention(torch.autograd.Function):
         return dQ, dK, dV, dlog_G, None, None
 
 
+def _like_queries(q, y):
+    """y as the queries' own tensor class, where torch's operators would have kept it (native code returns plain
+    tensors; a Parameter's results are plain ones too)."""
+    cls = type(q)
+    if cls is torch.Tensor or cls.__torch_function__ is torch._C._disabled_torch_function_impl:
+        return y
+    return y.as_subclass(cls)
+
+
 def _pad_head_dim(x, d_to):
     return torch.nn.functional.pad(x, (0, d_to - x.shape[-1]))
 
@@ -194,7 +203,7 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
         out = _lib.host().power_retention(Q, K, V, log_G, state, sok, return_final_state, int(deg), scale or 0.0,
                                           chunk_size, switch_over_seq_len, AUTO_CHUNK)
         if out is not None:
-            return out
+            return (_like_queries(Q, out[0]), out[1]) if return_final_state else _like_queries(Q, out)
     d_orig = Q.shape[-1]
     if d_orig in (16, 32, 48):
         if initial_state is not None or return_final_state:
@@ -271,4 +280,5 @@ def power_retention_inference(Q, K, V, log_G=None, initial_state=None, sum_of_ke
     """
     if deg != 2:
         raise PRError(f"deg={deg}: the state kernels implement deg=2")
-    return _lib.host().inference(Q, K, V, log_G, initial_state, sum_of_keys, scale, switch_over_seq_len)
+    out = _lib.host().inference(Q, K, V, log_G, initial_state, sum_of_keys, scale, switch_over_seq_len)
+    return out if type(Q) is torch.Tensor else (_like_queries(Q, out[0]), *out[1:])

@@ -202,3 +202,25 @@ def test_other_threads_run_while_a_launch_waits(cuda_device, name):
     if longest < 0.1:
         pytest.skip("no launch had to wait")
     assert max(gaps) < longest / 2
+
+
+def test_results_keep_the_queries_class(cuda_device):
+    import retention_integration_b200 as prb
+
+    class Marked(torch.Tensor):
+        pass
+
+    Q, K, V, G = _inputs(cuda_device, 1, 64, 2, 2)
+    q = Q.as_subclass(Marked)
+    assert type(prb.power_retention(q, K, V, G)) is Marked
+    y, (state, sok) = prb.power_retention(q, K, V, G, return_final_state=True)
+    assert type(y) is Marked and type(state) is torch.Tensor
+    y, s, n = prb.power_retention_inference(q, K, V, G, state, sok, switch_over_seq_len=None)
+    assert type(y) is Marked and s is state and n is sok
+    leaf = torch.nn.Parameter(Q)
+    out = prb.power_retention(leaf, K, V, G)
+    assert type(out) is torch.Tensor
+    want, = torch.autograd.grad(out.float().sum(), leaf)
+    marked = Q.clone().as_subclass(Marked).requires_grad_()
+    got, = torch.autograd.grad(prb.power_retention(marked, K, V, G).float().sum(), marked)
+    assert torch.equal(got.as_subclass(torch.Tensor), want)
