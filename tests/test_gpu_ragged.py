@@ -6,7 +6,8 @@ at most of these sizes, so 1e-2 bounds them with a factor of two.  On top of it 
 row sums divide: the backward takes <O, dO> from the rounded O, and the read-out's gradient from the rounded dO / l
 and the rounded state.  Each puts half a unit per element on a difference that cancels, and a row whose weights all
 happen to be tiny divides that by their small sum, so that one such row can carry a whole tensor's error.
-_rounding_bound adds it up from the exact weights."""
+_rounding_bound gives it row by row from the exact weights: rows where it is small are held to the plain 1e-2, and so
+are all rows of the last chunk together, which see enough tokens."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -33,10 +34,11 @@ def _grads(fn, leaves, dO):
 def _rounding_bound(leaves, dO, gold):
     """dQ_i is off by e_i sum_j M_ij k_j and dK_j by sum_i e_i M_ij q_i where <O_i, dO_i> is off by e_i, with
     M_ij = 2 (q_i.k_j) e^{a_i-a_j} / l_i.  e_i is a sum of independent roundings of up to half a unit, three per
-    element: three standard deviations are three half units times |O_i dO_i|.  Relative to the gradients' norms."""
+    element: three standard deviations are three half units times |O_i dO_i|.  The norm of every row, [b, t, heads]."""
     Q, K = (x.double() for x in leaves[:2])
     unit = 2.0 ** (-9 if leaves[0].dtype == torch.bfloat16 else -12)
-    r = Q.shape[2] // K.shape[2]
+    b, t, h, _ = K.shape
+    r = Q.shape[2] // h
     Kx = K.repeat_interleave(r, dim=2)
     s = torch.einsum("bihd,bjhd->bhij", Q, Kx)
     decay = torch.ones_like(s)
@@ -47,9 +49,9 @@ def _rounding_bound(leaves, dO, gold):
     l = (s * s * decay).sum(-1, keepdim=True)
     m = 2 * s * decay / l
     e = 3 * unit * (gold[0] * dO.double()).norm(dim=-1).transpose(1, 2)  # [b, hq, t]
-    dq = torch.einsum("bhi,bhij,bjhd->bihd", e, m, Kx)
-    dk = torch.einsum("bhi,bhij,bihd->bjhd", e ** 2, m ** 2, Q ** 2).sqrt()
-    return {"dQ": float(dq.norm() / gold[1].norm()), "dK": float(dk.norm() / gold[2].norm())}
+    dq = torch.einsum("bhi,bhij,bjhd->bihd", e, m, Kx).norm(dim=-1)
+    dk = torch.einsum("bhi,bhij,bihd->bjhd", e ** 2, m ** 2, Q ** 2).sum(-1)
+    return {"dQ": dq, "dK": dk.view(b, t, h, r).sum(-1).sqrt()}
 
 
 def _check(dev, b, t, h, r, d, chunk, gated, dtype=torch.bfloat16):
@@ -61,12 +63,22 @@ def _check(dev, b, t, h, r, d, chunk, gated, dtype=torch.bfloat16):
     gold = _grads(lambda *x: oracle.power_retention_quadratic(*x), [x.double() for x in leaves], dO)
     torch.cuda.synchronize()
     assert _lib.device_status(dev.index or 0) == 0
-    errs = {}
+    last = (t - 1) // chunk * chunk if chunk else 0  # first token of the last chunk
+    bound = _rounding_bound(leaves, dO, gold)
     for name, x, y in zip(("O", "dQ", "dK", "dV", "dlog_G"), ours, gold):
-        errs[name] = rel_l2(x.double().cpu(), y.cpu())
-    extra = _rounding_bound(leaves, dO, gold)
-    for name, err in errs.items():
-        assert err < 1e-2 + extra.get(name, 0.0), (name, err, extra)
+        x, y = (z if z.dim() == 4 else z[..., None] for z in (x.double(), y))
+        err, size = (x - y).norm(dim=-1), y.norm(dim=-1)
+        if name in bound:
+            sure = bound[name] < 1e-2 * size
+            assert sure.double().mean() > 0.75, name
+            rest = 1e-2 * size[~sure].norm() + bound[name][~sure].norm()
+            assert err[~sure].norm() <= rest, name
+            assert err[sure].norm() < 1e-2 * size[sure].norm(), name
+        else:
+            assert err.norm() < 1e-2 * size.norm(), name
+        # a gate's gradient is a difference of sums over the tokens; of the last few it may happen to be small
+        floor = size.square().mean().sqrt() if name == "dlog_G" else 0.0
+        assert err[:, last:].norm() < 1e-2 * max(size[:, last:].norm(), floor * size[:, last:].numel() ** 0.5), name
 
 
 @pytest.mark.parametrize("t,chunk", [(129, 128), (191, 64), (193, 64), (255, 128), (257, 128), (300, 192), (321, 320),
