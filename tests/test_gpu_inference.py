@@ -170,3 +170,22 @@ def test_decode_long_cache_both_dtypes(cuda_device, dtype, b, h, r, tk):
     gates keep the oldest cached tokens' weights alive, so a lost carry would show."""
     _decode_vs_oracle(cuda_device, b, h, r, tk, seed=3 * b + tk, check_rows=[(0, 0), (b - 1, h - 1)], dtype=dtype,
                       gate_shift=5.0)
+
+
+@pytest.mark.parametrize("b,h,r,tk", [(2, 3, 1, 33), (16, 32, 1, 0), (1, 2, 4, 70)])
+def test_decode_step_in_two_parts(cuda_device, b, h, r, tk):
+    """pr_decode_state followed by pr_decode_finish is the decode step.  Both round their 16-bit operands (2^-9 each)."""
+    import retention_integration_b200 as prb
+    from retention_integration_b200 import ops
+
+    g = torch.Generator().manual_seed(tk)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16().to(cuda_device)
+    Q, K, V = mk(b, 1, h * r, 64), mk(b, tk, h, 64), mk(b, tk, h, 64)
+    lg = F.logsigmoid(torch.randn(b, tk, h, generator=g) + 2.0).to(cuda_device)
+    state, sok = (x.to(cuda_device) for x in make_state(b, h, 64, 24, g))
+    state = state.bfloat16()
+    want, _, _ = prb.power_retention_inference(Q, K, V, lg, state, sok, switch_over_seq_len=None)
+    a = lg.cumsum(1) if tk else None
+    part = ops.decode_state(Q, state, sok, a[:, -1].contiguous() if tk else None, 0.125)
+    got = ops.decode_finish(Q, K if tk else None, V if tk else None, a, 0.125, *part, h)
+    assert rel_l2(got.float().cpu(), want.float().cpu()) < 1e-2
