@@ -11,12 +11,13 @@
 // Key side (gradient of the chunk state, retention/_update_state/reference.py:55-83):
 //   W = V, State = w (.) dS_m, Gs = dG_m + dG_m^T, g_i = 1, mult = 1, f_i = exp((A_m - a_i)/2).
 //
-// One CTA owns one row tile of 128 tokens of one (batch, chunk, head) and two CTAs share an SM
-// (Cfg<1>; Cfg<2> is the earlier shape, two row tiles in one CTA per SM, 7 % slower: measured
-// 0.302 vs 0.282 ms per launch at b1 t65536 h8).  The expansion gradient dphi is never written to
-// memory: tiles of 128 expanded rows are produced in tensor memory, two buffers per row tile, and
-// drained by the row tile's four warps while the tensor core fills the other buffer.  Each thread owns one token row and keeps x~ and dx~ in registers; the
-// triangle's (a, b) pattern is resolved at compile time, so the drain is two FMAs per entry.
+// One CTA owns one row tile of 128 tokens of one (batch, chunk, head) and two CTAs share an SM, so that one CTA's
+// prologue (operand loads, gating, Gram part) and write-out - a quarter of a CTA's life, all of it on the drain warps -
+// run while the other CTA drains.  (Two row tiles in one CTA per SM, where each state tile fetched from L2 feeds two
+// products, measured 7 % slower: 0.302 against 0.282 ms per launch at b1 t65536 h8.)  The expansion gradient dphi is
+// never written to memory: tiles of 128 expanded rows are produced in tensor memory, two buffers, and drained by four
+// warps while the tensor core fills the other buffer.  Each thread owns one token row and keeps x~ and dx~ in
+// registers; the triangle's (a, b) pattern is resolved at compile time, so the drain is two FMAs per entry.
 #include <type_traits>
 
 #include "host.cuh"
@@ -29,30 +30,16 @@ namespace eg {
 constexpr int HD = 64;
 constexpr int TILE_BYTES = 128 * 128;
 constexpr int G_BYTES = 64 * 128;
-// NRT row tiles of 128 tokens per CTA.  Warps: 4 NRT drain warps (one group of four per row tile), one
-// TMA warp, 2 NRT issuing warps (two threads per row tile).
-//   NRT = 2: one CTA per SM; each state tile fetched from L2 feeds two products.
-//   NRT = 1: two CTAs per SM, so that one CTA's prologue (operand loads, gating, Gram part) and epilogue
-//            (write-out) - a quarter of a CTA's life, all of it on the drain warps - run while the other
-//            CTA drains; the state tiles are fetched once per row tile, and the Gram operand borrows
-//            the last slot of the state ring until the Gram products have completed.
-template <int NRT>
-struct Cfg {
-  static constexpr int THREADS = 32 * (6 * NRT + 1);
-  static constexpr int ROWS = 128 * NRT;
-  static constexpr int NSS = NRT == 2 ? 4 : 2;  // state tiles in flight per CTA (64 KB per SM either way)
-  static constexpr bool G_IN_RING = NRT == 1;
-  static constexpr uint32_t TMEM_COLS = 256 * NRT;
-  static constexpr size_t SMEM =
-      1024 + (size_t)(2 * NRT + NSS) * TILE_BYTES + (G_IN_RING ? 0 : 2 * G_BYTES) + (size_t)NRT * 64 * 128 * 4;
-};
-#ifndef PR_EG_NRT
-#define PR_EG_NRT 1
-#endif
-// Tensor memory: two 128-column buffers per row tile, buffer b of row tile rt at (2 rt + b) * 128.
+constexpr int W_TMA = 4;                 // four drain warps, the TMA warp, two issuing warps (one per buffer)
+constexpr int THREADS = 32 * (W_TMA + 3);
+constexpr int ROWS = 128;
+constexpr int NSS = 2;                   // state tiles in flight; the Gram operand borrows the last slot first
+constexpr uint32_t TMEM_COLS = 256;
+constexpr size_t SMEM = 1024 + (size_t)(2 + NSS) * TILE_BYTES + (size_t)64 * 128 * 4;
+// Tensor memory: two 128-column buffers.
 // Before the first use of buffer 1 its columns hold the Gram part: the gated row as A operand
 // (32 columns at +0) and u = x~ Gs (64 columns at +64), read into the accumulators' initial value.
-__device__ __forceinline__ constexpr uint32_t col_d(int rt, int b) { return (uint32_t)((2 * rt + b) * 128); }
+__device__ __forceinline__ constexpr uint32_t col_d(int b) { return (uint32_t)(b * 128); }
 constexpr uint32_t OFF_XA = 0, OFF_U = 64;
 
 }  // namespace eg
@@ -75,17 +62,14 @@ struct ExpandGradParams {
   int* status;
 };
 
-template <typename T, int NRT>
-__global__ void __launch_bounds__(eg::Cfg<NRT>::THREADS, NRT == 1 ? 2 : 1)
+template <typename T>
+__global__ void __launch_bounds__(eg::THREADS, 2)
 expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap tm_w,
                    const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_s,
                    const __grid_constant__ CUtensorMap tm_ghi, const __grid_constant__ CUtensorMap tm_glo) {
   using namespace eg;
-  constexpr int THREADS = Cfg<NRT>::THREADS, ROWS = Cfg<NRT>::ROWS, NSS = Cfg<NRT>::NSS;
-  constexpr uint32_t TMEM_COLS = Cfg<NRT>::TMEM_COLS;
-  constexpr int W_TMA = 4 * NRT;  // the TMA warp; issuing warps follow
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t w_full, g_full, xa_full[2], u_full[2], s_full[NSS], s_empty[NSS], d_full[2][2], d_empty[2][2];
+  __shared__ uint64_t w_full, g_full, xa_full, u_full, s_full[NSS], s_empty[NSS], d_full[2], d_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
@@ -114,29 +98,26 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
 
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
-  uint8_t* smW = sm;                            // NRT x TILE_BYTES (one per row tile)
-  uint8_t* smX = smW + NRT * TILE_BYTES;        // NRT x TILE_BYTES
-  uint8_t* smS = smX + NRT * TILE_BYTES;        // NSS x TILE_BYTES (ring of state tiles)
-  // Gram operand (hi, lo): its own 16 KB, or the ring's last slot until the Gram products are done
-  uint8_t* smG = Cfg<NRT>::G_IN_RING ? smS + (NSS - 1) * TILE_BYTES : smS + NSS * TILE_BYTES;
-  // NRT x [64][128] fp32: dx~ terms indexed at run time
-  float* smR = reinterpret_cast<float*>(smS + NSS * TILE_BYTES + (Cfg<NRT>::G_IN_RING ? 0 : 2 * G_BYTES));
+  uint8_t* smW = sm;
+  uint8_t* smX = smW + TILE_BYTES;
+  uint8_t* smS = smX + TILE_BYTES;                // NSS x TILE_BYTES (ring of state tiles)
+  uint8_t* smG = smS + (NSS - 1) * TILE_BYTES;    // Gram operand (hi, lo): the ring's last slot until its products are done
+  static_assert(2 * G_BYTES <= TILE_BYTES, "the Gram operand fits a slot");
+  float* smR = reinterpret_cast<float*>(smS + NSS * TILE_BYTES);  // [64][128] fp32: dx~ terms indexed at run time
 
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&w_full, 1);
     mbar_init(&g_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&xa_full[s], 4);
-      mbar_init(&u_full[s], 1);
-      for (int b = 0; b < 2; ++b) {
-        mbar_init(&d_full[s][b], 1);
-        mbar_init(&d_empty[s][b], 4);
-      }
+    mbar_init(&xa_full, 4);
+    mbar_init(&u_full, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&d_full[b], 1);
+      mbar_init(&d_empty[b], 4);
     }
     for (int s = 0; s < NSS; ++s) {
       mbar_init(&s_full[s], 1);
-      mbar_init(&s_empty[s], NRT);  // one issuing thread per row tile releases a state tile
+      mbar_init(&s_empty[s], 1);
     }
     fence_mbar_init();
   }
@@ -152,11 +133,9 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
 
   if (warp == W_TMA) {
     if (elect_one()) {
-      mbar_expect_tx(&w_full, 2 * NRT * TILE_BYTES);
-      for (int rt = 0; rt < NRT; ++rt) {
-        tma_load_4d(smW + rt * TILE_BYTES, &tm_w, &w_full, 0, head, chunk * p.c + row0 + rt * 128, batch);
-        tma_load_4d(smX + rt * TILE_BYTES, &tm_x, &w_full, 0, head, chunk * p.c + row0 + rt * 128, batch);
-      }
+      mbar_expect_tx(&w_full, 2 * TILE_BYTES);
+      tma_load_4d(smW, &tm_w, &w_full, 0, head, chunk * p.c + row0, batch);
+      tma_load_4d(smX, &tm_x, &w_full, 0, head, chunk * p.c + row0, batch);
       mbar_expect_tx(&g_full, 2 * G_BYTES);
       tma_load_3d(smG, &tm_ghi, &g_full, 0, 0, ch);
       tma_load_3d(smG + G_BYTES, &tm_glo, &g_full, 0, 0, ch);
@@ -164,7 +143,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
         const int s = nt % NSS, ph = (nt / NSS) & 1;
         if (!mbar_wait(&s_empty[s], ph ^ 1, &abort_flag)) break;
         // the slot lent to the Gram operand is free once the Gram products have completed
-        if (Cfg<NRT>::G_IN_RING && nt == NSS - 1 && !mbar_wait(&u_full[0], 0, &abort_flag)) break;
+        if (nt == NSS - 1 && !mbar_wait(&u_full, 0, &abort_flag)) break;
         mbar_expect_tx(&s_full[s], TILE_BYTES);
         tma_load_2d(smS + s * TILE_BYTES, &tm_s, &s_full[s], 0, (ch * p.nt + nt) * 128);
       }
@@ -175,30 +154,30 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
     // traced timelines showed one thread per row tile setting the kernel's pace at ~1300 clocks per tile
     // against ~900 for the drain.
     if (elect_one()) {
-      const int rt = (warp - (W_TMA + 1)) >> 1, par = (warp - (W_TMA + 1)) & 1;
+      const int par = warp - (W_TMA + 1);
       bool ok = mbar_wait(&w_full, 0, &abort_flag);
       // prepared descriptors: a state tile on is TILE_BYTES >> 4 on in the address field
-      const uint64_t d_w = umma_desc_sw128(smem_u32(smW) + rt * TILE_BYTES, 16, 1024),
+      const uint64_t d_w = umma_desc_sw128(smem_u32(smW), 16, 1024),
                      d_s0 = umma_desc_sw128(smem_u32(smS), 16, 1024);
       const uint32_t idesc = umma_idesc(128, 128, Pack2<T>::is_bf16, false, false);
       for (int nt = par; nt < p.nt && ok; nt += 2) {
         const int s = nt % NSS, ph = (nt / NSS) & 1;
         const int b = par;
         // buffer 0 has been drained nt/2 times before tile nt; buffer 1 once more (the Gram part)
-        ok = mbar_wait(&d_empty[rt][b], ((nt >> 1) & 1) ^ (b ^ 1), &abort_flag) &&
+        ok = mbar_wait(&d_empty[b], ((nt >> 1) & 1) ^ (b ^ 1), &abort_flag) &&
              mbar_wait(&s_full[s], ph, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint64_t d_s = d_s0 + (uint32_t)s * (TILE_BYTES >> 4);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          umma_ss(tmem + col_d(rt, b), d_w + 2 * ks, d_s + 2 * ks, idesc, ks > 0 ? 1u : 0u);
-        umma_commit(&d_full[rt][b]);
+          umma_ss(tmem + col_d(b), d_w + 2 * ks, d_s + 2 * ks, idesc, ks > 0 ? 1u : 0u);
+        umma_commit(&d_full[b]);
         umma_commit(&s_empty[s]);
         if (nt == 0) {
           // Gram part: u = x~ (Gs_hi + Gs_lo), once per row tile, in the columns of buffer 1 (whose own
           // issuing thread waits until the rows have taken u out)
-          ok = mbar_wait(&g_full, 0, &abort_flag) && mbar_wait(&xa_full[rt], 0, &abort_flag);
+          ok = mbar_wait(&g_full, 0, &abort_flag) && mbar_wait(&xa_full, 0, &abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint32_t idesc_g = umma_idesc(128, HD, Pack2<T>::is_bf16, false, false);
@@ -207,18 +186,17 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
           for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              umma_ts(tmem + col_d(rt, 1) + OFF_U, tmem + col_d(rt, 1) + OFF_XA + ks * 8,
+              umma_ts(tmem + col_d(1) + OFF_U, tmem + col_d(1) + OFF_XA + ks * 8,
                       umma_desc_sw128(g_addr + half * G_BYTES + ks * 32, 16, 1024), idesc_g,
                       (half > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&u_full[rt]);
+          umma_commit(&u_full);
         }
       }
     }
   } else {
     // ------------------------------------------------------------ drain warps
-    const int rt = warp >> 2;                  // row tile owned by this warp group
     const int r = (warp & 3) * 32 + lane;      // token row inside the tile = TMEM lane
-    const int row = row0 + rt * 128 + r;
+    const int row = row0 + r;
     const bool row_valid = row < c;
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
 
@@ -230,7 +208,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
     bool ok = mbar_wait(&w_full, 0, &abort_flag);
     {
       uint32_t xp[32];
-      uint8_t* xs = smX + rt * TILE_BYTES;
+      uint8_t* xs = smX;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint4 v = *reinterpret_cast<const uint4*>(xs + swz128(r, j));
@@ -245,42 +223,42 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
       // run-time index in the drain)
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        *reinterpret_cast<uint4*>(smX + rt * TILE_BYTES + swz128(r, j)) =
+        *reinterpret_cast<uint4*>(smX + swz128(r, j)) =
             make_uint4(xp[4 * j], xp[4 * j + 1], xp[4 * j + 2], xp[4 * j + 3]);
       if (ok) {
-        tmem_st32(tmem + lane_addr + col_d(rt, 1) + OFF_XA, xp);
+        tmem_st32(tmem + lane_addr + col_d(1) + OFF_XA, xp);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&xa_full[rt]);
+        if (lane == 0) mbar_arrive(&xa_full);
       }
     }
     // Gram part first: dx~ starts at g_i * mult * (Gs x~)_i, which also frees buffer 1
     {
       float g = p.gram_mult;
       if (p.row_g != nullptr) g *= row_valid ? p.row_g[(tok0 + row) * p.hx + head] : 0.f;
-      if (ok) ok = mbar_wait(&u_full[rt], 0, &abort_flag);
+      if (ok) ok = mbar_wait(&u_full, 0, &abort_flag);
       tc_fence_after();
       uint32_t u[64];
       if (ok) {
-        tmem_ld32(tmem + lane_addr + col_d(rt, 1) + OFF_U, u);
-        tmem_ld32(tmem + lane_addr + col_d(rt, 1) + OFF_U + 32, u + 32);
+        tmem_ld32(tmem + lane_addr + col_d(1) + OFF_U, u);
+        tmem_ld32(tmem + lane_addr + col_d(1) + OFF_U + 32, u + 32);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&d_empty[rt][1]);
+        if (lane == 0) mbar_arrive(&d_empty[1]);
       }
       // dx~ lives in this thread's private column of shared memory (64 floats, stride 128): the
       // first-factor terms are added at a run-time index, and the second-factor terms of a
       // 16-block are kept in registers only while that block is being drained.  Keeping all 64
       // accumulators and the row itself in registers left the compiler no room to overlap the
       // FMAs of neighbouring entries.
-      float* sdx0 = smR + rt * 64 * 128 + r;
+      float* sdx0 = smR + r;
 #pragma unroll
       for (int e = 0; e < HD; ++e) sdx0[e * 128] = ok ? g * __uint_as_float(u[e]) : 0.f;
     }
-    float* sdx = smR + rt * 64 * 128 + r;
-    const uint8_t* xrow = smX + rt * TILE_BYTES;  // holds the gated row again (written above)
+    float* sdx = smR + r;
+    const uint8_t* xrow = smX;  // holds the gated row again (written above)
 
     int nt = 0;
     static_for<0, HD / 16>([&](auto yc) {
@@ -302,10 +280,10 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
 #pragma unroll 1
       for (int tt = 0; tt < 2 * (Y + 1); ++tt, ++nt) {
         const int b = nt & 1;
-        if (ok) ok = mbar_wait(&d_full[rt][b], (nt >> 1) & 1, &abort_flag);
+        if (ok) ok = mbar_wait(&d_full[b], (nt >> 1) & 1, &abort_flag);
         tc_fence_after();
         if (!ok) continue;
-        const uint32_t cd = tmem + lane_addr + col_d(rt, b);
+        const uint32_t cd = tmem + lane_addr + col_d(b);
         // the tile's eight first factors x~[8 tt .. 8 tt + 7] in one 16-byte load, and their gradient
         // terms collected in registers: the shared-memory column is touched once per tile, after the
         // loop, so no load of the loop has to wait behind a store to the same memory space
@@ -332,7 +310,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
             // all of this thread's reads of the buffer are done
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&d_empty[rt][b]);
+            if (lane == 0) mbar_arrive(&d_empty[b]);
           }
 #pragma unroll
           for (int aa = 0; aa < 2; ++aa) {
@@ -421,8 +399,7 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
   p.t = t;
   p.d = d;
   p.nt = ref_dim(d) / 128;
-  using C = Cfg<PR_EG_NRT>;
-  p.tiles_per_chunk = (c + C::ROWS - 1) / C::ROWS;
+  p.tiles_per_chunk = (c + ROWS - 1) / ROWS;
   p.chunk_lo = chunk_lo;
   p.chunk_hi = chunk_hi;
   p.query_side = query_side;
@@ -451,15 +428,15 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
     if ((rc = gram_tmap(&tm_ghi, g_hi, d, (uint64_t)b * n * h))) return rc;
     if ((rc = gram_tmap(&tm_glo, g_lo, d, (uint64_t)b * n * h))) return rc;
   }
-  const size_t smem = C::SMEM;
+  const size_t smem = SMEM;
   dim3 grid(p.tiles_per_chunk * n, hx, b);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == PR_BF16) {
-    PR_SMEM_ATTR((expand_grad_kernel<__nv_bfloat16, PR_EG_NRT>), smem, device, true);
-    expand_grad_kernel<__nv_bfloat16, PR_EG_NRT><<<grid, C::THREADS, smem, s>>>(p, tm_w, tm_x, tm_s, tm_ghi, tm_glo);
+    PR_SMEM_ATTR(expand_grad_kernel<__nv_bfloat16>, smem, device, true);
+    expand_grad_kernel<__nv_bfloat16><<<grid, THREADS, smem, s>>>(p, tm_w, tm_x, tm_s, tm_ghi, tm_glo);
   } else {
-    PR_SMEM_ATTR((expand_grad_kernel<__half, PR_EG_NRT>), smem, device, true);
-    expand_grad_kernel<__half, PR_EG_NRT><<<grid, C::THREADS, smem, s>>>(p, tm_w, tm_x, tm_s, tm_ghi, tm_glo);
+    PR_SMEM_ATTR(expand_grad_kernel<__half>, smem, device, true);
+    expand_grad_kernel<__half><<<grid, THREADS, smem, s>>>(p, tm_w, tm_x, tm_s, tm_ghi, tm_glo);
   }
   PR_CUDA(cudaGetLastError());
   return PR_OK;

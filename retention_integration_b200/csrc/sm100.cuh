@@ -96,22 +96,6 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
   return mbar_wait_slow(bar, parity, abort_flag, budget_ns);
 }
 
-// A wait for something that is far away (a whole phase of the kernel): polls with pauses in between,
-// so that the waiting warp leaves its issue slots to the warps that work.  Bounded like the others.
-static __device__ __noinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                      unsigned pause_ns = 500) {
-  const uint64_t t0 = globaltimer_ns();
-  for (;;) {
-    if (mbar_try_wait(bar, parity)) return true;
-    __nanosleep(pause_ns);
-    if (*abort_flag) return false;
-    if (globaltimer_ns() - t0 > PR_WAIT_BUDGET_NS) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
-}
-
 // The one thread of a converged warp that issues TMA copies and tcgen05.mma.  Not `lane == 0`: only elect.sync tells
 // the compiler that a single thread runs the branch, so that descriptors go straight into uniform registers.
 // Measured back to back at M = 128, N = 64, K = 16 with A in tensor memory: 32 clocks per product (the pipe's own
@@ -275,11 +259,6 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 32 lanes x N consecutive 32-bit columns; thread i of the warp gets lane (base lane + i).
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -441,9 +420,5 @@ __device__ __forceinline__ void expand_second(const uint8_t* tile, int r, int Y,
   x2[0] = lo.x; x2[1] = lo.y; x2[2] = lo.z; x2[3] = lo.w;
   x2[4] = hi.x; x2[5] = hi.y; x2[6] = hi.z; x2[7] = hi.w;
 }
-
-// duplicate the low / high 16-bit half of a packed pair into both halves
-__device__ __forceinline__ uint32_t dup_lo(uint32_t x) { return __byte_perm(x, x, 0x1010); }
-__device__ __forceinline__ uint32_t dup_hi(uint32_t x) { return __byte_perm(x, x, 0x3232); }
 
 }  // namespace pr
