@@ -528,13 +528,13 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
             }
           }
         }
-        // the query tile may be refilled (its last reads come before the async proxy's writes)
+        // The query tile may be refilled (its last reads come before the async proxy's writes).  After the meeting: a
+        // group that has no step in the tile has waited for nothing of it before, and could give the slot back twice
+        // while the other is still in a run of empty tiles.
         fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&q_free[it & 1]);
-
         sm_l[tiles & 1][grp][r] = l_acc;
         meet();
+        if (lane == 0) mbar_arrive(&q_free[it & 1]);
         if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
         tc_fence_after();
         // each group writes two pieces of 16 of the row's 64 columns, one 32-byte store each

@@ -95,11 +95,11 @@ def test_more_tiles_than_resident_ctas(cuda_device, b, t, h, r, d, chunk):
     _check(cuda_device, b, t, h, r, d, chunk, True)
 
 
-@pytest.mark.parametrize("t,r", [(1100, 1), (1025, 2)])
-def test_runs_of_empty_tiles_are_taken_over(cuda_device, t, r):
+@pytest.mark.parametrize("b,t,h,r", [(4, 1100, 24, 1), (4, 1025, 24, 2), (2, 2080, 8, 4)])
+def test_runs_of_empty_tiles_are_taken_over(cuda_device, b, t, h, r):
     """A last chunk of a tile or less leaves seven tiles in a row that hold no rows, in every head of many more tiles
     than the GPU holds CTAs: each CTA takes over such runs, and its warps must not lose step in them."""
-    _check(cuda_device, 4, t, 24, r, 64, 1024, True)
+    _check(cuda_device, b, t, h, r, 64, 1024, True)
 
 
 def test_final_state_of_a_ragged_sequence(cuda_device):
