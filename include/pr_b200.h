@@ -291,7 +291,7 @@ int pr_retention_fwd(const pr_problem* problem, const void* Q, const void* K, co
 
 /* The chunk size to run a request with (0 = no chunking asked for): same results, fewer and longer chunks.
  * The chunk size blocks the computation of retention/power_retention_maker.py:143-193 without changing its
- * result; on this hardware 1024 is fastest (5.3 ms per step at chunk 128 against 2.6 at 1024 for b1 t65536 h8).
+ * result; on this hardware 1024 is fastest (5.0 ms per step at chunk 128 against 2.5 at 1024 for b1 t65536 h8).
  * pr_retention_fwd / _bwd run whatever pr_problem.c says; a host that wants the fast blocking passes
  * c = pr_fast_chunk(t, its_chunk). */
 int pr_fast_chunk(long long t, int requested_chunk);
@@ -299,10 +299,11 @@ int pr_fast_chunk(long long t, int requested_chunk);
 /* Backward.  dO [b,t,hq,d] -> dQ, dK, dV (shapes of Q, K, V) and dlog_G [b,t,h] fp32 (NULL when
  * ungated).  `saved` as the forward left it; had_carry = 1 when the forward was given carries.
  * The query-side branch (expand_grad on the saved states, chunk_dq) runs on a second stream that
- * the library owns (one per device, created at the first call - make that call outside any
+ * the library owns (eight per device, picked by `stream`; created at the first call outside a
  * stream capture), forked from and joined back into `stream` with events, so everything is
- * complete in `stream` order when the call's work is; PR_BWD_OVERLAP=0 in the environment keeps
- * the whole pass on `stream`. */
+ * complete in `stream` order when the call's work is.  On `stream` alone where the second one
+ * belongs to another stream's capture, or does not exist yet during one; PR_BWD_OVERLAP=0 in the
+ * environment keeps every pass on `stream`. */
 int pr_retention_bwd(const pr_problem* problem, const void* Q, const void* K, const void* V, const float* log_G,
                      const void* O, const void* dO, int had_carry, void* saved, void* scratch, void* dQ, void* dK,
                      void* dV, float* dlog_G, int device, void* stream);

@@ -16,7 +16,8 @@
 // its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma.  One persistent CTA per SM takes over
 // tile after tile (ClcRing).  Bound by the latency of a step's chain (products, barrier, tensor-memory loads,
 // arithmetic, stores, barrier, product); two CTAs per SM with one row group each overlapped two of them and spent
-// a third of the time on set-up and write-out: 232 -> NEW us at b1 t65536 h8 with chunks of 1024.
+// a third of the time on set-up and write-out: 232 -> 220 us at b1 t65536 h8 with chunks of 1024
+// (94 -> 84 at b4 t5000 h2x4 fp16, 20.2 -> 12.6 at b1 t1024 h4).
 #include "host.cuh"
 #include "sm100.cuh"
 

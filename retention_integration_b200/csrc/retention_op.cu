@@ -1,9 +1,9 @@
 // Whole-operator entry points: the chunked forward and backward of power retention
 // (retention/power_retention_maker.py:96-197 and what autograd executes for it) as ONE call
-// each.  The launch sequence that the Python wrapper otherwise drives kernel by kernel lives
-// here in native code, so a host in any language runs the operator through three symbols
-// (pr_workspace_bytes, pr_retention_fwd, pr_retention_bwd) and a Python host pays one ctypes
-// call per pass instead of six / eleven.
+// each, and those of the state-free branch (:128-132), where one chunk holds the whole sequence.
+// The launch sequences live here in native code, so a host in any language runs the operator
+// through three symbols per branch (pr_workspace_bytes, pr_retention_fwd, pr_retention_bwd;
+// pr_attention_workspace_bytes, pr_attention_fwd, pr_attention_bwd).
 //
 // Memory: the caller allocates everything.  `saved` is what the backward needs from the
 // forward (gate sums, row sums, scanned states and Gram matrices); `scratch` is dead when the
@@ -211,18 +211,23 @@ class Fork {
 
 // The chunk size to run a request with.  The operator's result does not depend on the chunk size, its speed
 // does: every chunk's state is written, scanned and read again (1.3 GB per pass at chunk 128 against 0.17 GB at
-// 1024 for b1 t65536 h8), and above 1024 the intra-chunk attention grows.  Below 1024: the largest multiple of the
-// request up to 1024 that pads the sequence by at most 1/16 more than the request would; above: the largest divisor
-// of the request in [256, 1024]; 0 (no chunking) on more than 2048 tokens: 1024 or 512 if that pads by at most
-// 1/16, else 0.  Mirrors retention.py: effective_chunk, for hosts that do not go through the Python API.
+// 1024 for b1 t65536 h8), and above 1024 the intra-chunk attention grows.  Forward + backward of that shape in ms, as
+// asked: chunk 128 5.04, 256 3.42, 512 2.68, 1024 2.46, 2048 2.63, 4096 3.30.  Below 1024: the largest multiple of the
+// request up to 1024 that rounds the length up by at most 1/16 more than the request does; above: the largest divisor
+// of the request in [256, 1024]; 0 (no chunking) on more than 2048 tokens: 1024 or 512 if that rounds the length up by
+// at most 1/16, else 0.
+// The rounding was work while sequences were padded to whole chunks.  They no longer are, and by work the rule errs
+// where it still decides: t 2000 with chunk 128 takes two chunks of 1024 (115 us replayed from a graph, b1 h2) where
+// one without states takes 77, t 1100 three of 384 (90 us, b1 h4; 51), and t 7200 unchunked stays one (358 us, b1 h4)
+// where chunks of 1024 take 194.  Mirrors retention.py: effective_chunk, for hosts that do not go through the Python API.
 extern "C" int pr_fast_chunk(long long t, int requested) {
   const int fast = 1024;
   if (t <= 0 || requested < 0) return requested;
-  auto padded_to = [t](long long c) { return (t + c - 1) / c * c; };
+  auto rounded_to = [t](long long c) { return (t + c - 1) / c * c; };
   if (requested == 0) {
     if (t <= 2 * fast) return 0;
     for (int ce : {fast, fast / 2})
-      if (padded_to(ce) <= t + t / 16) return ce;
+      if (rounded_to(ce) <= t + t / 16) return ce;
     return 0;
   }
   if (requested > fast) {
@@ -231,10 +236,10 @@ extern "C" int pr_fast_chunk(long long t, int requested) {
     return requested;
   }
   if (requested == fast) return requested;
-  const long long padded = padded_to(requested);
+  const long long asked = rounded_to(requested);
   for (int m = fast / requested; m > 1; --m) {
     const long long ce = (long long)m * requested;
-    if (padded_to(ce) <= padded + padded / 16) return (int)ce;
+    if (rounded_to(ce) <= asked + asked / 16) return (int)ce;
   }
   return requested;
 }

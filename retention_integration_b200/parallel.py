@@ -230,7 +230,7 @@ def power_retention_sequence_parallel(Q, K, V, log_G=None, deg=2, scale=None, ch
     from . import retention
 
     if retention.AUTO_CHUNK and deg == 2 and chunk_size < 1024:
-        # as in power_retention: a small chunk is run with a multiple of it (here one that needs no padding)
+        # as in power_retention: a small chunk is run with a multiple of it (here one that divides the block)
         for m in range(1024 // chunk_size, 1, -1):
             if t % (m * chunk_size) == 0:
                 chunk_size = m * chunk_size

@@ -1,7 +1,7 @@
 """`power_retention` and `power_retention_inference` with the reference's signatures
 (retention/power_retention_maker.py:72-73 and :287-288), running on libpr_b200.so.
 
-The host side only validates arguments, pads, allocates and sequences kernel launches;
+The host side only validates arguments, allocates and sequences kernel launches;
 every arithmetic step of the path is a kernel of the C-ABI library.  That host side is native
 (csrc/binding.cpp); what is left here drives the same kernels one by one from Python.  There is no
 PyTorch or CPU fallback: inputs must be CUDA tensors of dtype bfloat16 or float16.
@@ -140,10 +140,10 @@ def _pad_head_dim(x, d_to):
 # to the same function for every chunk size, and so do the kernels here - tested).  Small chunks are slow on
 # this hardware for a reason the arithmetic does not care about: every chunk's state (2560 x 64 per head) is written,
 # scanned and read again, 1.3 GB per pass at chunk 128 against 0.17 GB at chunk 1024 for the benchmark's shape
-# (5.3 vs 2.6 ms per step).  With AUTO_CHUNK the Python API therefore runs a request for a chunk below 1024 with the
-# largest multiple of it that is at most 1024 and pads the sequence by at most 1/16 more than the request would
-# (padding tokens are zero keys and values behind gates of 1: they change neither the outputs of the real tokens nor
-# the state after the last one).  The C ABI (pr_retention_fwd) always takes the chunk it is given.
+# (5.0 vs 2.5 ms per step).  With AUTO_CHUNK the Python API therefore runs a request for a chunk below 1024 with the
+# largest multiple of it that is at most 1024 and rounds the length up by at most 1/16 more than the request does
+# (the sequence is not padded: its last chunk is shorter; csrc/retention_op.cu has the rule's figures, and where it
+# errs).  The C ABI (pr_retention_fwd) always takes the chunk it is given.
 AUTO_CHUNK = True
 _FAST_CHUNK = 1024
 
@@ -151,10 +151,10 @@ _FAST_CHUNK = 1024
 def effective_chunk(t: int, chunk_size, deg: int = 2):
     """The chunk size power_retention runs with for a sequence of t tokens and a requested chunk_size.
 
-    Below 1024: the largest multiple of the request up to 1024 that pads by at most 1/16 more.  Above 1024 (slower
-    again: the intra-chunk attention grows with the chunk): the largest divisor of the request in [256, 1024], which
-    leaves the padded length as it is.  None (no chunking) on a long sequence: 1024 or 512 if that pads by at most
-    1/16; the quadratic form otherwise.  deg 4 forms no states and is never chunked."""
+    Below 1024: the largest multiple of the request up to 1024 that rounds the length up by at most 1/16 more.  Above
+    1024 (slower again: the intra-chunk attention grows with the chunk): the largest divisor of the request in
+    [256, 1024], which leaves the rounded length as it is.  None (no chunking) on a long sequence: 1024 or 512 if that
+    rounds up by at most 1/16; the quadratic form otherwise.  deg 4 forms no states and is never chunked."""
     if not AUTO_CHUNK or deg != 2:
         return chunk_size
     if chunk_size is None:
@@ -171,10 +171,10 @@ def effective_chunk(t: int, chunk_size, deg: int = 2):
         return chunk_size
     if chunk_size == _FAST_CHUNK:
         return chunk_size
-    padded = -(-t // chunk_size) * chunk_size  # what the request itself pads to
+    asked = -(-t // chunk_size) * chunk_size  # what the request itself rounds up to
     for m in range(_FAST_CHUNK // chunk_size, 1, -1):
         ce = m * chunk_size
-        if -(-t // ce) * ce <= padded + padded // 16:
+        if -(-t // ce) * ce <= asked + asked // 16:
             return ce
     return chunk_size
 
