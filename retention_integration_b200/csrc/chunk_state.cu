@@ -8,16 +8,22 @@
 // Backward use (gradient of the state read-out, retention/_query_state/triton.py:337-448):
 //   x = gated queries, v = dO / l, weights off -> dZ_m; xs = x * dl -> gram = d(gram of Z).
 //
-// One CTA owns two tiles of 128 expanded rows, so every operand stage fetched from L2 feeds two
-// products.  The expansion is never written to shared or global memory: each thread owns the
-// expanded rows (a, b) and (a + 8, b) - the same row of both tiles, which share their second
-// factor - for half of the tokens of a stage, multiplies rows a, a + 8 and b of the transposed
-// operand (TMA-loaded, 128-byte swizzled) with packed 16-bit multiplies and stores the products
-// straight into tensor memory as the A operands of tcgen05.mma.  The kernel is bound by the
-// shared-memory reads that feed those multiplies (traced: ~1000 clocks per stage and SM against ~430
-// for the tensor core), which is why the second factor is read once for two products; the values come in by TMA as the MN-major B operand; fp32 accumulation in
-// tensor memory.  The last grid slot in x computes the Gram matrix with both operands
-// in shared memory.
+// An item is two tiles of 128 expanded rows of one state, so every operand stage fetched from L2 feeds two products, or a
+// state's Gram matrix.  The expansion is never written to shared or global memory: a thread owns the expanded rows
+// (a, b) and (a + 8, b) - the same row of both tiles, which share their second factor - multiplies rows a, a + 8 and b
+// of the transposed operand (TMA-loaded, 128-byte swizzled) with packed 16-bit multiplies and stores the products
+// straight into tensor memory as the A operands of tcgen05.mma; the values come in by TMA as the MN-major B operand;
+// fp32 accumulation in tensor memory.
+//
+// One persistent CTA per SM takes over item after item (ClcRing).  Four groups of four warps take the 64-token stages in
+// turn, each with a slot of its own in tensor memory; one thread per tile issues the products; four more warps write an
+// item out from the first pair of accumulators while the next one fills the second.  Before, two CTAs per SM expanded
+// every stage with all their warps into two slots: of a CTA's 24 thousand clocks at sixteen stages, half was set-up, first
+// loads, cold instructions and write-out, and a barrier round was paid for half a stage's work.  252 -> 232 us at
+// b1 t65536 h8 with chunks of 1024, 83 -> 60 at b4 t4096 h2 with four query heads summed, 406 -> 375 at b16 t2048 h32 in one
+// chunk, 15.1 -> 14.1 at b1 t2048 h2 (groups in turn alone: 238, 72, 375, 14.7).  A stage costs the shared-memory pipe
+// about 560 clocks (the operand reads, 8 for 16 products; the tensor core's own reads; tensor-memory stores), the
+// tensor pipe 256.
 //
 // EXACT (a token cache compressed into an inference state, retention/power_retention_maker.py:374-388): the read-out
 // writes the state in the exact layout, state * e^a_last + the cache's part in fp32, and sum_of_keys from the Gram
@@ -31,21 +37,24 @@ namespace pr {
 
 namespace cs {
 constexpr int HD = 64;          // head dim handled by this build of the kernel
-constexpr int NS = 4;           // shared-memory pipeline stages
-constexpr int NSA = 2;          // tensor-memory stages of each group's expansion ring
-constexpr int NG = 2;           // row tiles (groups of 4 warps) per CTA: each loaded stage feeds both
+constexpr int NT = 2;           // tiles of 128 expanded rows per item: every loaded stage feeds both
+constexpr int NG = 4;           // groups of 4 warps that expand the stages in turn
+constexpr int NS = 8;           // shared-memory pipeline stages
 constexpr int TOK = 64;         // tokens per stage
-constexpr int THREADS = 352;    // warps 0-3 / 4-7 expand + epilogue (one group per row tile), 8 TMA, 9 / 10 MMA of group 0 / 1
+constexpr int W_OUT = 4 * NG, W_TMA = W_OUT + 4, W_MMA = W_TMA + 1;  // four write-out warps, one issuing warp per tile
+constexpr int THREADS = 32 * (W_MMA + NT);
 constexpr int XT_BYTES = HD * TOK * 2;   // 8 KB
 constexpr int W_BYTES = TOK * HD * 2;    // 8 KB
-constexpr int GA_BYTES = 128 * TOK * 2;  // Gram A operand padded to 128 rows
-constexpr uint32_t TMEM_COLS = 256;
-constexpr uint32_t COL_ACC = 0;    // NG x 64 columns
-constexpr uint32_t COL_A = 128;    // NG rings of NSA x 32 columns
+constexpr int R_BYTES = XT_BYTES + W_BYTES;
+constexpr size_t SMEM = 1024 + NS * R_BYTES + XT_BYTES;  // + the rows past a Gram operand, which the products read for nothing
+constexpr uint32_t TMEM_COLS = 512;
+__device__ __forceinline__ constexpr uint32_t col_acc(int tb, int tile) { return (uint32_t)(tb * NT + tile) * 64u; }
+__device__ __forceinline__ constexpr uint32_t col_a(int grp, int tile) { return 256u + (uint32_t)(grp * NT + tile) * 32u; }
 }  // namespace cs
 
 struct ChunkStateParams {
-  int n_tiles;      // tiles of 128 expanded rows; grid.x = ceil(n_tiles / 2) + (gram ? 1 : 0)
+  int n_slots;      // items of two tiles of 128 expanded rows per state
+  int n_states;     // states (batch, chunk, head); grid.x = n_slots * n_states + (Gram matrices wanted ? n_states : 0)
   int nh;           // kv heads of the output
   int group;        // operand heads summed into one output head (GQA ratio in backward)
   int c, cp;        // chunk length, padded to 64
@@ -64,294 +73,355 @@ struct ChunkStateParams {
   int* status;
 };
 
+// What a CTA index stands for: two tiles of 128 expanded rows of one state, or its Gram matrix.  The tiles of a state
+// follow one another and share its operands through L2; the Gram matrices come last: they are short, which evens out
+// the end of the launch.
+struct StateItem {
+  int slot, chunk, head, batch, ch, kblocks, total;
+  bool gram;
+  __device__ __forceinline__ StateItem(const ChunkStateParams& p, unsigned cta) {
+    const unsigned n = (unsigned)p.n_slots * (unsigned)p.n_states;
+    gram = cta >= n;
+    const int which = (int)(gram ? cta - n : cta / (unsigned)p.n_slots);
+    slot = gram ? 0 : (int)(cta % (unsigned)p.n_slots);
+    head = which % p.nh;
+    chunk = p.chunk0 + (which / p.nh) % p.n_run;
+    batch = which / (p.nh * p.n_run);
+    ch = (batch * p.n_chunks + chunk) * p.nh + head;
+    kblocks = (min(p.c, p.t - chunk * p.c) + cs::TOK - 1) / cs::TOK;
+    total = kblocks * p.group;
+  }
+};
+
 template <typename T, bool EXACT>
-__global__ void __maxnreg__(80)
+__global__ void __launch_bounds__(cs::THREADS, 1)
 chunk_state_kernel(const ChunkStateParams p, const __grid_constant__ CUtensorMap tm_xt,
                    const __grid_constant__ CUtensorMap tm_xs, const __grid_constant__ CUtensorMap tm_w) {
   using namespace cs;
   extern __shared__ uint8_t smem_raw[];
-  // done[g][s]: the products of group g on stage s have completed.  ONE commit per stage and issuing thread
-  // serves both waiters - the expansion warps (their tensor-memory slot of two stages ago is free) and the TMA
-  // thread (the value tile of four stages ago is free): a commit costs the issuing thread ~150 clocks, a third
-  // of what the four products of a stage cost it.
-  __shared__ uint64_t x_full[NS], x_empty[NS], w_full[NS], w_empty[NS], a_full[NG][NSA], done[NG][NS], acc_done;
+  // full: a stage's operands have arrived.  a_full: a group has written the expansion of its stage.  done: the products
+  // of a stage have completed, which frees both the stage (TMA) and the group's slot in tensor memory.  A Gram matrix has
+  // no expansions: the groups report on a_full that they have seen their last phases of `done` before its products start,
+  // and wait for gram_done, or they could fall two phases behind, or be two ahead, on the ring's barriers.
+  // acc_full / acc_free: an item's accumulators are complete / read out.
+  __shared__ uint64_t full[NS], done[NS], a_full[NG], gram_done, acc_full[2], acc_free[2];
+  __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* sm = smem_raw + (sbase - smem_u32(smem_raw));
-  uint8_t* smX = sm;                          // NS x XT_BYTES (rows = features, 64 tokens)
-  uint8_t* smW = sm + NS * XT_BYTES;          // NS x W_BYTES  (rows = tokens, 64 features)
-  uint8_t* smG = smW;                         // Gram CTA only: 2 x GA_BYTES over the (unused) value ring
+  uint8_t* smR = smem_raw + (sbase - smem_u32(smem_raw));  // NS x (rows = features, 64 tokens; rows = tokens, 64 features)
 
-  // grid.x = slots * (batch, chunk, head) triples, slot fastest: the CTAs of one triple run together and
-  // share their operand tiles through L2, and the triple count is not bound by the 65535 limit of grid.y
-  const int n_tile_ctas = (p.n_tiles + NG - 1) / NG;
-  const int slots = n_tile_ctas + (EXACT || p.gram ? 1 : 0);
-  const int slot = (int)(blockIdx.x % (unsigned)slots);
-  const bool gram_cta = (slot == n_tile_ctas);
-  const int which = (int)(blockIdx.x / (unsigned)slots);
-  const int head = which % p.nh;
-  const int chunk = p.chunk0 + (which / p.nh) % p.n_run;
-  const int batch = which / (p.nh * p.n_run);
-  const int ch = (batch * p.n_chunks + chunk) * p.nh + head;
-  const int kblocks = (min(p.c, p.t - chunk * p.c) + TOK - 1) / TOK;
-  const int total = kblocks * p.group;
-
-  if (tid == 0) {
-    abort_flag = 0;
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(&x_full[s], 1);
-      mbar_init(&x_empty[s], 4 * NG);  // every expansion warp
-      mbar_init(&w_full[s], 1);
-      mbar_init(&w_empty[s], 1);  // Gram CTA only
-    }
-    for (int g = 0; g < NG; ++g)
-      for (int s = 0; s < NSA; ++s) {
-        mbar_init(&a_full[g][s], 4 * NG);  // every expansion warp fills its half of each tile's stage
+  if (warp == W_TMA) {
+    if (elect_one()) {
+      tma_prefetch_desc(&tm_xt);
+      tma_prefetch_desc(&tm_w);
+      abort_flag = 0;
+      for (int s = 0; s < NS; ++s) {
+        mbar_init(&full[s], 1);
+        mbar_init(&done[s], NT);
       }
-    for (int g = 0; g < NG; ++g)
-      for (int s = 0; s < NS; ++s) mbar_init(&done[g][s], 1);
-    mbar_init(&acc_done, gram_cta ? 1 : NG);
-    fence_mbar_init();
+      for (int g = 0; g < NG; ++g) mbar_init(&a_full[g], 4);
+      mbar_init(&gram_done, NT);
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(&acc_full[b], NT);
+        mbar_init(&acc_free[b], 4);
+      }
+      clc_init(&clc, 4 * NG + 4 + 1 + NT);
+      fence_mbar_init();
+    }
+    __syncwarp();
+    named_bar_arrive(1, THREADS);  // the first loads need not wait for the tensor memory
+  } else {
+    if (warp == 0) {
+      tmem_alloc(&tmem_base_s, TMEM_COLS);
+      tmem_relinquish();
+    }
+    tc_fence_before();
+    named_bar_sync(1, THREADS);
+    tc_fence_after();
   }
-  if (warp == 0) {
-    tmem_alloc(&tmem_base_s, TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
 
-  if (warp == 4 * NG) {
+  if (warp == W_TMA) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      for (int it = 0; it < total; ++it) {
-        const int s = it % NS, ph = (it / NS) & 1;
-        const int g = it / kblocks, kb = it % kblocks;
-        const int xhead = head * p.group + g;
-        const int xrow = ((batch * p.n_chunks + chunk) * (p.nh * p.group) + xhead) * p.d;
-        if (!gram_cta && !mbar_wait(&x_empty[s], ph ^ 1, &abort_flag)) break;
-        if (gram_cta) {
-          // two stages only: the padded A operand is twice the size of a value stage
-          const int gs = it & 1, gph = (it >> 1) & 1;
-          if (!mbar_wait(&w_empty[gs], gph ^ 1, &abort_flag)) break;
-          mbar_expect_tx(&w_full[gs], 2 * p.d * (TOK * 2));
-          tma_load_2d(smX + gs * XT_BYTES, &tm_xt, &w_full[gs], kb * TOK, xrow);
-          tma_load_2d(smG + gs * GA_BYTES, &tm_xs, &w_full[gs], kb * TOK, xrow);
-        } else {
-          mbar_expect_tx(&x_full[s], p.d * (TOK * 2));
-          tma_load_2d(smX + s * XT_BYTES, &tm_xt, &x_full[s], kb * TOK, xrow);
-          if (it >= NS && !(mbar_wait(&done[0][s], ph ^ 1, &abort_flag) && mbar_wait(&done[1][s], ph ^ 1, &abort_flag)))
-            break;
-          mbar_expect_tx(&w_full[s], W_BYTES);
-          tma_load_4d(smW + s * W_BYTES, &tm_w, &w_full[s], 0, xhead, chunk * p.c + kb * TOK, batch);
-        }
-      }
-    }
-  } else if (warp >= 4 * NG + 1) {
-    // ------------------------------------------------------------- MMA issuers
-    // One issuing thread per group: a single thread needs some 60-80 clocks per tcgen05.mma it
-    // issues and as many per commit or barrier wait, which made one thread serving both groups
-    // the slowest stage of the pipeline.
-    const int g = warp - (4 * NG + 1);
-    if ((!gram_cta || g == 0) && elect_one()) {
       bool ok = true;
-      if (gram_cta) {
-        const uint32_t idesc = umma_idesc(128, HD, Pack2<T>::is_bf16, false, false);
-        for (int it = 0; it < total && ok; ++it) {
-          const int gs = it & 1, gph = (it >> 1) & 1;
-          ok = mbar_wait(&w_full[gs], gph, &abort_flag);
+      dim3 cta = blockIdx;
+      int s = 0;
+      uint32_t ph = 1;
+      for (int it = 0; ok; ++it) {
+        const StateItem w(p, cta.x);
+        int kb = 0, xhead = w.head * p.group;
+        int xrow = ((w.batch * p.n_chunks + w.chunk) * (p.nh * p.group) + xhead) * p.d;
+        for (int i = 0; i < w.total && ok; ++i) {
+          ok = mbar_wait(&done[s], ph, &abort_flag);
           if (!ok) break;
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smG + gs * GA_BYTES), b_addr = smem_u32(smX + gs * XT_BYTES);
-#pragma unroll
-          for (int ks = 0; ks < TOK / 16; ++ks)
-            umma_ss(tmem + COL_ACC, umma_desc_sw128(a_addr + ks * 32, 16, 1024),
-                    umma_desc_sw128(b_addr + ks * 32, 16, 1024), idesc, (it > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&w_empty[gs]);
+          uint8_t* dst = smR + s * R_BYTES;
+          mbar_expect_tx(&full[s], p.d * (TOK * 2) + (w.gram ? p.d * (TOK * 2) : W_BYTES));
+          tma_load_2d(dst, &tm_xt, &full[s], kb * TOK, xrow);
+          if (w.gram)
+            tma_load_2d(dst + XT_BYTES, &tm_xs, &full[s], kb * TOK, xrow);
+          else
+            tma_load_4d(dst + XT_BYTES, &tm_w, &full[s], 0, xhead, w.chunk * p.c + kb * TOK, w.batch);
+          if (i == 0) ok = clc_ask(&clc, it, &abort_flag);
+          if (++kb == w.kblocks) kb = 0, ++xhead, xrow += p.d;
+          if (++s == NS) s = 0, ph ^= 1;
         }
-      } else {
-        const uint32_t idesc = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
-        const uint64_t d_w0 = umma_desc_sw128(smem_u32(smW), 8192, 1024);
-        for (int it = 0; it < total && ok; ++it) {
-          const int s = it % NS, ph = (it / NS) & 1;
-          const int sa = it % NSA, pha = (it / NSA) & 1;
-          ok = mbar_wait(&w_full[s], ph, &abort_flag) && mbar_wait(&a_full[g][sa], pha, &abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t d_w = d_w0 + (uint32_t)s * (W_BYTES >> 4);
-#pragma unroll
-          for (int ks = 0; ks < TOK / 16; ++ks)
-            umma_ts(tmem + COL_ACC + g * 64, tmem + COL_A + (g * NSA + sa) * 32 + ks * 8,
-                    d_w + ks * (2048 >> 4), idesc, (it > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&done[g][s]);
-        }
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
-      if (ok) umma_commit(&acc_done);
     }
-  } else {
-    // ------------------------------------------------- expansion + epilogue warps
-    const int grp = warp >> 2;
+  } else if (warp >= W_MMA) {
+    // ------------------------------------------------------------- MMA issuers
+    // One thread per tile: a stage's four products of a tile take the tensor pipe 128 clocks, about what one thread
+    // needs for the wait, the issue and the commit.
+    if (elect_one()) {
+      const uint32_t tmem = tmem_base_s;
+      const int tl = warp - W_MMA;
+      const uint32_t ring = smem_u32(smR);
+      const uint32_t idesc = umma_idesc(128, HD, Pack2<T>::is_bf16, false, true);
+      const uint32_t idesc_g = umma_idesc(128, HD / 2, Pack2<T>::is_bf16, false, false);
+      const uint64_t d_w0 = umma_desc_sw128(ring + XT_BYTES, 8192, 1024);
+      // the Gram matrix: each thread half of its columns
+      const uint64_t d_g0 = umma_desc_sw128(ring + XT_BYTES, 16, 1024),
+                     d_x0 = umma_desc_sw128(ring + tl * (HD / 2 * 128), 16, 1024);
+      bool ok = true;
+      dim3 cta = blockIdx;
+      int s = 0, grp = 0;
+      uint32_t ph = 0, a_ph = 0;
+      for (int it = 0; ok; ++it) {
+        const StateItem w(p, cta.x);
+        const int tb = it & 1;
+        if (it >= 2) ok = mbar_wait(&acc_free[tb], ((it >> 1) - 1) & 1, &abort_flag);
+        if (w.gram) {
+          const uint32_t acc = tmem + col_acc(tb, 0) + tl * (HD / 2);
+          for (int j = 0; j < NG && ok; ++j) {
+            ok = mbar_wait(&a_full[grp], a_ph, &abort_flag);
+            if (++grp == NG) grp = 0, a_ph ^= 1;
+          }
+          for (int i = 0; i < w.total && ok; ++i) {
+            ok = mbar_wait(&full[s], ph, &abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t off = (uint32_t)s * (R_BYTES >> 4);
+#pragma unroll
+            for (int ks = 0; ks < TOK / 16; ++ks)
+              umma_ss(acc, d_g0 + off + 2 * ks, d_x0 + off + 2 * ks, idesc_g, (i > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(&done[s]);
+            if (++s == NS) s = 0, ph ^= 1;
+          }
+          if (ok) umma_commit(&gram_done);
+        } else {
+          const uint32_t acc = tmem + col_acc(tb, tl);
+          for (int i = 0; i < w.total && ok; ++i) {
+            // the warps that wrote the operand have seen the stage's arrival
+            ok = mbar_wait(&a_full[grp], a_ph, &abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t d_w = d_w0 + (uint32_t)s * (R_BYTES >> 4);
+            const uint32_t ca = tmem + col_a(grp, tl);
+#pragma unroll
+            for (int ks = 0; ks < TOK / 16; ++ks)
+              umma_ts(acc, ca + ks * 8, d_w + ks * (2048 >> 4), idesc, (i > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(&done[s]);
+            if (++s == NS) s = 0, ph ^= 1;
+            if (++grp == NG) grp = 0, a_ph ^= 1;
+          }
+        }
+        if (ok) umma_commit(&acc_full[tb]);
+        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
+      }
+    }
+  } else if (warp >= W_OUT) {
+    // ------------------------------------------------------------------ write-out
+    const uint32_t tmem = tmem_base_s;
     const int row_in_tile = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    const int D2 = p.n_tiles * 128;
-    // expansion: this thread's row of both tiles (first factors a0 and a0 + 8, common second factor b),
-    // tokens [32 grp, 32 grp + 32) of every stage; epilogue: its row of tile `grp`
-    const int drow0 = slot * NG * 128 + row_in_tile;
-    int a0 = 0, b = 0;
-    if (!gram_cta && drow0 < D2) ref_decode(drow0, &a0, &b);
-    const int a1 = min(a0 + 8, HD - 1);  // the second tile of a pair lies in the same block of second factors
-    const int tile = slot * NG + grp;
-    const int drow = tile * 128 + row_in_tile;
-    const bool valid = !gram_cta && drow < D2;  // rows past the end still take part in the pipeline
-    const int a = grp ? a1 : a0;
     bool ok = true;
-    // swz128(row, j) = (row * 128 + ((row & 7) << 4)) ^ (j << 4): one XOR per address
-    const uint32_t a0_base = a0 * 128 + ((a0 & 7) << 4), a1_base = a1 * 128 + ((a1 & 7) << 4),
-                   b_base = b * 128 + ((b & 7) << 4);
-    if (!gram_cta) {
-      for (int it = 0; it < total; ++it) {
-        const int s = it % NS, ph = (it / NS) & 1;
-        ok = mbar_wait(&x_full[s], ph, &abort_flag);
-        if (!ok) break;
-        const uint8_t* xs = smX + s * XT_BYTES;
-        uint32_t r0[16], r1[16];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const uint32_t off = (uint32_t)((4 * grp + jj) << 4);
-          const uint4 vb = *reinterpret_cast<const uint4*>(xs + (b_base ^ off));
-          const uint4 va = *reinterpret_cast<const uint4*>(xs + (a0_base ^ off));
-          const uint4 vc = *reinterpret_cast<const uint4*>(xs + (a1_base ^ off));
-          r0[4 * jj + 0] = Pack2<T>::mul(va.x, vb.x);
-          r0[4 * jj + 1] = Pack2<T>::mul(va.y, vb.y);
-          r0[4 * jj + 2] = Pack2<T>::mul(va.z, vb.z);
-          r0[4 * jj + 3] = Pack2<T>::mul(va.w, vb.w);
-          r1[4 * jj + 0] = Pack2<T>::mul(vc.x, vb.x);
-          r1[4 * jj + 1] = Pack2<T>::mul(vc.y, vb.y);
-          r1[4 * jj + 2] = Pack2<T>::mul(vc.z, vb.z);
-          r1[4 * jj + 3] = Pack2<T>::mul(vc.w, vb.w);
+    dim3 cta = blockIdx;
+    for (int it = 0; ok; ++it) {
+      const StateItem w(p, cta.x);
+      const int tb = it & 1;
+      const float decay = !EXACT || p.state == nullptr ? 0.f : (p.a_last ? __expf(p.a_last[w.ch]) : 1.f);
+      ok = mbar_wait(&acc_full[tb], (it >> 1) & 1, &abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      int a, b;
+      ref_decode(w.slot * (NT * 128) + row_in_tile, &a, &b);
+#pragma unroll 1
+      for (int part = 0; part < 2 * NT; ++part) {
+        // 32 columns of the row in tile part / 2
+        const int tl = part >> 1, c0 = 32 * (part & 1);
+        uint32_t acc[32];
+        tmem_ld32(tmem + lane_addr + col_acc(tb, tl) + c0, acc);
+        tmem_wait_ld();
+        if (part == 2 * NT - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_free[tb]);
         }
-        const int sa = it % NSA;
-        if (it >= NSA) {
-          // both tiles' products of stage it - NSA have read this tensor-memory slot
-          const int sp = (it - NSA) % NS, php = ((it - NSA) / NS) & 1;
-          ok = mbar_wait(&done[0][sp], php, &abort_flag) && mbar_wait(&done[1][sp], php, &abort_flag);
-          if (!ok) break;
-        }
-        tc_fence_after();
-        tmem_st16(tmem + lane_addr + COL_A + (0 * NSA + sa) * 32 + 16 * grp, r0);
-        tmem_st16(tmem + lane_addr + COL_A + (1 * NSA + sa) * 32 + 16 * grp, r1);
-        // The shared-memory stage goes back to TMA only here: the stores above have consumed every
-        // product, so every load of the stage has delivered its data.  Released right after the
-        // loads were issued (a plain arrive), a refill could overtake loads still queued in this
-        // LDS-heavy kernel, and single rows of the state came out built from the wrong 64 tokens
-        // (seen only with two CTAs per SM at grids of thousands of CTAs).  The proxy fence orders
-        // this thread's generic-proxy reads before the async-proxy write that follows the release.
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&x_empty[s]);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&a_full[0][sa]);
-          mbar_arrive(&a_full[1][sa]);
-        }
-      }
-    }
-    if (ok) ok = mbar_wait(&acc_done, 0, &abort_flag);
-    tc_fence_after();
-    if (ok) {
-      uint32_t acc[64];
-      tmem_ld32(tmem + lane_addr + COL_ACC + grp * 64, acc);
-      tmem_ld32(tmem + lane_addr + COL_ACC + grp * 64 + 32, acc + 32);
-      tmem_wait_ld();
-      const float decay = !EXACT || p.state == nullptr ? 0.f : (p.a_last ? __expf(p.a_last[ch]) : 1.f);
-      if (gram_cta) {
-        if (EXACT) {
-          if (grp == 0 && row_in_tile < HD) {
-            // row a of the Gram matrix holds the pairs (a, b >= a), which lie side by side
-            const size_t at = (size_t)ch * exact_dim(HD) + exact_row(HD, row_in_tile, row_in_tile) - row_in_tile;
+        const int ar = a + 8 * tl;  // the two tiles share their second factors
+        if (w.gram) {
+          if (tl == 0 && row_in_tile < p.d) {
+            if (EXACT) {
+              // row a of the Gram matrix holds the pairs (a, b >= a), which lie side by side
+              const size_t at = (size_t)w.ch * exact_dim(HD) + exact_row(HD, row_in_tile, row_in_tile) - row_in_tile;
 #pragma unroll
-            for (int j = 0; j < HD; ++j)
-              if (j >= row_in_tile)
-                p.new_sok[at + j] = (p.sok != nullptr ? p.sok[at + j] * decay : 0.f) +
-                                    __uint_as_float(acc[j]) * (j == row_in_tile ? 1.f : 2.f);
-          }
-        } else if (grp == 0 && row_in_tile < p.d && p.gram != nullptr) {
-          float4* dst = reinterpret_cast<float4*>(p.gram + ((size_t)ch * p.d + row_in_tile) * p.d);
+              for (int j = 0; j < 32; ++j)
+                if (c0 + j >= row_in_tile)
+                  p.new_sok[at + c0 + j] = (p.sok != nullptr ? p.sok[at + c0 + j] * decay : 0.f) +
+                                           __uint_as_float(acc[j]) * (c0 + j == row_in_tile ? 1.f : 2.f);
+            } else {
+              float4* dst = reinterpret_cast<float4*>(p.gram + ((size_t)w.ch * p.d + row_in_tile) * p.d + c0);
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (4 * j < p.d) dst[j] = make_float4(__uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]),
-                                 __uint_as_float(acc[4 * j + 2]), __uint_as_float(acc[4 * j + 3]));
-        }
-      } else if (EXACT) {
-        if (valid && a <= b) {
-          const float wgt = a == b ? 1.f : 2.f;
-          const size_t at = ((size_t)ch * exact_dim(HD) + exact_row(HD, a, b)) * HD;
-          T* dst = static_cast<T*>(p.out) + at;
-          const T* old = static_cast<const T*>(p.state) + at;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 o[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-            if (p.state != nullptr) {
-              o[0] = *reinterpret_cast<const uint4*>(old + 16 * j);
-              o[1] = *reinterpret_cast<const uint4*>(old + 16 * j + 8);
+              for (int j = 0; j < 8; ++j)
+                if (c0 + 4 * j < p.d)
+                  dst[j] = make_float4(__uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]),
+                                       __uint_as_float(acc[4 * j + 2]), __uint_as_float(acc[4 * j + 3]));
             }
-            const uint32_t ow[8] = {o[0].x, o[0].y, o[0].z, o[0].w, o[1].x, o[1].y, o[1].z, o[1].w};
+          }
+        } else if (EXACT) {
+          if (ar <= b) {
+            const float wgt = ar == b ? 1.f : 2.f;
+            const size_t at = ((size_t)w.ch * exact_dim(HD) + exact_row(HD, ar, b)) * HD + c0;
+            T* dst = static_cast<T*>(p.out) + at;
+            const T* old = static_cast<const T*>(p.state) + at;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              uint4 o[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+              if (p.state != nullptr) {
+                o[0] = *reinterpret_cast<const uint4*>(old + 16 * j);
+                o[1] = *reinterpret_cast<const uint4*>(old + 16 * j + 8);
+              }
+              const uint32_t ow[8] = {o[0].x, o[0].y, o[0].z, o[0].w, o[1].x, o[1].y, o[1].z, o[1].w};
+              uint32_t v[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                // the reference rounds state * decay to the state's dtype before adding (:374-382)
+                const float2 raw = Pack2<T>::to_f32(ow[k]);
+                const float2 od = Pack2<T>::to_f32(Pack2<T>::from_f32(raw.x * decay, raw.y * decay));
+                v[k] = Pack2<T>::from_f32(od.x + wgt * __uint_as_float(acc[16 * j + 2 * k]),
+                                          od.y + wgt * __uint_as_float(acc[16 * j + 2 * k + 1]));
+              }
+              st_global_v8(dst + 16 * j, v);
+            }
+          }
+        } else {
+          const float wgt = p.key_weights ? ref_key_weight(ar, b) : 1.f;
+          T* dst = static_cast<T*>(p.out) + ((size_t)w.ch * (p.n_slots * NT * 128) + (w.slot * NT + tl) * 128 + row_in_tile) * p.d + c0;
+          // 32-byte stores: a full sector per thread and instruction
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (c0 + 16 * j >= p.d) break;
             uint32_t v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              // the reference rounds state * decay to the state's dtype before adding (:374-382)
-              const float2 raw = Pack2<T>::to_f32(ow[k]);
-              const float2 od = Pack2<T>::to_f32(Pack2<T>::from_f32(raw.x * decay, raw.y * decay));
-              v[k] = Pack2<T>::from_f32(od.x + wgt * __uint_as_float(acc[16 * j + 2 * k]),
-                                        od.y + wgt * __uint_as_float(acc[16 * j + 2 * k + 1]));
-            }
+            for (int k = 0; k < 8; ++k)
+              v[k] = Pack2<T>::from_f32(wgt * __uint_as_float(acc[16 * j + 2 * k]), wgt * __uint_as_float(acc[16 * j + 2 * k + 1]));
             st_global_v8(dst + 16 * j, v);
           }
         }
-      } else if (valid) {
-        const float wgt = p.key_weights ? ref_key_weight(a, b) : 1.f;
-        T* dst = static_cast<T*>(p.out) + ((size_t)ch * D2 + drow) * p.d;
-        // four 32-byte stores: a full sector per thread and instruction
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (16 * j >= p.d) break;
-          uint32_t v[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            v[k] = Pack2<T>::from_f32(wgt * __uint_as_float(acc[16 * j + 2 * k]), wgt * __uint_as_float(acc[16 * j + 2 * k + 1]));
-          asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 16 * j), "r"(v[0]), "r"(v[1]),
-                       "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-                       : "memory");
-        }
       }
+      if (!clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
+    }
+  } else {
+    // ------------------------------------------------------------------ expansion
+    const uint32_t tmem = tmem_base_s;
+    const int grp = warp >> 2;
+    const int row_in_tile = (warp & 3) * 32 + lane;
+    const uint32_t ca = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col_a(grp, 0);
+    bool ok = true;
+    dim3 cta = blockIdx;
+    int g0 = 0, u0 = 0;  // stages and expansions before the item; expansion u is group u % NG's
+    int grams = 0;       // Gram matrices so far
+    int last_g = -1;     // the stage of this group's latest expansion
+    auto slot_free = [&]() {  // its products have completed
+      if (last_g >= 0) ok = mbar_wait(&done[last_g % NS], (last_g / NS) & 1, &abort_flag);
+      tc_fence_after();
+    };
+    auto report = [&]() {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full[grp]);
+    };
+    for (int it = 0; ok; ++it) {
+      const StateItem w(p, cta.x);
+      if (!w.gram) {
+        // this thread's row of both tiles: first factors a0 and a0 + 8, common second factor b
+        int a0, b;
+        ref_decode(w.slot * (NT * 128) + row_in_tile, &a0, &b);
+        // swz128(row, j) = (row * 128 + ((row & 7) << 4)) ^ (j << 4): one XOR per address
+        const uint32_t a0_base = a0 * 128 + ((a0 & 7) << 4), a1_base = a0_base + 8 * 128,
+                       b_base = b * 128 + ((b & 7) << 4);
+        for (int i = (grp - u0) & (NG - 1); i < w.total; i += NG) {
+          const int g = g0 + i, s = g % NS;
+          ok = mbar_wait(&full[s], (g / NS) & 1, &abort_flag);
+          if (!ok) break;
+          const uint8_t* xs = smR + s * R_BYTES;
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            uint32_t r0[16], r1[16];
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) {
+              const uint32_t off = (uint32_t)((4 * hf + jj) << 4);
+              const uint4 vb = *reinterpret_cast<const uint4*>(xs + (b_base ^ off));
+              const uint4 va = *reinterpret_cast<const uint4*>(xs + (a0_base ^ off));
+              const uint4 vc = *reinterpret_cast<const uint4*>(xs + (a1_base ^ off));
+              r0[4 * jj + 0] = Pack2<T>::mul(va.x, vb.x);
+              r0[4 * jj + 1] = Pack2<T>::mul(va.y, vb.y);
+              r0[4 * jj + 2] = Pack2<T>::mul(va.z, vb.z);
+              r0[4 * jj + 3] = Pack2<T>::mul(va.w, vb.w);
+              r1[4 * jj + 0] = Pack2<T>::mul(vc.x, vb.x);
+              r1[4 * jj + 1] = Pack2<T>::mul(vc.y, vb.y);
+              r1[4 * jj + 2] = Pack2<T>::mul(vc.z, vb.z);
+              r1[4 * jj + 3] = Pack2<T>::mul(vc.w, vb.w);
+            }
+            if (hf == 0) {
+              slot_free();
+              if (!ok) break;
+            }
+            tmem_st16(ca + 16 * hf, r0);
+            tmem_st16(ca + 32 + 16 * hf, r1);
+          }
+          if (!ok) break;
+          last_g = g;
+          // The stage goes back to TMA once its products have completed, which is after these stores, and so after
+          // every load of it has delivered its data.  (Released right after the loads were issued, a refill overtook
+          // loads still queued: single rows of the state were built from the wrong 64 tokens.)  The proxy fence orders
+          // this thread's generic-proxy reads before the async-proxy write.
+          fence_async_smem();
+          tmem_wait_st();
+          tc_fence_before();
+          report();
+        }
+        u0 += w.total;
+      } else {
+        slot_free();
+        if (!ok) break;
+        last_g = -1;
+        report();
+        ok = mbar_wait(&gram_done, grams & 1, &abort_flag);
+        ++grams;
+      }
+      g0 += w.total;
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
     }
   }
-  if (tid == 0 && abort_flag) *p.status = ST_TIMEOUT;
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && abort_flag) *p.status = ST_TIMEOUT;
-  if (warp == 0) tmem_dealloc(tmem, cs::TMEM_COLS);
+  if (warp == 0) tmem_dealloc(tmem_base_s, TMEM_COLS);
 }
 
 template <typename T, bool EXACT>
-static int launch_chunk_state(const ChunkStateParams& p, int b, const CUtensorMap& tm_xt, const CUtensorMap& tm_xs,
+static int launch_chunk_state(const ChunkStateParams& p, const CUtensorMap& tm_xt, const CUtensorMap& tm_xs,
                               const CUtensorMap& tm_w, cudaStream_t stream) {
   using namespace cs;
-  const size_t smem = 1024 + NS * (XT_BYTES + W_BYTES);
-  static_assert(2 * GA_BYTES <= NS * W_BYTES, "Gram stages must fit in the value ring");
   int device = 0;
   PR_CUDA(cudaGetDevice(&device));  // the entry point has made the caller's device current
-  PR_SMEM_ATTR((chunk_state_kernel<T, EXACT>), smem, device, true);
-  const long long ctas = (long long)((p.n_tiles + NG - 1) / NG + (EXACT || p.gram ? 1 : 0)) * b * p.n_run * p.nh;
+  PR_SMEM_ATTR((chunk_state_kernel<T, EXACT>), SMEM, device, true);
+  const long long ctas = (long long)(p.n_slots + (EXACT || p.gram ? 1 : 0)) * p.n_states;
   PR_REQUIRE(ctas < (1ll << 31), PR_ERR_BAD_ARG, "%lld CTAs exceed the grid limit", ctas);
   dim3 grid((unsigned)ctas);
-  chunk_state_kernel<T, EXACT><<<grid, THREADS, smem, stream>>>(p, tm_xt, tm_xs, tm_w);
+  chunk_state_kernel<T, EXACT><<<grid, THREADS, SMEM, stream>>>(p, tm_xt, tm_xs, tm_w);
   PR_CUDA(cudaGetLastError());
   return PR_OK;
 }
@@ -364,7 +434,8 @@ static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, in
   PR_CUDA(cudaSetDevice(device));
   p.chunk0 = chunk0;
   p.n_run = n_run;
-  p.n_tiles = (ref_dim(d) + 127) / 128;
+  p.n_slots = ref_dim(d) / (cs::NT * 128);  // exact: 2, 6, 12 or 20 tiles
+  p.n_states = b * n_run * nh;
   p.nh = nh;
   p.group = group;
   p.c = c;
@@ -393,8 +464,8 @@ static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, in
     if (rc) return rc;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return dtype == PR_BF16 ? launch_chunk_state<__nv_bfloat16, EXACT>(p, b, tm_xt, tm_xs, tm_w, s)
-                          : launch_chunk_state<__half, EXACT>(p, b, tm_xt, tm_xs, tm_w, s);
+  return dtype == PR_BF16 ? launch_chunk_state<__nv_bfloat16, EXACT>(p, tm_xt, tm_xs, tm_w, s)
+                          : launch_chunk_state<__half, EXACT>(p, tm_xt, tm_xs, tm_w, s);
 }
 
 }  // namespace pr
