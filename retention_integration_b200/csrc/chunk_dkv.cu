@@ -13,14 +13,16 @@
 // key gradient (fp32, from the expansion-gradient kernel) and writes dK, dV.
 //
 // Three groups of four warps own the key rows, one row per thread in each group, and take the steps in turn, each in
-// its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma.  One persistent CTA per SM takes over
-// tile after tile (ClcRing).  A step is a serial chain - S and dP products, barrier, tensor-memory loads, arithmetic,
-// stores, barrier, dV and dK products - of about 4000 clocks in the earlier form, whose one buffer per CTA
-// made every part of it wait for the others; with three buffers the products of the next steps run while the rows work.
-// Per column of a step a thread reads two factors from shared memory, 1/l times the gate's and delta, where four were
-// read (a broadcast read costs the shared-memory pipe as much as a full one).
+// its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma; two warps make, step by step in turn and up to
+// six ahead, what the rows need of a step's queries (Cols).  One persistent CTA per SM takes over tile after tile
+// (ClcRing).  A step is a serial chain - S and dP products, barrier, tensor-memory loads, arithmetic, stores, barrier, dV and
+// dK products; with three buffers the products of the next steps run while the rows work.
 // 490 -> 470 us at b1 t65536 h8 with chunks of 1024 and states (144 -> 117 at b4 t5000 h2x4 fp16, 27.4 -> 17.2 at
-// b1 t1024 h4).
+// b1 t1024 h4) from the three groups.  Every row warp used to make the factors of its columns itself: loads, two divisions,
+// a logarithm and exponentials were a chain of 1000-1900 traced clocks in front of a step's 1000-1500, on all twelve
+// warps.  With warps of their own for it, and the next tile's gates and the state-path gradients fetched before the
+// write-out: 467 -> 413, 119 -> 102 (gated bf16), 80 -> 68 at b4 t2048 h8 in one chunk, 19.2 -> 17.2.  (One such warp, the
+// TMA warp: 483, 137, -, 21.3: it cannot keep up.)
 #include "host.cuh"
 #include "layout.cuh"
 #include "sm100.cuh"
@@ -31,14 +33,22 @@ namespace dkv {
 constexpr int HD = 64;
 constexpr int NG = 3;                    // row groups, each with its own buffer in tensor memory
 constexpr int NR = 7;                    // shared-memory ring: stages of 16 KB (a query and a dO tile, or two state blocks)
-constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
-constexpr int THREADS = 32 * (W_MMA + 1);
+constexpr int NF = 2;                    // warps that make the columns' factors, step by step in turn
+constexpr int NC = 2 * NG;               // steps whose factors are held; a multiple of NF
+constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1, W_COL = W_MMA + 1;
+constexpr int THREADS = 32 * (W_COL + NF);
 constexpr int TILE_BYTES = 128 * 128;   // 128 key rows x 64 features
 constexpr int TW = 64;                  // queries per step
 constexpr int QD_BYTES = TW * 128;      // one query or dO tile
 constexpr int Z_BYTES = 64 * 128;
 constexpr int R_BYTES = 2 * QD_BYTES;   // one ring stage
 constexpr size_t SMEM = 1024 + 4 * TILE_BYTES + NR * R_BYTES;
+// What the row warps need of a step's 64 queries: e^{a_i - r} / l_i (r = gate sum at the step's first query), 1 / l_i, a_i
+// and deg * delta_i; r, log of the largest l_i, largest a_i - r.
+struct alignas(16) Cols {
+  float fs[TW], il[TW], aq[TW], de[TW];
+  float4 top;
+};
 constexpr uint32_t TMEM_COLS = 512;
 // A buffer is 128 columns: S and dP, overwritten by P / l and dS (the first half of each); in the state phase 256
 // expanded entries.
@@ -162,15 +172,14 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
   using namespace dkv;
   extern __shared__ uint8_t smem_raw[];
   // kv_*: the key and value tiles, two pairs in flight.  r_*: the ring of operand tiles.  s_full: S and dP in a
-  // group's buffer; op_full: the group has written its A operands.  acc_full / acc_free: accumulators complete / read
-  // out; rows: the row warps meet.
-  __shared__ uint64_t kv_full[2], kv_free[2], r_full[NR], r_empty[NR], s_full[NG], op_full[NG], acc_full, acc_free, rows;
+  // group's buffer; op_full: the group has written its A operands.  c_full / c_free: a step's factors.  acc_full /
+  // acc_free: accumulators complete / read out; rows: the row warps meet.
+  __shared__ uint64_t kv_full[2], kv_free[2], r_full[NR], r_empty[NR], s_full[NG], op_full[NG], c_full[NC], c_free[NC],
+      acc_full, acc_free, rows;
   __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  // Per warp and step parity, each warp its own copy: e^{a_i - r} / l_i (r = gate sum at the step's first query),
-  // deg * delta_i, and a_i where the exponentials do not separate (the first is 1 / l_i then).
-  __shared__ __align__(16) float sm_fq[4 * NG][2][TW], sm_de[4 * NG][2][TW], sm_aq[4 * NG][TW];
+  __shared__ Cols sm_c[NC];
   __shared__ float sm_da[2][NG][128];
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
@@ -200,10 +209,14 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         mbar_init(&s_full[s], 1);
         mbar_init(&op_full[s], 4);
       }
+      for (int s = 0; s < NC; ++s) {
+        mbar_init(&c_full[s], 1);
+        mbar_init(&c_free[s], 4);
+      }
       mbar_init(&acc_full, 1);
       mbar_init(&acc_free, 4 * NG);
       mbar_init(&rows, 4 * NG);
-      clc_init(&clc, 4 * NG + 2);
+      clc_init(&clc, 4 * NG + 2 + NF);
       fence_mbar_init();
     }
     __syncwarp();
@@ -352,6 +365,67 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
     }
+  } else if (warp >= W_COL) {
+    // ------------------------------------------------------- the columns' factors
+    const bool gated = p.a != nullptr;
+    bool ok = true;
+    dim3 cta = blockIdx;
+    int n0 = 0;  // steps before the tile
+    for (int it = 0; ok; ++it) {
+      const DkvTile w(p, cta);
+      const size_t tok_base = (size_t)w.batch * p.t + w.tok_chunk;
+      const float* a_chunk = gated ? p.a + tok_base * p.h + w.kvhead : nullptr;
+      int st = (warp - W_COL - n0) & (NF - 1);
+      int I = w.qt0 + st / ratio, rem = st % ratio;  // the step's query tile, and its head within the group
+      // per-query values, two per lane, loaded one step ahead
+      float av[2], dlv[2], lv[2], rs = 0.f;
+      auto load_cols = [&]() {
+        rs = gated ? a_chunk[(size_t)(I * TW) * p.h] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int qp = I * TW + lane + 32 * k;
+          const bool v = qp < w.c;
+          const size_t ix = (tok_base + qp) * p.hq + w.kvhead * ratio + rem;
+          av[k] = !v ? -1e30f : gated ? a_chunk[(size_t)qp * p.h] : 0.f;
+          dlv[k] = v ? p.dl[ix] : 0.f;
+          lv[k] = v ? p.l[ix] : 0.f;  // 0: no such query
+        }
+      };
+      if (st < w.n_steps) load_cols();
+      for (; st < w.n_steps && ok; st += NF) {
+        const int n = n0 + st, slot = n % NC;
+        float log_l = 0.f;
+        if (gated)
+          log_l = __logf(__uint_as_float(
+              __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fabsf(lv[0]), fabsf(lv[1])), 1.f)))));
+        const float top = warp_max(fmaxf(av[0], av[1]) - rs);
+        float il[2], fs[2], de[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const bool v = I * TW + lane + 32 * k < w.c;
+          il[k] = v ? safe_recip(lv[k]) : 0.f;
+          fs[k] = v ? il[k] * __expf(av[k] - rs) : 0.f;
+          de[k] = (float)DEG * dlv[k] * lv[k];
+        }
+        if (n >= NC) ok = __all_sync(0xffffffffu, mbar_wait(&c_free[slot], (n / NC - 1) & 1, &abort_flag));
+        if (!ok) break;
+        Cols& cl = sm_c[slot];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          cl.fs[lane + 32 * k] = fs[k];
+          cl.il[lane + 32 * k] = il[k];
+          cl.aq[lane + 32 * k] = av[k];
+          cl.de[lane + 32 * k] = de[k];
+        }
+        if (lane == 0) cl.top = make_float4(rs, log_l, top, 0.f);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&c_full[slot]);
+        for (rem += NF; rem >= ratio; rem -= ratio) ++I;
+        if (st + NF < w.n_steps) load_cols();
+      }
+      n0 += w.n_steps;
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
+    }
   } else {
     const uint32_t tmem = tmem_base_s;
     const int grp = warp >> 2, r = tid & 127;  // row group, key row inside the tile
@@ -362,8 +436,8 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
     const float sdeg = DEG == 4 ? (p.scale * p.scale) * (p.scale * p.scale) : p.scale * p.scale;  // s^deg
     bool ok = true;
     dim3 cta = blockIdx;
-    int tiles = 0, own = 0;    // tiles with rows, operands of this group so far
-    int grp0 = 0, g0 = 0;      // group of the tile's first operand, ring stages before the tile
+    int tiles = 0;             // tiles with rows so far
+    int grp0 = 0, g0 = 0, n0 = 0;  // group of the tile's first operand, ring stages and steps before the tile
     int last_g = -1;           // last ring stage that this group's latest operand was multiplied with
     uint32_t s_ph = 0, row_ph = 0;
     // the row warps meet; bounded like every wait
@@ -379,39 +453,36 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       __syncwarp();
       if (lane == 0) mbar_arrive(&op_full[grp]);
       last_g = g;
-      ++own;
     };
+    // gate sums of this thread's row and of the whole chunk, loaded before the write-out of the tile before
+    float a_n = 0.f, A_n = 0.f;
+    auto load_row = [&](const DkvTile& w) {
+      a_n = A_n = 0.f;
+      if (gated && w.row0 + r < w.c) {
+        a_n = p.a[((size_t)w.batch * p.t + w.tok_chunk + w.row0 + r) * p.h + w.kvhead];
+        if (w.nI > 0) A_n = p.A[(w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead];
+      }
+    };
+    load_row(DkvTile(p, cta));
     for (int it = 0; ok; ++it) {
       const DkvTile w(p, cta);
+      bool more = false;
       if (!w.empty) {
         uint8_t* smK = smKV + (it & 1) * 2 * TILE_BYTES;
         const int row = w.row0 + r;  // key index inside the chunk
         const bool row_valid = row < w.c;
         const size_t tok_base = (size_t)w.batch * p.t + w.tok_chunk;
-        const float* a_chunk = gated ? p.a + tok_base * p.h + w.kvhead : nullptr;
-        const float a_j = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
+        const float a_j = a_n, A_c = A_n;
         float da = 0.f;  // deg times the row sum of p * dp
-        // per-query values of this warp's next step, two per lane, loaded one step ahead
-        float av[2], dlv[2], lv[2], r_n = 0.f;
-        auto load_cols = [&](int st) {
-          const int qp0 = (w.qt0 + st / ratio) * TW, qh = w.kvhead * ratio + st % ratio;
-          r_n = gated ? a_chunk[(size_t)qp0 * p.h] : 0.f;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int qp = qp0 + lane + 32 * k;
-            const bool v = qp < w.c;
-            av[k] = !v ? -1e30f : gated ? a_chunk[(size_t)qp * p.h] : 0.f;
-            dlv[k] = v ? p.dl[(tok_base + qp) * p.hq + qh] : 0.f;
-            lv[k] = v ? p.l[(tok_base + qp) * p.hq + qh] : 0.f;  // 0: no such query
-          }
-        };
         const int first = (grp - grp0 + NG) % NG;  // this group's first operand in the tile
-        if (first < w.n_steps) load_cols(first);
+        int I = w.qt0 + first / ratio, rem = first % ratio;
         for (int st = first; st < w.n_steps && ok; st += NG) {
-          const int qp0 = (w.qt0 + st / ratio) * TW;
-          float* fq = sm_fq[warp][own & 1];
-          float* de = sm_de[warp][own & 1];
-          const float rs = r_n;
+          const int qp0 = I * TW, n = n0 + st;
+          const Cols& cl = sm_c[n % NC];
+          ok = mbar_wait(&c_full[n % NC], (n / NC) & 1, &abort_flag);
+          if (!ok) break;
+          const float4 top = cl.top;
+          const float rs = top.x;
           // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
           // key and per query instead of one per pair (both exponents <= 0 off the diagonal for gates
           // <= 0; a warp falls back to the per-pair form if one exceeds 80).  The query's factor also holds 1 / l_i, so
@@ -421,22 +492,8 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
           // l_i >= e^{a_i - r} (s q_i.k_r)^deg, the weight of the key at r.  Steps whose queries all
           // come after this warp's keys need no mask; a warp whose keys all come after the step's
           // queries writes zeros without reading the scores.
-          float log_l = 0.f;
-          if (gated)
-            log_l = __logf(__uint_as_float(
-                __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fabsf(lv[0]), fabsf(lv[1])), 1.f)))));
-          const bool sep = !__any_sync(0xffffffffu, fmaxf(fmaxf(av[0], av[1]) - rs, rs - a_j + log_l) > 80.f);
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(top.z, rs - a_j + top.y) > 80.f);
           const float c_j = sep ? sdeg * __expf(rs - a_j) : sdeg;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const bool v = qp0 + lane + 32 * k < w.c;
-            const float il = v ? safe_recip(lv[k]) : 0.f;
-            fq[lane + 32 * k] = (sep && v) ? il * __expf(av[k] - rs) : il;
-            de[lane + 32 * k] = (float)DEG * dlv[k] * lv[k];
-            if (!sep) sm_aq[warp][lane + 32 * k] = av[k];
-          }
-          __syncwarp();
-          if (st + NG < w.n_steps) load_cols(st + NG);  // in flight while this step is computed
           ok = mbar_wait(&s_full[grp], s_ph, &abort_flag);
           s_ph ^= 1;
           if (!ok) break;
@@ -453,11 +510,13 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
           } else {
             const bool mask = (wrow0 + 31 > qp0) || (wrow0 + 31 >= w.c);
             const int lo = row_valid ? row - qp0 : TW;  // first query column this key keeps
-            if (!sep) dkv_step<T, DEG, false, true>(cb, fq, de, sm_aq[warp], c_j, a_j, lo, da);
-            else if (mask) dkv_step<T, DEG, true, true>(cb, fq, de, fq, c_j, a_j, lo, da);
-            else dkv_step<T, DEG, true, false>(cb, fq, de, fq, c_j, a_j, lo, da);
+            if (!sep) dkv_step<T, DEG, false, true>(cb, cl.il, cl.de, cl.aq, c_j, a_j, lo, da);
+            else if (mask) dkv_step<T, DEG, true, true>(cb, cl.fs, cl.de, cl.fs, c_j, a_j, lo, da);
+            else dkv_step<T, DEG, true, false>(cb, cl.fs, cl.de, cl.fs, c_j, a_j, lo, da);
           }
           operand_written(g0 + st);
+          if (lane == 0) mbar_arrive(&c_free[n % NC]);  // after the operand's __syncwarp
+          for (rem += NG; rem >= ratio; rem -= ratio) ++I;
         }
 
         if (w.nI > 0) {
@@ -466,7 +525,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
           // runtime index; each group does every third 16-byte piece.
           if (ok) ok = mbar_wait(&kv_full[it & 1], (it >> 1) & 1, &abort_flag);
           float f = 1.f;
-          if (gated) f = __expf(0.5f * (p.A[(w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead] - a_j));
+          if (gated) f = __expf(0.5f * (A_c - a_j));
           for (int j = grp; j < 8; j += NG) {
             uint4* slot = reinterpret_cast<uint4*>(smK + swz128(r, j));
             const uint4 v = *slot;
@@ -506,32 +565,39 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         meet();
         if (lane == 0) mbar_arrive(&kv_free[it & 1]);
 
+        // The groups share the write-out: 16 of the 64 columns of dV (units 0-3) or dK (units 4-7) at a time.  The
+        // state-path gradients come in while the last products run, and the next tile's gates too.
         const size_t tok = tok_base + row;
         const float* st = p.dk_state ? p.dk_state + (tok * p.h + w.kvhead) * p.d : nullptr;
+        constexpr int UNITS = (8 + NG - 1) / NG;
+        float4 add[UNITS - 1][4];
+#pragma unroll
+        for (int i = 1; i < UNITS; ++i) {
+          const int unit = grp + NG * i, c0 = 16 * (unit & 3);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            add[i - 1][j] = (st != nullptr && row_valid && unit >= 4 && unit < 8 && c0 < p.d)
+                                ? reinterpret_cast<const float4*>(st + c0)[j]
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
+        if (more) load_row(DkvTile(p, cta));
         if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
         tc_fence_after();
-        // the groups share the write-out: 16 of the 64 columns of dV (units 0-3) or dK (units 4-7) at a time
-        for (int unit = grp; ok && unit < 8; unit += NG) {
-          const int c0 = 16 * (unit & 3);
+#pragma unroll
+        for (int i = 0; i < UNITS; ++i) {
+          const int unit = grp + NG * i, c0 = 16 * (unit & 3);
+          if (!ok || unit >= 8) continue;
           uint32_t acc[16];
           tmem_ld16(tmem + lane_addr + 16 * unit, acc);
-          const bool mine = row_valid && c0 < p.d;
-          float4 add[4];
-          if (unit >= 4 && st != nullptr && mine) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) add[j] = reinterpret_cast<const float4*>(st + c0)[j];
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) add[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          }
           tmem_wait_ld();
-          if (mine) {
+          if (row_valid && c0 < p.d) {
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + add[j].x, __uint_as_float(acc[4 * j + 1]) + add[j].y);
-              v[2 * j + 1] =
-                  Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + add[j].z, __uint_as_float(acc[4 * j + 3]) + add[j].w);
+              const float4 ad = i > 0 ? add[i > 0 ? i - 1 : 0][j] : make_float4(0.f, 0.f, 0.f, 0.f);
+              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + ad.x, __uint_as_float(acc[4 * j + 1]) + ad.y);
+              v[2 * j + 1] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + ad.z, __uint_as_float(acc[4 * j + 3]) + ad.w);
             }
             T* dst = static_cast<T*>(unit < 4 ? p.dV : p.dK) + (tok * p.h + w.kvhead) * p.d + c0;
             if (p.aligned32) {
@@ -551,6 +617,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         }
         grp0 = (grp0 + w.n_steps + w.nI) % NG;
         g0 += w.n_steps + 2 * w.nI;
+        n0 += w.n_steps;
         ++tiles;
       } else {
         // Not before the producer has come to this tile, and so has seen the last phase of this slot's kv_free: in a
@@ -558,8 +625,10 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         ok = mbar_wait(&kv_full[it & 1], (it >> 1) & 1, &abort_flag);
         __syncwarp();
         if (lane == 0) mbar_arrive(&kv_free[it & 1]);
+        more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
+        if (more) load_row(DkvTile(p, cta));
       }
-      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
+      if (!more) break;
     }
   }
   tc_fence_before();

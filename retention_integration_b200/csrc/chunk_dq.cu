@@ -18,6 +18,10 @@
 // arithmetic, stores, barrier, product); two CTAs per SM with one row group each overlapped two of them and spent
 // a third of the time on set-up and write-out: 232 -> 220 us at b1 t65536 h8 with chunks of 1024
 // (94 -> 84 at b4 t5000 h2x4 fp16, 20.2 -> 12.6 at b1 t1024 h4).
+// Two more warps make, step by step in turn and up to six ahead, the gate factors of a step's keys (Cols), which every row
+// warp used to make for itself before it could look at the scores; a tile's row values are fetched before the
+// write-out of the tile before: 217 -> 202 us, 75.6 -> 72.7 (gated bf16), 56 -> 52 at b4 t2048 h8 in one chunk, the small
+// ones the same.
 #include "host.cuh"
 #include "sm100.cuh"
 
@@ -27,13 +31,20 @@ namespace dq {
 constexpr int HD = 64;
 constexpr int NG = 3;                    // row groups, each with its own buffer in tensor memory
 constexpr int NR = 6;                    // shared-memory ring: stages of a key and a value tile
-constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
-constexpr int THREADS = 32 * (W_MMA + 1);
+constexpr int NF = 2;                    // warps that make the columns' factors, step by step in turn
+constexpr int NC = 2 * NG;               // steps whose factors are held; a multiple of NF
+constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1, W_COL = W_MMA + 1;
+constexpr int THREADS = 32 * (W_COL + NF);
 constexpr int TILE_BYTES = 128 * 128;   // 128 query rows x 64 features
 constexpr int TW = 64;                  // keys per step
 constexpr int KV_BYTES = TW * 128;      // one key or value tile
 constexpr int R_BYTES = 2 * KV_BYTES;
 constexpr size_t SMEM = 1024 + 4 * TILE_BYTES + NR * R_BYTES;
+// What the row warps need of a step's 64 keys: e^{r - a_j} (r = gate sum at the step's last key) and a_j; r, smallest a_j.
+struct alignas(16) Cols {
+  float fk[TW], ak[TW];
+  float2 top;
+};
 constexpr uint32_t TMEM_COLS = 512;
 // the accumulator, then a buffer of 128 columns per group: S, overwritten by dS (its first half), and dP
 __device__ __forceinline__ constexpr uint32_t col_b(int grp) { return 128u + 128u * (uint32_t)grp; }
@@ -141,15 +152,14 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
   using namespace dq;
   extern __shared__ uint8_t smem_raw[];
   // q_*: the query and dO tiles, two pairs in flight.  r_*: the ring of key and value tiles.  s_full: S and dP in a
-  // group's buffer; op_full: the group has written dS.  acc_full / acc_free: accumulator complete / read out; rows: the
-  // row warps meet.
-  __shared__ uint64_t q_full[2], q_free[2], r_full[NR], r_empty[NR], s_full[NG], op_full[NG], acc_full, acc_free, rows;
+  // group's buffer; op_full: the group has written dS.  c_full / c_free: a step's factors.  acc_full / acc_free:
+  // accumulator complete / read out; rows: the row warps meet.
+  __shared__ uint64_t q_full[2], q_free[2], r_full[NR], r_empty[NR], s_full[NG], op_full[NG], c_full[NC], c_free[NC],
+      acc_full, acc_free, rows;
   __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  // Per warp and step parity, each warp its own copy: e^{r - a_j} of the step's keys, r = gate sum at its last key (or
-  // a_j itself where the exponentials do not separate).
-  __shared__ __align__(16) float sm_fk[4 * NG][2][TW];
+  __shared__ Cols sm_c[NC];
   __shared__ float sm_da[2][NG][128];
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
@@ -177,10 +187,14 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
         mbar_init(&s_full[s], 1);
         mbar_init(&op_full[s], 4);
       }
+      for (int s = 0; s < NC; ++s) {
+        mbar_init(&c_full[s], 1);
+        mbar_init(&c_free[s], 4);
+      }
       mbar_init(&acc_full, 1);
       mbar_init(&acc_free, 4 * NG);
       mbar_init(&rows, 4 * NG);
-      clc_init(&clc, 4 * NG + 2);
+      clc_init(&clc, 4 * NG + 2 + NF);
       fence_mbar_init();
     }
     __syncwarp();
@@ -291,6 +305,46 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
         if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
       }
     }
+  } else if (warp >= W_COL) {
+    // ------------------------------------------------------- the columns' factors
+    const bool gated = p.a != nullptr;
+    bool ok = true;
+    dim3 cta = blockIdx;
+    int n0 = 0;  // steps before the tile
+    for (int it = 0; ok; ++it) {
+      const DqTile w(p, cta);
+      const float* a_chunk = gated ? p.a + ((size_t)w.batch * p.t + w.tok_chunk) * p.h + w.kvhead : nullptr;
+      int J = (warp - W_COL - n0) & (NF - 1);
+      // gate sums, two keys per lane, loaded one step ahead
+      float av0 = 0.f, av1 = 0.f, rs = 0.f;
+      auto load_gates = [&]() {
+        if (gated) {
+          const int kp = J * TW + lane;
+          rs = a_chunk[(size_t)min(J * TW + TW - 1, w.c - 1) * p.h];
+          av0 = kp < w.c ? a_chunk[(size_t)kp * p.h] : 0.f;
+          av1 = kp + 32 < w.c ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
+        }
+      };
+      if (J < w.nJ) load_gates();
+      while (J < w.nJ && ok) {
+        const int n = n0 + J, slot = n % NC;
+        const float low = warp_min(fminf(av0, av1)), f0 = __expf(rs - av0), f1 = __expf(rs - av1);
+        if (n >= NC) ok = __all_sync(0xffffffffu, mbar_wait(&c_free[slot], (n / NC - 1) & 1, &abort_flag));
+        if (!ok) break;
+        Cols& cl = sm_c[slot];
+        cl.fk[lane] = f0;
+        cl.fk[lane + 32] = f1;
+        cl.ak[lane] = av0;
+        cl.ak[lane + 32] = av1;
+        if (lane == 0) cl.top = make_float2(rs, low);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&c_full[slot]);
+        J += NF;
+        if (J < w.nJ) load_gates();
+      }
+      n0 += w.nJ;
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
+    }
   } else {
     const uint32_t tmem = tmem_base_s;
     const int grp = warp >> 2, r = tid & 127;  // row group, query row inside the tile
@@ -301,48 +355,48 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
     const float sdeg = DEG == 4 ? 4.f * (p.scale * p.scale) * (p.scale * p.scale) : 2.f * p.scale * p.scale;  // deg s^deg
     bool ok = true;
     dim3 cta = blockIdx;
-    int tiles = 0, own = 0, grp0 = 0;  // tiles with rows, steps of this group so far; group of the tile's first step
+    int tiles = 0, own = 0, n0 = 0, grp0 = 0;  // tiles with rows, steps of this group and of all so far; group of the first
     uint32_t row_ph = 0;
+    // this thread's row: gate sum, dl and row sum, loaded before the write-out of the tile before
+    float a_n = 0.f, dl_n = 0.f, l_n = 0.f;
+    auto load_row = [&](const DqTile& w) {
+      a_n = dl_n = l_n = 0.f;
+      if (w.row0 + r < w.c) {
+        const size_t tok = (size_t)w.batch * p.t + w.tok_chunk + w.row0 + r;
+        if (gated) a_n = p.a[tok * p.h + w.kvhead];
+        dl_n = p.dl[tok * p.hq + w.qhead];
+        l_n = p.l[tok * p.hq + w.qhead];
+      }
+    };
+    load_row(DqTile(p, cta));
     for (int it = 0; ok; ++it) {
       const DqTile w(p, cta);
+      bool more = false;
       if (!w.empty) {
         const int row = w.row0 + r;
         const bool row_valid = row < w.c;
         const size_t tok0 = (size_t)w.batch * p.t + w.tok_chunk;
         const size_t ix = (tok0 + row) * p.hq + w.qhead;
-        const float* a_chunk = gated ? p.a + tok0 * p.h + w.kvhead : nullptr;
-        const float a_i = (gated && row_valid) ? a_chunk[(size_t)row * p.h] : 0.f;
-        const float dl_i = row_valid ? p.dl[ix] : 0.f;
-        const float inv_l = row_valid ? safe_recip(p.l[ix]) : 0.f;
+        const float a_i = a_n, dl_i = dl_n;
+        const float inv_l = row_valid ? safe_recip(l_n) : 0.f;
         const int wrow0 = w.row0 + wrow;  // first row of this warp
         float da = 0.f;                   // deg times the row sum of p * dp
-        // gate sums of this warp's next step, two keys per lane, loaded one step ahead
-        float av0 = 0.f, av1 = 0.f, r_n = 0.f;
-        auto load_gates = [&](int J) {
-          if (gated) {
-            const int kp = J * TW + lane;
-            r_n = a_chunk[(size_t)min(J * TW + TW - 1, w.c - 1) * p.h];
-            av0 = kp < w.c ? a_chunk[(size_t)kp * p.h] : 0.f;
-            av1 = kp + 32 < w.c ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
-          }
-        };
         const int first = (grp - grp0 + NG) % NG;  // this group's first step in the tile
-        if (first < w.nJ) load_gates(first);
         for (int J = first; J < w.nJ && ok; J += NG, ++own) {
           const int kp0 = J * TW;
-          float* fk = sm_fk[warp][own & 1];
-          const float rs = r_n;
+          const int n = n0 + J;
+          const Cols& cl = sm_c[n % NC];
+          ok = mbar_wait(&c_full[n % NC], (n / NC) & 1, &abort_flag);
+          if (!ok) break;
+          const float2 top = cl.top;
+          const float rs = top.x;
           // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential
           // per row and per key instead of one per pair.  Both exponents are <= 0 below the
           // diagonal for gates <= 0; if one exceeds 80 (growing gates) the warp takes the per-pair
           // form.  Steps wholly below the diagonal need no mask; a warp whose rows all precede the
           // step's keys writes zeros without reading the scores.
-          const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - fminf(av0, av1), a_i - rs) > 80.f);
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - top.y, a_i - rs) > 80.f);
           const float c_i = sep ? sdeg * __expf(a_i - rs) : sdeg;
-          fk[lane] = sep ? __expf(rs - av0) : av0;
-          fk[lane + 32] = sep ? __expf(rs - av1) : av1;
-          __syncwarp();
-          if (J + NG < w.nJ) load_gates(J + NG);  // in flight while this step is computed
           ok = mbar_wait(&s_full[grp], own & 1, &abort_flag);
           if (!ok) break;
           tc_fence_after();
@@ -355,14 +409,17 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
           } else {
             const bool mask = (kp0 + TW - 1 > wrow0) || (kp0 + TW - 1 >= w.c);
             const int lim = min(row, w.c - 1) - kp0;  // last column this row keeps
-            if (!sep) dq_step<T, DEG, false, true>(cb, fk, c_i, a_i, inv_l, dl_i, lim, da);
-            else if (mask) dq_step<T, DEG, true, true>(cb, fk, c_i, a_i, inv_l, dl_i, lim, da);
-            else dq_step<T, DEG, true, false>(cb, fk, c_i, a_i, inv_l, dl_i, lim, da);
+            if (!sep) dq_step<T, DEG, false, true>(cb, cl.ak, c_i, a_i, inv_l, dl_i, lim, da);
+            else if (mask) dq_step<T, DEG, true, true>(cb, cl.fk, c_i, a_i, inv_l, dl_i, lim, da);
+            else dq_step<T, DEG, true, false>(cb, cl.fk, c_i, a_i, inv_l, dl_i, lim, da);
           }
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&op_full[grp]);
+          if (lane == 0) {
+            mbar_arrive(&op_full[grp]);
+            mbar_arrive(&c_free[n % NC]);
+          }
         }
         sm_da[tiles & 1][first][r] = da;  // by step, not by group: a fixed order of the sum whatever the CTA did before
         // the row warps meet; bounded like every wait
@@ -379,6 +436,8 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
             add[q][j] = (st != nullptr && row_valid && c0 < p.d && c0 < HD) ? reinterpret_cast<const float4*>(st + c0)[j]
                                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
+        if (more) load_row(DqTile(p, cta));
         if (ok) ok = mbar_wait(&rows, row_ph, &abort_flag);
         row_ph ^= 1;
         if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
@@ -413,9 +472,13 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
         if (grp == NG - 1 && row_valid)
           p.da_q[ix] = (1.f / DEG) * ((sm_da[tiles & 1][0][r] + sm_da[tiles & 1][1][r]) + sm_da[tiles & 1][2][r]);
         grp0 = (grp0 + w.nJ) % NG;
+        n0 += w.nJ;
         ++tiles;
+      } else {
+        more = clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
+        if (more) load_row(DqTile(p, cta));
       }
-      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
+      if (!more) break;
     }
   }
   tc_fence_before();

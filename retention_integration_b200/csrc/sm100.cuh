@@ -358,6 +358,18 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
+// the largest / smallest of a converged warp's values, in one instruction
+__device__ __forceinline__ float warp_max(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float warp_min(float x) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // 1 / l guarded against an exact zero only.  Row sums of real states are positive, but a
 // caller may hand over any state, and the reference divides by negative sums too.
 __device__ __forceinline__ float safe_recip(float l) {
