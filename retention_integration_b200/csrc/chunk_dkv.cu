@@ -21,7 +21,8 @@
 // b1 t1024 h4) from the three groups.  Every row warp used to make the factors of its columns itself: loads, two divisions,
 // a logarithm and exponentials were a chain of 1000-1900 traced clocks in front of a step's 1000-1500, on all twelve
 // warps.  With warps of their own for it, and the next tile's gates and the state-path gradients fetched before the
-// write-out: 467 -> 413, 119 -> 102 (gated bf16), 80 -> 68 at b4 t2048 h8 in one chunk, 19.2 -> 17.2.  (One such warp, the
+// write-out: 467 -> 413, 119 -> 102 (gated bf16), 80 -> 68 at b4 t2048 h8 in one chunk, 19.2 -> 17.2; without divisions
+// between the tiles 395, 98, 67, 17.  (One such warp, the
 // TMA warp: 483, 137, -, 21.3: it cannot keep up.)
 #include "host.cuh"
 #include "layout.cuh"
@@ -58,6 +59,8 @@ __device__ __forceinline__ constexpr uint32_t col_b(int grp) { return 128u + 128
 
 struct ChunkDkvParams {
   int hq, h, n_chunks, c, tiles_per_chunk;
+  int ratio;               // query heads per kv head
+  Div by_tiles, by_ratio;
   int t, d;               // tokens (the last chunk may be shorter), features (a multiple of 16)
   int nblk;               // stages of 64 expanded rows of a state
   int state_chunk_hi;     // chunks <= this have a state-path dV term
@@ -83,8 +86,8 @@ struct DkvTile {
   bool empty;   // past the end of a shorter last chunk
   __device__ __forceinline__ DkvTile(const ChunkDkvParams& p, const dim3& cta) {
     const int x = (int)cta.x;
-    const int tile_j = x % p.tiles_per_chunk;  // the longest tiles of a head first
-    chunk = x / p.tiles_per_chunk;
+    int tile_j;
+    p.by_tiles.of(x, &chunk, &tile_j);  // the longest tiles of a head first
     kvhead = (int)cta.y;
     batch = (int)cta.z;
     row0 = tile_j * 128;
@@ -92,7 +95,7 @@ struct DkvTile {
     c = min(p.c, p.t - tok_chunk);
     empty = row0 >= c;
     qt0 = row0 / dkv::TW;
-    n_steps = empty ? 0 : ((c + dkv::TW - 1) / dkv::TW - qt0) * (p.hq / p.h);
+    n_steps = empty ? 0 : ((c + dkv::TW - 1) / dkv::TW - qt0) * p.ratio;
     nI = (!empty && chunk <= p.state_chunk_hi) ? p.nblk / 4 : 0;
   }
 };
@@ -230,7 +233,7 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
     named_bar_sync(1, THREADS);
     tc_fence_after();
   }
-  const int ratio = p.hq / p.h;
+  const int ratio = p.ratio;
 
   if (warp == W_TMA) {
     if (elect_one()) {
@@ -255,12 +258,13 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
           mbar_expect_tx(&kv_full[it & 1], 2 * TILE_BYTES);
           tma_load_4d(kv, &tm_k, &kv_full[it & 1], 0, w.kvhead, w.tok_chunk + w.row0, w.batch);
           tma_load_4d(kv + TILE_BYTES, &tm_v, &kv_full[it & 1], 0, w.kvhead, w.tok_chunk + w.row0, w.batch);
+          int I = w.qt0, qh = w.kvhead * ratio;
           for (int st = 0; st < w.n_steps && ok; ++st) {
-            const int I = w.qt0 + st / ratio, qh = w.kvhead * ratio + st % ratio;
             uint8_t* dst = next_stage();
             if (!ok) break;
             tma_load_4d(dst, &tm_q, &r_full[s], 0, qh, w.tok_chunk + I * TW, w.batch);
             tma_load_4d(dst + QD_BYTES, &tm_dy, &r_full[s], 0, qh, w.tok_chunk + I * TW, w.batch);
+            if (++qh == (w.kvhead + 1) * ratio) qh = w.kvhead * ratio, ++I;
             advance();
             if (st == 0) ok = clc_ask(&clc, it, &abort_flag);
           }
@@ -376,7 +380,9 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
       const size_t tok_base = (size_t)w.batch * p.t + w.tok_chunk;
       const float* a_chunk = gated ? p.a + tok_base * p.h + w.kvhead : nullptr;
       int st = (warp - W_COL - n0) & (NF - 1);
-      int I = w.qt0 + st / ratio, rem = st % ratio;  // the step's query tile, and its head within the group
+      int I, rem;  // the step's query tile, and its head within the group
+      p.by_ratio.of(st, &I, &rem);
+      I += w.qt0;
       // per-query values, two per lane, loaded one step ahead
       float av[2], dlv[2], lv[2], rs = 0.f;
       auto load_cols = [&]() {
@@ -475,7 +481,9 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         const float a_j = a_n, A_c = A_n;
         float da = 0.f;  // deg times the row sum of p * dp
         const int first = (grp - grp0 + NG) % NG;  // this group's first operand in the tile
-        int I = w.qt0 + first / ratio, rem = first % ratio;
+        int I, rem;
+        p.by_ratio.of(first, &I, &rem);
+        I += w.qt0;
         for (int st = first; st < w.n_steps && ok; st += NG) {
           const int qp0 = I * TW, n = n0 + st;
           const Cols& cl = sm_c[n % NC];
@@ -668,6 +676,9 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   p.nblk = ref_dim(d) / 64;
   p.c = c;
   p.tiles_per_chunk = (c + 127) / 128;
+  p.ratio = hq / h;
+  p.by_tiles = Div(p.tiles_per_chunk);
+  p.by_ratio = Div(p.ratio);
   p.state_chunk_hi = wdS ? state_chunk_hi : -1;
   p.scale = scale;
   p.a = a;

@@ -52,6 +52,7 @@ __device__ __forceinline__ constexpr uint32_t col_b(int grp) { return 128u + 128
 
 struct ChunkDqParams {
   int hq, h, n_chunks, c, tiles_per_chunk;
+  Div by_tiles, by_ratio;  // by tiles_per_chunk, by query heads per kv head
   int t, d;               // tokens (the last chunk may be shorter), features (a multiple of 16)
   float scale;
   const float* a;         // [b, t, h] or null
@@ -72,11 +73,12 @@ struct DqTile {
   __device__ __forceinline__ DqTile(const ChunkDqParams& p, const dim3& cta) {
     const int x = (int)cta.x;
     // the longest tiles of a head first
-    const int tile_i = p.tiles_per_chunk - 1 - x % p.tiles_per_chunk;
-    chunk = x / p.tiles_per_chunk;
+    int tile_i;
+    p.by_tiles.of(x, &chunk, &tile_i);
+    tile_i = p.tiles_per_chunk - 1 - tile_i;
     qhead = (int)cta.y;
     batch = (int)cta.z;
-    kvhead = qhead / (p.hq / p.h);
+    kvhead = p.by_ratio.of(qhead);
     row0 = tile_i * 128;
     tok_chunk = chunk * p.c;
     c = min(p.c, p.t - tok_chunk);
@@ -514,6 +516,8 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   p.d = d;
   p.c = c;
   p.tiles_per_chunk = (c + 127) / 128;
+  p.by_tiles = Div(p.tiles_per_chunk);
+  p.by_ratio = Div(hq / h);
   p.scale = scale;
   p.a = a;
   p.dl = dl;

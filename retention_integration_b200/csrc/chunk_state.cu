@@ -21,7 +21,8 @@
 // every stage with all their warps into two slots: of a CTA's 24 thousand clocks at sixteen stages, half was set-up, first
 // loads, cold instructions and write-out, and a barrier round was paid for half a stage's work.  252 -> 232 us at
 // b1 t65536 h8 with chunks of 1024, 83 -> 60 at b4 t4096 h2 with four query heads summed, 406 -> 375 at b16 t2048 h32 in one
-// chunk, 15.1 -> 14.1 at b1 t2048 h2 (groups in turn alone: 238, 72, 375, 14.7).  A stage costs the shared-memory pipe
+// chunk, 15.1 -> 14.1 at b1 t2048 h2 (groups in turn alone: 238, 72, 375, 14.7); without divisions between the items 201,
+// 56, 9 % less, 14.  A stage costs the shared-memory pipe
 // about 560 clocks (the operand reads, 8 for 16 products; the tensor core's own reads; tensor-memory stores), the
 // tensor pipe 256.
 //
@@ -55,6 +56,7 @@ __device__ __forceinline__ constexpr uint32_t col_a(int grp, int tile) { return 
 struct ChunkStateParams {
   int n_slots;      // items of two tiles of 128 expanded rows per state
   int n_states;     // states (batch, chunk, head); grid.x = n_slots * n_states + (Gram matrices wanted ? n_states : 0)
+  Div by_slots, by_heads, by_run;  // by n_slots, nh, n_run
   int nh;           // kv heads of the output
   int group;        // operand heads summed into one output head (GQA ratio in backward)
   int c, cp;        // chunk length, padded to 64
@@ -82,11 +84,12 @@ struct StateItem {
   __device__ __forceinline__ StateItem(const ChunkStateParams& p, unsigned cta) {
     const unsigned n = (unsigned)p.n_slots * (unsigned)p.n_states;
     gram = cta >= n;
-    const int which = (int)(gram ? cta - n : cta / (unsigned)p.n_slots);
-    slot = gram ? 0 : (int)(cta % (unsigned)p.n_slots);
-    head = which % p.nh;
-    chunk = p.chunk0 + (which / p.nh) % p.n_run;
-    batch = which / (p.nh * p.n_run);
+    int which = (int)(cta - n), rest;
+    slot = 0;
+    if (!gram) p.by_slots.of((int)cta, &which, &slot);
+    p.by_heads.of(which, &rest, &head);
+    p.by_run.of(rest, &batch, &chunk);
+    chunk += p.chunk0;
     ch = (batch * p.n_chunks + chunk) * p.nh + head;
     kblocks = (min(p.c, p.t - chunk * p.c) + cs::TOK - 1) / cs::TOK;
     total = kblocks * p.group;
@@ -436,6 +439,9 @@ static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, in
   p.n_run = n_run;
   p.n_slots = ref_dim(d) / (cs::NT * 128);  // exact: 2, 6, 12 or 20 tiles
   p.n_states = b * n_run * nh;
+  p.by_slots = Div(p.n_slots);
+  p.by_heads = Div(nh);
+  p.by_run = Div(n_run);
   p.nh = nh;
   p.group = group;
   p.c = c;
