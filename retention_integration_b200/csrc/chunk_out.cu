@@ -14,7 +14,8 @@
 //
 // Warp roles: two groups of four warps own the query rows, one row per thread in each group, and take the steps in
 // turn (scores -> weights P, expansion phi(q~)); there is no running maximum, so a row's partial sums are simply
-// added at the end.  One more warp issues TMA loads and one tcgen05.mma.
+// added at the end.  One more warp issues TMA loads and makes the gate factors of a step's keys for all rows (Cols), which
+// every row warp used to make for itself; one issues tcgen05.mma.
 //
 // What bounded the earlier form (one row group per CTA, 637 us at b16 t2048 h32 without states, 317 us at
 // b1 t65536 h8 with chunks of 1024 and states): the latency of a step's chain, about 2000 clocks traced for a 64-key
@@ -25,7 +26,9 @@
 // rotating across tiles; and the issuing thread keeps running positions and prepared descriptors, since every
 // instruction it executes between two batches leaves the tensor pipe idle (with divisions and a second commit per
 // operand: 459, 301 us).  Now 451 and 265 us.  Slower: three groups per CTA (520 us); 256 rows per CTA at one CTA per SM
-// (439 us, but 360 with states, where every gap of the one or two issuing threads is exposed).
+// (439 us, but 360 with states, where every gap of the one or two issuing threads is exposed).  With the keys' factors made
+// by the TMA warp, the next tile's gates fetched before the write-out, and no divisions between the tiles: 477 -> 392 and
+// 261 -> 258 us (without the last 400, 266).
 //   S = Q K_J^T        : A, B K-major in shared memory (TMA, 128-byte swizzle)
 //   acc += P V_J       : A = P written to tensor memory by the row threads, B = V_J MN-major
 //   acc += phi(q~) Z   : A = expansion written to tensor memory 64 rows at a time,
@@ -45,12 +48,18 @@ constexpr int NR = 4;                  // ring stages of 16 KB (key and value ti
 constexpr int W_TMA = 4 * NG, W_MMA = W_TMA + 1;
 constexpr int THREADS = 32 * (W_MMA + 1);
 constexpr uint32_t TMEM_COLS = 256;    // two CTAs per SM
-constexpr size_t SMEM = 1024 + 2 * 128 * 128 + NR * 16384;
 constexpr int TILE_BYTES = 128 * 128;  // 128 rows x 64 16-bit features
 constexpr int TW = 64;                 // keys per attention step
 constexpr int KV_BYTES = TW * 128;     // one key or value tile
 constexpr int Z_BYTES = 64 * 128;      // 64 expanded rows x 64 features
 constexpr int R_BYTES = 2 * KV_BYTES;  // one ring stage
+// What the row warps need of a step's 64 keys, made by the TMA warp while the tiles are on their way: e^{r - a_j} (r = gate
+// sum at the step's last key) and a_j; r, smallest a_j.
+struct alignas(16) Cols {
+  float fk[TW], ak[TW];
+  float2 top;
+};
+constexpr size_t SMEM = 1024 + 2 * TILE_BYTES + NR * (R_BYTES + sizeof(Cols));
 // Tensor memory: the accumulator, then the buffers.  A buffer holds scores, overwritten by their weights P; in the
 // state read-out 128 expanded entries, and for a while u = q~ Zg.  Operand number u of a CTA goes to buffer u % NB and
 // is written by group u % NG.
@@ -65,6 +74,7 @@ struct ChunkOutParams {
   int d;                // features (a multiple of 16; TMA fills the tiles' columns up to 64 with zeros)
   int nblk;             // stages of 64 expanded rows of a state: ref_dim(d) / 64
   int tiles_per_chunk;  // ceil(cq / 128)
+  Div by_tiles, by_ratio;  // by tiles_per_chunk, by query heads per kv head
   int state_from_chunk; // chunks >= this read the state (n_chunks: never)
   int q_gate_last;      // 1: gate the state read-out with the gate at the last key (inference)
   int normalize;        // 1: O = y / l; 0: O = y (l is written either way when l_out != null)
@@ -87,11 +97,12 @@ struct OutTile {
   __device__ __forceinline__ OutTile(const ChunkOutParams& p, const dim3& cta) {
     const int x = (int)cta.x;
     // the longest tiles of a head first
-    const int tile_i = p.tiles_per_chunk - 1 - x % p.tiles_per_chunk;
-    chunk = x / p.tiles_per_chunk;
+    int tile_i;
+    p.by_tiles.of(x, &chunk, &tile_i);
+    tile_i = p.tiles_per_chunk - 1 - tile_i;
     qhead = (int)cta.y;
     batch = (int)cta.z;
-    kvhead = qhead / (p.hq / p.h);
+    kvhead = p.by_ratio.of(qhead);
     cq = min(p.cq, p.tq - chunk * p.cq);
     ck = min(p.ck, p.tk - chunk * p.ck);
     q_off = ck - cq;
@@ -164,18 +175,14 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   using namespace co;
   extern __shared__ uint8_t smem_raw[];
   // q_*: the query tiles, two in flight.  r_*: the ring of operand tiles; operand number u takes stage u % NR, and
-  // r_empty says that the products that read both have completed.  s_full: scores in a buffer; op_full: a group has
+  // r_empty says that the products that read both have completed; c_full: a step's factors.  s_full: scores in a buffer; op_full: a group has
   // written an A operand (weights, q~, expansion) into it.  u_full: the Gram product; acc_full / acc_free:
   // accumulator complete / read out; rows: the row warps meet.
-  __shared__ uint64_t q_full[2], q_free[2], r_full[NR], r_empty[NR], s_full[NB], op_full[NB];
+  __shared__ uint64_t q_full[2], q_free[2], r_full[NR], r_empty[NR], c_full[NR], s_full[NB], op_full[NB];
   __shared__ uint64_t u_full, acc_full, acc_free, rows;
   __shared__ ClcRing clc;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  // Per warp and step parity: e^{r - a_j} of the step's keys, r = gate sum at its last key (or a_j itself where the
-  // exponentials do not separate).  Every warp makes its own copy, two keys per lane, so that no barrier ties the
-  // warps of a step together.
-  __shared__ __align__(16) float sm_fk[4 * NG][2][TW];
   __shared__ float sm_l[2][NG][128];            // row sums of the groups
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
@@ -186,6 +193,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   // on with the same stage counter, two 64-row state blocks per stage, and so does the next tile, so the operands of
   // what comes next stream in while the last steps are still being computed.
   uint8_t* smR = smQ0 + 2 * TILE_BYTES;       // NR x R_BYTES
+  Cols* smC = reinterpret_cast<Cols*>(smR + NR * R_BYTES);  // NR
 
   if (warp == W_TMA) {
     if (elect_one()) {
@@ -199,6 +207,7 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       }
       for (int s = 0; s < NR; ++s) {
         mbar_init(&r_full[s], 1);
+        mbar_init(&c_full[s], 1);
         mbar_init(&r_empty[s], 1);
       }
       for (int s = 0; s < NB; ++s) {
@@ -225,27 +234,48 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
   }
 
   if (warp == W_TMA) {
-    // ------------------------------------------------------------ TMA producer
-    if (elect_one()) {
-      bool ok = true;
-      dim3 cta = blockIdx;
-      int g = 0;  // ring stages so far
-      for (int it = 0; ok; ++it) {
-        const OutTile w(p, cta);
-        if (ok && it >= 2) ok = mbar_wait(&q_free[it & 1], ((it >> 1) - 1) & 1, &abort_flag);
-        if (!ok) break;
-        if (!w.empty) {
+    // -------------------------------------- TMA producer, and the factors of the keys
+    const bool lead = elect_one();
+    const bool gated = p.a != nullptr;
+    bool ok = true;
+    dim3 cta = blockIdx;
+    int g = 0;  // ring stages so far
+    auto ask = [&](int it) { ok = __all_sync(0xffffffffu, ok && (!lead || clc_ask(&clc, it, &abort_flag))); };
+    for (int it = 0; ok; ++it) {
+      const OutTile w(p, cta);
+      if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&q_free[it & 1], ((it >> 1) - 1) & 1, &abort_flag));
+      if (!ok) break;
+      if (!w.empty) {
+        if (lead) {
           mbar_expect_tx(&q_full[it & 1], TILE_BYTES);
           tma_load_4d(smQ0 + (it & 1) * TILE_BYTES, &tm_q, &q_full[it & 1], 0, w.qhead, w.chunk * p.cq + w.row0, w.batch);
-          const int ch = (w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead;
-          for (int i = 0; i < w.nJ + w.nI && ok; ++i, ++g) {
-            if (i == 1) ok = clc_ask(&clc, it, &abort_flag);  // after the loads that the tile starts with
-            const int s = g % NR;
-            ok = ok && mbar_wait(&r_empty[s], ((g / NR) & 1) ^ 1, &abort_flag);
-            if (!ok) break;
+        }
+        const int ch = (w.batch * p.n_chunks + w.chunk) * p.h + w.kvhead;
+        const float* a_chunk =
+            gated ? p.a + ((size_t)w.batch * p.tk + (size_t)w.chunk * p.ck) * p.h + w.kvhead : nullptr;
+        // gate sums of the next step, two keys per lane, loaded one step ahead
+        float av0 = 0.f, av1 = 0.f, r_n = 0.f;
+        auto load_gates = [&](int J) {
+          if (gated) {
+            const int kp = J * TW + lane;
+            r_n = a_chunk[(size_t)min(J * TW + TW - 1, w.ck - 1) * p.h];
+            av0 = kp < w.ck ? a_chunk[(size_t)kp * p.h] : 0.f;
+            av1 = kp + 32 < w.ck ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
+          }
+        };
+        if (w.nJ > 0) load_gates(0);
+        for (int i = 0; i < w.nJ + w.nI && ok; ++i, ++g) {
+          if (i == 1) ask(it);  // after the loads that the tile starts with
+          const int s = g % NR;
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(&r_empty[s], ((g / NR) & 1) ^ 1, &abort_flag));
+          if (!ok) break;
+          uint8_t* dst = smR + s * R_BYTES;
+          const int k = i - w.nJ;
+          // c_full passes with every stage, so that its phases are the ring's; where there are no factors, before the loads
+          if (k >= 0 && lane == 0) mbar_arrive(&c_full[s]);
+          __syncwarp();
+          if (lead) {
             mbar_expect_tx(&r_full[s], R_BYTES);
-            uint8_t* dst = smR + s * R_BYTES;
-            const int k = i - w.nJ;
             if (k < 0) {
               tma_load_4d(dst, &tm_k, &r_full[s], 0, w.kvhead, w.chunk * p.ck + i * TW, w.batch);
               tma_load_4d(dst + KV_BYTES, &tm_v, &r_full[s], 0, w.kvhead, w.chunk * p.ck + i * TW, w.batch);
@@ -257,13 +287,25 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
               tma_load_2d(dst + Z_BYTES, &tm_z, &r_full[s], 0, (ch * p.nblk + 2 * (k - 1) + 1) * 64);
             }
           }
-          if (ok && w.nJ + w.nI == 1) ok = clc_ask(&clc, it, &abort_flag);
-        } else {
-          mbar_arrive(&q_full[it & 1]);  // nothing to load: the phase passes all the same
-          ok = clc_ask(&clc, it, &abort_flag);
+          if (k < 0) {
+            Cols& cl = smC[s];
+            cl.fk[lane] = __expf(r_n - av0);
+            cl.fk[lane + 32] = __expf(r_n - av1);
+            cl.ak[lane] = av0;
+            cl.ak[lane + 32] = av1;
+            const float low = warp_min(fminf(av0, av1));
+            if (lane == 0) cl.top = make_float2(r_n, low);
+            if (i + 1 < w.nJ) load_gates(i + 1);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c_full[s]);
+          }
         }
-        if (!ok || !clc_next(&clc, it, &cta, true, false, &abort_flag)) break;
+        if (w.nJ + w.nI == 1) ask(it);
+      } else {
+        if (lead) mbar_arrive(&q_full[it & 1]);  // nothing to load: the phase passes all the same
+        ask(it);
       }
+      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
     }
   } else if (warp == W_MMA) {
     const uint32_t tmem = tmem_base_s;
@@ -383,46 +425,43 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
       if (ok && u >= NB) ok = mbar_wait(&r_empty[(u - NB) % NR], ((u - NB) / NR) & 1, &abort_flag);
       tc_fence_after();
     };
+    // gate sum of this thread's row, loaded before the write-out of the tile before
+    float a_n = 0.f;
+    auto load_row = [&](const OutTile& w) {
+      a_n = (gated && w.row0 + r < w.cq)
+                ? p.a[((size_t)w.batch * p.tk + (size_t)w.chunk * p.ck + w.row0 + r + w.q_off) * p.h + w.kvhead]
+                : 0.f;
+    };
+    load_row(OutTile(p, cta));
     for (int it = 0; ok; ++it) {
       const OutTile w(p, cta);
+      bool more = false;
       if (!w.empty) {
         uint8_t* smQ = smQ0 + (it & 1) * TILE_BYTES;
         const float* a_chunk =
             gated ? p.a + ((size_t)w.batch * p.tk + (size_t)w.chunk * p.ck) * p.h + w.kvhead : nullptr;
         const int row = w.row0 + r;             // query index inside the chunk
         const int qpos = row + w.q_off;         // its key position
-        const float a_i = (gated && row < w.cq) ? a_chunk[(size_t)qpos * p.h] : 0.f;
+        const float a_i = a_n;
         float l_acc = 0.f;
-        // gate sums of this warp's next step, loaded one step ahead
-        float av0 = 0.f, av1 = 0.f, r_n = 0.f;
-        auto load_gates = [&](int J) {
-          if (gated) {
-            const int kp = J * TW + lane;
-            r_n = a_chunk[(size_t)min(J * TW + TW - 1, w.ck - 1) * p.h];
-            av0 = kp < w.ck ? a_chunk[(size_t)kp * p.h] : 0.f;
-            av1 = kp + 32 < w.ck ? a_chunk[(size_t)(kp + 32) * p.h] : 0.f;
-          }
-        };
         const int first = (u0 + grp) & 1;       // this group's first operand in the tile
         static_assert(NG == 2, "the group of operand u is u & 1");
-        if (first < w.nJ) load_gates(first);
 
         for (int J = first; J < w.nJ && ok; J += NG) {
           const int u = u0 + J, b = u % NB;
           const int kp0 = J * TW;
-          float* fk = sm_fk[warp][(J >> 1) & 1];
-          const float rs = r_n;
+          const Cols& cl = smC[u % NR];
+          ok = mbar_wait(&c_full[u % NR], (u / NR) & 1, &abort_flag);
+          if (!ok) break;
+          const float2 top = cl.top;
+          const float rs = top.x;
           // The gate factor separates, e^{a_i - a_j} = e^{a_i - r} * e^{r - a_j}: one exponential per
           // row and per key instead of one per pair (both exponents <= 0 below the diagonal for gates
           // <= 0; a warp falls back to the per-pair form if one exceeds 80).  Steps wholly below the
           // diagonal need no mask; a warp whose rows all precede the step's keys writes zeros
           // without reading the scores.
-          const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - fminf(av0, av1), a_i - rs) > 80.f);
+          const bool sep = !__any_sync(0xffffffffu, fmaxf(rs - top.y, a_i - rs) > 80.f);
           const float c_i = sep ? s2 * __expf(a_i - rs) : s2;
-          fk[lane] = sep ? __expf(rs - av0) : av0;
-          fk[lane + 32] = sep ? __expf(rs - av1) : av1;
-          __syncwarp();
-          if (J + NG < w.nJ) load_gates(J + NG);  // in flight while this step is computed
           ok = mbar_wait(&s_full[b], ((s_base >> b) + J / NB) & 1, &abort_flag);
           if (!ok) break;
           tc_fence_after();
@@ -437,9 +476,9 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
           } else {
             const bool mask = (kp0 + TW - 1 > wq0) || (kp0 + TW - 1 >= w.ck);
             const int lim = min(qpos, w.ck - 1) - kp0;  // last column this row keeps
-            if (!sep) out_step<T, DEG, false, true>(cs, fk, c_i, a_i, lim, l_acc);
-            else if (mask) out_step<T, DEG, true, true>(cs, fk, c_i, a_i, lim, l_acc);
-            else out_step<T, DEG, true, false>(cs, fk, c_i, a_i, lim, l_acc);
+            if (!sep) out_step<T, DEG, false, true>(cs, cl.ak, c_i, a_i, lim, l_acc);
+            else if (mask) out_step<T, DEG, true, true>(cs, cl.fk, c_i, a_i, lim, l_acc);
+            else out_step<T, DEG, true, false>(cs, cl.fk, c_i, a_i, lim, l_acc);
           }
           operand_written(u);
         }
@@ -535,6 +574,8 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         sm_l[tiles & 1][grp][r] = l_acc;
         meet();
         if (lane == 0) mbar_arrive(&q_free[it & 1]);
+        more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
+        if (more) load_row(OutTile(p, cta));
         if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
         tc_fence_after();
         // each group writes two pieces of 16 of the row's 64 columns, one 32-byte store each
@@ -582,8 +623,10 @@ chunk_out_kernel(const ChunkOutParams p, const __grid_constant__ CUtensorMap tm_
         ok = mbar_wait(&q_full[it & 1], (it >> 1) & 1, &abort_flag);
         __syncwarp();
         if (lane == 0) mbar_arrive(&q_free[it & 1]);
+        more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
+        if (more) load_row(OutTile(p, cta));
       }
-      if (!ok || !clc_next(&clc, it, &cta, lane == 0, true, &abort_flag)) break;
+      if (!more) break;
     }
   }
   tc_fence_before();
@@ -628,6 +671,8 @@ int pr::chunk_out(int dtype, int b, int tq, int tk, int cq, int ck, int hq, int 
   p.d = d;
   p.nblk = ref_dim(d) / 64;
   p.tiles_per_chunk = (cq + 127) / 128;
+  p.by_tiles = Div(p.tiles_per_chunk);
+  p.by_ratio = Div(hq / h);
   p.state_from_chunk = with_state ? state_from_chunk : n_chunks;
   p.q_gate_last = q_gate_last;
   p.normalize = normalize;
