@@ -226,6 +226,10 @@ StatePair final_state(const Tensor& S, const Tensor& gram, int64_t b, int64_t h,
 // autograd.Function for this case, which the tracer records as one node: the entry points answer None.
 bool being_traced() { return at::tracer::impl::is_dispatch_enabled(); }
 
+// Up to this length a sequence without states runs in the quadratic form whatever chunk was asked for (retention.py has
+// the reason and figures).
+constexpr int64_t kQuadraticTokens = 2048;
+
 using Retained = std::variant<Tensor, std::tuple<Tensor, StatePair>>;  // with a final state: (output, pair)
 
 // power_retention with the blocking chosen here.  Returns None for the head dims that the caller has to widen first, and
@@ -246,7 +250,11 @@ std::optional<Retained> power_retention(Tensor Q, Tensor K, Tensor V, const OptT
     throw PrError("states are kept for head dim 64 only (got " + std::to_string(d) + ")");
   if (d == 48) return std::nullopt;
   int64_t c = (auto_chunk && deg == 2) ? pr_fast_chunk(t, (int)std::min<int64_t>(chunk, std::numeric_limits<int>::max())) : chunk;
-  if (c != chunk || !switch_over.has_value()) switch_over = c ? std::optional<double>((double)c) : std::nullopt;
+  if (c != chunk || !switch_over.has_value()) {
+    // the blocking is this function's own choice: one chunk is the quadratic form, and so are short sequences
+    switch_over = c ? std::optional<double>((double)c) : std::nullopt;
+    if (auto_chunk && deg == 2 && !with_state && t <= kQuadraticTokens) c = 0;
+  }
   const bool quadratic = !switch_over.has_value() || c == 0 || (double)((t + c - 1) / c * c) <= *switch_over;
   if (deg != 2 && !(deg == 4 && quadratic && !with_state))
     throw PrError("deg=" + std::to_string(deg) +

@@ -146,6 +146,12 @@ def _pad_head_dim(x, d_to):
 # errs).  The C ABI (pr_retention_fwd) always takes the chunk it is given.
 AUTO_CHUNK = True
 _FAST_CHUNK = 1024
+# Up to two such chunks the quadratic form is less work than the states between them (per token and head 0.9 against 1.3
+# MFLOP forward and backward at 2048) and six launches instead of fourteen, so with AUTO_CHUNK sequences of up to that
+# length that carry no state run in it, whatever chunk was asked for; csrc/binding.cpp has the same number.
+# Forward and backward in us, one quadratic chunk / chunks of 1024: b1 t2000 h2 112 / 151, b8 t2048 h16 476 / 863,
+# b16 t1100 h32 733 / 2079, b8 t2048 h4x8 868 / 1094, b1 t2048 h2x12 315 / 311; at 4096 (b1 h4) 156 / 123.
+QUADRATIC_TOKENS = 2048
 
 
 def effective_chunk(t: int, chunk_size, deg: int = 2):
@@ -217,11 +223,12 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     h = K.shape[2]
     requested = chunk_size
     chunk_size = effective_chunk(t, chunk_size, deg)
-    if chunk_size != requested:
-        # the blocking is this function's own choice: one chunk is the quadratic form, several the chunked one
+    if chunk_size != requested or (chunk_size is not None and switch_over_seq_len is None):
+        # the blocking is this function's own choice: one chunk is the quadratic form, and so are short sequences;
+        # several chunks are the chunked one
         switch_over_seq_len = chunk_size
-    elif chunk_size is not None and switch_over_seq_len is None:
-        switch_over_seq_len = chunk_size
+        if AUTO_CHUNK and deg == 2 and t <= QUADRATIC_TOKENS and initial_state is None and not return_final_state:
+            chunk_size = None
     t_padded = t if chunk_size is None else -(-t // chunk_size) * chunk_size
     state_free = (switch_over_seq_len is None or t_padded <= switch_over_seq_len or chunk_size is None) and \
         initial_state is None and not return_final_state
