@@ -12,12 +12,17 @@
 //   W = V, State = w (.) dS_m, Gs = dG_m + dG_m^T, g_i = 1, mult = 1, f_i = exp((A_m - a_i)/2).
 //
 // One CTA owns one row tile of 128 tokens of one (batch, chunk, head) and two CTAs share an SM, so that one CTA's
-// prologue (operand loads, gating, Gram part) and write-out - a quarter of a CTA's life, all of it on the drain warps -
+// prologue (operand loads, gating) and write-out (with the Gram part) - a quarter of a CTA's life, all of it on the drain warps -
 // run while the other CTA drains.  (Two row tiles in one CTA per SM, where each state tile fetched from L2 feeds two
 // products, measured 7 % slower: 0.302 against 0.282 ms per launch at b1 t65536 h8.)  The expansion gradient dphi is
 // never written to memory: tiles of 128 expanded rows are produced in tensor memory, two buffers, and drained by four
-// warps while the tensor core fills the other buffer.  Each thread owns one token row and keeps x~ and dx~ in
-// registers; the triangle's (a, b) pattern is resolved at compile time, so the drain is two FMAs per entry.
+// warps while the tensor core fills the other buffer.  Each thread owns one token row; the second factors of a 16-block and
+// their gradients are in registers while the block is drained, two FMAs per entry.  The Gram part comes last, as one
+// more tile: at the start it held up the first state tile (272 -> 268 us, 79.7 -> 78.4 at b4 t5000 h2x4, 25.8 -> 25.2 with
+// one head per group).  A tile takes a drain warp about 1000 clocks, where its FMAs and tensor-memory loads alone take 365
+// (packed FMAs with three distinct operand pairs issue every 2.8 clocks).  Measured and not kept: one CTA per SM with
+// four row tiles, four groups of drain warps, W in tensor memory and pieces of 64 rows: 266 us, but 85 and 27.2 for the
+// other two.
 #include <type_traits>
 
 #include "host.cuh"
@@ -33,14 +38,11 @@ constexpr int G_BYTES = 64 * 128;
 constexpr int W_TMA = 4;                 // four drain warps, the TMA warp, two issuing warps (one per buffer)
 constexpr int THREADS = 32 * (W_TMA + 3);
 constexpr int ROWS = 128;
-constexpr int NSS = 2;                   // state tiles in flight; the Gram operand borrows the last slot first
+constexpr int NSS = 2;                   // state tiles in flight; the Gram operand comes last
 constexpr uint32_t TMEM_COLS = 256;
 constexpr size_t SMEM = 1024 + (size_t)(2 + NSS) * TILE_BYTES + (size_t)64 * 128 * 4;
-// Tensor memory: two 128-column buffers.
-// Before the first use of buffer 1 its columns hold the Gram part: the gated row as A operand
-// (32 columns at +0) and u = x~ Gs (64 columns at +64), read into the accumulators' initial value.
+// Tensor memory: two 128-column buffers; in the end u = x~ Gs comes in the first one.
 __device__ __forceinline__ constexpr uint32_t col_d(int b) { return (uint32_t)(b * 128); }
-constexpr uint32_t OFF_XA = 0, OFF_U = 64;
 
 }  // namespace eg
 
@@ -50,6 +52,7 @@ struct ExpandGradParams {
   int t, d;              // tokens (the last chunk may be shorter), features (a multiple of 16)
   int nt;                // tiles of 128 expanded rows (8 first factors x 16) of a state
   int tiles_per_chunk;
+  Div by_tiles, by_ratio;  // by tiles_per_chunk, by hx / h
   int chunk_lo, chunk_hi;  // chunks in [lo, hi] have a state term; the others get zeros
   int query_side;
   float scale;           // s (query side only)
@@ -69,15 +72,15 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
                    const __grid_constant__ CUtensorMap tm_ghi, const __grid_constant__ CUtensorMap tm_glo) {
   using namespace eg;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t w_full, g_full, xa_full, u_full, s_full[NSS], s_empty[NSS], d_full[2], d_empty[2];
+  __shared__ uint64_t w_full, x_in, s_full[NSS], s_empty[NSS], d_full[2], d_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
-  const int tile_i = blockIdx.x % p.tiles_per_chunk;
-  const int chunk = blockIdx.x / p.tiles_per_chunk;
+  int tile_i, chunk;
+  p.by_tiles.of((int)blockIdx.x, &chunk, &tile_i);
   const int head = blockIdx.y, batch = blockIdx.z;
-  const int gh = head / (p.hx / p.h);
+  const int gh = p.by_ratio.of(head);
   const int row0 = tile_i * ROWS;
   const size_t tok0 = (size_t)batch * p.t + (size_t)chunk * p.c;
   const int c = min(p.c, p.t - chunk * p.c);  // tokens of this chunk
@@ -101,16 +104,13 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
   uint8_t* smW = sm;
   uint8_t* smX = smW + TILE_BYTES;
   uint8_t* smS = smX + TILE_BYTES;                // NSS x TILE_BYTES (ring of state tiles)
-  uint8_t* smG = smS + (NSS - 1) * TILE_BYTES;    // Gram operand (hi, lo): the ring's last slot until its products are done
-  static_assert(2 * G_BYTES <= TILE_BYTES, "the Gram operand fits a slot");
+  static_assert(2 * G_BYTES == TILE_BYTES, "the Gram operand (hi, lo) is one more stage of the ring");
   float* smR = reinterpret_cast<float*>(smS + NSS * TILE_BYTES);  // [64][128] fp32: dx~ terms indexed at run time
 
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&w_full, 1);
-    mbar_init(&g_full, 1);
-    mbar_init(&xa_full, 4);
-    mbar_init(&u_full, 1);
+    mbar_init(&x_in, 4);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&d_full[b], 1);
       mbar_init(&d_empty[b], 4);
@@ -136,16 +136,16 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
       mbar_expect_tx(&w_full, 2 * TILE_BYTES);
       tma_load_4d(smW, &tm_w, &w_full, 0, head, chunk * p.c + row0, batch);
       tma_load_4d(smX, &tm_x, &w_full, 0, head, chunk * p.c + row0, batch);
-      mbar_expect_tx(&g_full, 2 * G_BYTES);
-      tma_load_3d(smG, &tm_ghi, &g_full, 0, 0, ch);
-      tma_load_3d(smG + G_BYTES, &tm_glo, &g_full, 0, 0, ch);
-      for (int nt = 0; nt < p.nt; ++nt) {
+      for (int nt = 0; nt <= p.nt; ++nt) {
         const int s = nt % NSS, ph = (nt / NSS) & 1;
         if (!mbar_wait(&s_empty[s], ph ^ 1, &abort_flag)) break;
-        // the slot lent to the Gram operand is free once the Gram products have completed
-        if (nt == NSS - 1 && !mbar_wait(&u_full, 0, &abort_flag)) break;
         mbar_expect_tx(&s_full[s], TILE_BYTES);
-        tma_load_2d(smS + s * TILE_BYTES, &tm_s, &s_full[s], 0, (ch * p.nt + nt) * 128);
+        if (nt < p.nt) {
+          tma_load_2d(smS + s * TILE_BYTES, &tm_s, &s_full[s], 0, (ch * p.nt + nt) * 128);
+        } else {
+          tma_load_3d(smS + s * TILE_BYTES, &tm_ghi, &s_full[s], 0, 0, ch);
+          tma_load_3d(smS + s * TILE_BYTES + G_BYTES, &tm_glo, &s_full[s], 0, 0, ch);
+        }
       }
     }
   } else if (warp > W_TMA) {
@@ -163,9 +163,7 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
       for (int nt = par; nt < p.nt && ok; nt += 2) {
         const int s = nt % NSS, ph = (nt / NSS) & 1;
         const int b = par;
-        // buffer 0 has been drained nt/2 times before tile nt; buffer 1 once more (the Gram part)
-        ok = mbar_wait(&d_empty[b], ((nt >> 1) & 1) ^ (b ^ 1), &abort_flag) &&
-             mbar_wait(&s_full[s], ph, &abort_flag);
+        ok = mbar_wait(&d_empty[b], ((nt >> 1) & 1) ^ 1, &abort_flag) && mbar_wait(&s_full[s], ph, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint64_t d_s = d_s0 + (uint32_t)s * (TILE_BYTES >> 4);
@@ -174,22 +172,23 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
           umma_ss(tmem + col_d(b), d_w + 2 * ks, d_s + 2 * ks, idesc, ks > 0 ? 1u : 0u);
         umma_commit(&d_full[b]);
         umma_commit(&s_empty[s]);
-        if (nt == 0) {
-          // Gram part: u = x~ (Gs_hi + Gs_lo), once per row tile, in the columns of buffer 1 (whose own
-          // issuing thread waits until the rows have taken u out)
-          ok = mbar_wait(&g_full, 0, &abort_flag) && mbar_wait(&xa_full, 0, &abort_flag);
-          if (!ok) break;
+      }
+      if (par == 0 && ok) {
+        // Gram part: u = x~ (Gs_hi + Gs_lo), as one more tile; the number of tiles is even
+        const int s = p.nt % NSS;
+        ok = mbar_wait(&d_empty[0], ((p.nt >> 1) & 1) ^ 1, &abort_flag) &&
+             mbar_wait(&s_full[s], (p.nt / NSS) & 1, &abort_flag) && mbar_wait(&x_in, 0, &abort_flag);
+        if (ok) {
           tc_fence_after();
           const uint32_t idesc_g = umma_idesc(128, HD, Pack2<T>::is_bf16, false, false);
-          const uint32_t g_addr = smem_u32(smG);
+          const uint64_t d_x = umma_desc_sw128(smem_u32(smX), 16, 1024), d_g = d_s0 + (uint32_t)s * (TILE_BYTES >> 4);
 #pragma unroll
           for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              umma_ts(tmem + col_d(1) + OFF_U, tmem + col_d(1) + OFF_XA + ks * 8,
-                      umma_desc_sw128(g_addr + half * G_BYTES + ks * 32, 16, 1024), idesc_g,
+              umma_ss(tmem + col_d(0), d_x + 2 * ks, d_g + half * (G_BYTES >> 4) + 2 * ks, idesc_g,
                       (half > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&u_full);
+          umma_commit(&d_full[0]);
         }
       }
     }
@@ -206,59 +205,31 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
       f *= p.query_side ? __expf(0.5f * a_i) : __expf(0.5f * (p.A[ch] - a_i));
     }
     bool ok = mbar_wait(&w_full, 0, &abort_flag);
-    {
-      uint32_t xp[32];
-      uint8_t* xs = smX;
+    // the gated row replaces the raw one in this thread's slot of the tile: the drain fetches factors from it by a
+    // run-time index, and it is the Gram product's A operand
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(xs + swz128(r, j));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    for (int j = 0; j < 8; ++j) {
+      uint4* slot = reinterpret_cast<uint4*>(smX + swz128(r, j));
+      const uint4 v = *slot;
+      uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 raw = Pack2<T>::to_f32(w[k]);
-          xp[4 * j + k] = Pack2<T>::from_f32(raw.x * f, raw.y * f);
-        }
+      for (int k = 0; k < 4; ++k) {
+        const float2 raw = Pack2<T>::to_f32(w[k]);
+        w[k] = Pack2<T>::from_f32(raw.x * f, raw.y * f);
       }
-      // the gated row replaces the raw one in this thread's slot of the tile (fetched by a
-      // run-time index in the drain)
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        *reinterpret_cast<uint4*>(smX + swz128(r, j)) =
-            make_uint4(xp[4 * j], xp[4 * j + 1], xp[4 * j + 2], xp[4 * j + 3]);
-      if (ok) {
-        tmem_st32(tmem + lane_addr + col_d(1) + OFF_XA, xp);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&xa_full);
-      }
+      *slot = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    // Gram part first: dx~ starts at g_i * mult * (Gs x~)_i, which also frees buffer 1
-    {
-      float g = p.gram_mult;
-      if (p.row_g != nullptr) g *= row_valid ? p.row_g[(tok0 + row) * p.hx + head] : 0.f;
-      if (ok) ok = mbar_wait(&u_full, 0, &abort_flag);
-      tc_fence_after();
-      uint32_t u[64];
-      if (ok) {
-        tmem_ld32(tmem + lane_addr + col_d(1) + OFF_U, u);
-        tmem_ld32(tmem + lane_addr + col_d(1) + OFF_U + 32, u + 32);
-        tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&d_empty[1]);
-      }
-      // dx~ lives in this thread's private column of shared memory (64 floats, stride 128): the
-      // first-factor terms are added at a run-time index, and the second-factor terms of a
-      // 16-block are kept in registers only while that block is being drained.  Keeping all 64
-      // accumulators and the row itself in registers left the compiler no room to overlap the
-      // FMAs of neighbouring entries.
-      float* sdx0 = smR + r;
-#pragma unroll
-      for (int e = 0; e < HD; ++e) sdx0[e * 128] = ok ? g * __uint_as_float(u[e]) : 0.f;
-    }
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&x_in);
+    float g = p.gram_mult;
+    if (p.row_g != nullptr) g *= row_valid ? p.row_g[(tok0 + row) * p.hx + head] : 0.f;
+    // dx~ lives in this thread's private column of shared memory (64 floats, stride 128): the first-factor terms are
+    // added at a run-time index, and the second-factor terms of a 16-block are kept in registers only while that block
+    // is being drained.  Keeping all 64 accumulators and the row itself in registers left the compiler no room to overlap
+    // the FMAs of neighbouring entries.
     float* sdx = smR + r;
-    const uint8_t* xrow = smX;  // holds the gated row again (written above)
+    const uint8_t* xrow = smX;
 
     int nt = 0;
     static_for<0, HD / 16>([&](auto yc) {
@@ -330,8 +301,14 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
             rsum[2 * q + aa] = (ra0.x + ra0.y) + (ra1.x + ra1.y);
           }
         }
+        // the block's own entries come up as first factors for the first time here
+        if (tt < 2 * Y) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sdx[(8 * tt + j) * 128] += rsum[j];
+          for (int j = 0; j < 8; ++j) sdx[(8 * tt + j) * 128] += rsum[j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sdx[(8 * tt + j) * 128] = rsum[j];
+        }
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -340,7 +317,13 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
       }
     });
 
-    if (ok && row_valid) {
+    if (ok) ok = mbar_wait(&d_full[0], (p.nt >> 1) & 1, &abort_flag);
+    tc_fence_after();
+    if (ok) {
+      uint32_t u[64];
+      tmem_ld32(tmem + lane_addr + col_d(0), u);
+      tmem_ld32(tmem + lane_addr + col_d(0) + 32, u + 32);
+      tmem_wait_ld();
       float dot = 0.f;
       float4* dst = reinterpret_cast<float4*>(p.dX + ((tok0 + row) * p.hx + head) * p.d);
 #pragma unroll
@@ -352,18 +335,19 @@ expand_grad_kernel(const ExpandGradParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const float2 f2 = Pack2<T>::to_f32(w[k]);
-          d8[2 * k] = sdx[(8 * j + 2 * k) * 128];
-          d8[2 * k + 1] = sdx[(8 * j + 2 * k + 1) * 128];
+          d8[2 * k] = fmaf(g, __uint_as_float(u[8 * j + 2 * k]), sdx[(8 * j + 2 * k) * 128]);
+          d8[2 * k + 1] = fmaf(g, __uint_as_float(u[8 * j + 2 * k + 1]), sdx[(8 * j + 2 * k + 1) * 128]);
           dot = fmaf(f2.x, d8[2 * k], dot);
           dot = fmaf(f2.y, d8[2 * k + 1], dot);
         }
         // one 32-byte store: a full sector per thread and instruction
-        asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 2 * j), "f"(d8[0] * f),
+        if (row_valid)
+          asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 2 * j), "f"(d8[0] * f),
                      "f"(d8[1] * f), "f"(d8[2] * f), "f"(d8[3] * f), "f"(d8[4] * f), "f"(d8[5] * f), "f"(d8[6] * f),
                      "f"(d8[7] * f)
                      : "memory");
       }
-      p.gdot[(tok0 + row) * p.hx + head] = 0.5f * dot;
+      if (row_valid) p.gdot[(tok0 + row) * p.hx + head] = 0.5f * dot;
     }
   }
   tc_fence_before();
@@ -400,6 +384,8 @@ extern "C" int pr_expand_grad(int dtype, int b, int t, int h, int hx, int d, int
   p.d = d;
   p.nt = ref_dim(d) / 128;
   p.tiles_per_chunk = (c + ROWS - 1) / ROWS;
+  p.by_tiles = Div(p.tiles_per_chunk);
+  p.by_ratio = Div(hx / h);
   p.chunk_lo = chunk_lo;
   p.chunk_hi = chunk_hi;
   p.query_side = query_side;

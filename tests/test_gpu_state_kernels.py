@@ -51,3 +51,39 @@ def test_chunk_state(cuda_device, b, n, nh, group, c, weights, gram):
         if gram:
             xg = xs[:, m].view(b, nh, group, 64, c).double()
             assert rel_l2(G[:, m].double(), torch.einsum("bhgai,bhgei->bhae", xg, x.double())) < 2e-5, m
+
+
+@pytest.mark.parametrize("b,n,h,r,c", [(1, 2, 1, 1, 64), (1, 2, 1, 1, 512), (1, 3, 2, 2, 384), (2, 4, 4, 2, 200),
+                                       (1, 12, 8, 1, 1024)])
+@pytest.mark.parametrize("query_side", [True, False])
+def test_expand_grad(cuda_device, b, n, h, r, c, query_side):
+    from retention_integration_b200 import ops
+
+    g = torch.Generator(cuda_device).manual_seed(n + c)
+    hx, t, dev = h * r, n * c, cuda_device
+    R = lambda *s: torch.randn(*s, generator=g, device=dev)
+    W, X = R(b, t, hx, 64).bfloat16(), R(b, t, hx, 64).bfloat16()
+    S, hi, lo = R(b, n, h, 2560, 64).bfloat16(), R(b, n, h, 64, 64).bfloat16(), (0.01 * R(b, n, h, 64, 64)).bfloat16()
+    row_g = R(b, t, hx) if query_side else None
+    scale, mult = (0.125, 2.0) if query_side else (1.0, 1.0)
+    first, last = (1, n - 1) if query_side else (0, n - 2)
+    args = (W, X, S, hi, lo, None, None, row_g, c, h, query_side, scale, mult, first, last)
+    dX, gdot = ops.expand_grad(*args)
+    dX2, gdot2 = ops.expand_grad(*args)
+    assert _status(cuda_device) == 0
+    assert torch.equal(dX, dX2) and torch.equal(gdot, gdot2)
+    fa, fb = _pairs(dev)
+    for m in range(n):
+        rows = slice(m * c, (m + 1) * c)
+        if not first <= m <= last:
+            assert torch.count_nonzero(dX[:, rows]) == 0 and torch.count_nonzero(gdot[:, rows]) == 0
+            continue
+        for k in range(hx):
+            x = (X[:, rows, k].float() * scale).bfloat16().double()
+            dphi = torch.einsum("bie,bDe->biD", W[:, rows, k].double(), S[:, m, k // r].double())
+            Gs = hi[:, m, k // r].double() + lo[:, m, k // r].double()
+            gx = mult * torch.einsum("bae,bie->bia", Gs, x) * (row_g[:, rows, k].double()[..., None] if query_side else 1)
+            gx.index_add_(2, fa, dphi * x[:, :, fb])
+            gx.index_add_(2, fb, dphi * x[:, :, fa])
+            assert rel_l2(dX[:, rows, k].double(), gx * scale) < 2e-5, (m, k)
+            assert rel_l2(gdot[:, rows, k].double(), 0.5 * (gx * x).sum(-1)) < 2e-5, (m, k)
