@@ -22,7 +22,8 @@
 // a logarithm and exponentials were a chain of 1000-1900 traced clocks in front of a step's 1000-1500, on all twelve
 // warps.  With warps of their own for it, and the next tile's gates and the state-path gradients fetched before the
 // write-out: 467 -> 413, 119 -> 102 (gated bf16), 80 -> 68 at b4 t2048 h8 in one chunk, 19.2 -> 17.2; without divisions
-// between the tiles 395, 98, 67, 17.  (One such warp, the
+// between the tiles 395, 98, 67, 17; with the state-path gradients fetched 32 bytes a lane, before the rows meet, 373: a
+// tile's end, traced at 7400 clocks of 21000 at first, is bound by rows 2 KB apart, a line per lane and instruction.  (One such warp, the
 // TMA warp: 483, 137, -, 21.3: it cannot keep up.)
 #include "host.cuh"
 #include "layout.cuh"
@@ -73,6 +74,7 @@ struct ChunkDkvParams {
   void* dK;
   void* dV;
   int aligned32;          // dK and dV start on 32-byte boundaries
+  int state_aligned32;    // dk_state does
   float* da_k;            // [b, t, h]
   int* status;
 };
@@ -570,24 +572,36 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
         // that read them have completed with the scores)
         fence_async_smem();
         sm_da[tiles & 1][first][r] = da;  // by step, not by group: a fixed order of the sum whatever the CTA did before
-        meet();
-        if (lane == 0) mbar_arrive(&kv_free[it & 1]);
-
         // The groups share the write-out: 16 of the 64 columns of dV (units 0-3) or dK (units 4-7) at a time.  The
-        // state-path gradients come in while the last products run, and the next tile's gates too.
+        // state-path gradients come in while the rows meet and the last products run, and the next tile's gates too.
         const size_t tok = tok_base + row;
         const float* st = p.dk_state ? p.dk_state + (tok * p.h + w.kvhead) * p.d : nullptr;
         constexpr int UNITS = (8 + NG - 1) / NG;
-        float4 add[UNITS - 1][4];
+        float add[UNITS - 1][2][8];
 #pragma unroll
         for (int i = 1; i < UNITS; ++i) {
           const int unit = grp + NG * i, c0 = 16 * (unit & 3);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            add[i - 1][j] = (st != nullptr && row_valid && unit >= 4 && unit < 8 && c0 < p.d)
-                                ? reinterpret_cast<const float4*>(st + c0)[j]
-                                : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) add[i - 1][j][k] = 0.f;
+            if (st != nullptr && row_valid && unit >= 4 && unit < 8 && c0 < p.d) {
+              if (p.state_aligned32) {
+                ld_global_v8(st + c0 + 8 * j, add[i - 1][j]);
+              } else {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const float4 v = reinterpret_cast<const float4*>(st + c0 + 8 * j)[k];
+                  add[i - 1][j][4 * k] = v.x, add[i - 1][j][4 * k + 1] = v.y;
+                  add[i - 1][j][4 * k + 2] = v.z, add[i - 1][j][4 * k + 3] = v.w;
+                }
+              }
+            }
+          }
         }
+        meet();
+        if (lane == 0) mbar_arrive(&kv_free[it & 1]);
+
         more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
         if (more) load_row(DkvTile(p, cta));
         if (ok) ok = mbar_wait(&acc_full, tiles & 1, &abort_flag);
@@ -603,9 +617,12 @@ chunk_dkv_kernel(const ChunkDkvParams p, const __grid_constant__ CUtensorMap tm_
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const float4 ad = i > 0 ? add[i > 0 ? i - 1 : 0][j] : make_float4(0.f, 0.f, 0.f, 0.f);
-              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + ad.x, __uint_as_float(acc[4 * j + 1]) + ad.y);
-              v[2 * j + 1] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + ad.z, __uint_as_float(acc[4 * j + 3]) + ad.w);
+              float ad[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) ad[k] = i > 0 ? add[i > 0 ? i - 1 : 0][j >> 1][4 * (j & 1) + k] : 0.f;
+              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + ad[0], __uint_as_float(acc[4 * j + 1]) + ad[1]);
+              v[2 * j + 1] =
+                  Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + ad[2], __uint_as_float(acc[4 * j + 3]) + ad[3]);
             }
             T* dst = static_cast<T*>(unit < 4 ? p.dV : p.dK) + (tok * p.h + w.kvhead) * p.d + c0;
             if (p.aligned32) {
@@ -689,6 +706,7 @@ extern "C" int pr_chunk_dkv(int dtype, int b, int t, int hq, int h, int d, int c
   p.dK = dK;
   p.dV = dV;
   p.aligned32 = aligned32(dK) && aligned32(dV);
+  p.state_aligned32 = aligned32(dk_state);
   p.da_k = da_k;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;

@@ -21,7 +21,7 @@
 // Two more warps make, step by step in turn and up to six ahead, the gate factors of a step's keys (Cols), which every row
 // warp used to make for itself before it could look at the scores; a tile's row values are fetched before the
 // write-out of the tile before: 217 -> 202 us, 75.6 -> 72.7 (gated bf16), 56 -> 52 at b4 t2048 h8 in one chunk, the small
-// ones the same.
+// ones the same; 198 without divisions between the tiles, 196 with the state-path gradient read 32 bytes a lane.
 #include "host.cuh"
 #include "sm100.cuh"
 
@@ -61,6 +61,7 @@ struct ChunkDqParams {
   const float* dq_state;  // [b, t, hq, d] fp32 or null
   void* dQ;               // [b, t, hq, d]
   int aligned32;          // dQ starts on a 32-byte boundary
+  int state_aligned32;    // dq_state does
   float* da_q;            // [b, t, hq]
   int* status;
 };
@@ -429,14 +430,27 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
         if (lane == 0) mbar_arrive(&rows);
         // the groups share the write-out, 16 of the 64 columns at a time; the state-path gradient comes in meanwhile
         const float* st = p.dq_state ? p.dq_state + ix * p.d : nullptr;
-        float4 add[2][4];
+        float add[2][2][8];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const int c0 = 16 * (grp + NG * q);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            add[q][j] = (st != nullptr && row_valid && c0 < p.d && c0 < HD) ? reinterpret_cast<const float4*>(st + c0)[j]
-                                                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) add[q][j][k] = 0.f;
+            if (st != nullptr && row_valid && c0 < p.d && c0 < HD) {
+              if (p.state_aligned32) {
+                ld_global_v8(st + c0 + 8 * j, add[q][j]);
+              } else {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const float4 v = reinterpret_cast<const float4*>(st + c0 + 8 * j)[k];
+                  add[q][j][4 * k] = v.x, add[q][j][4 * k + 1] = v.y;
+                  add[q][j][4 * k + 2] = v.z, add[q][j][4 * k + 3] = v.w;
+                }
+              }
+            }
+          }
         }
         more = ok && clc_next(&clc, it, &cta, lane == 0, true, &abort_flag);
         if (more) load_row(DqTile(p, cta));
@@ -455,9 +469,10 @@ chunk_dq_kernel(const ChunkDqParams p, const __grid_constant__ CUtensorMap tm_q,
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + add[q][j].x, __uint_as_float(acc[4 * j + 1]) + add[q][j].y);
+              const float* ad = add[q][j >> 1] + 4 * (j & 1);
+              v[2 * j] = Pack2<T>::from_f32(__uint_as_float(acc[4 * j]) + ad[0], __uint_as_float(acc[4 * j + 1]) + ad[1]);
               v[2 * j + 1] =
-                  Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + add[q][j].z, __uint_as_float(acc[4 * j + 3]) + add[q][j].w);
+                  Pack2<T>::from_f32(__uint_as_float(acc[4 * j + 2]) + ad[2], __uint_as_float(acc[4 * j + 3]) + ad[3]);
             }
             T* dst = static_cast<T*>(p.dQ) + ix * p.d + c0;
             if (p.aligned32) {
@@ -525,6 +540,7 @@ extern "C" int pr_chunk_dq(int dtype, int b, int t, int hq, int h, int d, int c,
   p.dq_state = dq_state;
   p.dQ = dQ;
   p.aligned32 = aligned32(dQ);
+  p.state_aligned32 = aligned32(dq_state);
   p.da_q = da_q;
   int rc = status_word(device, &p.status, nullptr);
   if (rc) return rc;

@@ -240,6 +240,13 @@ __device__ __forceinline__ void st_global_v8(void* dst, const uint32_t (&v)[8]) 
                : "memory");
 }
 
+// the same for a load of eight floats
+__device__ __forceinline__ void ld_global_v8(const float* src, float (&v)[8]) {
+  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(src));
+}
+
 // -------------------------------------------------------------------- TMEM
 // One full warp calls alloc / dealloc.  ncols: power of two in [32, 512].
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
