@@ -421,9 +421,7 @@ static int launch_chunk_state(const ChunkStateParams& p, const CUtensorMap& tm_x
   int device = 0;
   PR_CUDA(cudaGetDevice(&device));  // the entry point has made the caller's device current
   PR_SMEM_ATTR((chunk_state_kernel<T, EXACT>), SMEM, device, true);
-  const long long ctas = (long long)(p.n_slots + (EXACT || p.gram ? 1 : 0)) * p.n_states;
-  PR_REQUIRE(ctas < (1ll << 31), PR_ERR_BAD_ARG, "%lld CTAs exceed the grid limit", ctas);
-  dim3 grid((unsigned)ctas);
+  dim3 grid((unsigned)((p.n_slots + (EXACT || p.gram ? 1 : 0)) * p.n_states));
   chunk_state_kernel<T, EXACT><<<grid, THREADS, SMEM, stream>>>(p, tm_xt, tm_xs, tm_w);
   PR_CUDA(cudaGetLastError());
   return PR_OK;
@@ -434,10 +432,14 @@ template <bool EXACT>
 static int run_chunk_state(int dtype, int b, int t, int nh, int group, int d, int c, const void* xt, const void* xts,
                            const void* v, ChunkStateParams p, int chunk0, int n_run, int device, void* stream) {
   if (n_run <= 0) return PR_OK;
+  p.n_slots = ref_dim(d) / (cs::NT * 128);  // exact: 2, 6, 12 or 20 tiles
+  // the items' indices are 32-bit (StateItem): counted before anything is narrowed
+  const long long most = ((1ll << 31) - 1) / (p.n_slots + (EXACT || p.gram ? 1 : 0));
+  PR_REQUIRE((long long)b * n_run <= most && (long long)b * n_run * nh <= most, PR_ERR_BAD_ARG,
+             "b=%d, %d chunks and %d heads exceed the grid limit of %lld states", b, n_run, nh, most);
   PR_CUDA(cudaSetDevice(device));
   p.chunk0 = chunk0;
   p.n_run = n_run;
-  p.n_slots = ref_dim(d) / (cs::NT * 128);  // exact: 2, 6, 12 or 20 tiles
   p.n_states = b * n_run * nh;
   p.by_slots = Div(p.n_slots);
   p.by_heads = Div(nh);
