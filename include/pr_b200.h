@@ -293,15 +293,8 @@ int pr_retention_fwd(const pr_problem* problem, const void* Q, const void* K, co
  * The chunk size blocks the computation of retention/power_retention_maker.py:143-193 without changing its
  * result; on this hardware 1024 is fastest (5.0 ms per step at chunk 128 against 2.5 at 1024 for b1 t65536 h8).
  * pr_retention_fwd / _bwd run whatever pr_problem.c says; a host that wants the fast blocking passes
- * c = pr_fast_chunk(t, its_chunk) where a state comes in or goes out, and asks pr_blocking where none does. */
+ * c = pr_fast_chunk(t, its_chunk). */
 int pr_fast_chunk(long long t, int requested_chunk);
-
-/* The blocking to run a sequence with that neither starts from a state nor returns one: 0 = the quadratic form
- * (pr_attention_fwd / _bwd), else the chunk length for pr_retention_fwd / _bwd.  One chunk is the quadratic form; where
- * there would be several, up to `longest_quadratic` tokens (the Python API says 2048), the form that is less work for these
- * heads and this width; beyond, pr_fast_chunk's choice.  Host arithmetic only; deg 2.  Sizes that the operator refuses come
- * back as pr_fast_chunk has them. */
-int pr_blocking(int b, long long t, int h, int hq, int d, int requested_chunk, int longest_quadratic);
 
 /* Backward.  dO [b,t,hq,d] -> dQ, dK, dV (shapes of Q, K, V) and dlog_G [b,t,h] fp32 (NULL when
  * ungated).  `saved` as the forward left it; had_carry = 1 when the forward was given carries.

@@ -8,7 +8,6 @@
 // Memory: the caller allocates everything.  `saved` is what the backward needs from the
 // forward (gate sums, row sums, scanned states and Gram matrices); `scratch` is dead when the
 // call returns its work to the stream and may be reused by the next call on the same stream.
-#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -218,8 +217,9 @@ class Fork {
 // of the request in [256, 1024]; 0 (no chunking) on more than 2048 tokens: 1024 or 512 if that rounds the length up by
 // at most 1/16, else 0.
 // The rounding was work while sequences were padded to whole chunks.  They no longer are, and by work the rule errs
-// where it still decides: t 7200 unchunked stays one chunk (358 us, b1 h4) where chunks of 1024 take 194.  Short sequences
-// without states have pr_blocking.  Mirrors retention.py: effective_chunk, for hosts that do not go through the Python API.
+// where it still decides: t 7200 unchunked stays one chunk (358 us, b1 h4) where chunks of 1024 take 194, and up to
+// 2048 tokens without states no chunks are better whatever was asked for, which the Python API does
+// (retention.py: QUADRATIC_TOKENS; a C host asks for c = 0).  Mirrors retention.py: effective_chunk, for hosts that do not go through the Python API.
 extern "C" int pr_fast_chunk(long long t, int requested) {
   const int fast = 1024;
   if (t <= 0 || requested < 0) return requested;
@@ -242,50 +242,6 @@ extern "C" int pr_fast_chunk(long long t, int requested) {
     if (rounded_to(ce) <= asked + asked / 16) return (int)ce;
   }
   return requested;
-}
-
-namespace pr {
-namespace {
-
-// Row tiles of 128 queries of t tokens, and the 64-key steps that they take between them.
-double row_tiles(long long t) { return (double)((t + 127) / 128); }
-double row_steps(long long t) {
-  const double n = row_tiles(t);
-  return n * (n + 1) - (2 * n - (double)((t + 63) / 64));
-}
-
-// What the quadratic form saves forward and backward against chunks of c < t tokens, in us, from what the kernels run:
-// attention is 64 features wide at every head dim, a state has ref_dim(d) rows.
-//   - attention, per SM: the row steps of all tiles and query heads, but no less than 0.3 of the steps of the longest
-//     key tile, which one CTA of chunk_dkv takes alone (128 keys against all later queries of their group): 1.4 us a step
-//   - state work that goes away, per SM: 128 tokens x 64 state rows, read and differentiated for every query head, made and
-//     differentiated for every kv head: 0.6 us
-//   - the start and end of a row tile, per SM: 6 us; eight launches fewer: 20 us
-// Fitted to 485 shapes (d 16, 32, 64, 300-2048 tokens, chunks of 128-1031, 1-1024 query heads, ratios 1-16; replayed).  What
-// it picks is the faster form or within 3 % of it in 464 of them, and up to a fifth slower in the others, narrow heads in
-// three or four ragged chunks that take 80-180 us.  By tokens alone, quadratic up to 2048, 99 were slower and up to a
-// half: quadratic / chunks d 16 b16 t2048 h32x2 2842 / 2339, d 32 b16 t1999 h4x12 2284 / 1881, d 64 b1 t1999 h1x16 322 / 238.
-double quadratic_saves_us(double b, long long t, double h, double hq, int d, long long c) {
-  const double sms = 148, ratio = hq / h;
-  const long long m = (t + c - 1) / c, last = t - (m - 1) * c;
-  const double full = row_tiles(c), tail = row_tiles(last), before = (double)(m - 1);
-  auto attention = [&](double steps, long long longest) {
-    return std::max(b * hq * steps / sms, 0.3 * ratio * (double)((longest + 63) / 64));
-  };
-  const double more = attention(row_steps(t), t) - attention(before * row_steps(c) + row_steps(last), c);
-  const double tiles = b * hq * (before * full + tail) / sms;
-  const double states = b * (hq * ((before - 1) * full + tail) + h * before * full) * (ref_dim(d) / 64) / sms;
-  return 20 + 6 * tiles + 0.6 * states - 1.4 * more;
-}
-
-}  // namespace
-}  // namespace pr
-
-extern "C" int pr_blocking(int b, long long t, int h, int hq, int d, int requested, int longest_quadratic) {
-  const int c = pr_fast_chunk(t, requested);
-  if (t <= c) return 0;
-  if (c <= 0 || t > longest_quadratic || b <= 0 || h <= 0 || hq < h || !pr::head_dim_ok(d)) return c;
-  return pr::quadratic_saves_us(b, t, h, hq, d, c) > 0 ? 0 : c;
 }
 
 extern "C" int pr_workspace_bytes(const pr_problem* prob, int what, size_t* out) {

@@ -8,7 +8,6 @@ PyTorch or CPU fallback: inputs must be CUDA tensors of dtype bfloat16 or float1
 """
 from __future__ import annotations
 
-import ctypes
 import math
 
 import torch
@@ -147,13 +146,16 @@ def _pad_head_dim(x, d_to):
 # errs).  The C ABI (pr_retention_fwd) always takes the chunk it is given.
 AUTO_CHUNK = True
 _FAST_CHUNK = 1024
-# The longest sequence that AUTO_CHUNK may run in the quadratic form although several chunks were asked for (blocking).
+# Up to two such chunks the quadratic form is less work than the states between them (per token and head 0.9 against 1.3
+# MFLOP forward and backward at 2048) and six launches instead of fourteen, so with AUTO_CHUNK sequences of up to that
+# length that carry no state run in it, whatever chunk was asked for; csrc/binding.cpp has the same number.
+# Forward and backward in us, one quadratic chunk / chunks of 1024: b1 t2000 h2 112 / 151, b8 t2048 h16 476 / 863,
+# b16 t1100 h32 733 / 2079, b8 t2048 h4x8 868 / 1094, b1 t2048 h2x12 315 / 311; at 4096 (b1 h4) 156 / 123.
 QUADRATIC_TOKENS = 2048
 
 
 def effective_chunk(t: int, chunk_size, deg: int = 2):
-    """The chunk size of the chunked form for a sequence of t tokens and a requested chunk_size: what power_retention runs
-    with where a state comes in or goes out.  Without states `blocking` chooses between this and the quadratic form.
+    """The chunk size power_retention runs with for a sequence of t tokens and a requested chunk_size.
 
     Below 1024: the largest multiple of the request up to 1024 that rounds the length up by at most 1/16 more.  Above
     1024 (slower again: the intra-chunk attention grows with the chunk): the largest divisor of the request in
@@ -183,25 +185,6 @@ def effective_chunk(t: int, chunk_size, deg: int = 2):
     return chunk_size
 
 
-def blocking(b: int, t: int, h: int, hq: int, d: int, chunk_size):
-    """The chunk size power_retention runs a sequence without states with (deg 2); None: the quadratic form.
-
-    Both forms compute the same function.  The quadratic form has fewer launches (six instead of fourteen) and no states to
-    form, scan and read, but more attention, which runs 64 features wide at every head dim, while a state has 2560 / 768 /
-    256 rows at d = 64 / 32 / 16.  pr_blocking (csrc/retention_op.cu) counts both, for sequences of up to QUADRATIC_TOKENS.
-    Forward and backward replayed in us, one quadratic chunk / chunks of 1024, * = taken: d = 64 b1 t2000 h2 70* / 105,
-    b8 t2048 h16 467* / 817, b8 t2048 h4x8 820* / 1034, b1 t2048 h1x12 264 / 246*; d = 32 b8 t2048 h16 446* / 492, b16 t2048 h4x12
-    2119 / 1936*; d = 16 b16 t2048 h32 1492 / 1371*, b1 t2048 h2 61* / 79.  At 4096 (b1 h4, d = 64) 141 / 122."""
-    if not AUTO_CHUNK:
-        return chunk_size
-
-    def i(x):  # sizes are tensors while a call is traced
-        return ctypes.c_int(min(int(x), 2**31 - 1))
-
-    return _lib.lib().pr_blocking(i(b), ctypes.c_longlong(int(t)), i(h), i(hq), i(d), i(chunk_size or 0),
-                                  i(QUADRATIC_TOKENS)) or None
-
-
 def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=False, deg=2, scale=None,
                     chunk_size=None, switch_over_seq_len=None):
     """Symmetric power retention, training forward (differentiable).
@@ -224,7 +207,7 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     if NATIVE_SEQUENCER and not ops.launch_log.timing:
         state, sok = initial_state if initial_state is not None else (None, None)
         out = _lib.host().power_retention(Q, K, V, log_G, state, sok, return_final_state, int(deg), scale or 0.0,
-                                          chunk_size, switch_over_seq_len, AUTO_CHUNK, QUADRATIC_TOKENS)
+                                          chunk_size, switch_over_seq_len, AUTO_CHUNK)
         if out is not None:
             return (_like_queries(Q, out[0]), out[1]) if return_final_state else _like_queries(Q, out)
     d_orig = Q.shape[-1]
@@ -241,10 +224,11 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     requested = chunk_size
     chunk_size = effective_chunk(t, chunk_size, deg)
     if chunk_size != requested or (chunk_size is not None and switch_over_seq_len is None):
-        # the blocking is this function's own choice: one chunk is the quadratic form
+        # the blocking is this function's own choice: one chunk is the quadratic form, and so are short sequences;
+        # several chunks are the chunked one
         switch_over_seq_len = chunk_size
-        if AUTO_CHUNK and deg == 2 and initial_state is None and not return_final_state:
-            chunk_size = blocking(b, t, h, hq, d, requested)
+        if AUTO_CHUNK and deg == 2 and t <= QUADRATIC_TOKENS and initial_state is None and not return_final_state:
+            chunk_size = None
     t_padded = t if chunk_size is None else -(-t // chunk_size) * chunk_size
     state_free = (switch_over_seq_len is None or t_padded <= switch_over_seq_len or chunk_size is None) and \
         initial_state is None and not return_final_state
