@@ -226,10 +226,6 @@ StatePair final_state(const Tensor& S, const Tensor& gram, int64_t b, int64_t h,
 // autograd.Function for this case, which the tracer records as one node: the entry points answer None.
 bool being_traced() { return at::tracer::impl::is_dispatch_enabled(); }
 
-// Up to this length a sequence without states runs in the quadratic form whatever chunk was asked for (retention.py has
-// the reason and figures).
-constexpr int64_t kQuadraticTokens = 2048;
-
 using Retained = std::variant<Tensor, std::tuple<Tensor, StatePair>>;  // with a final state: (output, pair)
 
 // power_retention with the blocking chosen here.  Returns None for the head dims that the caller has to widen first, and
@@ -237,7 +233,7 @@ using Retained = std::variant<Tensor, std::tuple<Tensor, StatePair>>;  // with a
 std::optional<Retained> power_retention(Tensor Q, Tensor K, Tensor V, const OptTensor& log_G, const OptTensor& state,
                                         const OptTensor& sok, bool want_final, int64_t deg, double scale,
                                         std::optional<int64_t> chunk_size, std::optional<double> switch_over,
-                                        bool auto_chunk) {
+                                        bool auto_chunk, int64_t quadratic_tokens) {
   if (being_traced()) return std::nullopt;
   require(deg % 2 == 0, "deg must be even");
   pr_require(!chunk_size.has_value() || *chunk_size > 0, "chunk_size must be positive");
@@ -251,9 +247,9 @@ std::optional<Retained> power_retention(Tensor Q, Tensor K, Tensor V, const OptT
   if (d == 48) return std::nullopt;
   int64_t c = (auto_chunk && deg == 2) ? pr_fast_chunk(t, (int)std::min<int64_t>(chunk, std::numeric_limits<int>::max())) : chunk;
   if (c != chunk || !switch_over.has_value()) {
-    // the blocking is this function's own choice: one chunk is the quadratic form, and so are short sequences
+    // the blocking is this function's own choice: one chunk is the quadratic form, and so is what the caller says is short
     switch_over = c ? std::optional<double>((double)c) : std::nullopt;
-    if (auto_chunk && deg == 2 && !with_state && t <= kQuadraticTokens) c = 0;
+    if (auto_chunk && deg == 2 && !with_state && t <= quadratic_tokens) c = 0;
   }
   const bool quadratic = !switch_over.has_value() || c == 0 || (double)((t + c - 1) / c * c) <= *switch_over;
   if (deg != 2 && !(deg == 4 && quadratic && !with_state))

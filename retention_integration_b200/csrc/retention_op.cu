@@ -217,9 +217,9 @@ class Fork {
 // of the request in [256, 1024]; 0 (no chunking) on more than 2048 tokens: 1024 or 512 if that rounds the length up by
 // at most 1/16, else 0.
 // The rounding was work while sequences were padded to whole chunks.  They no longer are, and by work the rule errs
-// where it still decides: t 7200 unchunked stays one chunk (358 us, b1 h4) where chunks of 1024 take 194, and up to
-// 2048 tokens without states no chunks are better whatever was asked for, which the Python API does
-// (retention.py: QUADRATIC_TOKENS; a C host asks for c = 0).  Mirrors retention.py: effective_chunk, for hosts that do not go through the Python API.
+// where it still decides: t 2000 with chunk 128 takes two chunks of 1024 (105 us replayed from a graph, b1 h2) where
+// one without states takes 68, t 1100 three of 384 (87 us, b1 h4; 49), and t 7200 unchunked stays one (334 us, b1 h4)
+// where chunks of 1024 take 177.  Mirrors retention.py: effective_chunk, for hosts that do not go through the Python API.
 extern "C" int pr_fast_chunk(long long t, int requested) {
   const int fast = 1024;
   if (t <= 0 || requested < 0) return requested;

@@ -146,12 +146,13 @@ def _pad_head_dim(x, d_to):
 # errs).  The C ABI (pr_retention_fwd) always takes the chunk it is given.
 AUTO_CHUNK = True
 _FAST_CHUNK = 1024
-# Up to two such chunks the quadratic form is less work than the states between them (per token and head 0.9 against 1.3
-# MFLOP forward and backward at 2048) and six launches instead of fourteen, so with AUTO_CHUNK sequences of up to that
-# length that carry no state run in it, whatever chunk was asked for; csrc/binding.cpp has the same number.
-# Forward and backward in us, one quadratic chunk / chunks of 1024: b1 t2000 h2 112 / 151, b8 t2048 h16 476 / 863,
-# b16 t1100 h32 733 / 2079, b8 t2048 h4x8 868 / 1094, b1 t2048 h2x12 315 / 311; at 4096 (b1 h4) 156 / 123.
-QUADRATIC_TOKENS = 2048
+# Sequences of up to this length that carry no state run in the quadratic form whatever chunk was asked for (with AUTO_CHUNK,
+# deg 2).  0: none, the chunk decides.  Up to two chunks of 1024 the quadratic form is mostly faster at head dim 64 (forward and
+# backward replayed in us, one quadratic chunk / chunks: b1 t2000 h2 68 / 105, b8 t2048 h16 470 / 817, b16 t1100 h32 727 /
+# 2208, but b1 t2048 h1x16 342 / 310) and mostly slower with narrow heads in number (d 16, b16 t2048 h32 1492 / 1371).  Both
+# are as near to exact results (dlog_G of b1 t2000 h2: 3.61e-3 / 3.65e-3), but they round differently, 1e-3 in that float32
+# gradient, so it is the caller's choice; a single call of up to 2048 tokens makes it by chunk_size=None.
+QUADRATIC_TOKENS = 0
 
 
 def effective_chunk(t: int, chunk_size, deg: int = 2):
@@ -207,7 +208,7 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     if NATIVE_SEQUENCER and not ops.launch_log.timing:
         state, sok = initial_state if initial_state is not None else (None, None)
         out = _lib.host().power_retention(Q, K, V, log_G, state, sok, return_final_state, int(deg), scale or 0.0,
-                                          chunk_size, switch_over_seq_len, AUTO_CHUNK)
+                                          chunk_size, switch_over_seq_len, AUTO_CHUNK, QUADRATIC_TOKENS)
         if out is not None:
             return (_like_queries(Q, out[0]), out[1]) if return_final_state else _like_queries(Q, out)
     d_orig = Q.shape[-1]
@@ -224,8 +225,8 @@ def power_retention(Q, K, V, log_G=None, initial_state=None, return_final_state=
     requested = chunk_size
     chunk_size = effective_chunk(t, chunk_size, deg)
     if chunk_size != requested or (chunk_size is not None and switch_over_seq_len is None):
-        # the blocking is this function's own choice: one chunk is the quadratic form, and so are short sequences;
-        # several chunks are the chunked one
+        # the blocking is this function's own choice: one chunk is the quadratic form, and so is what QUADRATIC_TOKENS says
+        # is short; several chunks are the chunked one
         switch_over_seq_len = chunk_size
         if AUTO_CHUNK and deg == 2 and t <= QUADRATIC_TOKENS and initial_state is None and not return_final_state:
             chunk_size = None
