@@ -453,17 +453,22 @@ extern "C" int pr_attention_bwd(const pr_problem* prob, int deg, const void* Q, 
   if ((rc = dout_prep(p.dtype, (long long)p.b * p.t * p.hq, p.d, O, dO, l, nullptr, dl, device, stream))) return rc;
   Fork fork;
   if ((rc = fork.begin(device, stream))) return rc;
-  // The key side is enqueued first.  Both kernels hold one CTA per SM while they have tiles; chunk_dkv's are fewer (one
-  // per key tile of a kv head) and longer, so in front they leave SMs to chunk_dq from the start, and behind it they run
-  // alone at the end.  Eager launches came out in this order anyway; a replayed graph keeps the one they were recorded
-  // in.  Replayed forward and backward in us, chunk_dq / chunk_dkv first: b4 t2048 h2x4 239 / 154, b4 t2048 h2x12 639 / 351,
-  // b1 t2048 h2x12 472 / 288, b2 t1024 h8 60 / 56, b1 t1024 h4 41 / 41, b1 t7200 h4 325 / 334 (one stream: 193, 460, 326, 55,
-  // 51, 405).
-  rc = pr_chunk_dkv(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.t, Q, dO, K, V, nullptr, a, nullptr, dl, l, nullptr, -1,
-                    p.scale, deg, dK, dV, dak, device, stream);
+  // Both kernels hold one CTA per SM while they have tiles.  With grouped queries chunk_dkv's tiles, one per key tile of a
+  // kv head, are fewer and longer: in front they leave SMs to chunk_dq from the start, behind it they run alone at the
+  // end.  Eager launches come out in that order anyway, a replayed graph keeps the one they were recorded in.  With as many
+  // kv heads as query heads the grids are equal and either order is within 4 % of the other.  Replayed forward and
+  // backward in us, chunk_dq / chunk_dkv first: b4 t2048 h2x4 239 / 154, b4 t2048 h2x12 639 / 351, b1 t2048 h2x12 472 / 288,
+  // b8 t1024 h4x8 332 / 272; b1 t2048 h4 64 / 64, b4 t2048 h8 170 / 166, b4 t2000 h4 119 / 123, b1 t7200 h4 325 / 334.
+  const bool keys_first = p.hq > p.h;
+  auto query_side = [&] {
+    return pr_chunk_dq(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.t, Q, dO, K, V, a, dl, l, nullptr, p.scale, deg, dQ, daq, device,
+                       fork.side());
+  };
+  if (!keys_first) rc = query_side();
   if (!rc)
-    rc = pr_chunk_dq(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.t, Q, dO, K, V, a, dl, l, nullptr, p.scale, deg, dQ, daq, device,
-                     fork.side());
+    rc = pr_chunk_dkv(p.dtype, p.b, p.t, p.hq, p.h, p.d, p.t, Q, dO, K, V, nullptr, a, nullptr, dl, l, nullptr, -1,
+                      p.scale, deg, dK, dV, dak, device, stream);
+  if (keys_first && !rc) rc = query_side();
   fork.side_done();
   rc = fork.join(rc);
   if (rc || log_G == nullptr) return rc;
