@@ -291,7 +291,7 @@ int pr_retention_fwd(const pr_problem* problem, const void* Q, const void* K, co
 
 /* The chunk size to run a request with (0 = no chunking asked for): same results, fewer and longer chunks.
  * The chunk size blocks the computation of retention/power_retention_maker.py:143-193 without changing its
- * result; on this hardware 1024 is fastest (5.0 ms per step at chunk 128 against 2.5 at 1024 for b1 t65536 h8).
+ * result; on this hardware 1024 is fastest (4.5 ms per step at chunk 128 against 2.2 at 1024 for b1 t65536 h8).
  * pr_retention_fwd / _bwd run whatever pr_problem.c says; a host that wants the fast blocking passes
  * c = pr_fast_chunk(t, its_chunk). */
 int pr_fast_chunk(long long t, int requested_chunk);

@@ -15,16 +15,14 @@
 // Three groups of four warps own the key rows, one row per thread in each group, and take the steps in turn, each in
 // its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma; two warps make, step by step in turn and up to
 // six ahead, what the rows need of a step's queries (Cols).  One persistent CTA per SM takes over tile after tile
-// (ClcRing).  A step is a serial chain - S and dP products, barrier, tensor-memory loads, arithmetic, stores, barrier, dV and
-// dK products; with three buffers the products of the next steps run while the rows work.
-// 490 -> 470 us at b1 t65536 h8 with chunks of 1024 and states (144 -> 117 at b4 t5000 h2x4 fp16, 27.4 -> 17.2 at
-// b1 t1024 h4) from the three groups.  Every row warp used to make the factors of its columns itself: loads, two divisions,
-// a logarithm and exponentials were a chain of 1000-1900 traced clocks in front of a step's 1000-1500, on all twelve
-// warps.  With warps of their own for it, and the next tile's gates and the state-path gradients fetched before the
-// write-out: 467 -> 413, 119 -> 102 (gated bf16), 80 -> 68 at b4 t2048 h8 in one chunk, 19.2 -> 17.2; without divisions
-// between the tiles 395, 98, 67, 17; with the state-path gradients fetched 32 bytes a lane, before the rows meet, 373: a
-// tile's end, traced at 7400 clocks of 21000 at first, is bound by rows 2 KB apart, a line per lane and instruction.  (One such warp, the
-// TMA warp: 483, 137, -, 21.3: it cannot keep up.)
+// (ClcRing); the next tile's gates and the state-path gradients are fetched before the write-out.
+// Bound by the latency of a step's serial chain - S and dP products, barrier, tensor-memory loads, arithmetic, stores,
+// barrier, dV and dK products - of which the three buffers overlap three, and by the end of a tile, where rows lie 2 KB
+// apart, a line per lane and instruction.  The columns' factors (loads, two divisions, a logarithm, exponentials) are a
+// chain of 1000-1900 clocks: on the row warps it stood in front of a step's own 1000-1500, and the TMA warp alone cannot
+// keep up with it (467 -> 483 us).
+// 490 -> 373 us at b1 t65536 h8 with chunks of 1024 and states (one group per CTA -> now); the factors on warps of their own
+// instead of the row warps: 467 -> 413, 80 -> 68 at b4 t2048 h8 in one chunk, 119 -> 102 at b4 t5000 h2x4.
 #include "host.cuh"
 #include "layout.cuh"
 #include "sm100.cuh"

@@ -13,15 +13,12 @@
 // state-path gradient (fp32, from the expansion-gradient kernel) and writes dQ.
 //
 // Three groups of four warps own the query rows, one row per thread in each group, and take the steps in turn, each in
-// its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma.  One persistent CTA per SM takes over
-// tile after tile (ClcRing).  Bound by the latency of a step's chain (products, barrier, tensor-memory loads,
-// arithmetic, stores, barrier, product); two CTAs per SM with one row group each overlapped two of them and spent
-// a third of the time on set-up and write-out: 232 -> 220 us at b1 t65536 h8 with chunks of 1024
-// (94 -> 84 at b4 t5000 h2x4 fp16, 20.2 -> 12.6 at b1 t1024 h4).
-// Two more warps make, step by step in turn and up to six ahead, the gate factors of a step's keys (Cols), which every row
-// warp used to make for itself before it could look at the scores; a tile's row values are fetched before the
-// write-out of the tile before: 217 -> 202 us, 75.6 -> 72.7 (gated bf16), 56 -> 52 at b4 t2048 h8 in one chunk, the small
-// ones the same; 198 without divisions between the tiles, 196 with the state-path gradient read 32 bytes a lane.
+// its own tensor-memory buffer; one warp issues TMA loads, one tcgen05.mma; two warps make, step by step in turn and up to
+// six ahead, the gate factors of a step's keys (Cols).  One persistent CTA per SM takes over tile after tile (ClcRing);
+// a tile's row values are fetched before the write-out of the tile before.  Bound by the latency of a step's chain
+// (products, barrier, tensor-memory loads, arithmetic, stores, barrier, product).
+// 232 -> 196 us at b1 t65536 h8 with chunks of 1024 (one group per CTA, two CTAs per SM -> now); the factors on warps of their
+// own instead of every row warp: 217 -> 202, 56 -> 52 at b4 t2048 h8 in one chunk.
 #include "host.cuh"
 #include "sm100.cuh"
 

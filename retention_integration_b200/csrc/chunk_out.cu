@@ -12,23 +12,19 @@
 // Because both terms share one fp32 accumulator in tensor memory, the reference's
 // rowmax / sqrt(D) range management is not needed.
 //
-// Warp roles: two groups of four warps own the query rows, one row per thread in each group, and take the steps in
-// turn (scores -> weights P, expansion phi(q~)); there is no running maximum, so a row's partial sums are simply
-// added at the end.  One more warp issues TMA loads and makes the gate factors of a step's keys for all rows (Cols), which
-// every row warp used to make for itself; one issues tcgen05.mma.
-//
-// What bounded the earlier form (one row group per CTA, 637 us at b16 t2048 h32 without states, 317 us at
-// b1 t65536 h8 with chunks of 1024 and states): the latency of a step's chain, about 2000 clocks traced for a 64-key
-// step whose products take 320 - two groups and three buffers overlap four such chains per SM (494, 287 us) -
-// and then, for a third of the time, 10 thousand clocks per CTA of set-up, first loads, cold instructions and
-// write-out.  So the kernel is persistent: two CTAs per SM take over tile after tile (ClcRing), the loads and the
-// first scores of a tile overlap the write-out of the one before, and ring stages, buffers and groups go on
-// rotating across tiles; and the issuing thread keeps running positions and prepared descriptors, since every
-// instruction it executes between two batches leaves the tensor pipe idle (with divisions and a second commit per
-// operand: 459, 301 us).  Now 451 and 265 us.  Slower: three groups per CTA (520 us); 256 rows per CTA at one CTA per SM
-// (439 us, but 360 with states, where every gap of the one or two issuing threads is exposed).  With the keys' factors made
-// by the TMA warp, the next tile's gates fetched before the write-out, and no divisions between the tiles: 477 -> 392 and
-// 261 -> 258 us (without the last 400, 266).
+// Two groups of four warps own the query rows, one row per thread in each group, and take the steps in turn (scores ->
+// weights P, expansion phi(q~)); there is no running maximum, so a row's partial sums are simply added at the end.  One
+// more warp issues TMA loads and makes the gate factors of a step's keys for all rows (Cols); one issues tcgen05.mma.  Two
+// persistent CTAs per SM take over tile after tile (ClcRing): the loads and the first scores of a tile overlap the
+// write-out of the one before, and ring stages, buffers and groups go on rotating across tiles.  The issuing thread keeps
+// running positions and prepared descriptors, since what it executes between two batches leaves the tensor pipe idle.
+// Bound by the latency of a step's chain, about 2000 clocks for a 64-key step whose products take 320: two groups in two
+// CTAs overlap four such chains per SM.
+// 637 -> 392 us (one group and one tile per CTA -> now) at b16 t2048 h32 without states, 317 -> 257 at b1 t65536 h8 with
+// chunks of 1024 and states.  The factors on the TMA warp against every row warp making its own: 477 -> 400 without states;
+// with states 261 -> 266, and 257 once tiles are found without divisions; a few steps in front of a state are 0.25 us slower
+// (b1 t4096 h4 c256 14.5 -> 14.75).  Slower: three groups per CTA; 256 rows per CTA at one CTA per SM; factors three
+// stages behind the loads; all loads that have room before a tile's first gates are waited for (257 -> 277).
 //   S = Q K_J^T        : A, B K-major in shared memory (TMA, 128-byte swizzle)
 //   acc += P V_J       : A = P written to tensor memory by the row threads, B = V_J MN-major
 //   acc += phi(q~) Z   : A = expansion written to tensor memory 64 rows at a time,

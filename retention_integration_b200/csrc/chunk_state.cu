@@ -17,14 +17,12 @@
 //
 // One persistent CTA per SM takes over item after item (ClcRing).  Four groups of four warps take the 64-token stages in
 // turn, each with a slot of its own in tensor memory; one thread per tile issues the products; four more warps write an
-// item out from the first pair of accumulators while the next one fills the second.  Before, two CTAs per SM expanded
-// every stage with all their warps into two slots: of a CTA's 24 thousand clocks at sixteen stages, half was set-up, first
-// loads, cold instructions and write-out, and a barrier round was paid for half a stage's work.  252 -> 232 us at
-// b1 t65536 h8 with chunks of 1024, 83 -> 60 at b4 t4096 h2 with four query heads summed, 406 -> 375 at b16 t2048 h32 in one
-// chunk, 15.1 -> 14.1 at b1 t2048 h2 (groups in turn alone: 238, 72, 375, 14.7); without divisions between the items 201,
-// 56, 9 % less, 14.  A stage costs the shared-memory pipe
-// about 560 clocks (the operand reads, 8 for 16 products; the tensor core's own reads; tensor-memory stores), the
-// tensor pipe 256.
+// item out from the first pair of accumulators while the next one fills the second.  A CTA per item spent half of its
+// life on set-up, first loads and write-out.
+// Bound by the shared-memory pipe, about 560 clocks a stage (the operand reads, 8 wavefronts for 16 products; the tensor
+// core's own reads; tensor-memory stores) against 256 of the tensor pipe, and by 1500 clocks at the change of items.
+// 252 -> 201 us (a CTA per item -> now) at b1 t65536 h8 with chunks of 1024, 83 -> 56 at b4 t4096 h2 with four query heads
+// summed, 406 -> 365 at b16 t2048 h32 in one chunk, 15.1 -> 14.1 at b1 t2048 h2.
 //
 // EXACT (a token cache compressed into an inference state, retention/power_retention_maker.py:374-388): the read-out
 // writes the state in the exact layout, state * e^a_last + the cache's part in fp32, and sum_of_keys from the Gram

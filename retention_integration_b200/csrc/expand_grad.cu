@@ -11,18 +11,16 @@
 // Key side (gradient of the chunk state, retention/_update_state/reference.py:55-83):
 //   W = V, State = w (.) dS_m, Gs = dG_m + dG_m^T, g_i = 1, mult = 1, f_i = exp((A_m - a_i)/2).
 //
-// One CTA owns one row tile of 128 tokens of one (batch, chunk, head) and two CTAs share an SM, so that one CTA's
-// prologue (operand loads, gating) and write-out (with the Gram part) - a quarter of a CTA's life, all of it on the drain warps -
-// run while the other CTA drains.  (Two row tiles in one CTA per SM, where each state tile fetched from L2 feeds two
-// products, measured 7 % slower: 0.302 against 0.282 ms per launch at b1 t65536 h8.)  The expansion gradient dphi is
-// never written to memory: tiles of 128 expanded rows are produced in tensor memory, two buffers, and drained by four
-// warps while the tensor core fills the other buffer.  Each thread owns one token row; the second factors of a 16-block and
-// their gradients are in registers while the block is drained, two FMAs per entry.  The Gram part comes last, as one
-// more tile: at the start it held up the first state tile (272 -> 268 us, 79.7 -> 78.4 at b4 t5000 h2x4, 25.8 -> 25.2 with
-// one head per group).  A tile takes a drain warp about 1000 clocks, where its FMAs and tensor-memory loads alone take 365
-// (packed FMAs with three distinct operand pairs issue every 2.8 clocks).  Measured and not kept: one CTA per SM with
-// four row tiles, four groups of drain warps, W in tensor memory and pieces of 64 rows: 266 us, but 85 and 27.2 for the
-// other two.
+// One CTA owns one row tile of 128 tokens of one (batch, chunk, head) and two CTAs share an SM, so that one CTA's prologue
+// (operand loads, gating) and write-out (with the Gram part, which comes last as one more tile), over a quarter of a CTA's
+// life and all of it on the drain warps, run while the other CTA drains.  The expansion gradient dphi is never written to
+// memory: tiles of 128 expanded rows are produced in tensor memory, two buffers, and drained by four warps while the
+// tensor core fills the other buffer.  Each thread owns one token row; the second factors of a 16-block and their
+// gradients are in registers while the block is drained, two FMAs per entry.
+// Bound by the drain: a tile takes a drain warp about 1000 clocks, of which its FMAs and tensor-memory loads alone are 365
+// (packed FMAs with three distinct operand pairs issue every 2.8 clocks).  302 -> 268 us (two row tiles per CTA, Gram part
+// first -> now) at b1 t65536 h8, 79.7 -> 78.4 at b4 t5000 h2x4 (Gram part first -> last).  Slower there: one CTA per SM with
+// four row tiles (266 us, but 85).
 #include <type_traits>
 
 #include "host.cuh"

@@ -212,7 +212,7 @@ class Fork {
 // The chunk size to run a request with.  The operator's result does not depend on the chunk size, its speed
 // does: every chunk's state is written, scanned and read again (1.3 GB per pass at chunk 128 against 0.17 GB at
 // 1024 for b1 t65536 h8), and above 1024 the intra-chunk attention grows.  Forward + backward of that shape in ms, as
-// asked: chunk 128 5.04, 256 3.42, 512 2.68, 1024 2.46, 2048 2.63, 4096 3.30.  Below 1024: the largest multiple of the
+// asked: chunk 128 4.46, 256 3.01, 512 2.38, 1024 2.24, 2048 2.46, 4096 2.97.  Below 1024: the largest multiple of the
 // request up to 1024 that rounds the length up by at most 1/16 more than the request does; above: the largest divisor
 // of the request in [256, 1024]; 0 (no chunking) on more than 2048 tokens: 1024 or 512 if that rounds the length up by
 // at most 1/16, else 0.

@@ -140,7 +140,7 @@ def _pad_head_dim(x, d_to):
 # to the same function for every chunk size, and so do the kernels here - tested).  Small chunks are slow on
 # this hardware for a reason the arithmetic does not care about: every chunk's state (2560 x 64 per head) is written,
 # scanned and read again, 1.3 GB per pass at chunk 128 against 0.17 GB at chunk 1024 for the benchmark's shape
-# (5.0 vs 2.5 ms per step).  With AUTO_CHUNK the Python API therefore runs a request for a chunk below 1024 with the
+# (4.5 vs 2.2 ms per step).  With AUTO_CHUNK the Python API therefore runs a request for a chunk below 1024 with the
 # largest multiple of it that is at most 1024 and rounds the length up by at most 1/16 more than the request does
 # (the sequence is not padded: its last chunk is shorter; csrc/retention_op.cu has the rule's figures, and where it
 # errs).  The C ABI (pr_retention_fwd) always takes the chunk it is given.
